@@ -175,7 +175,8 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
   if (z_stride < p->h || delta_stride < p->r || (act_out && act_stride < p->h)) return SKV_ERR_SHAPE;
   const int impl = resolve(*p);
   if (impl < 0) return impl;
-  if (impl == SKV_IMPL_TCGEN05) {
+  const bool small = p->impl == SKV_IMPL_AUTO && p->N <= small_forward_tokens(*p);
+  if (impl == SKV_IMPL_TCGEN05 && !small) {
     if (!aligned(z, 16) || !aligned(C, 16) || !aligned(delta_out, 16) || (act_out && !aligned(act_out, 16)) ||
         z_stride % 8 || delta_stride % (p->delta_f32 ? 4 : 8) || (act_out && act_stride % 8)) {
       if (p->impl == SKV_IMPL_TCGEN05) return SKV_ERR_ALIGN;
@@ -184,7 +185,7 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
       return tc_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
     }
   }
-  return simt_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride);
+  return simt_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
 }
 
 int skv_feature_backward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, const void* g_act,

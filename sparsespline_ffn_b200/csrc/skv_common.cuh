@@ -124,7 +124,8 @@ struct LaunchCtx {
 // CUDA-core kernel family (any N, h, L, r <= 256; bf16 or float32).
 size_t simt_scratch_bytes(const skv_problem& p, int op);
 int simt_forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* act_out, int64_t as,
-                 void* delta_out, int64_t ds);
+                 void* delta_out, int64_t ds, void* scratch, size_t scratch_bytes);
+int64_t small_forward_tokens(const skv_problem& p);
 int simt_backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const void* g_act, int64_t gas,
                   const void* g_delta, int64_t gds, void* dz, int64_t dzs, float* dC, void* dC_cast,
                   void* scratch, size_t scratch_bytes);

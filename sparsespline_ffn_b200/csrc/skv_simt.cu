@@ -1,255 +1,677 @@
-// CUDA-core kernels of the spline-KV feature operator: any N, h, L and r <= 256,
-// bf16 or float32 I/O, float32 arithmetic.  They are the float32 tier of the
-// library and the path for shapes the tcgen05 kernels do not cover.
+// CUDA-core kernels of the spline-KV feature operator: any N, h, L and r <= 256, bf16 or float32
+// I/O, float32 arithmetic, quadratic or linear spline.  They are the float32 tier of the library, the
+// path for shapes the tcgen05 kernels do not cover, and the path of the smallest forwards.
 //
-// Mapping used by all three: one warp works on one (token, 32-key group) or
-// (key, 32-token group) at a time; each lane evaluates the knot interval and
-// B-spline weights of one (token, key) pair, then the warp walks the 32 pairs
-// with the lanes spread over the r code channels, reading the code-table rows
-// C[j, bin + k, :] from a float32 copy of the current key chunk in shared memory.
+// They use the sparsity the tensor-core kernels cannot: a (token, key) pair touches order + 1 knot
+// rows of r channels, nothing else.  A row is read with 16-byte loads by LPT neighbouring lanes, so
+// a warp works on 32 / LPT tokens of one key at a time; knot interval and weights of a pair are
+// computed once by one lane and handed to the LPT lanes through shared memory (a 16-byte broadcast).
 #include "skv_common.cuh"
 
 namespace skv {
 namespace {
 
 constexpr int kWarp = 32;
-constexpr int kMaxRIter = 8;          // r <= 256
 constexpr unsigned kFull = 0xffffffffu;
+constexpr int kWarps = 8;             // warps per CTA of the token-major kernels
+constexpr int kGroups = 4;            // token groups a warp of the staged forward keeps accumulators for
+constexpr int kSmallEntries = 256;    // pair weights per warp of the small forward (tokens x keys of a pass)
 
 __host__ __device__ inline int64_t cdiv64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// ---------------------------------------------------------------------------------------------
-// Forward: grid.x = token blocks of TB tokens.  The CTA walks the keys in chunks of KCH keys,
-// each warp owns TB/8 tokens and keeps their delta rows in shared memory.
-// ---------------------------------------------------------------------------------------------
-template <typename T, typename TD>
-__global__ void __launch_bounds__(256)
-simt_forward_kernel(const T* __restrict__ z, int64_t zs, const T* __restrict__ C,
-                    T* __restrict__ act_out, int64_t as, TD* __restrict__ delta_out, int64_t ds,
-                    int64_t N, int h, int L, int r, GridParams g, float lambda, int act, int TB, int KCH) {
-  extern __shared__ float smem[];
-  float* Cs = smem;                                   // [KCH][L][r]
-  float* dacc = smem + (size_t)KCH * L * r;           // [TB][r]
-  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp, nwarps = blockDim.x / kWarp;
-  const int64_t n0 = (int64_t)blockIdx.x * TB;
-  const int riter = (r + kWarp - 1) / kWarp;
-  const bool three = g.order != 1;                    // the linear spline has no third row
-
-  for (int i = threadIdx.x; i < TB * r; i += blockDim.x) dacc[i] = 0.0f;
-
-  for (int j0 = 0; j0 < h; j0 += KCH) {
-    const int kc = min(KCH, h - j0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < kc * L * r; i += blockDim.x)
-      Cs[i] = ld_f32<T>(C + (size_t)j0 * L * r + i);
-    __syncthreads();
-
-    for (int t = warp; t < TB; t += nwarps) {
-      const int64_t n = n0 + t;
-      if (n >= N) break;
-      float acc[kMaxRIter];
+// 16 bytes of a table row as float32.
+template <typename T> struct Vec;
+template <> struct Vec<float> {
+  static constexpr int n = 4;
+  static __device__ __forceinline__ void cvt(const uint4& v, float* f) {
+    f[0] = __uint_as_float(v.x); f[1] = __uint_as_float(v.y); f[2] = __uint_as_float(v.z); f[3] = __uint_as_float(v.w);
+  }
+};
+template <> struct Vec<__nv_bfloat16> {
+  static constexpr int n = 8;
+  static __device__ __forceinline__ void cvt(const uint4& v, float* f) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int ci = 0; ci < kMaxRIter; ++ci) acc[ci] = 0.0f;
-      for (int jg = 0; jg < kc; jg += kWarp) {
-        const int jl = jg + lane;
-        int bin = 0;
-        float B0 = 0.f, B1 = 0.f, B2 = 0.f;
-        if (jl < kc) {
-          float zz = ld_f32<T>(z + n * zs + j0 + jl);
-          Knot k = knot_of(zz, g);
-          basis_weights(k, B0, B1, B2, g.order);
-          bin = k.bin;
-          if (act_out) st_f32<T>(act_out + n * as + j0 + jl, act_fwd(zz, act));
-        }
-        const int cnt = min(kWarp, kc - jg);
-        for (int q = 0; q < cnt; ++q) {
-          const int b = __shfl_sync(kFull, bin, q);
-          const float w0 = __shfl_sync(kFull, B0, q);
-          const float w1 = __shfl_sync(kFull, B1, q);
-          const float w2 = __shfl_sync(kFull, B2, q);
-          const float* row = Cs + ((size_t)(jg + q) * L + b) * r;
-#pragma unroll
-          for (int ci = 0; ci < kMaxRIter; ++ci) {
-            if (ci < riter) {
-              const int c = ci * kWarp + lane;
-              if (c < r) acc[ci] += w0 * row[c] + w1 * row[r + c] + (three ? w2 * row[2 * r + c] : 0.0f);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int ci = 0; ci < kMaxRIter; ++ci) {
-        if (ci < riter) {
-          const int c = ci * kWarp + lane;
-          if (c < r) dacc[t * r + c] += acc[ci];
-        }
-      }
+    for (int i = 0; i < 4; ++i) {
+      f[2 * i] = __uint_as_float(w[i] << 16);
+      f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < TB * r; i += blockDim.x) {
-    const int t = i / r, c = i % r;
-    const int64_t n = n0 + t;
-    if (n < N) st_f32<TD>(delta_out + n * ds + c, lambda * dacc[i]);
+};
+
+// Rows [0, rows) of r elements, contiguous in global memory, into shared rows of `pitch` elements.
+// The pad columns are not written (the caller zeroes the buffer once).
+template <typename T>
+__device__ __forceinline__ void stage_rows(T* dst, const T* __restrict__ src, int rows, int r, int pitch) {
+  if (r == pitch && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    const int n16 = (int)((size_t)rows * r * sizeof(T) / 16);
+    for (int i = threadIdx.x; i < n16; i += blockDim.x)
+      reinterpret_cast<uint4*>(dst)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+  } else {
+    // `per` threads copy one row (the largest power of two not above r, at most a warp)
+    int per = 32;
+    while (per > r) per >>= 1;
+    const int c0 = threadIdx.x & (per - 1);
+    for (int row = threadIdx.x / per; row < rows; row += blockDim.x / per)
+      for (int c = c0; c < r; c += per) dst[(size_t)row * pitch + c] = src[(size_t)row * r + c];
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// dz: same walk as the forward; per pair the lanes hold g[n, c] * sum_k dB_k C[j, bin+k, c] for
-// their channels, a butterfly transpose-reduce turns 32 such per-lane partials into one sum per
-// lane (lane q ends up with the pair q), which then takes the base-path term and is stored.
-// ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256)
-simt_dz_kernel(const T* __restrict__ z, int64_t zs, const T* __restrict__ C,
-               const T* __restrict__ g_act, int64_t gas, const T* __restrict__ g_delta, int64_t gds,
-               T* __restrict__ dz, int64_t dzs, int64_t N, int h, int L, int r, GridParams g,
-               float lambda, int act, int TB, int KCH) {
-  extern __shared__ float smem[];
-  float* Cs = smem;                                   // [KCH][L][r]
-  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp, nwarps = blockDim.x / kWarp;
-  const int64_t n0 = (int64_t)blockIdx.x * TB;
-  const int riter = (r + kWarp - 1) / kWarp;
-  const float coef = lambda * g.scale;
-  const bool three = g.order != 1;
+__device__ __forceinline__ void zero16(void* p, size_t bytes) {
+  for (size_t i = threadIdx.x; i < bytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+}
 
-  for (int j0 = 0; j0 < h; j0 += KCH) {
-    const int kc = min(KCH, h - j0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < kc * L * r; i += blockDim.x)
-      Cs[i] = ld_f32<T>(C + (size_t)j0 * L * r + i);
-    __syncthreads();
+struct FwdArgs {
+  const void* z;
+  int64_t zs;
+  const void* C;
+  void* act_out;
+  int64_t as;
+  void* delta_out;
+  int64_t ds;
+  float* partial;            // [splits][N][r], or null when one CTA covers all keys of its tokens
+  int64_t N;
+  int h, L, r;
+  GridParams g;
+  float lambda;
+  int act;
+  int kch;                   // staged: keys per slab; small: keys per warp
+  int keys_per_split;
+  int groups;                // staged: token groups per warp (1..kGroups); small: tokens per warp
+};
 
-    for (int t = warp; t < TB; t += nwarps) {
-      const int64_t n = n0 + t;
-      if (n >= N) break;
-      float gd[kMaxRIter];
-#pragma unroll
-      for (int ci = 0; ci < kMaxRIter; ++ci) {
-        const int c = ci * kWarp + lane;
-        gd[ci] = (ci < riter && c < r) ? ld_f32<T>(g_delta + n * gds + c) : 0.0f;
-      }
-      for (int jg = 0; jg < kc; jg += kWarp) {
-        const int jl = jg + lane;
-        int bin = 0;
-        float d0 = 0.f, d1 = 0.f, d2 = 0.f, zz = 0.f;
-        if (jl < kc) {
-          zz = ld_f32<T>(z + n * zs + j0 + jl);
-          Knot k = knot_of(zz, g);
-          basis_derivs(k, d0, d1, d2, g.order);
-          bin = k.bin;
-        }
-        float v[kWarp];
-        const int cnt = min(kWarp, kc - jg);
-#pragma unroll
-        for (int q = 0; q < kWarp; ++q) {
-          float p = 0.0f;
-          if (q < cnt) {
-            const int b = __shfl_sync(kFull, bin, q);
-            const float w0 = __shfl_sync(kFull, d0, q);
-            const float w1 = __shfl_sync(kFull, d1, q);
-            const float w2 = __shfl_sync(kFull, d2, q);
-            const float* row = Cs + ((size_t)(jg + q) * L + b) * r;
-#pragma unroll
-            for (int ci = 0; ci < kMaxRIter; ++ci) {
-              if (ci < riter) {
-                const int c = ci * kWarp + lane;
-                if (c < r) p += gd[ci] * (w0 * row[c] + w1 * row[r + c] + (three ? w2 * row[2 * r + c] : 0.0f));
-              }
-            }
-          }
-          v[q] = p;
-        }
-        // butterfly transpose-reduce: afterwards v[0] on lane q is the sum over lanes of v[q]
-#pragma unroll
-        for (int s = 16; s >= 1; s >>= 1) {
-#pragma unroll
-          for (int i = 0; i < s; ++i) {
-            const bool up = (lane & s) != 0;
-            const float send = up ? v[i] : v[i + s];
-            const float keep = up ? v[i + s] : v[i];
-            v[i] = keep + __shfl_xor_sync(kFull, send, s);
-          }
-        }
-        if (jl < kc) {
-          float out = coef * v[0];
-          if (g_act) out += ld_f32<T>(g_act + n * gas + j0 + jl) * act_grad(zz, act);
-          st_f32<T>(dz + n * dzs + j0 + jl, out);
-        }
-      }
-    }
-  }
+// Weights of one pair for the gather loop: B_0..B_2 and the element offset of row `bin`.
+__device__ __forceinline__ float4 pair_weights(float zz, const GridParams& g, int key_row, int pitch) {
+  const Knot k = knot_of(zz, g);
+  float B0, B1, B2;
+  basis_weights(k, B0, B1, B2, g.order);
+  return make_float4(B0, B1, B2, __int_as_float((key_row + k.bin) * pitch));
 }
 
 // ---------------------------------------------------------------------------------------------
-// dC partials: grid = (key groups of KD keys, token splits).  One warp per key; the warp owns a
-// private [L][r] float32 accumulator in shared memory, so no atomics are needed and the sum
-// order is fixed.  z and g_delta tiles of TT tokens are staged in shared memory.
-// part[split][h][L][r] is written; simt_dc_reduce_kernel sums the splits.
+// Forward over a staged table: grid = (token tiles, key splits).  A CTA walks the keys of its split in
+// slabs whose table rows it copies to shared memory; a warp owns `groups` groups of 32 / LPT tokens and
+// keeps their residuals in registers over all slabs.
+//
+// Bound: shared-memory bandwidth (three rows of r channels per pair, 128 bytes a clock), which is why a
+// bf16 table stays bf16 there.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(512)
-simt_dc_partial_kernel(const T* __restrict__ z, int64_t zs, const T* __restrict__ g_delta, int64_t gds,
-                       float* __restrict__ part, int64_t N, int h, int L, int r, GridParams g,
-                       int KD, int TT, int64_t tokens_per_split) {
-  extern __shared__ float smem[];
-  float* acc = smem;                                  // [KD][L][r]
-  float* gs = acc + (size_t)KD * L * r;               // [TT][r]
-  float* zt = gs + (size_t)TT * r;                    // [TT][KD]
+template <typename T, typename TD, int LPT, int CV>
+__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const FwdArgs P) {
+  constexpr int V = Vec<T>::n;
+  constexpr int TPW = kWarp / LPT;
+  constexpr int pitch = LPT * V * CV;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  float4* wbuf = reinterpret_cast<float4*>(smem_raw);                     // [warp][TPW][32]
+  T* Cs = reinterpret_cast<T*>(wbuf + kWarps * TPW * kWarp);               // [kch][L][pitch]
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  const int j0 = blockIdx.x * KD;
-  const int kd = min(KD, h - j0);
-  const int64_t nb = (int64_t)blockIdx.y * tokens_per_split;
-  const int64_t ne = min(N, nb + tokens_per_split);
-  const int riter = (r + kWarp - 1) / kWarp;
+  const int sub = lane / LPT, sl = lane % LPT;
+  float4* my = wbuf + warp * TPW * kWarp;
+  const T* z = static_cast<const T*>(P.z);
+  T* act_out = static_cast<T*>(P.act_out);
+  const int64_t tile0 = (int64_t)blockIdx.x * (kWarps * TPW * P.groups);
+  const int kbeg = blockIdx.y * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
+  const int rowstep = pitch;
+  const bool three = P.g.order != 1;
 
-  const bool three = g.order != 1;
-  for (int i = threadIdx.x; i < KD * L * r; i += blockDim.x) acc[i] = 0.0f;
-  float* my = acc + (size_t)warp * L * r;
+  if (pitch != P.r) zero16(Cs, (size_t)P.kch * P.L * pitch * sizeof(T));
+  float acc[kGroups][CV][V];
+#pragma unroll
+  for (int m = 0; m < kGroups; ++m)
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[m][c][i] = 0.0f;
 
-  for (int64_t t0 = nb; t0 < ne; t0 += TT) {
-    const int tt = (int)min((int64_t)TT, ne - t0);
+  for (int j0 = kbeg; j0 < kend; j0 += P.kch) {
+    const int kc = min(P.kch, kend - j0);
     __syncthreads();
-    for (int i = threadIdx.x; i < tt * r; i += blockDim.x)
-      gs[i] = ld_f32<T>(g_delta + (t0 + i / r) * gds + i % r);
-    for (int i = threadIdx.x; i < tt * KD; i += blockDim.x) {
-      const int t = i / KD, k = i % KD;
-      zt[i] = k < kd ? ld_f32<T>(z + (t0 + t) * zs + j0 + k) : 0.0f;
-    }
+    stage_rows(Cs, static_cast<const T*>(P.C) + (size_t)j0 * P.L * P.r, kc * P.L, P.r, pitch);
     __syncthreads();
-    if (warp < kd) {
-      for (int tg = 0; tg < tt; tg += kWarp) {
-        int bin = 0;
-        float B0 = 0.f, B1 = 0.f, B2 = 0.f;
-        if (tg + lane < tt) {
-          Knot k = knot_of(zt[(tg + lane) * KD + warp], g);
-          basis_weights(k, B0, B1, B2, g.order);
-          bin = k.bin;
+#pragma unroll
+    for (int m = 0; m < kGroups; ++m) {
+      if (m >= P.groups) break;
+      const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+      if (n0 >= P.N) break;
+      __syncwarp();
+#pragma unroll 4
+      for (int t = 0; t < TPW; ++t) {
+        float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (lane < kc && n0 + t < P.N) {
+          const float zz = ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
+          w = pair_weights(zz, P.g, lane * P.L, pitch);
+          if (act_out) st_f32<T>(act_out + (n0 + t) * P.as + j0 + lane, act_fwd(zz, P.act));
         }
-        const int cnt = min(kWarp, tt - tg);
-        for (int q = 0; q < cnt; ++q) {
-          const int b = __shfl_sync(kFull, bin, q);
-          const float w0 = __shfl_sync(kFull, B0, q);
-          const float w1 = __shfl_sync(kFull, B1, q);
-          const float w2 = __shfl_sync(kFull, B2, q);
-          float* row = my + (size_t)b * r;
-          const float* gr = gs + (size_t)(tg + q) * r;
-          for (int ci = 0; ci < riter; ++ci) {
-            const int c = ci * kWarp + lane;
-            if (c < r) {
-              const float gv = gr[c];
-              row[c] += w0 * gv;
-              row[r + c] += w1 * gv;
-              if (three) row[2 * r + c] += w2 * gv;
-            }
+        my[t * kWarp + lane] = w;
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int q = 0; q < kc; ++q) {
+        const float4 w = my[sub * kWarp + q];
+        const T* row = Cs + __float_as_int(w.w) + sl * V;
+#pragma unroll
+        for (int c = 0; c < CV; ++c) {
+          const T* rc = row + c * (LPT * V);
+          float f0[V], f1[V], f2[V];
+          Vec<T>::cvt(*reinterpret_cast<const uint4*>(rc), f0);
+          Vec<T>::cvt(*reinterpret_cast<const uint4*>(rc + rowstep), f1);
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[m][c][i] = fmaf(w.y, f1[i], fmaf(w.x, f0[i], acc[m][c][i]));
+          if (three) {
+            Vec<T>::cvt(*reinterpret_cast<const uint4*>(rc + 2 * rowstep), f2);
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[m][c][i] = fmaf(w.z, f2[i], acc[m][c][i]);
           }
         }
       }
     }
   }
+#pragma unroll
+  for (int m = 0; m < kGroups; ++m) {
+    if (m >= P.groups) break;
+    const int64_t n = tile0 + (int64_t)(m * kWarps + warp) * TPW + sub;
+    if (n >= P.N) continue;
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int col = c * (LPT * V) + sl * V + i;
+        if (col < P.r) {
+          if (P.partial) P.partial[((size_t)blockIdx.y * P.N + n) * P.r + col] = acc[m][c][i];
+          else st_f32<TD>(static_cast<TD*>(P.delta_out) + n * P.ds + col, P.lambda * acc[m][c][i]);
+        }
+      }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Forward that reads the table rows where they are: grid = (token groups, key splits).  For few tokens
+// most of the table is never touched, so nothing is copied or packed first; each warp takes `kch` keys
+// of up to 32 / LPT tokens, spare lane groups share the keys of the tokens there are, and the warps'
+// sums are added in shared memory.  Also the path of a table too large per key for shared memory.
+//
+// Bound: the latency of one dependent chain (z -> knot -> row), so keys are spread over as many
+// warps as the chip holds and four rows' loads are in flight per lane.
+// ---------------------------------------------------------------------------------------------
+template <typename T, int CV, bool VECLD>
+__device__ __forceinline__ void load_row(const T* __restrict__ row, int col, int r, float (&f)[Vec<T>::n]) {
+  if constexpr (VECLD) {
+    Vec<T>::cvt(__ldg(reinterpret_cast<const uint4*>(row + col)), f);
+  } else {
+#pragma unroll
+    for (int i = 0; i < Vec<T>::n; ++i) f[i] = col + i < r ? ld_f32<T>(row + col + i) : 0.0f;
+  }
+}
+
+template <typename T, typename TD, int LPT, int CV, bool VECLD>
+__global__ void __launch_bounds__(kWarps * kWarp) simt_forward_small_kernel(const FwdArgs P) {
+  constexpr int V = Vec<T>::n;
+  constexpr int TPW = kWarp / LPT;
+  constexpr int pitch = LPT * V * CV;
+  __shared__ float4 wbuf[kWarps][kSmallEntries];
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int sub = lane / LPT, sl = lane % LPT;
+  const int TG = P.groups;                            // tokens of a warp: a power of two up to TPW
+  const int tok = sub & (TG - 1), ks = sub / TG, kstep = TPW / TG;
+  const T* z = static_cast<const T*>(P.z);
+  const T* C = static_cast<const T*>(P.C);
+  T* act_out = static_cast<T*>(P.act_out);
+  const int64_t n0 = (int64_t)blockIdx.x * TG;
+  const int kbeg = blockIdx.y * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
+  const bool three = P.g.order != 1;
+  float4* my = wbuf[warp];
+
+  float acc[CV][V];
+#pragma unroll
+  for (int c = 0; c < CV; ++c)
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[c][i] = 0.0f;
+
+  const int kw = P.kch;                               // keys of a warp per pass: 4, 8, 16 or 32
+  for (int j0 = kbeg + warp * kw; j0 < kend; j0 += kWarps * kw) {
+    const int kc = min(kw, kend - j0);
+    __syncwarp();
+    for (int e = lane; e < TG * kw; e += kWarp) {
+      const int t = e / kw, k = e % kw;
+      float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (k < kc && n0 + t < P.N) {
+        const float zz = ld_f32<T>(z + (n0 + t) * P.zs + j0 + k);
+        w = pair_weights(zz, P.g, k * P.L, P.r);
+        if (act_out) st_f32<T>(act_out + (n0 + t) * P.as + j0 + k, act_fwd(zz, P.act));
+      }
+      my[e] = w;
+    }
+    __syncwarp();
+    const T* base = C + (size_t)j0 * P.L * P.r;
+#pragma unroll 4
+    for (int q = ks; q < kc; q += kstep) {
+      const float4 w = my[tok * kw + q];
+      const T* row = base + __float_as_int(w.w);
+#pragma unroll
+      for (int c = 0; c < CV; ++c) {
+        const int col = c * (LPT * V) + sl * V;
+        if (col < P.r) {
+          float f0[V], f1[V], f2[V];
+          load_row<T, CV, VECLD>(row, col, P.r, f0);
+          load_row<T, CV, VECLD>(row + P.r, col, P.r, f1);
+          if (three) load_row<T, CV, VECLD>(row + 2 * P.r, col, P.r, f2);
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            acc[c][i] = fmaf(w.y, f1[i], fmaf(w.x, f0[i], acc[c][i]));
+            if (three) acc[c][i] = fmaf(w.z, f2[i], acc[c][i]);
+          }
+        }
+      }
+    }
+  }
+  // lanes that shared a token, then the warps, in a fixed order
+  for (int s = LPT * TG; s < kWarp; s <<= 1) {
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[c][i] += __shfl_xor_sync(kFull, acc[c][i], s);
+  }
+  float* red = reinterpret_cast<float*>(&wbuf[0][0]);  // [warp][TG][pitch]
   __syncthreads();
-  float* dst = part + ((size_t)blockIdx.y * h + j0) * L * r;
-  for (int i = threadIdx.x; i < kd * L * r; i += blockDim.x) dst[i] = acc[i];
+  if (ks == 0) {
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) red[((size_t)warp * TG + tok) * pitch + c * (LPT * V) + sl * V + i] = acc[c][i];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < TG * P.r; e += blockDim.x) {
+    const int t = e / P.r, col = e % P.r;
+    if (n0 + t >= P.N) break;
+    float s = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) s += red[((size_t)w * TG + t) * pitch + col];
+    if (P.partial) P.partial[((size_t)blockIdx.y * P.N + n0 + t) * P.r + col] = s;
+    else st_f32<TD>(static_cast<TD*>(P.delta_out) + (n0 + t) * P.ds + col, P.lambda * s);
+  }
+}
+
+// Sum of the key splits' partial residuals in a fixed order, lambda, cast.  A CTA takes 32 elements;
+// its eight warps each add every eighth split, so that a sum over many splits is not one serial chain.
+template <typename TD>
+__global__ void __launch_bounds__(256) simt_finalize_kernel(const float* __restrict__ partial, int splits, int64_t N,
+                                                            int r, float lambda, TD* __restrict__ out, int64_t ds) {
+  __shared__ float part[8][kWarp];
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int64_t total = N * r;
+  for (int64_t b = (int64_t)blockIdx.x * kWarp; b < total; b += (int64_t)gridDim.x * kWarp) {
+    const int64_t i = b + lane;
+    float s = 0.0f;
+    if (i < total) {
+#pragma unroll 4
+      for (int k = warp; k < splits; k += 8) s += partial[(size_t)k * total + i];
+    }
+    __syncthreads();
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < total) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) s += part[w][lane];
+      st_f32<TD>(out + (i / r) * ds + (i % r), lambda * s);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dz: grid = (token tiles, key slabs).  The derivative of the quadratic spline is linear between the knots,
+//     sum_k B_k' C[bin + k] = (1 - tau) D[bin] + tau D[bin + 1],   D[b] = C[b + 1] - C[b]
+// (the linear spline: D[bin] alone), so the slab is staged as its differences D in float32 and a pair
+// reads two rows instead of three.  The lanes of a token hold partial sums of LPT keys and one
+// transpose-reduce turns them into one key's sum per lane; 32 keys' results go through shared memory so
+// that z, g_act and dz are read and written by whole rows of 32 keys.
+//
+// Bound: shared-memory bandwidth, two float32 rows of r channels per pair.
+// ---------------------------------------------------------------------------------------------
+struct DzArgs {
+  const void* z;
+  int64_t zs;
+  const void* C;
+  const void* g_act;
+  int64_t gas;
+  const void* g_delta;
+  int64_t gds;
+  void* dz;
+  int64_t dzs;
+  int64_t N;
+  int h, L, r;
+  GridParams g;
+  float coef;                // lambda * scale
+  int act;
+  int kch;                   // keys per slab, at most 32
+  int groups;                // token groups per warp
+};
+
+// STAGED = false: a key's differences do not fit shared memory; they are formed from the table itself.
+template <typename T, int LPT, int CV, bool STAGED>
+__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs P) {
+  constexpr int V = 4;
+  constexpr int TPW = kWarp / LPT;
+  constexpr int pitch = LPT * V * CV;
+  constexpr int kRes = kWarp + 4;                                          // pitch of the result rows
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  float2* wbuf = reinterpret_cast<float2*>(smem_raw);                     // [warp][TPW][32]  (tau, row offset)
+  float* rbuf = reinterpret_cast<float*>(wbuf + kWarps * TPW * kWarp);     // [warp][TPW][kRes]
+  float* Ds = rbuf + kWarps * TPW * kRes;                                  // [kch][rows][pitch]
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int sub = lane / LPT, sl = lane % LPT;
+  float2* my = wbuf + warp * TPW * kWarp;
+  float* res = rbuf + warp * TPW * kRes;
+  const T* z = static_cast<const T*>(P.z);
+  const T* C = static_cast<const T*>(P.C);
+  const T* g_act = static_cast<const T*>(P.g_act);
+  const T* g_delta = static_cast<const T*>(P.g_delta);
+  T* dz = static_cast<T*>(P.dz);
+  const bool two = P.g.order != 1;
+  const int R = P.L - 1;                                                   // difference rows per key
+  const int64_t tile0 = (int64_t)blockIdx.x * (kWarps * TPW * P.groups);
+  const int j0 = blockIdx.y * P.kch, kc = min(P.kch, P.h - j0);
+
+  if constexpr (STAGED) {
+    int per = 32;
+    while (per > P.r) per >>= 1;
+    const int c0 = threadIdx.x & (per - 1);
+    for (int row = threadIdx.x / per; row < kc * R; row += blockDim.x / per) {
+      const T* src = C + ((size_t)(j0 + row / R) * P.L + row % R) * P.r;
+      for (int c = c0; c < pitch; c += per)
+        Ds[(size_t)row * pitch + c] = c < P.r ? ld_f32<T>(src + P.r + c) - ld_f32<T>(src + c) : 0.0f;
+    }
+  }
+  __syncthreads();
+
+  for (int m = 0; m < P.groups; ++m) {
+    const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+    if (n0 >= P.N) break;
+    float zz[TPW];
+    uint32_t live = 0u;                                                    // bit t: 0 <= u <= G-1 for (t, lane)
+#pragma unroll
+    for (int t = 0; t < TPW; ++t) {
+      float2 w = make_float2(0.0f, 0.0f);
+      zz[t] = 0.0f;
+      if (lane < kc && n0 + t < P.N) {
+        zz[t] = ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
+        const Knot k = knot_of(zz[t], P.g);
+        w = make_float2(k.tau, __int_as_float(STAGED ? (lane * R + k.bin) * pitch : (lane * P.L + k.bin) * P.r));
+        if (k.clamp_active) live |= 1u << t;
+      }
+      my[t * kWarp + lane] = w;
+    }
+    float gd[CV][V];
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int col = c * (LPT * V) + sl * V + i;
+        gd[c][i] = (n0 + sub < P.N && col < P.r) ? ld_f32<T>(g_delta + (n0 + sub) * P.gds + col) : 0.0f;
+      }
+    __syncwarp();
+#pragma unroll 1
+    for (int q0 = 0; q0 < kc; q0 += LPT) {
+      float v[LPT];
+#pragma unroll
+      for (int q = 0; q < LPT; ++q) {
+        const float2 w = my[sub * kWarp + q0 + q];                          // keys past kc: row 0, result unused
+        float s = 0.0f;
+#pragma unroll
+        for (int c = 0; c < CV; ++c) {
+          float d[V], e[V];
+          if constexpr (STAGED) {
+            const float* row = Ds + __float_as_int(w.y) + sl * V + c * (LPT * V);
+            const float4 a = *reinterpret_cast<const float4*>(row);
+            d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;
+            if (two) {
+              const float4 b = *reinterpret_cast<const float4*>(row + pitch);
+              e[0] = b.x; e[1] = b.y; e[2] = b.z; e[3] = b.w;
+            }
+          } else {
+            const T* row = C + (size_t)j0 * P.L * P.r + __float_as_int(w.y);
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              const int col = c * (LPT * V) + sl * V + i;
+              const float c1 = col < P.r ? ld_f32<T>(row + P.r + col) : 0.0f;
+              d[i] = col < P.r ? c1 - ld_f32<T>(row + col) : 0.0f;
+              e[i] = two && col < P.r ? ld_f32<T>(row + 2 * P.r + col) - c1 : 0.0f;
+            }
+          }
+          if (two) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) d[i] = fmaf(w.x, e[i] - d[i], d[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < V; ++i) s = fmaf(gd[c][i], d[i], s);
+        }
+        v[q] = s;
+      }
+      // afterwards v[0] of lane sl is the sum over the token's lanes of v[sl]
+#pragma unroll
+      for (int s = LPT / 2; s >= 1; s >>= 1) {
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+          const bool up = (sl & s) != 0;
+          const float send = up ? v[i] : v[i + s];
+          const float keep = up ? v[i + s] : v[i];
+          v[i] = keep + __shfl_xor_sync(kFull, send, s);
+        }
+      }
+      res[sub * kRes + q0 + sl] = v[0];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < TPW; ++t) {
+      if (lane < kc && n0 + t < P.N) {
+        float o = (live >> t) & 1u ? P.coef * res[t * kRes + lane] : 0.0f;
+        if (g_act) o = fmaf(ld_f32<T>(g_act + (n0 + t) * P.gas + j0 + lane), act_grad(zz[t], P.act), o);
+        st_f32<T>(dz + (n0 + t) * P.dzs + j0 + lane, o);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dC: grid = (key groups, token splits), one warp per key.  A tile of up to 256 tokens is staged (g rows in
+// float32 and the CTA's columns of z); the warp sorts the tile's tokens by knot interval (a counting sort
+// over warp votes, so the order, and with it the result, is always the same) and walks the intervals: the
+// order + 1 rows of an interval are summed in registers over all of its tokens and added to the key's
+// accumulator once per interval, where adding every token to its rows would read and write three rows
+// of shared memory for each.  Tokens outside the grid have no weight and leave the lists.
+//
+// Bound: instruction issue (about seven warp instructions per pair at r = 32) and one row of g per pair.
+// ---------------------------------------------------------------------------------------------
+struct DcArgs {
+  const void* z;
+  int64_t zs;
+  const void* g_delta;
+  int64_t gds;
+  float* part;               // [splits][h][L][r]; null: the sums are final and go to dC / dC_cast
+  float* dC;
+  void* dC_cast;
+  int64_t N;
+  int h, L, r;
+  GridParams g;
+  float lambda;
+  int TT;                    // tokens per tile, a multiple of 32
+  int64_t tokens_per_split;
+};
+
+constexpr int kMaxTile = 256;
+
+// GACC = true: a key's accumulator does not fit shared memory and lives in the partial buffer.
+template <typename T, int LPT, int CV, bool GACC>
+__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs P) {
+  constexpr int V = 4;
+  constexpr int S = kWarp / LPT;
+  constexpr int pitch = LPT * V * CV;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int W = blockDim.x / kWarp, TT = P.TT, nb = P.L - P.g.order, r = P.r;
+  const int zp = W + 1;
+  float* gs = reinterpret_cast<float*>(smem_raw);                          // [TT][pitch]
+  float4* ent_all = reinterpret_cast<float4*>(gs + (size_t)TT * pitch);    // [W][TT]  (w0, w1, w2, token)
+  float* acc_all = reinterpret_cast<float*>(ent_all + (size_t)W * TT);     // [W][L][pitch] unless GACC
+  float* zt = acc_all + (GACC ? 0 : (size_t)W * P.L * pitch);              // [TT][zp]
+  int* off_all = reinterpret_cast<int*>(zt + (size_t)TT * zp);             // [W][nb + 1]
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int sub = lane / LPT, sl = lane % LPT;
+  const int j0 = blockIdx.x * W, kd = min(W, P.h - j0);
+  const int64_t nbeg = (int64_t)blockIdx.y * P.tokens_per_split, nend = min(P.N, nbeg + P.tokens_per_split);
+  const T* z = static_cast<const T*>(P.z);
+  const T* g_delta = static_cast<const T*>(P.g_delta);
+  const bool three = P.g.order != 1;
+  const bool mine = warp < kd;
+  float4* ent = ent_all + (size_t)warp * TT;
+  int* off = off_all + warp * (nb + 1);
+  float* acc = GACC ? P.part + (((size_t)blockIdx.y * P.h + j0 + (mine ? warp : 0)) * P.L) * r
+                    : acc_all + (size_t)warp * P.L * pitch;
+  const int ap = GACC ? r : pitch;
+
+  if constexpr (GACC) {
+    if (mine)
+      for (int i = lane; i < P.L * r; i += kWarp) acc[i] = 0.0f;
+  } else {
+    zero16(acc_all, (size_t)W * P.L * pitch * sizeof(float));
+  }
+  int per = 32;
+  while (per > r) per >>= 1;
+  const int c0 = threadIdx.x & (per - 1);
+  if (r != pitch) zero16(gs, (size_t)TT * pitch * sizeof(float));
+
+  for (int64_t t0 = nbeg; t0 < nend; t0 += TT) {
+    const int tt = (int)min((int64_t)TT, nend - t0);
+    __syncthreads();
+    for (int t = threadIdx.x / per; t < tt; t += blockDim.x / per)
+      for (int c = c0; c < r; c += per) gs[(size_t)t * pitch + c] = ld_f32<T>(g_delta + (t0 + t) * P.gds + c);
+    for (int i = threadIdx.x; i < tt * W; i += blockDim.x) {
+      const int t = i / W, k = i % W;
+      zt[t * zp + k] = k < kd ? ld_f32<T>(z + (t0 + t) * P.zs + j0 + k) : 0.0f;
+    }
+    for (int i = lane; i <= nb; i += kWarp) off[i] = 0;
+    __syncthreads();
+    if (!mine) continue;
+
+    // ---- rank of every token within its interval, counts per interval
+    int bins[kMaxTile / kWarp], pos[kMaxTile / kWarp];
+    float tau[kMaxTile / kWarp];
+#pragma unroll
+    for (int i = 0; i < kMaxTile / kWarp; ++i) {
+      bins[i] = -1;
+      if (i * kWarp < tt) {
+        const int t = i * kWarp + lane;
+        if (t < tt) {
+          const Knot k = knot_of(zt[t * zp + warp], P.g);
+          tau[i] = k.tau;
+          if (k.in_range) bins[i] = k.bin;
+        }
+        const unsigned same = __match_any_sync(kFull, bins[i]);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        const int base = bins[i] >= 0 ? off[bins[i]] : 0;
+        __syncwarp();
+        if (bins[i] >= 0 && rank == 0) off[bins[i]] = base + __popc(same);
+        __syncwarp();
+        pos[i] = base + rank;
+      }
+    }
+    // ---- counts -> first entry of each interval (off[nb] = number of entries)
+    int carry = 0;
+    for (int b0 = 0; b0 <= nb; b0 += kWarp) {
+      const int b = b0 + lane;
+      const int c = b < nb ? off[b] : 0;
+      int x = c;
+#pragma unroll
+      for (int s = 1; s < kWarp; s <<= 1) {
+        const int y = __shfl_up_sync(kFull, x, s);
+        if (lane >= s) x += y;
+      }
+      if (b <= nb) off[b] = carry + x - c;
+      carry += __shfl_sync(kFull, x, kWarp - 1);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kMaxTile / kWarp; ++i) {
+      if (bins[i] >= 0) {
+        Knot k;
+        k.tau = tau[i];
+        k.in_range = true;
+        float B0, B1, B2;
+        basis_weights(k, B0, B1, B2, P.g.order);
+        ent[off[bins[i]] + pos[i]] = make_float4(B0, B1, B2, __int_as_float(i * kWarp + lane));
+      }
+    }
+    __syncwarp();
+    // ---- one interval at a time
+    int end = off[0];
+    for (int b = 0; b < nb; ++b) {
+      const int beg = end;
+      end = off[b + 1];
+      if (beg == end) continue;
+      float a[3][CV][V];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int c = 0; c < CV; ++c)
+#pragma unroll
+          for (int i = 0; i < V; ++i) a[k][c][i] = 0.0f;
+#pragma unroll 2
+      for (int p = beg + sub; p < end; p += S) {
+        const float4 e = ent[p];
+        const float* gr = gs + (size_t)__float_as_int(e.w) * pitch + sl * V;
+#pragma unroll
+        for (int c = 0; c < CV; ++c) {
+          const float4 g4 = *reinterpret_cast<const float4*>(gr + c * (LPT * V));
+          const float gv[V] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            a[0][c][i] = fmaf(e.x, gv[i], a[0][c][i]);
+            a[1][c][i] = fmaf(e.y, gv[i], a[1][c][i]);
+            a[2][c][i] = fmaf(e.z, gv[i], a[2][c][i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k == 2 && !three) break;
+#pragma unroll
+        for (int c = 0; c < CV; ++c) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+#pragma unroll
+            for (int s = LPT; s < kWarp; s <<= 1) a[k][c][i] += __shfl_xor_sync(kFull, a[k][c][i], s);
+          }
+          if (sub == 0) {
+            float* dst = acc + (size_t)(b + k) * ap + sl * V + c * (LPT * V);
+            if constexpr (GACC) {
+#pragma unroll
+              for (int i = 0; i < V; ++i)
+                if (sl * V + c * (LPT * V) + i < r) dst[i] += a[k][c][i];
+            } else {
+              float4 d = *reinterpret_cast<float4*>(dst);
+              d.x += a[k][c][0]; d.y += a[k][c][1]; d.z += a[k][c][2]; d.w += a[k][c][3];
+              *reinterpret_cast<float4*>(dst) = d;
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  if (!mine) return;
+  const size_t row0 = (size_t)(j0 + warp) * P.L;
+  if (P.part) {
+    if constexpr (!GACC) {
+      float* dst = P.part + ((size_t)blockIdx.y * P.h * P.L + row0) * r;
+      for (int i = lane; i < P.L * r; i += kWarp) dst[i] = acc[(size_t)(i / r) * pitch + i % r];
+    }
+  } else {
+    for (int i = lane; i < P.L * r; i += kWarp) {
+      const float v = P.lambda * acc[(size_t)(i / r) * pitch + i % r];
+      if (P.dC) P.dC[row0 * r + i] = v;
+      if (P.dC_cast) st_f32<T>(static_cast<T*>(P.dC_cast) + row0 * r + i, v);
+    }
+  }
 }
 
 template <typename T>
@@ -257,6 +679,7 @@ __global__ void simt_dc_reduce_kernel(const float* __restrict__ part, int splits
                                       float* __restrict__ dC, T* __restrict__ dC_cast) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < elems; i += (size_t)gridDim.x * blockDim.x) {
     float s = 0.0f;
+#pragma unroll 4
     for (int k = 0; k < splits; ++k) s += part[(size_t)k * elems + i];
     s *= lambda;
     if (dC) dC[i] = s;
@@ -275,43 +698,140 @@ __global__ void simt_knot_index_kernel(const T* __restrict__ z, int64_t zs, int6
   }
 }
 
-constexpr size_t kSmemBudget = 160 * 1024;
+// =================================================================================================
+// plans and launches
+// =================================================================================================
+constexpr int kPlanSMs = 148;                            // B200; only used to balance launch shapes
+constexpr size_t kSmemHalf = 110 * 1024;                 // two CTAs per SM
+constexpr size_t kSmemFull = 216 * 1024;
+constexpr size_t kFwdScratchCap = SKV_NOALLOC_SCRATCH_BYTES;   // the key splits' partials stay below this
 
-struct FwdPlan { int TB, KCH; size_t smem; };
-FwdPlan plan_token_major(const skv_problem& p, bool with_dacc) {
+// Lanes per token (a power of two from 2 to 32) and 16-byte pieces per lane for rows of r elements.
+void lanes_for(int r, int v, int* lpt, int* cv) {
+  int l = 2;
+  while (l < 32 && l * v < r) l <<= 1;
+  *lpt = l;
+  *cv = l * v < r ? 2 : 1;
+}
+
+struct FwdPlan { bool small; int lpt, cv, kch, groups, splits, keys_per_split; int64_t tiles; size_t smem; };
+
+FwdPlan plan_forward(const skv_problem& p) {
   FwdPlan f;
-  f.TB = 128;
-  const size_t per_key = (size_t)p.L * p.r * sizeof(float);
-  const size_t dacc = with_dacc ? (size_t)f.TB * p.r * sizeof(float) : 0;
-  size_t kch = (kSmemBudget - dacc) / per_key;
-  if (kch >= 32) kch = kch / 32 * 32;
-  if (kch > 64) kch = 64;
-  if (kch > (size_t)p.h) kch = p.h;
-  if (kch < 1) kch = 1;
-  f.KCH = (int)kch;
-  f.smem = kch * per_key + dacc;
+  const int size = p.dtype == SKV_BF16 ? 2 : 4, v = 16 / size;
+  lanes_for(p.r, v, &f.lpt, &f.cv);
+  const int tpw = kWarp / f.lpt, pitch = f.lpt * v * f.cv;
+  const int64_t N = p.N > 0 ? p.N : 1;
+  const size_t wb = (size_t)kWarps * tpw * kWarp * 16, per_key = (size_t)p.L * pitch * size;
+  size_t kch = kSmemHalf > wb ? (kSmemHalf - wb) / per_key : 0;
+  if (kch < 8) kch = (kSmemFull - wb) / per_key;
+  f.kch = (int)(kch > 32 ? 32 : kch);
+  f.small = f.kch < 1 || N <= small_forward_tokens(p);
+  const size_t part_bytes = (size_t)N * p.r * sizeof(float);
+  if (f.small) {
+    int tg = 1;
+    while (tg < tpw && tg < N) tg <<= 1;
+    f.groups = tg;
+    f.tiles = cdiv64(N, tg);
+    // the largest pass that still gives two CTAs per SM, so that few partials are left to add
+    int kw = 4;
+    while (kw < tpw / tg) kw <<= 1;
+    while (kw < 32 && 2 * kw * tg <= kSmallEntries && f.tiles * cdiv64(p.h, kWarps * kw * 2) >= 2 * kPlanSMs) kw <<= 1;
+    f.kch = kw;
+    int64_t splits = cdiv64(p.h, kWarps * kw);
+    const int64_t most = (int64_t)(kFwdScratchCap / part_bytes);
+    if (splits > most) splits = most > 1 ? most : 1;
+    f.keys_per_split = (int)(cdiv64(cdiv64(p.h, splits), kWarps * kw) * kWarps * kw);
+    f.splits = (int)cdiv64(p.h, f.keys_per_split);
+    f.smem = 0;
+    return f;
+  }
+  f.smem = wb + (size_t)f.kch * per_key;
+  const int slots = kPlanSMs * (f.smem <= kSmemHalf + 1024 ? 2 : 1);
+  const int slabs = (int)cdiv64(p.h, f.kch);
+  // clocks: a slab's copy, the work of one token group on it, and the partials' round trip
+  const double copy = (double)f.kch * per_key / 32.0;
+  const double work = (double)kWarps * tpw * f.kch * (pitch * size / 64.0 + 0.5);
+  double best = 0.0;
+  for (int groups = kGroups; groups >= 1; groups >>= 1) {
+    const int64_t tiles = cdiv64(N, (int64_t)kWarps * tpw * groups);
+    for (int per = slabs; per >= 1; --per) {
+      const int splits = (int)cdiv64(slabs, per);
+      if (splits > 1 && splits * part_bytes > kFwdScratchCap) break;
+      if (per < slabs && cdiv64(slabs, per + 1) == splits) continue;
+      const double t = (double)cdiv64(tiles * splits, slots) * per * (copy + groups * work) +
+                       (splits > 1 ? 4000.0 + (double)splits * part_bytes / 1500.0 : 0.0);
+      if (best == 0.0 || t < best) {
+        best = t;
+        f.groups = groups;
+        f.tiles = tiles;
+        f.splits = splits;
+        f.keys_per_split = per * f.kch;
+      }
+    }
+  }
   return f;
 }
 
-struct DcPlan { int KD, TT, splits; int64_t tokens_per_split; size_t smem; };
-DcPlan plan_dc(const skv_problem& p, int num_sms) {
+struct DzPlan { bool staged; int lpt, cv, kch, groups; int64_t tiles; size_t smem; };
+DzPlan plan_dz(const skv_problem& p) {
+  DzPlan d;
+  lanes_for(p.r, 4, &d.lpt, &d.cv);
+  const int tpw = kWarp / d.lpt, pitch = d.lpt * 4 * d.cv;
+  const size_t bufs = (size_t)kWarps * tpw * (kWarp * 8 + (kWarp + 4) * 4), per_key = (size_t)(p.L - 1) * pitch * 4;
+  size_t kch = (kSmemHalf - bufs) / per_key;
+  if (kch < 8) kch = (kSmemFull - bufs) / per_key;
+  d.staged = kch >= 1;
+  if (kch > 32 || !d.staged) kch = 32;
+  while (kch > 8 && kch % 8) --kch;
+  d.kch = (int)kch;
+  d.smem = bufs + (d.staged ? kch * per_key : 0);
+  const int slots = kPlanSMs * (d.smem <= kSmemHalf + 1024 ? 2 : 1);
+  const int64_t N = p.N > 0 ? p.N : 1, slabs = cdiv64(p.h, d.kch), unit = (int64_t)kWarps * tpw;
+  const double copy = d.staged ? (double)kch * per_key / 24.0 : 0.0;
+  const double work = (double)unit * kch * (pitch / 16.0 + 0.5);
+  double best = 0.0;
+  for (int64_t groups = 1; groups <= 64; groups <<= 1) {
+    const int64_t tiles = cdiv64(N, unit * groups);
+    const double t = (double)cdiv64(tiles * slabs, slots) * (copy + groups * work);
+    if (best == 0.0 || t < best) { best = t; d.groups = (int)groups; d.tiles = tiles; }
+    if (tiles == 1) break;
+  }
+  return d;
+}
+
+struct DcPlan { bool gacc; int lpt, cv, W, TT, splits; int64_t tokens_per_split; size_t smem; };
+DcPlan plan_dc(const skv_problem& p) {
   DcPlan d;
-  const size_t per_key = (size_t)p.L * p.r * sizeof(float);
-  d.TT = 64;
-  int kd = 16;
-  while (kd > 1 && kd * per_key + (size_t)d.TT * (p.r + kd) * sizeof(float) > kSmemBudget) kd /= 2;
-  d.KD = kd;
-  d.smem = kd * per_key + (size_t)d.TT * (p.r + kd) * sizeof(float);
-  const int64_t groups = cdiv64(p.h, kd);
-  int64_t splits = cdiv64(2 * (int64_t)num_sms, groups);
-  const int64_t max_splits = cdiv64(p.N, 256);
-  if (splits > max_splits) splits = max_splits;
-  if (splits > 16) splits = 16;
-  if (splits < 1) splits = 1;
-  d.tokens_per_split = cdiv64(cdiv64(p.N, splits), d.TT) * d.TT;
-  if (d.tokens_per_split < d.TT) d.tokens_per_split = d.TT;
-  d.splits = (int)cdiv64(p.N, d.tokens_per_split);
-  if (d.splits < 1) d.splits = 1;
+  lanes_for(p.r, 4, &d.lpt, &d.cv);
+  const int pitch = d.lpt * 4 * d.cv, nb = p.L - 1;
+  const size_t per_acc = (size_t)p.L * pitch * 4;
+  auto bytes = [&](int W, int TT, bool gacc) {
+    return (size_t)TT * pitch * 4 + (size_t)W * TT * 16 + (gacc ? 0 : W * per_acc) + (size_t)TT * (W + 1) * 4 +
+           (size_t)W * (nb + 2) * 4;
+  };
+  // eight keys and 256 tokens with two CTAs per SM where that fits, then smaller tiles, then fewer keys
+  d.gacc = false;
+  d.W = kWarps;
+  d.TT = kMaxTile;
+  while (d.TT > 64 && bytes(d.W, d.TT, false) > kSmemHalf) d.TT >>= 1;
+  if (bytes(d.W, d.TT, false) > kSmemHalf) d.TT = 128;
+  while (d.W > 1 && bytes(d.W, d.TT, false) > kSmemFull) d.W >>= 1;
+  if (bytes(d.W, d.TT, false) > kSmemFull) { d.gacc = true; d.W = kWarps; d.TT = 64; }
+  d.smem = bytes(d.W, d.TT, d.gacc);
+  const int slots = kPlanSMs * (d.smem <= kSmemHalf + 1024 ? 2 : 1);
+  const int64_t N = p.N > 0 ? p.N : 1, groups = cdiv64(p.h, d.W), tiles = cdiv64(N, d.TT);
+  const double elems = (double)p.h * p.L * p.r;
+  double best = 0.0;
+  for (int64_t per = tiles; per >= 1; --per) {
+    const int64_t splits = cdiv64(tiles, per);
+    if (splits > 16) break;
+    if (per < tiles && cdiv64(tiles, per + 1) == splits) continue;
+    // clocks: a tile per warp about 7 instructions per pair and 40 per interval; partials' round trip
+    const double t = (double)cdiv64(groups * splits, slots) * per * (d.TT * 14.0 * d.cv + 4000.0) +
+                     (splits > 1 ? 4000.0 + splits * elems * 8 / 1500.0 : 0.0);
+    if (best == 0.0 || t < best) { best = t; d.splits = (int)splits; d.tokens_per_split = per * d.TT; }
+  }
   return d;
 }
 
@@ -326,17 +846,49 @@ int set_smem(K kernel, size_t bytes) {
   return SKV_OK;
 }
 
+// One case per (lanes per token, pieces per lane) that rows of up to 256 elements need.
+#define SKV_LANES(LPT_, CV_, CALL)                                    \
+  if (CV_ == 2) CALL(32, 2)                                           \
+  else if (LPT_ == 2) CALL(2, 1)                                      \
+  else if (LPT_ == 4) CALL(4, 1)                                      \
+  else if (LPT_ == 8) CALL(8, 1)                                      \
+  else if (LPT_ == 16) CALL(16, 1)                                    \
+  else CALL(32, 1)
+
 template <typename T, typename TD>
 int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* act_out, int64_t as,
-              void* delta_out, int64_t ds) {
+              void* delta_out, int64_t ds, void* scratch, size_t scratch_bytes) {
   const skv_problem& p = c.p;
-  FwdPlan f = plan_token_major(p, true);
-  if (int e = set_smem(simt_forward_kernel<T, TD>, f.smem)) return e;
-  const unsigned grid = (unsigned)cdiv64(p.N, f.TB);
-  simt_forward_kernel<T, TD><<<grid, 256, f.smem, c.stream>>>(
-      (const T*)z, zs, (const T*)C, (T*)act_out, as, (TD*)delta_out, ds, p.N, p.h, p.L, p.r, c.g,
-      p.lambda_scale, p.activation, f.TB, f.KCH);
+  FwdPlan f = plan_forward(p);
+  if (f.splits > 1 && (!scratch || scratch_bytes < (size_t)f.splits * p.N * p.r * sizeof(float))) {
+    f.splits = 1;                                        // no room for partials: a CTA covers all keys
+    f.keys_per_split = p.h;
+  }
+  FwdArgs a;
+  a.z = z; a.zs = zs; a.C = C; a.act_out = act_out; a.as = as; a.delta_out = delta_out; a.ds = ds;
+  a.partial = f.splits > 1 ? static_cast<float*>(scratch) : nullptr;
+  a.N = p.N; a.h = p.h; a.L = p.L; a.r = p.r; a.g = c.g; a.lambda = p.lambda_scale; a.act = p.activation;
+  a.kch = f.kch; a.keys_per_split = f.keys_per_split; a.groups = f.groups;
+  const dim3 grid((unsigned)f.tiles, (unsigned)f.splits);
+  const bool vec = p.r % Vec<T>::n == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  int e = SKV_OK;
+#define SKV_CALL(LPT_, CV_)                                                                                     \
+  {                                                                                                             \
+    if (f.small && vec) simt_forward_small_kernel<T, TD, LPT_, CV_, true><<<grid, kWarps * kWarp, 0, c.stream>>>(a);  \
+    else if (f.small) simt_forward_small_kernel<T, TD, LPT_, CV_, false><<<grid, kWarps * kWarp, 0, c.stream>>>(a);   \
+    else if ((e = set_smem(simt_forward_kernel<T, TD, LPT_, CV_>, f.smem)) == SKV_OK)                           \
+      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, kWarps * kWarp, f.smem, c.stream>>>(a);                     \
+  }
+  SKV_LANES(f.lpt, f.cv, SKV_CALL)
+#undef SKV_CALL
+  if (e) return e;
   note_launches(1);
+  if (f.splits > 1) {
+    const int64_t blocks = cdiv64(p.N * p.r, kWarp);
+    simt_finalize_kernel<TD><<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, c.stream>>>(
+        a.partial, f.splits, p.N, p.r, p.lambda_scale, static_cast<TD*>(delta_out), ds);
+    note_launches(1);
+  }
   return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }
 
@@ -346,30 +898,60 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
                void* scratch, size_t scratch_bytes) {
   const skv_problem& p = c.p;
   if (dz) {
-    FwdPlan f = plan_token_major(p, false);
-    if (int e = set_smem(simt_dz_kernel<T>, f.smem)) return e;
-    const unsigned grid = (unsigned)cdiv64(p.N, f.TB);
-    simt_dz_kernel<T><<<grid, 256, f.smem, c.stream>>>(
-        (const T*)z, zs, (const T*)C, (const T*)g_act, gas, (const T*)g_delta, gds, (T*)dz, dzs, p.N, p.h, p.L,
-        p.r, c.g, p.lambda_scale, p.activation, f.TB, f.KCH);
+    const DzPlan d = plan_dz(p);
+    DzArgs a;
+    a.z = z; a.zs = zs; a.C = C; a.g_act = g_act; a.gas = gas; a.g_delta = g_delta; a.gds = gds; a.dz = dz; a.dzs = dzs;
+    a.N = p.N; a.h = p.h; a.L = p.L; a.r = p.r; a.g = c.g; a.coef = p.lambda_scale * c.g.scale; a.act = p.activation;
+    a.kch = d.kch; a.groups = d.groups;
+    const dim3 grid((unsigned)d.tiles, (unsigned)cdiv64(p.h, d.kch));
+    int e = SKV_OK;
+#define SKV_CALL(LPT_, CV_)                                                                              \
+  {                                                                                                      \
+    if (!d.staged) {                                                                                     \
+      if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, false>, d.smem)) == SKV_OK)                         \
+        simt_dz_kernel<T, LPT_, CV_, false><<<grid, kWarps * kWarp, d.smem, c.stream>>>(a);              \
+    } else if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, true>, d.smem)) == SKV_OK)                     \
+      simt_dz_kernel<T, LPT_, CV_, true><<<grid, kWarps * kWarp, d.smem, c.stream>>>(a);                 \
+  }
+    SKV_LANES(d.lpt, d.cv, SKV_CALL)
+#undef SKV_CALL
+    if (e) return e;
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
   }
   if (dC || dC_cast) {
-    DcPlan d = plan_dc(p, c.num_sms);
+    const DcPlan d = plan_dc(p);
     const size_t elems = (size_t)p.h * p.L * p.r;
-    if (!scratch || scratch_bytes < (size_t)d.splits * elems * sizeof(float)) return SKV_ERR_SCRATCH;
-    if (int e = set_smem(simt_dc_partial_kernel<T>, d.smem)) return e;
-    dim3 grid((unsigned)cdiv64(p.h, d.KD), (unsigned)d.splits);
-    simt_dc_partial_kernel<T><<<grid, d.KD * kWarp, d.smem, c.stream>>>(
-        (const T*)z, zs, (const T*)g_delta, gds, (float*)scratch, p.N, p.h, p.L, p.r, c.g, d.KD, d.TT,
-        d.tokens_per_split);
+    const bool parts = d.splits > 1 || d.gacc;
+    if (parts && (!scratch || scratch_bytes < (size_t)d.splits * elems * sizeof(float))) return SKV_ERR_SCRATCH;
+    DcArgs a;
+    a.z = z; a.zs = zs; a.g_delta = g_delta; a.gds = gds;
+    a.part = parts ? static_cast<float*>(scratch) : nullptr;
+    a.dC = dC; a.dC_cast = dC_cast;
+    a.N = p.N; a.h = p.h; a.L = p.L; a.r = p.r; a.g = c.g; a.lambda = p.lambda_scale;
+    a.TT = d.TT; a.tokens_per_split = d.tokens_per_split;
+    const dim3 grid((unsigned)cdiv64(p.h, d.W), (unsigned)d.splits);
+    int e = SKV_OK;
+#define SKV_CALL(LPT_, CV_)                                                                              \
+  {                                                                                                      \
+    if (d.gacc) {                                                                                        \
+      if ((e = set_smem(simt_dc_kernel<T, LPT_, CV_, true>, d.smem)) == SKV_OK)                          \
+        simt_dc_kernel<T, LPT_, CV_, true><<<grid, d.W * kWarp, d.smem, c.stream>>>(a);                  \
+    } else if ((e = set_smem(simt_dc_kernel<T, LPT_, CV_, false>, d.smem)) == SKV_OK)                    \
+      simt_dc_kernel<T, LPT_, CV_, false><<<grid, d.W * kWarp, d.smem, c.stream>>>(a);                   \
+  }
+    SKV_LANES(d.lpt, d.cv, SKV_CALL)
+#undef SKV_CALL
+    if (e) return e;
+    note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
-    const unsigned rgrid = (unsigned)((elems + 255) / 256 < 4096 ? (elems + 255) / 256 : 4096);
-    simt_dc_reduce_kernel<T><<<rgrid, 256, 0, c.stream>>>((const float*)scratch, d.splits, elems,
-                                                           p.lambda_scale, dC, (T*)dC_cast);
-    note_launches(2);
-    if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
+    if (parts) {
+      const unsigned rgrid = (unsigned)((elems + 255) / 256 < 4096 ? (elems + 255) / 256 : 4096);
+      simt_dc_reduce_kernel<T><<<rgrid, 256, 0, c.stream>>>(a.part, d.splits, elems, p.lambda_scale, dC,
+                                                            static_cast<T*>(dC_cast));
+      note_launches(1);
+      if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
+    }
   }
   return SKV_OK;
 }
@@ -377,20 +959,26 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
 }  // namespace
 
 size_t simt_scratch_bytes(const skv_problem& p, int op) {
-  if (op != SKV_OP_BACKWARD) return 0;
-  // independent of the SM count actually present: sized for the largest split count plan_dc can pick
-  DcPlan d = plan_dc(p, 148);
-  int splits = d.splits;
-  DcPlan d2 = plan_dc(p, 256);
-  if (d2.splits > splits) splits = d2.splits;
-  return (size_t)splits * p.h * p.L * p.r * sizeof(float);
+  if (op == SKV_OP_BACKWARD) {
+    const DcPlan d = plan_dc(p);
+    return d.splits > 1 || d.gacc ? (size_t)d.splits * p.h * p.L * p.r * sizeof(float) : 0;
+  }
+  const FwdPlan f = plan_forward(p);
+  return f.splits > 1 ? (size_t)f.splits * (p.N > 0 ? p.N : 1) * p.r * sizeof(float) : 0;
+}
+
+int64_t small_forward_tokens(const skv_problem& p) {
+  (void)p;
+  return 64;
 }
 
 int simt_forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* act_out, int64_t as,
-                 void* delta_out, int64_t ds) {
-  if (c.p.dtype == SKV_F32) return forward_t<float, float>(c, z, zs, C, act_out, as, delta_out, ds);
-  return c.p.delta_f32 ? forward_t<__nv_bfloat16, float>(c, z, zs, C, act_out, as, delta_out, ds)
-                       : forward_t<__nv_bfloat16, __nv_bfloat16>(c, z, zs, C, act_out, as, delta_out, ds);
+                 void* delta_out, int64_t ds, void* scratch, size_t scratch_bytes) {
+  if (c.p.dtype == SKV_F32)
+    return forward_t<float, float>(c, z, zs, C, act_out, as, delta_out, ds, scratch, scratch_bytes);
+  return c.p.delta_f32
+             ? forward_t<__nv_bfloat16, float>(c, z, zs, C, act_out, as, delta_out, ds, scratch, scratch_bytes)
+             : forward_t<__nv_bfloat16, __nv_bfloat16>(c, z, zs, C, act_out, as, delta_out, ds, scratch, scratch_bytes);
 }
 
 int simt_backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const void* g_act, int64_t gas,
