@@ -38,6 +38,7 @@ class SplineKVError(RuntimeError):
 
 
 _lib = None
+_host = None
 
 
 def load() -> ctypes.CDLL:
@@ -80,6 +81,21 @@ def load() -> ctypes.CDLL:
         raise RuntimeError("libsplinekv_b200.so has an unexpected ABI version; rebuild it")
     _lib = lib
     return lib
+
+
+def host():
+    """The native host path of the operators (``csrc/skv_host.cpp``), loaded on top of the library."""
+    global _host
+    if _host is None:
+        load()
+        import torch  # noqa: F401  (its libraries have to be in the process first)
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(f"sparsespline_ffn_b200/_host.so is missing or cannot be loaded ({e}): build it with "
+                               "`python -m sparsespline_ffn_b200.build`.") from e
+        _host = module
+    return _host
 
 
 def check(code: int) -> None:

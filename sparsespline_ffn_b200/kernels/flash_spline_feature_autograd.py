@@ -13,6 +13,9 @@ unchanged.  What differs, on purpose:
   ``SPARSE_SPLINE_FWD_KERNEL`` environment override is honoured the same way.
 * There is no CPU and no eager path: ``use_kernel=False``, CPU tensors or a missing library raise
   ``RuntimeError`` instead of running PyTorch code.
+* A plain call (CUDA tensors of one dtype, shapes that agree) never enters Python beyond ``apply``: checks,
+  allocation, launch and the autograd node are native (``csrc/skv_host.cpp``).  The ``forward`` /
+  ``backward`` below serve every other call: casts, odd strides, errors, the slow-family warning.
 * ``grad_output`` is consumed in place (no ``.contiguous()`` copies of its two halves) and the
   lambda chain-rule factor is applied inside the kernels in float32.
 """
@@ -22,7 +25,7 @@ import os
 
 import torch
 
-from .. import ops
+from .. import _lib, ops
 
 # kernel names the reference accepts (flash_spline_feature_autograd.py:47-51, 83-131, 176-225)
 _REFERENCE_FWD = {"auto", "triton", "wgmma_cuda", "v10_cuda", "v11_cuda"}
@@ -36,6 +39,18 @@ def _impl_of(name: str, vocabulary: set[str], what: str) -> str:
     if name in vocabulary:
         return "auto"
     raise ValueError(f"unknown {what} {name!r}; expected one of {sorted(vocabulary | _OURS)}")
+
+
+_FWD_IMPL = {**{n: 0 for n in _REFERENCE_FWD}, **{n: _lib.SKV_IMPL[n] for n in _OURS}}
+_BWD_IMPL = {**{n: 0 for n in _REFERENCE_BWD}, **{n: _lib.SKV_IMPL[n] for n in _OURS}}
+
+
+def _native(z, C, grid_lo, grid_hi, G, activation, lambda_scale, fwd_impl, bwd_impl, spline_order, with_base):
+    """The call on the native host path, or None when it is not a plain one."""
+    act = _lib.SKV_ACT.get(activation)
+    if act is None or fwd_impl is None or bwd_impl is None or torch._C._are_functorch_transforms_active():
+        return None
+    return _lib.host().feature(z, C, grid_lo, grid_hi, lambda_scale, G, act, fwd_impl, bwd_impl, spline_order, with_base)
 
 
 def _require_kernel(use_kernel: bool, z: torch.Tensor) -> None:
@@ -61,6 +76,15 @@ def _capture_safe_dC_return(C: torch.Tensor, dC: torch.Tensor | None):
 
 class FlashSplineFeature(torch.autograd.Function):
     """``f = [phi(z); lambda * delta(z, C)]`` as ``[N, h + r]`` in the dtype of ``z``."""
+
+    @classmethod
+    def apply(cls, z, C, grid_lo, grid_hi, G, activation, lambda_scale, use_kernel,
+              bwd_kernel="triton", fwd_kernel="auto"):
+        f = _native(z, C, grid_lo, grid_hi, G, activation, lambda_scale, _FWD_IMPL.get(fwd_kernel),
+                    _BWD_IMPL.get(bwd_kernel), 2, True) if use_kernel else None
+        if f is not None:
+            return f
+        return super().apply(z, C, grid_lo, grid_hi, G, activation, lambda_scale, use_kernel, bwd_kernel, fwd_kernel)
 
     @staticmethod
     def forward(ctx, z, C, grid_lo, grid_hi, G, activation, lambda_scale, use_kernel,
@@ -100,6 +124,11 @@ class SplineFeatureOfOrder(torch.autograd.Function):
     runs in PyTorch only), so this is a separate Function and :class:`FlashSplineFeature` keeps the
     reference's argument list."""
 
+    @classmethod
+    def apply(cls, z, C, grid_lo, grid_hi, G, activation, lambda_scale, spline_order):
+        f = _native(z, C, grid_lo, grid_hi, G, activation, lambda_scale, 0, 0, spline_order, True)
+        return f if f is not None else super().apply(z, C, grid_lo, grid_hi, G, activation, lambda_scale, spline_order)
+
     @staticmethod
     def forward(ctx, z, C, grid_lo, grid_hi, G, activation, lambda_scale, spline_order):
         _require_kernel(True, z)
@@ -138,6 +167,12 @@ def flash_spline_feature(z, C, grid_lo=-3.0, grid_hi=3.0, G=20, activation="relu
 class FlashSplineDelta(torch.autograd.Function):
     """Spline residual only: ``lambda * delta(z, C)`` as ``[N, r]``; no base path in either
     direction (reference: flash_spline_feature_autograd.py:295-429)."""
+
+    @classmethod
+    def apply(cls, z, C, grid_lo, grid_hi, G, lambda_scale, bwd_kernel):
+        impl = _BWD_IMPL.get(bwd_kernel)
+        d = _native(z, C, grid_lo, grid_hi, G, "identity", lambda_scale, impl, impl, 2, False)
+        return d if d is not None else super().apply(z, C, grid_lo, grid_hi, G, lambda_scale, bwd_kernel)
 
     @staticmethod
     def forward(ctx, z, C, grid_lo, grid_hi, G, lambda_scale, bwd_kernel):

@@ -13,7 +13,6 @@ import torch
 from . import _lib
 
 _DTYPES = {torch.bfloat16: _lib.SKV_BF16, torch.float32: _lib.SKV_F32}
-_status_words: dict[int, torch.Tensor] = {}
 
 
 def grid_scale(grid_lo: float, grid_hi: float, G: int) -> float:
@@ -25,11 +24,7 @@ def grid_scale(grid_lo: float, grid_hi: float, G: int) -> float:
 def status_word(device: torch.device) -> torch.Tensor:
     """Per-device int32 the kernels write to when a bounded wait runs out (0 = healthy)."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    t = _status_words.get(idx)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = t
-    return t
+    return _lib.host().status_word(idx)
 
 
 def check_status(device: torch.device) -> None:
@@ -178,9 +173,13 @@ def feature_forward(z, C, grid_lo, grid_hi, G, activation="relu_sq", lambda_scal
 def feature_readout_forward(z, C, W_out, grid_lo, grid_hi, G, activation="relu_sq", lambda_scale=1.0):
     """``y = [phi(z); lambda*delta] @ W_out.T`` as ``[N, d_out]`` without the feature in memory.
 
-    bf16 only (``z``, ``C`` and ``W_out`` are cast as the reference's wrapper casts them,
+    bf16 only (plain calls take the native host path, ``csrc/skv_host.cpp``; ``z``, ``C`` and ``W_out`` are cast as the reference's wrapper casts them,
     src/sparsespline_ffn/cuda_ext/__init__.py:626-632); ``W_out`` is ``[d_out, h + r]``, the layout of
     ``torch.nn.Linear.weight``.  Forward only."""
+    if activation in ("relu_sq", "identity"):
+        y = _lib.host().readout(z, C, W_out, grid_lo, grid_hi, lambda_scale, G, _lib.SKV_ACT[activation])
+        if y is not None:
+            return y
     lib = _lib.load()
     if not (z.is_cuda and C.is_cuda and W_out.is_cuda):
         raise RuntimeError("CUDA-only")
