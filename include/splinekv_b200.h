@@ -41,10 +41,11 @@ enum skv_error {
 
 enum skv_dtype { SKV_BF16 = 0, SKV_F32 = 1 };
 enum skv_activation { SKV_ACT_RELU_SQ = 0, SKV_ACT_IDENTITY = 1, SKV_ACT_GELU = 2 };
-/* SKV_IMPL_AUTO picks the tcgen05 kernels when the shape is eligible (bf16, r a multiple of 16
- * up to 128, L up to 64, h a multiple of 8, 16-byte aligned rows) and the CUDA-core kernels
- * otherwise.  The CUDA-core kernels are the float32 tier and a correctness fallback, tens of
- * times slower at production sizes: skv_resolve_impl tells which family a problem gets. */
+/* SKV_IMPL_AUTO picks the tcgen05 kernels when the shape is eligible (bf16, r up to 128, L up to 64, either
+ * spline order; other h and r than multiples of 8 and 16 are padded inside the scratch) and the CUDA-core
+ * kernels otherwise, and for forwards of a few tokens.  The CUDA-core kernels are the float32 tier and the path of
+ * the remaining shapes, several times slower at production sizes: skv_resolve_impl tells which family a
+ * problem gets. */
 enum skv_impl { SKV_IMPL_AUTO = 0, SKV_IMPL_SIMT = 1, SKV_IMPL_TCGEN05 = 2 };
 enum skv_op { SKV_OP_FORWARD = 0, SKV_OP_BACKWARD = 1 };
 
@@ -70,7 +71,7 @@ typedef struct skv_problem {
   int32_t spline_order; /* 0 or 2: quadratic B-spline, L = G + 2 (the operator of the reference's kernels);
                           1: linear B-spline, L = G + 1, weights 1 - tau and tau at rows bin, bin + 1
                           (_b1_basis_and_bins, src/sparsespline_ffn/rl_spline_kv_reference.py:125-142, which the
-                          reference evaluates in PyTorch only); runs on the CUDA-core kernels */
+                          reference evaluates in PyTorch only) */
 } skv_problem;
 
 /* ABI version of the loaded library (SKV_ABI_VERSION). */

@@ -52,7 +52,7 @@ int validate(const skv_problem* p) {
 
 int resolve(const skv_problem& p) {
   if (p.impl == SKV_IMPL_SIMT) return SKV_IMPL_SIMT;
-  const bool ok = p.spline_order != 1 && tc_eligible(p);      // the linear spline runs on the CUDA-core kernels
+  const bool ok = tc_eligible(p);
   if (p.impl == SKV_IMPL_TCGEN05) return ok ? (int)SKV_IMPL_TCGEN05 : (int)SKV_ERR_UNSUPPORTED;
   return ok ? (int)SKV_IMPL_TCGEN05 : (int)SKV_IMPL_SIMT;
 }
@@ -100,6 +100,14 @@ int make_ctx(const skv_problem* p, void* stream, int32_t* status, LaunchCtx* c) 
 }
 
 bool aligned(const void* p, size_t a) { return ((uintptr_t)p % a) == 0; }
+
+// Whether the token-major rows of this shape ([N][h] and [N][h + r] tensors) start on 16-byte boundaries and hold
+// whole chunks of keys.  Where they do not, the tensor-core kernels work on padded copies, and the
+// scratch size includes them.
+bool rows_fit(const skv_problem& p) { return p.h % 8 == 0 && p.r % 8 == 0; }
+
+// The rows of one array as a call passes it: pointer and stride in 16-byte pieces.
+bool row_ok(const void* p, int64_t stride, int64_t per16) { return !p || (aligned(p, 16) && stride % per16 == 0); }
 
 }  // namespace
 
@@ -156,13 +164,7 @@ size_t skv_scratch_bytes(const skv_problem* p, int op) {
   const int impl = resolve(*p);
   if (impl == SKV_IMPL_SIMT) return simt_scratch_bytes(*p, op);
   if (impl != SKV_IMPL_TCGEN05) return 0;
-  size_t need = tc_scratch_bytes(*p, op);
-  if (p->impl == SKV_IMPL_AUTO) {
-    // AUTO falls back to the CUDA-core kernels when a pointer or stride is not 16-byte aligned
-    const size_t alt = simt_scratch_bytes(*p, op);
-    if (alt > need) need = alt;
-  }
-  return need;
+  return tc_scratch_bytes(*p, op, rows_fit(*p));
 }
 
 int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, void* act_out,
@@ -177,13 +179,14 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
   if (impl < 0) return impl;
   const bool small = p->impl == SKV_IMPL_AUTO && p->N <= small_forward_tokens(*p);
   if (impl == SKV_IMPL_TCGEN05 && !small) {
-    if (!aligned(z, 16) || !aligned(C, 16) || !aligned(delta_out, 16) || (act_out && !aligned(act_out, 16)) ||
-        z_stride % 8 || delta_stride % (p->delta_f32 ? 4 : 8) || (act_out && act_stride % 8)) {
-      if (p->impl == SKV_IMPL_TCGEN05) return SKV_ERR_ALIGN;
-    } else {
-      if (!scratch || scratch_bytes < tc_scratch_bytes(*p, SKV_OP_FORWARD)) return SKV_ERR_SCRATCH;
-      return tc_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
+    const bool ok = p->h % 8 == 0 && row_ok(z, z_stride, 8) && row_ok(act_out, act_stride, 8);
+    const bool copies = !ok && scratch_bytes >= tc_scratch_bytes(*p, SKV_OP_FORWARD, false);
+    if (ok || copies || rows_fit(*p) == false) {
+      if (!scratch || scratch_bytes < tc_scratch_bytes(*p, SKV_OP_FORWARD, ok)) return SKV_ERR_SCRATCH;
+      return tc_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, ok);
     }
+    // rows of a fitting shape passed at odd addresses or strides: there is no room for copies
+    if (p->impl == SKV_IMPL_TCGEN05) return SKV_ERR_ALIGN;
   }
   return simt_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
 }
@@ -210,15 +213,15 @@ int skv_feature_backward(const skv_problem* p, const void* z, int64_t z_stride, 
   const bool dz32 = p->dz_f32 && p->dtype == SKV_BF16;          // float32 dz of a bf16 problem: tcgen05 kernels only
   if (dz32 && impl != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;
   if (impl == SKV_IMPL_TCGEN05) {
-    if (!aligned(z, 16) || !aligned(C, 16) || !aligned(g_delta, 16) || (g_act && !aligned(g_act, 16)) ||
-        (dz && !aligned(dz, 16)) || z_stride % 8 || gdelta_stride % 8 || (g_act && gact_stride % 8) ||
-        (dz && dz_stride % (dz32 ? 4 : 8))) {
-      if (p->impl == SKV_IMPL_TCGEN05 || dz32) return SKV_ERR_ALIGN;
-    } else {
-      if (!scratch || scratch_bytes < tc_scratch_bytes(*p, SKV_OP_BACKWARD)) return SKV_ERR_SCRATCH;
+    const bool ok = p->h % 8 == 0 && row_ok(z, z_stride, 8) && row_ok(g_act, gact_stride, 8) &&
+                    row_ok(dz, dz_stride, dz32 ? 4 : 8);
+    const bool copies = !ok && scratch_bytes >= tc_scratch_bytes(*p, SKV_OP_BACKWARD, false);
+    if (ok || copies || rows_fit(*p) == false) {
+      if (!scratch || scratch_bytes < tc_scratch_bytes(*p, SKV_OP_BACKWARD, ok)) return SKV_ERR_SCRATCH;
       return tc_backward(c, z, z_stride, C, g_act, gact_stride, g_delta, gdelta_stride, dz, dz_stride, dC_f32,
-                         dC_cast, scratch, scratch_bytes);
+                         dC_cast, scratch, ok);
     }
+    if (p->impl == SKV_IMPL_TCGEN05 || dz32) return SKV_ERR_ALIGN;
   }
   return simt_backward(c, z, z_stride, C, g_act, gact_stride, g_delta, gdelta_stride, dz, dz_stride, dC_f32,
                        dC_cast, scratch, scratch_bytes);

@@ -131,13 +131,14 @@ int simt_backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, 
                   void* scratch, size_t scratch_bytes);
 int simt_knot_index(const LaunchCtx& c, const void* z, int64_t zs, int32_t* bins);
 
-// tcgen05 kernel family (bf16, eligible shapes only).
+// tcgen05 kernel family (bf16, eligible shapes only).  `rows_ok`: the rows of z, act_out, g_act and dz start
+// on 16-byte boundaries and hold whole chunks of eight keys; otherwise they are copied to rows that do.
 bool tc_eligible(const skv_problem& p);
-size_t tc_scratch_bytes(const skv_problem& p, int op);
+size_t tc_scratch_bytes(const skv_problem& p, int op, bool rows_ok);
 int tc_forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* act_out, int64_t as,
-               void* delta_out, int64_t ds, void* scratch, size_t scratch_bytes);
+               void* delta_out, int64_t ds, void* scratch, bool rows_ok);
 int tc_backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const void* g_act, int64_t gas,
                 const void* g_delta, int64_t gds, void* dz, int64_t dzs, float* dC, void* dC_cast,
-                void* scratch, size_t scratch_bytes);
+                void* scratch, bool rows_ok);
 
 }  // namespace skv

@@ -99,8 +99,8 @@ Tensor forward(const Tensor& z, const Tensor& C, const skv_problem& p, bool with
   const int64_t esz = f.element_size();
   char* base = static_cast<char*>(f.data_ptr());
   void* delta = base + (with_base ? p.h * esz : 0);
-  if (slow_family(p, aligned16(z.data_ptr(), z.stride(0) * esz) && aligned16(C.data_ptr(), 0) &&
-                         aligned16(delta, width * esz)))
+  if (slow_family(p, p.h % 8 || p.r % 8 ||
+                         (aligned16(z.data_ptr(), z.stride(0) * esz) && (!with_base || aligned16(base, width * esz)))))
     return Tensor();
   const size_t need = skv_scratch_bytes(&p, SKV_OP_FORWARD);
   Tensor scratch = scratch_for(need, z);

@@ -42,12 +42,19 @@ extern "C" int skv_feature_forward_noalloc(const skv_problem* p, const void* z, 
   const int impl = skv_resolve_impl(p);
   if (impl < 0) return impl;
   const size_t need = skv_scratch_bytes(p, SKV_OP_FORWARD);
-  if (need > (size_t)SKV_NOALLOC_SCRATCH_BYTES) return SKV_ERR_NOALLOC_LIMIT;
+  skv_problem q = *p;
+  if (need > (size_t)SKV_NOALLOC_SCRATCH_BYTES) {
+    // the CUDA-core forward makes do with any scratch; it is the path of shapes whose tensor-core form needs
+    // padding or the linear spline's images
+    if (p->impl != SKV_IMPL_AUTO || (p->h % 8 == 0 && p->r % 16 == 0 && p->spline_order != 1 && p->L <= 49))
+      return SKV_ERR_NOALLOC_LIMIT;
+    q.impl = SKV_IMPL_SIMT;
+  }
   void* scratch = nullptr;
   if (int e = scratch_address(&scratch)) return e;
   // Nothing in the array has to start at zero: the forward writes the whole operand image and
   // every partial-residual row it later reads before reading them, so leftovers of the previous
   // call are never observed.
-  return skv_feature_forward(p, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch,
+  return skv_feature_forward(&q, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch,
                              (size_t)SKV_NOALLOC_SCRATCH_BYTES, status, stream);
 }

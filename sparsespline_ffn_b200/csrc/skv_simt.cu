@@ -755,10 +755,12 @@ FwdPlan plan_forward(const skv_problem& p) {
   double best = 0.0;
   for (int groups = kGroups; groups >= 1; groups >>= 1) {
     const int64_t tiles = cdiv64(N, (int64_t)kWarps * tpw * groups);
-    for (int per = slabs; per >= 1; --per) {
-      const int splits = (int)cdiv64(slabs, per);
+    int last = 0;
+    for (int s = 1; s <= slabs && s <= 64; ++s) {
+      const int per = (int)cdiv64(slabs, s), splits = (int)cdiv64(slabs, per);
       if (splits > 1 && splits * part_bytes > kFwdScratchCap) break;
-      if (per < slabs && cdiv64(slabs, per + 1) == splits) continue;
+      if (splits == last) continue;
+      last = splits;
       const double t = (double)cdiv64(tiles * splits, slots) * per * (copy + groups * work) +
                        (splits > 1 ? 4000.0 + (double)splits * part_bytes / 1500.0 : 0.0);
       if (best == 0.0 || t < best) {
@@ -823,10 +825,11 @@ DcPlan plan_dc(const skv_problem& p) {
   const int64_t N = p.N > 0 ? p.N : 1, groups = cdiv64(p.h, d.W), tiles = cdiv64(N, d.TT);
   const double elems = (double)p.h * p.L * p.r;
   double best = 0.0;
-  for (int64_t per = tiles; per >= 1; --per) {
-    const int64_t splits = cdiv64(tiles, per);
-    if (splits > 16) break;
-    if (per < tiles && cdiv64(tiles, per + 1) == splits) continue;
+  int64_t last = 0;
+  for (int64_t s = 1; s <= 16; ++s) {
+    const int64_t per = cdiv64(tiles, s), splits = cdiv64(tiles, per);
+    if (splits == last) continue;
+    last = splits;
     // clocks: a tile per warp about 7 instructions per pair and 40 per interval; partials' round trip
     const double t = (double)cdiv64(groups * splits, slots) * per * (d.TT * 14.0 * d.cv + 4000.0) +
                      (splits > 1 ? 4000.0 + splits * elems * 8 / 1500.0 : 0.0);
@@ -920,10 +923,16 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
     if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
   }
   if (dC || dC_cast) {
-    const DcPlan d = plan_dc(p);
+    DcPlan d = plan_dc(p);
     const size_t elems = (size_t)p.h * p.L * p.r;
+    const int64_t room = scratch ? (int64_t)(scratch_bytes / (elems * sizeof(float))) : 0;
+    if (d.gacc && room < 1) return SKV_ERR_SCRATCH;
+    if (d.splits > room) {                               // fewer splits where there is less room for partials
+      d.splits = room > 1 ? (int)room : 1;
+      d.tokens_per_split = cdiv64(cdiv64(p.N, d.splits), d.TT) * d.TT;
+      d.splits = (int)cdiv64(p.N, d.tokens_per_split);
+    }
     const bool parts = d.splits > 1 || d.gacc;
-    if (parts && (!scratch || scratch_bytes < (size_t)d.splits * elems * sizeof(float))) return SKV_ERR_SCRATCH;
     DcArgs a;
     a.z = z; a.zs = zs; a.g_delta = g_delta; a.gds = gds;
     a.part = parts ? static_cast<float*>(scratch) : nullptr;

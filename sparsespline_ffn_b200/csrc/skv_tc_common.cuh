@@ -257,49 +257,6 @@ __device__ __forceinline__ void pow2_scales(uint32_t amax_bits, float& scale, fl
 // Words of the 256-byte header at the start of a call's scratch: bit patterns of max|g_delta| and max|C|.
 constexpr int kAmaxG = 0, kAmaxC = 8;
 
-namespace {
-// Largest magnitude (as a float32 bit pattern, NaN skipped) of a [rows][cols] bf16 array with row stride.
-__global__ void tc_amax_kernel(const __nv_bfloat16* __restrict__ a, int64_t stride, int64_t rows, int cols,
-                               uint32_t* __restrict__ amax_bits) {
-  const int64_t total = rows * cols;
-  uint32_t m = 0;
-  if (stride == cols && (reinterpret_cast<uintptr_t>(a) & 15) == 0) {
-    // contiguous: 16-byte loads; |x| of a bf16 as a float32 bit pattern is its 15 low bits shifted up
-    const int64_t n8 = total / 8;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + i);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t lo = (w[q] << 16) & 0x7fff0000u, hi = w[q] & 0x7fff0000u;
-        if (lo <= 0x7f800000u) m = max(m, lo);          // NaN patterns lie above infinity: skipped
-        if (hi <= 0x7f800000u) m = max(m, hi);
-      }
-    }
-    for (int64_t i = n8 * 8 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const float v = fabsf(__bfloat162float(a[i]));
-      if (v == v) m = max(m, __float_as_uint(v));
-    }
-  } else {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-      const float v = fabsf(__bfloat162float(a[(i / cols) * stride + (i % cols)]));
-      if (v == v) m = max(m, __float_as_uint(v));
-    }
-  }
-  // one atomic per CTA: thousands of per-warp atomics on one word serialise in L2
-  __shared__ uint32_t wmax[32];
-  for (int s = 16; s >= 1; s >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x + 31) / 32 ? wmax[threadIdx.x] : 0u;
-    for (int s = 16; s >= 1; s >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
-    if (threadIdx.x == 0 && m) atomicMax(amax_bits, m);
-  }
-}
-}  // namespace
-
 // Two float32 -> packed f16x2 (low half = a) as a 32-bit word.
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
@@ -333,19 +290,23 @@ __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 
 // ---------------------------------------------------------------------------------------------
 // `kw` is the word distance between consecutive 16-byte chunks of a row minus 4: 508 for tiles of
 // 128 token rows (2048 bytes per chunk column), 252 for tiles of 64.
+// LIN: the linear spline's weights 1 - tau and tau.  Its last interval's second word would lie past the
+// key's segment; it is zero then (as for every even interval), and both offsets are the first word's, so a caller
+// that stores x1 before x0 writes the segment's own words only.
+template <bool LIN = false>
 __device__ __forceinline__ void phi_pair(float zz, const GridParams& g, uint32_t wq, uint32_t& x0, uint32_t& x1,
                                          uint32_t& wo0, uint32_t& wo1, uint32_t kw = 508u) {
   const Knot k = knot_of(zz, g);
   const float t = k.tau, omt = 1.0f - t;
   const float hm = k.in_range ? 0.5f : 0.0f;
-  const float B0 = (hm * omt) * omt;
-  const float B2 = (hm * t) * t;
-  const float B1 = fmaf(2.0f, hm, -B0) - B2;          // (m - B0) - B2 with m = 2 * hm, same roundings
+  const float B0 = LIN ? 2.0f * hm * omt : (hm * omt) * omt;
+  const float B2 = LIN ? 0.0f : (hm * t) * t;
+  const float B1 = LIN ? 2.0f * hm * t : fmaf(2.0f, hm, -B0) - B2;   // (m - B0) - B2 with m = 2 * hm, same roundings
   const uint32_t p01 = pack_h2(B0, B1), p2 = pack_h2(B2, 0.0f);
   const uint32_t sh = (k.tbits & 1u) << 4;
   x0 = p01 << sh;
   x1 = __funnelshift_l(p01, p2, sh);
-  const uint32_t s0 = wq + ((uint32_t)k.bin >> 1), s1 = s0 + 1u;
+  const uint32_t s0 = wq + ((uint32_t)k.bin >> 1), s1 = s0 + (LIN ? k.tbits & 1u : 1u);
   wo0 = s0 + (s0 >> 2) * kw;
   wo1 = s1 + (s1 >> 2) * kw;
 }
@@ -366,29 +327,13 @@ __device__ __forceinline__ void phi_pair_s(float zz, const GridParams& g, uint32
   s0 = wq + ((uint32_t)k.bin >> 1);
 }
 
-// Knot-dependent part of phi_pair only: the two f16x2 words and the index (bin >> 1) of the first
-// one within the key's L/2 words, returned with the bias kWordBias (the callers fold the bias into
-// the constants they compare or add it to, which saves an instruction per pair).
+// Index (bin >> 1) of a pair's first word within its key's L/2 words carries the bias kWordBias (the
+// callers fold it into the constants they compare or add it to, which saves an instruction per pair).
 constexpr uint32_t kWordBias = kKnotBias >> 1;
-__device__ __forceinline__ void phi_pair_words(float zz, const GridParams& g, uint32_t& x0, uint32_t& x1,
-                                               uint32_t& wp) {
-  const Knot k = knot_of(zz, g);
-  const float t = k.tau, omt = 1.0f - t;
-  const float hm = k.in_range ? 0.5f : 0.0f;
-  const float B0 = (hm * omt) * omt;
-  const float B2 = (hm * t) * t;
-  const float B1 = fmaf(2.0f, hm, -B0) - B2;          // (m - B0) - B2 with m = 2 * hm, same roundings
-  const uint32_t p01 = pack_h2(B0, B1), p2 = pack_h2(B2, 0.0f);
-  const uint32_t sh = (k.tbits & 1u) << 4;
-  x0 = p01 << sh;
-  x1 = __funnelshift_l(p01, p2, sh);
-  wp = k.tbits >> 1;
-}
-
-// phi_pair_words for the two keys held in one packed bf16 word (low half = first key), with the
+// The two f16x2 words and the biased word index of the two keys held in one packed bf16 word (low half = first key), with the
 // float32 arithmetic issued as two-wide instructions (add / sub / mul / fma .f32x2 of sm_100: each half
 // is the same IEEE operation with the same rounding as the scalar instruction, so every result is bit
-// for bit that of phi_pair_words).
+// for bit that of the scalar form).  LIN: the linear spline's two weights, B2 = 0.
 __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -397,6 +342,7 @@ __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
+template <bool LIN>
 __device__ __forceinline__ void phi_pair_words2(uint32_t zw, const GridParams& g, uint32_t (&x0)[2], uint32_t (&x1)[2],
                                                 uint32_t (&wp)[2]) {
   unsigned long long v, u2, t2, tau2, omt2, b0, b2, b1;
@@ -404,21 +350,28 @@ __device__ __forceinline__ void phi_pair_words2(uint32_t zw, const GridParams& g
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(u2) : "l"(v), "l"(f2_pack(g.scale, g.scale)), "l"(0ull));
   float ua, ub;
   f2_unpack(u2, ua, ub);
-  const float hma = __float_as_uint(ua) <= __float_as_uint(g.Gf) ? 0.5f : 0.0f;
-  const float hmb = __float_as_uint(ub) <= __float_as_uint(g.Gf) ? 0.5f : 0.0f;
+  constexpr float kIn = LIN ? 1.0f : 0.5f;
+  const float hma = __float_as_uint(ua) <= __float_as_uint(g.Gf) ? kIn : 0.0f;
+  const float hmb = __float_as_uint(ub) <= __float_as_uint(g.Gf) ? kIn : 0.0f;
   const unsigned long long uc2 = f2_pack(fminf(fmaxf(ua, 0.0f), g.Gm1f), fminf(fmaxf(ub, 0.0f), g.Gm1f));
   const unsigned long long big2 = f2_pack(8388608.0f, 8388608.0f), hm2 = f2_pack(hma, hmb);
   asm("add.rm.f32x2 %0, %1, %2;" : "=l"(t2) : "l"(uc2), "l"(big2));
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(t2), "l"(big2));
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(tau2) : "l"(uc2), "l"(v));
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(omt2) : "l"(f2_pack(1.0f, 1.0f)), "l"(tau2));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(hm2), "l"(omt2));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b0) : "l"(v), "l"(omt2));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(hm2), "l"(tau2));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b2) : "l"(v), "l"(tau2));
-  asm("add.rn.f32x2 %0, %1, %1;" : "=l"(v) : "l"(hm2));                                    // 2 * hm, exact
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(b0), "l"(f2_pack(-1.0f, -1.0f)), "l"(v));  // 2 hm - B0, one rounding
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(b1) : "l"(v), "l"(b2));
+  if constexpr (LIN) {
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b0) : "l"(hm2), "l"(omt2));                       // hm is the mask itself
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b1) : "l"(hm2), "l"(tau2));
+    b2 = 0ull;
+  } else {
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(hm2), "l"(omt2));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b0) : "l"(v), "l"(omt2));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(hm2), "l"(tau2));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(b2) : "l"(v), "l"(tau2));
+    asm("add.rn.f32x2 %0, %1, %1;" : "=l"(v) : "l"(hm2));                                    // 2 * hm, exact
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(b0), "l"(f2_pack(-1.0f, -1.0f)), "l"(v));  // 2 hm - B0, one rounding
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(b1) : "l"(v), "l"(b2));
+  }
   float ta, tb, B0a, B0b, B1a, B1b, B2a, B2b;
   f2_unpack(t2, ta, tb);
   f2_unpack(b0, B0a, B0b);

@@ -1,0 +1,10 @@
+// Forward kernels of the quadratic spline, ReLU^2 base path.
+#include "skv_tc_fwd_kernel.cuh"
+
+namespace skv {
+namespace tc {
+cudaError_t fwd_launch_quad_relu(int groups, int words, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
+  return fwd_launch<SKV_ACT_RELU_SQ, false>(groups, words, P, grid, smem, stream);
+}
+}  // namespace tc
+}  // namespace skv

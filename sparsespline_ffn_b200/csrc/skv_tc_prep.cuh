@@ -1,0 +1,73 @@
+// Operand images of one call and the sums of its partial results, as the tensor-core kernels share them.
+#pragma once
+
+#include "skv_launch.cuh"
+#include "skv_tc_common.cuh"
+
+namespace skv {
+namespace tc {
+
+constexpr int kChunkKeys = 8;
+constexpr int kPlanSMs = 148;                 // B200; only used to balance launch shapes
+constexpr size_t kSmemLimit = 227 * 1024;
+// The contraction kernels run one CTA per SM.  A kernel started while its predecessor still occupies the chip
+// is placed unevenly, and a second CTA on an SM would only wait there for the first one's tensor memory while
+// other SMs idle (2495 x 2048, L = 42: 221 us per step instead of 184), so each asks for more than half of the
+// shared memory.
+constexpr size_t kSmemOnePerSM = 116 * 1024;
+
+// Header at the start of a call's scratch: the final maxima (kAmaxG, kAmaxC), then the maxima of the blocks
+// that scanned C and g_delta.
+constexpr size_t kHeaderBytes = 4096;
+constexpr int kBlockMax = 64;                 // first word of the block maxima
+constexpr int kMaxBlocks = 296;               // scanning blocks per array
+
+// The kernels work on whole chunks of keys and whole K = 16 steps of code channels; the images (and, when the
+// rows of z cannot be read in 16-byte pieces, padded copies of the token-major arrays) carry the padding.
+inline int padded_h(const skv_problem& p) { return (p.h + kChunkKeys - 1) / kChunkKeys * kChunkKeys; }
+inline int padded_r(const skv_problem& p) { return (p.r + 15) / 16 * 16; }
+
+inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// One [N][h] bf16 array copied to [N][hp] (pad columns zero); with act_out also phi of it at that pointer.
+struct CopyJob {
+  const __nv_bfloat16* src;
+  int64_t ss;
+  __nv_bfloat16* dst;        // null: no job
+  __nv_bfloat16* act_out;
+  int64_t as;
+};
+
+struct PrepParams {
+  const __nv_bfloat16* C;
+  int h, hp, L, r, rp;
+  int lpc;                   // rows per key of the code-table image, 0: none wanted
+  __half* cimg;
+  int lpt;                   // rows per key of the transformed-table image, 0: none wanted
+  __half* timg;
+  const __nv_bfloat16* g;    // null: no gradient image
+  int64_t gds, N, tiles;     // tiles of 128 tokens in the image
+  __half* gimg;
+  CopyJob copy[2];
+  int act;
+  uint32_t* hdr;
+  int scan_c, scan_g;        // blocks that scan each array
+  int blocks_c, blocks_t, blocks_g, blocks_copy;
+};
+
+// Maxima, then images and copies: two launches.
+int launch_prep(PrepParams& P, cudaStream_t stream);
+
+// out[n][c] = lambda * 2^-k * sum over splits of partial[split][n][c], c < r of the rp partial columns.
+int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,
+                    void* out, int64_t ds, bool out_f32, cudaStream_t stream);
+
+// dC = lambda * 2^-k * sum over splits of part[split][row][c] for `rows` knot rows.
+int launch_dc_reduce(const float* part, int splits, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
+                     const uint32_t* hdr, float* dC, void* dC_cast, cudaStream_t stream);
+
+// dst[n][j] = src[n][j], j < h, from padded rows.
+int launch_unpad(const void* src, int64_t ss, void* dst, int64_t ds, int64_t N, int h, bool f32, cudaStream_t stream);
+
+}  // namespace tc
+}  // namespace skv

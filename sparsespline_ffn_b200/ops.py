@@ -72,11 +72,11 @@ _warned_slow: set[tuple] = set()
 
 def _warn_if_slow_family(lib, p: _lib.Problem, z: torch.Tensor, aligned_fn) -> None:
     """One warning per shape when a large bf16 problem is about to run on the CUDA-core kernels
-    (r not a multiple of 16, h not a multiple of 8, a pointer or stride that is not 16-byte
-    aligned, ...): they are a correctness fallback, tens of times slower than the tcgen05 kernels."""
+    (r above 128, more than 64 knot rows, or rows of a fitting shape at an odd address or stride): they are
+    several times slower than the tcgen05 kernels."""
     if z.dtype != torch.bfloat16 or p.impl != _lib.SKV_IMPL["auto"] or p.N * p.h < (1 << 24):
         return
-    aligned = bool(aligned_fn())
+    aligned = bool(p.h % 8 or p.r % 8 or aligned_fn())      # shapes that do not fit are padded by the library
     if aligned and lib.skv_resolve_impl(ctypes.byref(p)) == _lib.SKV_IMPL["tcgen05"]:
         return
     key = (p.h, p.L, p.r, aligned)
@@ -85,10 +85,9 @@ def _warn_if_slow_family(lib, p: _lib.Problem, z: torch.Tensor, aligned_fn) -> N
     _warned_slow.add(key)
     import warnings
     why = ("a tensor whose base address or row stride is not 16-byte aligned" if not aligned else
-           f"a shape outside the tcgen05 kernels' range (h={p.h}, L={p.L}, r={p.r}: need r % 16 == 0, r <= 128, "
-           "h % 8 == 0, L <= 64)")
+           f"a shape outside the tcgen05 kernels' range (h={p.h}, L={p.L}, r={p.r}: need r <= 128, L <= 64)")
     warnings.warn(f"splinekv_b200: {p.N} x {p.h} bf16 problem runs on the CUDA-core fallback kernels because of "
-                  f"{why}; expect it to be tens of times slower", RuntimeWarning, stacklevel=3)
+                  f"{why}; expect it to be several times slower", RuntimeWarning, stacklevel=3)
 
 
 def _aligned16(*tensors) -> bool:
@@ -159,8 +158,8 @@ def feature_forward(z, C, grid_lo, grid_hi, G, activation="relu_sq", lambda_scal
             delta_ptr = ctypes.c_void_p(f.data_ptr() + (h * f.element_size() if with_base else 0))
             act_stride = delta_stride = f.stride(0)
             result = f
-        _warn_if_slow_family(lib, p, z, lambda: _aligned16(z, C) and (delta_ptr.value or 0) % 16 == 0
-                             and (delta_stride * (4 if delta_f32 else z.element_size())) % 16 == 0)
+        _warn_if_slow_family(lib, p, z, lambda: _aligned16(z) and (act_ptr is None or (act_ptr.value or 0) % 16 == 0)
+                             and (act_stride * z.element_size()) % 16 == 0)
         scratch, nbytes = _scratch(lib, p, _lib.SKV_OP_FORWARD, z.device)
         code = lib.skv_feature_forward(
             ctypes.byref(p), _ptr(z), z.stride(0), _ptr(C), act_ptr, act_stride, delta_ptr, delta_stride,
@@ -253,9 +252,7 @@ def feature_backward(z, C, grad_out, grid_lo, grid_hi, G, activation="relu_sq", 
         dC_cast = None
         if need_dC and cast_dC and z.dtype != torch.float32:
             dC_cast = torch.empty((h, L, r), dtype=z.dtype, device=z.device)
-        _warn_if_slow_family(lib, p, z, lambda: _aligned16(z, C) and (gdelta_ptr.value or 0) % 16 == 0
-                             and (gact_ptr is None or (gact_ptr.value or 0) % 16 == 0)
-                             and (gdelta_stride * z.element_size()) % 16 == 0
+        _warn_if_slow_family(lib, p, z, lambda: _aligned16(z) and (gact_ptr is None or (gact_ptr.value or 0) % 16 == 0)
                              and (gact_stride * z.element_size()) % 16 == 0)
         scratch, nbytes = _scratch(lib, p, _lib.SKV_OP_BACKWARD, z.device)
         code = lib.skv_feature_backward(
