@@ -37,23 +37,29 @@ Split best_split(int64_t tiles, int64_t units, int64_t most, double unit, double
 bool make_dz_plan(const skv_problem& p, DzPlan* o) {
   const int lb = (p.L - 1 + 7) / 8, rp = padded_r(p);    // 8-column blocks per key; columns L-1.. are padding
   if (lb < 1 || lb > 8) return false;
-  const int ncols = kChunkKeys * 8 * lb;
-  const int groups = 2 * ncols <= 512 ? 2 : 1;
-  o->groups = groups;
   o->lb = lb;
-  int tstages = kTStages;
-  auto smem_for = [&](int ts) { return (size_t)groups * 128 * rp * 2 + (size_t)ts * kChunkKeys * 8 * lb * rp * 2 + 256; };
-  while (tstages > 2 && smem_for(tstages) > kSmemLimit) --tstages;
-  o->tstages = tstages;
-  o->smem = smem_for(tstages);
-  if (o->smem > kSmemLimit) return false;
+  // two token groups where their rows, g and the table ring fit shared memory
+  bool fits = false;
+  for (int groups = 2; groups >= 1 && !fits; --groups)
+    for (int rs = kRowStages; rs >= 2 && !fits; --rs)
+      for (int ts = kTStages; ts >= 2 && !fits; --ts) {
+        o->groups = groups;
+        o->rstages = rs;
+        o->tstages = ts;
+        o->smem = 1024 + (size_t)groups * rs * 2 * kBoxBytes + (size_t)groups * 128 * rp * 2 +
+                  (size_t)ts * kChunkKeys * 8 * lb * rp * 2 + 512;
+        fits = o->smem <= kSmemLimit;
+      }
+  if (!fits) return false;
+  const int groups = o->groups;
   if (o->smem < kSmemOnePerSM) o->smem = kSmemOnePerSM;
   const int chunks = padded_h(p) / kChunkKeys;
   const int64_t tiles = ((p.N > 0 ? p.N : 1) + 128 * groups - 1) / (128 * groups);
   // 1.0 us per chunk of two groups at L = 22, r = 32; the MMAs grow with r
   const double chunk = 0.5 * groups * lb / 3.0 * (0.8 + rp / 160.0);
-  const Split s = best_split(tiles, chunks, (chunks + 3) / 4, chunk, 4.5, 0.0);
-  o->chunks_per_split = s.per;
+  const int boxes = (chunks + kBoxChunks - 1) / kBoxChunks;                  // a split is a whole number of boxes
+  const Split s = best_split(tiles, boxes, boxes, chunk * kBoxChunks, 4.5, 0.0);
+  o->chunks_per_split = s.per * kBoxChunks;
   o->splits = s.splits;
   return true;
 }
@@ -211,6 +217,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Z.chunks_total = hp / kChunkKeys;
   Z.chunks_per_split = b.dz.chunks_per_split;
   Z.tstages = b.dz.tstages;
+  Z.rstages = b.dz.rstages;
   Z.dz_f32 = p.dz_f32;
   Z.wait_cycles = wait_cycle_limit();
   Z.status = c.status;

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) tc_bwd_fused_kernel(const BfPar
     reg_dec<kRegsAux>();
     if (warp == kAux0) {
       // ---------------------------------------------------------------- S MMAs (both groups)
-      if (lane == 0 && (P.roles & 1)) {
+      if ((P.roles & 1) && elect_one()) {
         mbar_wait(tfull, 0, wc);
         const uint32_t rb = (uint32_t)(r / 8) * 128u;
         const uint32_t a_hi = desc_hi(128u), b_hi = desc_hi(rb);
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) tc_bwd_fused_kernel(const BfPar
       }
     } else if (warp == kAux0 + 1) {
       // ---------------------------------------------------------------- dC MMAs (both groups)
-      if (lane == 0 && (P.roles & 2)) {
+      if ((P.roles & 2) && elect_one()) {
         const uint32_t idesc = instr_desc(0, 0, 1, 1, 128, r);
         const uint32_t a_hi = desc_hi(1024u), b_hi = desc_hi(2048u);
         int it[2] = {0, 0};
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) tc_bwd_fused_kernel(const BfPar
       }
     } else if (warp == kAux0 + 2) {
       // ---------------------------------------------------------------- loader
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_arrive_expect_tx(tfull, 2 * t_bytes);
         bulk_g2s(t_base, reinterpret_cast<const uint8_t*>(P.timg) + (size_t)(key0 / kChunkKeys) * t_bytes,
                  2 * t_bytes, tfull);

@@ -30,6 +30,20 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in one lane of the (converged) warp, always the same one.  The compiler knows that a branch on it holds a
+// single thread; behind `lane == 0` it cannot tell, and wraps every tcgen05 and TMA instruction, whose
+// operands live in registers of the whole warp, in a loop over the lanes that might be active.  Issuing two MMAs and a
+// commit took the dz kernel's thread 300 to 400 cycles that way.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256 + 64, 1) tc_dc_kernel(const DcParams P) {
     tc_fence_before();
   } else if (warp == 8) {
     // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc(0, 0, 1, 1, 128, r);
       const uint32_t ab_hi = desc_hi(2048u);
       int guse[2] = {0, 0}, puse[2] = {0, 0};
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256 + 64, 1) tc_dc_kernel(const DcParams P) {
     }
   } else {
     // ------------------------------------------------------------------ gradient-tile loader
-    if (lane == 0) {
+    if (elect_one()) {
       int guse[2] = {0, 0};
       for (int ti = 0; ti < ntiles; ++ti) {
         const int pg = ti & 1;

@@ -12,6 +12,7 @@
 #pragma once
 
 #include "skv_tc_prep.cuh"
+#include "skv_tma.cuh"
 
 namespace skv {
 namespace tc {
@@ -33,6 +34,7 @@ struct DzParams {
   float coef;                // lambda * scale
   int chunks_total, chunks_per_split;
   int tstages;               // depth of the transformed-table ring (2..kTStages)
+  int rstages;               // boxes of z and g_act per token group (2 or 3)
   int dz_f32;                // dz is float32 [N][dzs] instead of bf16
   int32_t* status;
   long long wait_cycles;     // limit of every bounded wait, in clock cycles
@@ -124,30 +126,60 @@ __device__ __forceinline__ float dz_key_sum(const uint32_t (&r)[LB][8], float uc
 }
 
 constexpr int kTStages = 4;
+constexpr int kRowStages = 3;                 // boxes of z (and g_act) per token group, two where wide r needs the room
+constexpr int kBoxChunks = kBoxKeys / kChunkKeys;
 
+// Keys of one S block: S columns of a token group are computed and consumed in blocks of 4 keys (2 from 33 knot
+// columns on), two blocks in tensor memory per group.
+__host__ __device__ constexpr int dz_block_keys(int lb) { return lb <= 4 ? 4 : 2; }
+
+// Launch shape: grid = (token tiles of 128*GROUPS tokens, key splits).  Per token group
+//   eight consumer warps, two threads per token, one for each S buffer: z and g_act from their boxes, S from
+//                        tensor memory, dz into the place of z
+//   one warp (lane 0)    issues the group's S MMAs, a block ahead of the consumers
+//   one warp (lane 0)    moves the group's boxes: loads of z and g_act, stores of dz
+// and one loader warp for the transformed table.
+//
+// Bound: instruction issue of the consumers (64 instructions per 32 pairs, 42 of them the saturating adds and the
+// packed FMAs).  What it took to get near it, at the d20 shape: MMAs issued by an elected thread (300-400 cycles
+// per pair of MMAs before, 150 now), which is what makes smaller S blocks affordable; two blocks per group, so that
+// one is computed while the other is read (with one block of 8 keys a group waited 670 cycles per chunk); a
+// block given back as soon as its last key is in registers; the boxes' copies on a warp of their own (a consumer
+// warp that also moved them held its group up by 680 cycles per box).
+//
 // RELU: the base path is ReLU^2 (compile-time, so that the code of the other activations stays
 // out of the hot loop); otherwise P.act (identity or gelu) is evaluated at run time.
 // LIN: the derivative of the linear spline is C[bin+1] - C[bin]; with the same table its column weights
 // are the steps 1[bin >= m + 1] = sat(bin - m), so the only change is bin in the place of u_c.
 template <int GROUPS, int LB, int NC, bool RELU, bool LIN>
-__global__ void __launch_bounds__(128 * GROUPS + 64, 1) tc_dz_kernel(const DzParams P) {
-  extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __launch_bounds__(320 * GROUPS + 32, 1)
+    tc_dz_kernel(const DzParams P, const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_ga,
+                 const __grid_constant__ CUtensorMap map_dz) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* row_base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // [group][rstages][z, g_act]
+  const int RS = P.rstages;
+  uint8_t* smem = row_base + (size_t)GROUPS * RS * 2 * kBoxBytes;
   const int r = P.r;
   constexpr int LP = 8 * LB;                                         // padded knot columns per key
+  constexpr int KB = dz_block_keys(LB);
+  constexpr int NBLK = kChunkKeys / KB;                              // blocks per chunk
+  constexpr bool DB = LB <= 4;                                       // two keys' columns in registers
   const uint32_t g_bytes = (uint32_t)(128 * r * 2);
   const uint32_t t_bytes = (uint32_t)(kChunkKeys * LP * r * 2);
-  constexpr uint32_t ncols = (uint32_t)(kChunkKeys * LP);            // S columns per group
+  constexpr uint32_t bcols = (uint32_t)(KB * LP);                    // columns of one S block
   uint8_t* g_base = smem;                                             // [group][g_bytes]
   uint8_t* t_base = smem + (size_t)GROUPS * g_bytes;                  // [kTStages][t_bytes]
   const int TS = P.tstages;
   uint64_t* bars = reinterpret_cast<uint64_t*>(t_base + (size_t)TS * t_bytes);
-  uint64_t* gfull = bars;                    // [1]
-  uint64_t* tfull = gfull + 1;               // [kTStages]
-  uint64_t* tempty = tfull + kTStages;       // [kTStages]
-  uint64_t* sfull = tempty + kTStages;       // [GROUPS]  MMA -> consumers
-  uint64_t* sempty = sfull + GROUPS;         // [GROUPS]  consumers -> MMA
-  uint64_t* done = sempty + GROUPS;          // [1]       all MMAs of this CTA complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* gfull = bars;                       // [1]
+  uint64_t* tfull = gfull + 1;                  // [kTStages]
+  uint64_t* tempty = tfull + kTStages;          // [kTStages]           one arrival per group
+  uint64_t* sfull = tempty + kTStages;          // [GROUPS][2]          MMA -> consumers
+  uint64_t* sempty = sfull + 2 * GROUPS;        // [GROUPS][2]          consumers -> MMA
+  uint64_t* done = sempty + 2 * GROUPS;         // [GROUPS]             all MMAs of the group complete
+  uint64_t* zfull = done + GROUPS;              // [GROUPS][kRowStages] box landed
+  uint64_t* zdone = zfull + GROUPS * kRowStages;  // [GROUPS][kRowStages] box consumed, dz in place
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(zdone + GROUPS * kRowStages);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wc{abort_flag, P.status, kStatusTimeoutDz, P.wait_cycles};
 
@@ -156,17 +188,18 @@ __global__ void __launch_bounds__(128 * GROUPS + 64, 1) tc_dz_kernel(const DzPar
   const int nch = min(P.chunks_per_split, P.chunks_total - chunk_begin);
   const int64_t tile_base = (int64_t)blockIdx.x * (128 * GROUPS);
   uint32_t tmem_cols = 32;
-  while (tmem_cols < GROUPS * ncols) tmem_cols <<= 1;
+  while (tmem_cols < GROUPS * 2 * bcols) tmem_cols <<= 1;
 
   if (tid == 0) {
     mbar_init(gfull, 1);
-    for (int i = 0; i < kTStages; ++i) { mbar_init(tfull + i, 1); mbar_init(tempty + i, 1); }
-    for (int i = 0; i < GROUPS; ++i) { mbar_init(sfull + i, 1); mbar_init(sempty + i, 4); }
-    mbar_init(done, 1);
+    for (int i = 0; i < kTStages; ++i) { mbar_init(tfull + i, 1); mbar_init(tempty + i, GROUPS); }
+    for (int i = 0; i < 2 * GROUPS; ++i) { mbar_init(sfull + i, 1); mbar_init(sempty + i, 4); }
+    for (int i = 0; i < GROUPS; ++i) mbar_init(done + i, 1);
+    for (int i = 0; i < GROUPS * kRowStages; ++i) { mbar_init(zfull + i, 1); mbar_init(zdone + i, 8); }
     *abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 4 * GROUPS) tmem_alloc(tmem_slot, tmem_cols);
+  if (warp == 8 * GROUPS) tmem_alloc(tmem_slot, tmem_cols);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -175,117 +208,165 @@ __global__ void __launch_bounds__(128 * GROUPS + 64, 1) tc_dz_kernel(const DzPar
   pdl_launch();
   pdl_wait();
 
-  if (warp < 4 * GROUPS) {
-    // ------------------------------------------------------------------ one thread per token
-    const int grp = warp >> 2;
+  if (warp < 8 * GROUPS) {
+    // ------------------------------------------------------------------ two threads per token, one per S buffer
+    const int grp = warp >> 3, half = (warp >> 2) & 1;
     const int t = tid & 127;
     const int64_t n = tile_base + grp * 128 + t;
-    const bool valid = n < P.N;
-    const int64_t nn = valid ? n : 0;
-    const __nv_bfloat16* zrow = P.z + nn * P.zs + (int64_t)chunk_begin * kChunkKeys;
-    const __nv_bfloat16* garow = P.g_act ? P.g_act + nn * P.gas + (int64_t)chunk_begin * kChunkKeys : nullptr;
-    __nv_bfloat16* dzrow = P.dz + nn * P.dzs + (int64_t)chunk_begin * kChunkKeys;
+    const bool has_ga = P.g_act != nullptr;
     float gscale, ginv;
     pow2_scales(*P.amax_bits, gscale, ginv);
     float cscale, cinv;
     pow2_scales(P.amax_bits[kAmaxC], cscale, cinv);
     const float coef = P.coef * ginv * cinv;
     const int act = P.act;
-    const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)grp * ncols;
-    uint4 znext = valid && nch > 0 ? ld16(zrow) : make_uint4(0, 0, 0, 0);
-    uint4 ganext = valid && nch > 0 && garow ? ld16(garow) : make_uint4(0, 0, 0, 0);
+    const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(grp * 2 + half) * bcols;
+    uint64_t* sf = sfull + 2 * grp + half;
+    uint64_t* se = sempty + 2 * grp + half;
+    const uint32_t boxes = smem_u32(row_base + (size_t)grp * RS * 2 * kBoxBytes);
+    int st = 0;
+    uint32_t zpar = 0u;                                // stage and phase of the current box
 
     for (int ci = 0; ci < nch; ++ci) {
-      const uint4 zc = znext, gac = ganext;
-      if (ci + 1 < nch && valid) {
-        znext = ld16(zrow + (ci + 1) * kChunkKeys);
-        if (garow) ganext = ld16(garow + (ci + 1) * kChunkKeys);
+      if (ci % kBoxChunks == 0) mbar_wait(zfull + grp * kRowStages + st, zpar, wc);
+      const uint32_t zaddr = boxes + (uint32_t)st * 2u * kBoxBytes + box_piece((uint32_t)t, (uint32_t)(ci % kBoxChunks)) +
+                             (uint32_t)half * (KB == 4 ? 8u : 4u);
+      // this thread's four keys of the chunk: two packed words of z and of g_act
+      uint32_t zw[2], gw[2] = {0u, 0u};
+      if constexpr (KB == 4) {
+        lds64(zaddr, zw);
+        if (has_ga) lds64(zaddr + kBoxBytes, gw);
+      } else {
+        zw[0] = lds32(zaddr);
+        zw[1] = lds32(zaddr + 8u);
+        if (has_ga) { gw[0] = lds32(zaddr + kBoxBytes); gw[1] = lds32(zaddr + kBoxBytes + 8u); }
       }
-      const uint32_t zw[4] = {zc.x, zc.y, zc.z, zc.w};
-      const uint32_t gw[4] = {gac.x, gac.y, gac.z, gac.w};
-      uint32_t bufa[LB][8], bufb[LB][8];
-      float outv[kChunkKeys];
-      mbar_wait(sfull + grp, (uint32_t)ci & 1u, wc);
-      tc_fence_after();
-      tmem_ld_key<LB, NC>(trow, bufa);
+      float outv[4];
+      uint32_t buf[DB ? 2 : 1][LB][8];
 #pragma unroll
-      for (int q = 0; q < kChunkKeys; ++q) {
-        // the loads of key q are in flight; wait, start the loads of key q+1, then do key q's math
-        if (q & 1) tmem_wait_key<LB, NC>(bufb); else tmem_wait_key<LB, NC>(bufa);
-        if (q + 1 < kChunkKeys) {
-          if (q & 1) tmem_ld_key<LB, NC>(trow + (uint32_t)((q + 1) * LP), bufa);
-          else tmem_ld_key<LB, NC>(trow + (uint32_t)((q + 1) * LP), bufb);
+      for (int i = 0; i < 4; ++i) {
+        constexpr int kAlt = DB ? 1 : 0;
+        if (i % KB == 0) {                             // first key of a block
+          mbar_wait(sf, (uint32_t)(ci * (4 / KB) + i / KB) & 1u, wc);
+          tc_fence_after();
+          tmem_ld_key<LB, NC>(trow, buf[(i & kAlt)]);
+        } else if (!DB) {
+          tmem_ld_key<LB, NC>(trow + (uint32_t)((i % KB) * LP), buf[0]);
         }
-        const float zz = (q & 1) ? bf_hi(zw[q >> 1]) : bf_lo(zw[q >> 1]);
+        tmem_wait_key<LB, NC>(buf[i & kAlt]);
+        if (i % KB == KB - 1) {                        // the last key of the block is in registers: hand it back
+          tc_fence_before();
+          mbar_arrive_warp(se);
+        } else if (DB) {
+          tmem_ld_key<LB, NC>(trow + (uint32_t)((i % KB + 1) * LP), buf[(i + 1) & kAlt]);
+        }
+        const float zz = (i & 1) ? bf_hi(zw[i >> 1]) : bf_lo(zw[i >> 1]);
         // same u and the same single-comparison range test as knot_of
         const float u = __fmaf_rn(__fsub_rn(zz, P.g.lo), P.g.scale, 0.0f);
         const bool active = __float_as_uint(u) <= __float_as_uint(P.g.Gm1f);
         float uc = fminf(fmaxf(u, 0.0f), P.g.Gm1f);
         if constexpr (LIN) uc = __fsub_rn(__fadd_rd(uc, 8388608.0f), 8388608.0f);
-        const float acc = (q & 1) ? dz_key_sum<LB, NC>(bufb, uc) : dz_key_sum<LB, NC>(bufa, uc);
+        const float acc = dz_key_sum<LB, NC>(buf[i & kAlt], uc);
         float o = active ? coef * acc : 0.0f;
-        if (garow) {
-          const float ga = (q & 1) ? bf_hi(gw[q >> 1]) : bf_lo(gw[q >> 1]);
+        if (has_ga) {
+          const float ga = (i & 1) ? bf_hi(gw[i >> 1]) : bf_lo(gw[i >> 1]);
           const float dphi = RELU ? 2.0f * fmaxf(zz, 0.0f) : act_grad(zz, act);
           o = fmaf(ga, dphi, o);
         }
-        outv[q] = o;
+        outv[i] = o;
       }
-      // (Handing the S columns back two keys earlier, with the loads running two keys ahead in a third
-      // register buffer, was measured slower: 1.14 ms against 1.11 ms at the d20 shape.)
-      tc_fence_before();
-      mbar_arrive_warp(sempty + grp);
-      if (valid) {
-        if (P.dz_f32) {
-          float* o = reinterpret_cast<float*>(P.dz) + nn * P.dzs + (int64_t)(chunk_begin + ci) * kChunkKeys;
-          *reinterpret_cast<float4*>(o) = make_float4(outv[0], outv[1], outv[2], outv[3]);
-          *reinterpret_cast<float4*>(o + 4) = make_float4(outv[4], outv[5], outv[6], outv[7]);
-        } else {
-          *reinterpret_cast<uint4*>(dzrow + ci * kChunkKeys) =
-              make_uint4(pack_bf2(outv[0], outv[1]), pack_bf2(outv[2], outv[3]), pack_bf2(outv[4], outv[5]),
-                         pack_bf2(outv[6], outv[7]));
+      if (P.dz_f32) {
+        if (n < P.N) {
+          float* o = reinterpret_cast<float*>(P.dz) + n * P.dzs + (int64_t)(chunk_begin + ci) * kChunkKeys + half * KB;
+          *reinterpret_cast<float2*>(o) = make_float2(outv[0], outv[1]);
+          *reinterpret_cast<float2*>(o + (KB == 4 ? 2 : 4)) = make_float2(outv[2], outv[3]);
         }
+      } else {
+        // dz takes the place of the z words this thread has read
+        const uint32_t w0 = pack_bf2(outv[0], outv[1]), w1 = pack_bf2(outv[2], outv[3]);
+        if constexpr (KB == 4) sts64(zaddr, w0, w1);
+        else { sts32(zaddr, w0); sts32(zaddr + 8u, w1); }
+      }
+      if (ci % kBoxChunks == kBoxChunks - 1 || ci + 1 == nch) {
+        fence_async_smem();
+        mbar_arrive_warp(zdone + grp * kRowStages + st);
+        if (++st == RS) { st = 0; zpar ^= 1u; }
       }
     }
-  } else if (warp == 4 * GROUPS) {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+  } else if (warp < 9 * GROUPS) {
+    // ------------------------------------------------------------------ MMA issue, one warp per token group
+    if (elect_one()) {
+      const int grp = warp - 8 * GROUPS;
       mbar_wait(gfull, 0, wc);
       const uint32_t rb = (uint32_t)(r / 8) * 128u;          // bytes between 8-row groups of the T image
       const uint32_t a_hi = desc_hi(128u), b_hi = desc_hi(rb);
-      // The groups are served in a fixed order.  (Serving whichever group has released its S columns
-      // first, by polling both, was measured slower: 1.32 ms against 1.21 ms at the d20 shape.)
-      for (int ci = 0; ci < nch; ++ci) {
-        const int s = ci % TS;
-        bool drain = mbar_wait(tfull + s, (uint32_t)(ci / TS) & 1u, wc);
-        const uint32_t b_addr = smem_u32(t_base + (size_t)s * t_bytes);
-        for (int grp = 0; grp < GROUPS && !drain; ++grp) {
-          if (ci > 0) drain = mbar_wait(sempty + grp, (uint32_t)(ci - 1) & 1u, wc);
-          if (drain) break;                          // draining: issue nothing more
+      constexpr uint32_t idesc = instr_desc(0, 0, 0, 0, 128, (int)bcols);
+      const uint32_t a_lo0 = desc_lo(smem_u32(g_base + (size_t)grp * g_bytes), 2048u);
+      const uint32_t d0 = tmem_base + (uint32_t)grp * 2u * bcols;
+      const int ksteps = r / 16;
+      uint64_t* sf = sfull + 2 * grp;
+      uint64_t* se = sempty + 2 * grp;
+      bool drain = false;
+      int ts = 0;
+      uint32_t tpar = 0u;
+      for (int ci = 0; ci < nch && !drain; ++ci) {
+        drain = mbar_wait(tfull + ts, tpar, wc);
+        uint32_t b_blk = desc_lo(smem_u32(t_base + (size_t)ts * t_bytes), 128u);
+#pragma unroll
+        for (int b = 0; b < NBLK; ++b) {
+          const uint32_t use = (uint32_t)(ci * NBLK + b) >> 1;
+          if (use > 0) drain = drain || mbar_wait(se + (b & 1), (use - 1u) & 1u, wc);
+          if (drain) break;                            // draining: issue nothing more
           tc_fence_after();
-          const uint32_t a_lo0 = desc_lo(smem_u32(g_base + (size_t)grp * g_bytes), 2048u);
-          for (uint32_t c0 = 0; c0 < ncols; c0 += 256) {
-            const uint32_t npiece = min(256u, ncols - c0);
-            const uint32_t idesc = instr_desc(0, 0, 0, 0, 128, (int)npiece);
-            uint32_t a_lo = a_lo0;
-            uint32_t b_lo = desc_lo(b_addr + (c0 / 8) * rb, 128u);
-            const uint32_t d_addr = tmem_base + (uint32_t)grp * ncols + c0;
-            for (int ks = 0; ks < r / 16; ++ks) {
-              umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, ks > 0 ? 1u : 0u);
-              a_lo += 4096u >> 4;
-              b_lo += 256u >> 4;
-            }
+          uint32_t a_lo = a_lo0, b_lo = b_blk;
+          const uint32_t d_addr = d0 + (uint32_t)(b & 1) * bcols;
+          for (int ks = 0; ks < ksteps; ++ks) {
+            umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, ks > 0 ? 1u : 0u);
+            a_lo += 4096u >> 4;
+            b_lo += 256u >> 4;
           }
-          umma_commit(sfull + grp);
+          umma_commit(sf + (b & 1));
+          b_blk += ((bcols / 8u) * rb) >> 4;
         }
-        if (drain) break;
-        umma_commit(tempty + s);
+        if (!drain) umma_commit(tempty + ts);
+        if (++ts == TS) { ts = 0; tpar ^= 1u; }
       }
-      umma_commit(done);
+      umma_commit(done + grp);
+    }
+  } else if (warp < 10 * GROUPS) {
+    // ------------------------------------------------------------------ boxes of z, g_act and dz, one warp per group
+    if (elect_one()) {
+      const int grp = warp - 9 * GROUPS;
+      const int row0 = (int)(tile_base + grp * 128);
+      const bool has_ga = P.g_act != nullptr, store = !P.dz_f32 && row0 < P.N;
+      const int steps = (nch + kBoxChunks - 1) / kBoxChunks, key_begin = chunk_begin * kChunkKeys;
+      auto load = [&](int step, int st) {
+        uint8_t* box = row_base + (size_t)(grp * RS + st) * 2 * kBoxBytes;
+        uint64_t* bar = zfull + grp * kRowStages + st;
+        mbar_arrive_expect_tx(bar, has_ga ? 2 * kBoxBytes : kBoxBytes);
+        tma_load_2d(box, &map_z, key_begin + step * kBoxKeys, row0, bar);
+        if (has_ga) tma_load_2d(box + kBoxBytes, &map_ga, key_begin + step * kBoxKeys, row0, bar);
+      };
+      for (int i = 0; i < RS && i < steps; ++i) load(i, i);
+      int st = 0;
+      uint32_t par = 0u;
+      for (int step = 0; step < steps; ++step) {
+        if (mbar_wait(zdone + grp * kRowStages + st, par, wc)) break;
+        if (store)
+          tma_store_2d(&map_dz, row_base + (size_t)(grp * RS + st) * 2 * kBoxBytes, key_begin + step * kBoxKeys, row0);
+        bulk_commit();
+        bulk_wait_read<0>();                           // before the stage is loaded again, and before the CTA ends
+        if (step + RS < steps) load(step + RS, st);
+        if (++st == RS) { st = 0; par ^= 1u; }
+      }
+      if (*abort_flag) {                               // loads of a drained CTA may be in flight
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {}
+      }
     }
   } else {
-    // ------------------------------------------------------------------ loader
-    if (lane == 0) {
+    // ------------------------------------------------------------------ table loader
+    if (elect_one()) {
       mbar_arrive_expect_tx(gfull, GROUPS * g_bytes);
       for (int grp = 0; grp < GROUPS; ++grp)
         bulk_g2s(g_base + (size_t)grp * g_bytes,
@@ -308,31 +389,38 @@ __global__ void __launch_bounds__(128 * GROUPS + 64, 1) tc_dz_kernel(const DzPar
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4 * GROUPS) {
-    mbar_wait_drain(done, 0, P.wait_cycles);
+  if (warp == 8 * GROUPS) {
+    for (int i = 0; i < GROUPS; ++i) mbar_wait_drain(done + i, 0, P.wait_cycles);
     tc_fence_after();
     tmem_free(tmem_base, tmem_cols);
   }
 }
 
-struct DzPlan { int groups, lb, splits, chunks_per_split, tstages; size_t smem; };
+struct DzPlan { int groups, lb, splits, chunks_per_split, tstages, rstages; size_t smem; };
 
 // NC_ = L - 1 useful columns per key for the knot counts in common use, all 8 * LB_ otherwise.
 template <bool LIN>
 cudaError_t dz_launch(const DzPlan& zp, int L, bool relu, const DzParams& P, dim3 grid, cudaStream_t stream) {
-  const unsigned threads = 128 * zp.groups + 64;
+  CUtensorMap mz, mg, md;
+  if (!make_box_map(&mz, P.z, P.N, P.h, P.zs) || (P.g_act && !make_box_map(&mg, P.g_act, P.N, P.h, P.gas)) ||
+      (!P.dz_f32 && !make_box_map(&md, P.dz, P.N, P.h, P.dzs)))
+    return cudaErrorInvalidValue;
+  if (!P.g_act) mg = mz;
+  if (P.dz_f32) md = mz;
+  const unsigned threads = 320 * zp.groups + 32;
 #define SKV_DZ_CASE(G_, LB_, NC_, COND_)                                                                           \
   if (zp.groups == G_ && zp.lb == LB_ && (COND_))                                                                  \
-    return relu ? launch_chained<tc_dz_kernel<G_, LB_, NC_, true, LIN>>(grid, threads, zp.smem, stream, P)         \
-                : launch_chained<tc_dz_kernel<G_, LB_, NC_, false, LIN>>(grid, threads, zp.smem, stream, P);
+    return relu ? launch_chained<tc_dz_kernel<G_, LB_, NC_, true, LIN>>(grid, threads, zp.smem, stream, P, mz, mg, md)         \
+                : launch_chained<tc_dz_kernel<G_, LB_, NC_, false, LIN>>(grid, threads, zp.smem, stream, P, mz, mg, md);
   if constexpr (LIN) {
     SKV_DZ_CASE(2, 3, 20, L == 21)
   } else {
-    SKV_DZ_CASE(2, 3, 21, L == 22) SKV_DZ_CASE(2, 2, 15, L == 16) SKV_DZ_CASE(1, 6, 41, L == 42)
+    SKV_DZ_CASE(2, 3, 21, L == 22) SKV_DZ_CASE(2, 2, 15, L == 16) SKV_DZ_CASE(2, 6, 41, L == 42)
   }
   SKV_DZ_CASE(2, 1, 8, true) SKV_DZ_CASE(2, 2, 16, true) SKV_DZ_CASE(2, 3, 24, true) SKV_DZ_CASE(2, 4, 32, true)
-  SKV_DZ_CASE(1, 5, 40, true) SKV_DZ_CASE(1, 6, 48, true)
-  SKV_DZ_CASE(1, 7, 56, true) SKV_DZ_CASE(1, 8, 64, true)
+  SKV_DZ_CASE(2, 5, 40, true) SKV_DZ_CASE(2, 6, 48, true) SKV_DZ_CASE(2, 7, 56, true) SKV_DZ_CASE(2, 8, 64, true)
+  SKV_DZ_CASE(1, 1, 8, true) SKV_DZ_CASE(1, 2, 16, true) SKV_DZ_CASE(1, 3, 24, true) SKV_DZ_CASE(1, 4, 32, true)
+  SKV_DZ_CASE(1, 5, 40, true) SKV_DZ_CASE(1, 6, 48, true) SKV_DZ_CASE(1, 7, 56, true) SKV_DZ_CASE(1, 8, 64, true)
 #undef SKV_DZ_CASE
   return cudaErrorInvalidValue;
 }

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
   } else if (warp < 5 * GROUPS) {
     // ------------------------------------------------------------------ MMA issue, one warp per token group
     // (one thread cannot issue N = r MMAs faster than about one per 45 cycles)
-    if (lane == 0) {
+    if (elect_one()) {
       const int grp = warp - 4 * GROUPS;
       const uint32_t idesc = instr_desc(0, 0, 0, 1, 128, r);
       const uint32_t b_hi = desc_hi(P.b_sbo);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
     }
   } else {
     // ------------------------------------------------------------------ code-table loader
-    if (lane == 0) {
+    if (elect_one()) {
       const uint8_t* src = reinterpret_cast<const uint8_t*>(P.cimg) + (size_t)chunk_begin * c_bytes;
       for (int ci = 0; ci < nch; ++ci) {
         const int s = ci % CS;

@@ -29,10 +29,7 @@
 // stores back to shared memory and no A reads from it): 0.72 ms, because a 128 x 256 tile needs 48 KB
 // from L2 per 4.2 MFLOP against 64 KB per 8.4 MFLOP here, and both kernels take in about 90 GB/s per
 // SM, which looks like the limit of the L2-to-SM path.)
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
-#include "skv_tc_common.cuh"
+#include "skv_tma.cuh"
 
 namespace skv {
 namespace tc {
@@ -87,25 +84,6 @@ __global__ void tc_pack_w_kernel(const __nv_bfloat16* __restrict__ W, int64_t ws
     }
     img[idx] = ok ? __ldg(reinterpret_cast<const uint4*>(W + n * ws + k)) : make_uint4(0, 0, 0, 0);
   }
-}
-
-__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-
-// Tiled TMA load, to this CTA alone, of one box of `map` at element coordinates (x, y) into this CTA's shared
-// memory; x * 2 bytes is a multiple of 16 at every call site (x is a multiple of 64).
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
 }
 
 template <bool RELU>
@@ -164,7 +142,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
             for (int j = 0; j < kPerThread; ++j) {
               v[j].x = relu_sq_bf2(v[j].x); v[j].y = relu_sq_bf2(v[j].y);
               v[j].z = relu_sq_bf2(v[j].z); v[j].w = relu_sq_bf2(v[j].w);
-              sts128(src + (uint32_t)j * 4096u, v[j]);
+              sts128(src + (uint32_t)j * 4096u, v[j].x, v[j].y, v[j].z, v[j].w);
             }
             fence_async_smem();
           }
@@ -200,7 +178,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
     }
   } else if (warp == 8) {
     // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       // A: K-major tile whose rows are one swizzle span (128 or 64 bytes) long, 8-row groups 8 rows apart;
       // a K step of 16 elements advances the start address by 32 bytes inside the swizzled row.
       constexpr uint32_t kRowBytes = kRoK * 2;
@@ -237,7 +215,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
     }
   } else {
     // ------------------------------------------------------------------ loader
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool stop = false;
       for (int64_t t = blockIdx.x; t < P.tiles && !stop; t += step) {
@@ -268,32 +246,9 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   }
 }
 
-PFN_cuTensorMapEncodeTiled tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
-    else
-      cudaGetLastError();
-  }
-  return fn;
-}
-
-// Map of a [rows][cols] bf16 matrix with row pitch `pitch` elements; boxes of 256 rows x kRoK columns,
-// the swizzle span of one row, zeros outside the matrix.
+// Boxes of 256 rows x kRoK columns, the swizzle span of one row.
 bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch) {
-  PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
-  if (!enc) return false;
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {pitch * 2};
-  const cuuint32_t box[2] = {kRoK, 256};
-  const cuuint32_t es[2] = {1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, kRoK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return make_map_2d(m, base, rows, cols, pitch, kRoK, 256, kRoK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 }  // namespace
