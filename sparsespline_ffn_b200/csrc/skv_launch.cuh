@@ -24,6 +24,17 @@ __device__ __forceinline__ uint4 ld16(const void* p) {
   return v;
 }
 
+__device__ __forceinline__ uint2 ld8(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld4(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Raises the kernel's dynamic shared-memory limit to all the device has, once per kernel and device.
 template <auto Kernel>
 cudaError_t allow_all_smem() {

@@ -65,23 +65,27 @@ bool make_dz_plan(const skv_problem& p, DzPlan* o) {
 }
 
 bool make_dc_plan(const skv_problem& p, DcPlan* o) {
-  const int LR = (p.L + 1) & ~1, rp = padded_r(p), hp = padded_h(p);
-  for (int kch = 16; kch >= 8; kch /= 2) {
-    const int mtiles = (kch * LR + 127) / 128;
-    if (mtiles > 3) continue;
-    const size_t smem = 2 * (size_t)mtiles * 16 * 2048 + 2 * (size_t)128 * rp * 2 + 256;
-    if (smem > kSmemLimit) continue;
+  const int words = (p.L + 1) / 2, rp = padded_r(p), hp = padded_h(p);
+  for (int kj = 4; kj >= 2; kj /= 2) {
+    const int kch = 4 * kj, mtiles = (kch * 2 * words + 127) / 128;
+    if (mtiles * rp > 512) continue;
+    // as many producer groups (stages) as fit shared memory; two of eight warps where it cannot be three of four
+    int ng = kDcMaxGroups;
+    auto smem_for = [&](int n) { return (size_t)n * (dc_stage_bytes(mtiles) + (size_t)kDcTokens * rp * 2) + 256; };
+    while (ng > 1 && smem_for(ng) > kSmemLimit) --ng;
+    if (ng < 2) continue;
+    o->kj = kj;
+    o->gw = ng >= 3 ? 4 : 8;
+    o->ngroups = ng;
+    o->mtiles = mtiles;
+    o->smem = smem_for(ng) < kSmemOnePerSM ? kSmemOnePerSM : smem_for(ng);
     int most = 512 / (mtiles * rp);
-    if (most < 1) continue;
     if (most > 8) most = 8;
     const int chunks = (hp + kch - 1) / kch;
-    o->kch = kch;
-    o->mtiles = mtiles;
-    o->smem = smem < kSmemOnePerSM ? kSmemOnePerSM : smem;
-    o->tiles_total = ((p.N > 0 ? p.N : 1) + 127) / 128;
-    // 1.2 us per tile and chunk of 16 keys at L = 22, r = 32 (1.6 at r = 128) and the wait for a tile's g; a
+    o->tiles_total = ((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens;
+    // 0.38 us per tile and chunk of 16 keys at L = 22, r = 32, and the wait for a tile's g; a
     // CTA's prologue and epilogue; a split's partials written and read again through L2 or HBM
-    const double unit = 1.2 * kch / 16.0 * LR / 22.0 * (0.89 + rp / 290.0), tile = 0.004 * rp;
+    const double unit = 0.38 * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
     const double per_split = (double)hp * p.L * rp * 8.0 / 5.0e6;
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
@@ -248,8 +252,8 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.L = p.L;
       P.r = rp;
       P.g = c.g;
-      P.LR = (p.L + 1) & ~1;
-      P.kch = b.dc.kch;
+      P.words = (p.L + 1) / 2;
+      P.ngroups = b.dc.ngroups;
       P.mtiles = b.dc.mtiles;
       P.slab_chunks = b.dc.slab_chunks;
       P.tiles_per_split = b.dc.tiles_per_split;

@@ -292,40 +292,11 @@ __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w <<
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // ---------------------------------------------------------------------------------------------
-// Expanded-basis (Phi) row segment of one (token, key) pair.
-//
-// A token's Phi row is stored K-major in the un-swizzled canonical layout: 32-bit word w of the
-// row (knot columns 2w, 2w+1 as f16x2) lives at byte (w >> 2) * 2048 + (w & 3) * 4 from the
-// token's row base, i.e. at word offset w + (w >> 2) * 508.  The three non-zero weights sit at
-// columns bin..bin+2 of the key's L columns and always fall into two consecutive words.
-// phi_pair returns those two words and their word offsets; `wq` is the word index at which the
-// key's segment starts (key-in-chunk * L / 2).
-// The weights use B1 = 1 - B0 - B2 (partition of unity), masked by 0 <= u <= G.
+// Expanded basis (Phi) of one (token, key) pair: the non-zero weights sit at knot rows bin..bin+2 of the key's L
+// rows and always fall into two consecutive f16x2 words (rows 2w, 2w + 1).  The weights use
+// B1 = 1 - B0 - B2 (partition of unity), masked by 0 <= u <= G.
 // ---------------------------------------------------------------------------------------------
-// `kw` is the word distance between consecutive 16-byte chunks of a row minus 4: 508 for tiles of
-// 128 token rows (2048 bytes per chunk column), 252 for tiles of 64.
-// LIN: the linear spline's weights 1 - tau and tau.  Its last interval's second word would lie past the
-// key's segment; it is zero then (as for every even interval), and both offsets are the first word's, so a caller
-// that stores x1 before x0 writes the segment's own words only.
-template <bool LIN = false>
-__device__ __forceinline__ void phi_pair(float zz, const GridParams& g, uint32_t wq, uint32_t& x0, uint32_t& x1,
-                                         uint32_t& wo0, uint32_t& wo1, uint32_t kw = 508u) {
-  const Knot k = knot_of(zz, g);
-  const float t = k.tau, omt = 1.0f - t;
-  const float hm = k.in_range ? 0.5f : 0.0f;
-  const float B0 = LIN ? 2.0f * hm * omt : (hm * omt) * omt;
-  const float B2 = LIN ? 0.0f : (hm * t) * t;
-  const float B1 = LIN ? 2.0f * hm * t : fmaf(2.0f, hm, -B0) - B2;   // (m - B0) - B2 with m = 2 * hm, same roundings
-  const uint32_t p01 = pack_h2(B0, B1), p2 = pack_h2(B2, 0.0f);
-  const uint32_t sh = (k.tbits & 1u) << 4;
-  x0 = p01 << sh;
-  x1 = __funnelshift_l(p01, p2, sh);
-  const uint32_t s0 = wq + ((uint32_t)k.bin >> 1), s1 = s0 + (LIN ? k.tbits & 1u : 1u);
-  wo0 = s0 + (s0 >> 2) * kw;
-  wo1 = s1 + (s1 >> 2) * kw;
-}
-
-// phi_pair with the word index s0 of the first word (the second is s0 + 1) instead of offsets.
+// The two words and the index s0 of the first; `wq` is the word index at which the key's segment starts.
 __device__ __forceinline__ void phi_pair_s(float zz, const GridParams& g, uint32_t wq, uint32_t& x0, uint32_t& x1,
                                            uint32_t& s0) {
   const Knot k = knot_of(zz, g);

@@ -1,17 +1,18 @@
-// dC kernels: keys per chunk and, for L = 21 / 22, words per key known at compile time.
+// dC kernels: keys per lane and warps per producer group.
 #include "skv_tc_dc_kernel.cuh"
 
 namespace skv {
 namespace tc {
 
 cudaError_t dc_launch(const DcPlan& dp, bool lin, const DcParams& P, dim3 grid, cudaStream_t stream) {
-#define SKV_DC_CASE(KCH_, HLC_)                                                                      \
-  return lin ? launch_chained<tc_dc_kernel<KCH_, HLC_, true>>(grid, 320, dp.smem, stream, P)         \
-             : launch_chained<tc_dc_kernel<KCH_, HLC_, false>>(grid, 320, dp.smem, stream, P);
-  if (dp.kch == 16 && P.LR == 22) SKV_DC_CASE(16, 11)
-  if (dp.kch == 16) SKV_DC_CASE(16, 0)
-  SKV_DC_CASE(8, 0)
+  const unsigned threads = (unsigned)(dp.ngroups * dp.gw + 2) * 32;
+#define SKV_DC_CASE(KJ_, GW_)                                                                              \
+  if (dp.kj == KJ_ && dp.gw == GW_)                                                                        \
+    return lin ? launch_chained<tc_dc_kernel<KJ_, GW_, true>>(grid, threads, dp.smem, stream, P)           \
+               : launch_chained<tc_dc_kernel<KJ_, GW_, false>>(grid, threads, dp.smem, stream, P);
+  SKV_DC_CASE(4, 4) SKV_DC_CASE(4, 8) SKV_DC_CASE(2, 4) SKV_DC_CASE(2, 8)
 #undef SKV_DC_CASE
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace tc
