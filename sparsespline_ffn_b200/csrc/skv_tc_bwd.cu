@@ -69,16 +69,20 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
   for (int kj = 4; kj >= 2; kj /= 2) {
     const int kch = 4 * kj, mtiles = (kch * 2 * words + 127) / 128;
     if (mtiles * rp > 512) continue;
-    // as many producer groups (stages) as fit shared memory; two of eight warps where it cannot be three of four
+    // as many producer groups (stages) as fit shared memory beside a longer ring of g tiles; two groups of eight
+    // warps where it cannot be three of four
+    const size_t stage = dc_stage_bytes(mtiles), slot = (size_t)kDcTokens * rp * 2;
     int ng = kDcMaxGroups;
-    auto smem_for = [&](int n) { return (size_t)n * (dc_stage_bytes(mtiles) + (size_t)kDcTokens * rp * 2) + 256; };
-    while (ng > 1 && smem_for(ng) > kSmemLimit) --ng;
+    while (ng > 1 && ng * stage + (ng + 1) * slot + 512 > kSmemLimit) --ng;
     if (ng < 2) continue;
     o->kj = kj;
     o->gw = ng >= 3 ? 4 : 8;
     o->ngroups = ng;
+    int ring = (int)((kSmemLimit - 512 - ng * stage) / slot);
+    o->gring = ring > kDcMaxRing ? kDcMaxRing : ring;
     o->mtiles = mtiles;
-    o->smem = smem_for(ng) < kSmemOnePerSM ? kSmemOnePerSM : smem_for(ng);
+    o->smem = ng * stage + o->gring * slot + 512;
+    if (o->smem < kSmemOnePerSM) o->smem = kSmemOnePerSM;
     int most = 512 / (mtiles * rp);
     if (most > 8) most = 8;
     const int chunks = (hp + kch - 1) / kch;
@@ -254,6 +258,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.g = c.g;
       P.words = (p.L + 1) / 2;
       P.ngroups = b.dc.ngroups;
+      P.gring = b.dc.gring;
       P.mtiles = b.dc.mtiles;
       P.slab_chunks = b.dc.slab_chunks;
       P.tiles_per_split = b.dc.tiles_per_split;

@@ -5,7 +5,7 @@ namespace skv {
 namespace tc {
 
 cudaError_t dc_launch(const DcPlan& dp, bool lin, const DcParams& P, dim3 grid, cudaStream_t stream) {
-  const unsigned threads = (unsigned)(dp.ngroups * dp.gw + 2) * 32;
+  const unsigned threads = (unsigned)(dp.ngroups * dp.gw + kDcIssuers + 1) * 32;
 #define SKV_DC_CASE(KJ_, GW_)                                                                              \
   if (dp.kj == KJ_ && dp.gw == GW_)                                                                        \
     return lin ? launch_chained<tc_dc_kernel<KJ_, GW_, true>>(grid, threads, dp.smem, stream, P)           \

@@ -30,6 +30,7 @@ struct DcParams {
   GridParams g;
   int words;                 // f16x2 words per key in the Phi^T tile: L / 2 rounded up (an odd L's last row is zero)
   int ngroups;               // producer groups, one stage each
+  int gring;                 // slots of the ring of g tiles, more than groups
   int mtiles;                // 128-row MMA tiles per chunk
   int slab_chunks;           // chunks per CTA slab
   int64_t tiles_per_split;   // 64-token tiles per token split
@@ -41,12 +42,14 @@ struct DcParams {
 constexpr int kDcTokens = 64;                        // tokens per tile
 constexpr uint32_t kDcUnit = kDcTokens * 16;         // bytes of one 8-row group of a tile
 constexpr int kDcMaxGroups = 4;
+constexpr int kDcMaxRing = 8;                        // slots of the ring of g tiles
+constexpr int kDcIssuers = 3;                        // warps that issue MMAs, each for every third M tile
 // One unit behind a stage: the linear spline's last interval stores a zero word there.
 __host__ __device__ constexpr uint32_t dc_stage_bytes(int mtiles) { return (uint32_t)mtiles * 16u * kDcUnit + kDcUnit; }
 
 // KJ = keys per lane and token (a chunk is 4 * KJ keys), GW = warps per producer group.
 template <int KJ, int GW, bool LIN>
-__global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
+__global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int KCH = 4 * KJ;
   constexpr int TI = kDcTokens / GW / 8;                            // tokens per lane
@@ -54,13 +57,14 @@ __global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
   const uint32_t phi_bytes = dc_stage_bytes(P.mtiles);             // [m groups][8 token groups][8 tok][8 m]
   const uint32_t g_bytes = (uint32_t)(kDcTokens * r * 2);
   uint8_t* phi_base = smem;                                         // [NG][phi_bytes]
-  uint8_t* g_base = smem + NG * (size_t)phi_bytes;                  // [NG][g_bytes]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(g_base + NG * (size_t)g_bytes);
+  const int GR = P.gring;
+  uint8_t* g_base = smem + NG * (size_t)phi_bytes;                  // [GR][g_bytes]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(g_base + GR * (size_t)g_bytes);
   uint64_t* pfull = bars;                       // [NG] producers -> MMA
   uint64_t* pempty = pfull + kDcMaxGroups;      // [NG] MMA -> producers
-  uint64_t* gfull = pempty + kDcMaxGroups;      // [NG] TMA -> MMA
-  uint64_t* gempty = gfull + kDcMaxGroups;      // [NG] MMA -> TMA
-  uint64_t* done = gempty + kDcMaxGroups;       // [1]
+  uint64_t* gfull = pempty + kDcMaxGroups;      // [GR] TMA -> MMA
+  uint64_t* gempty = gfull + kDcMaxRing;        // [GR] MMA -> TMA
+  uint64_t* done = gempty + kDcMaxRing;         // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wc{abort_flag, P.status, kStatusTimeoutDc, P.wait_cycles};
@@ -77,11 +81,13 @@ __global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
   if (tid == 0) {
     for (int i = 0; i < kDcMaxGroups; ++i) {
       mbar_init(pfull + i, GW);
-      mbar_init(pempty + i, 1);
-      mbar_init(gfull + i, 1);
-      mbar_init(gempty + i, 1);
+      mbar_init(pempty + i, kDcIssuers);
     }
-    mbar_init(done, 1);
+    for (int i = 0; i < kDcMaxRing; ++i) {
+      mbar_init(gfull + i, 1);
+      mbar_init(gempty + i, kDcIssuers);
+    }
+    mbar_init(done, kDcIssuers);
     *abort_flag = 0;
     mbar_init_fence();
   }
@@ -194,37 +200,45 @@ __global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
       }
     }
     tc_fence_before();
-  } else if (warp == mma_warp) {
+  } else if (warp < mma_warp + kDcIssuers) {
     // ------------------------------------------------------------------ MMA issue
     if (elect_one()) {
+      const int m0 = warp - mma_warp;
       const uint32_t idesc = instr_desc(0, 0, 1, 1, 128, r);
       const uint32_t ab_hi = desc_hi(kDcUnit);
+      const uint32_t a_tile0 = desc_lo(smem_u32(phi_base) + (uint32_t)m0 * 16u * kDcUnit, 128u);
+      const uint32_t b_ring = desc_lo(smem_u32(g_base), 128u);
       uint32_t fills = 0;                              // of every group so far
+      int slot0 = 0;                                   // ring slot and phase of the round's first tile
+      uint32_t gpar0 = 0u;
       bool drain = false;
       for (int tp = 0; tp < ntiles && !drain; tp += NG) {
         const int npg = min(NG, ntiles - tp);
-        const uint32_t gpar = (uint32_t)(tp / NG) & 1u;
         for (int ch = 0; ch < nchunks && !drain; ++ch, ++fills) {
+          int slot = slot0;
+          uint32_t gpar = gpar0;
           for (int pg = 0; pg < npg; ++pg) {
-            if (ch == 0) drain = drain || mbar_wait(gfull + pg, gpar, wc);
+            if (ch == 0) drain = drain || mbar_wait(gfull + slot, gpar, wc);
             drain = drain || mbar_wait(pfull + pg, fills & 1u, wc);
             if (drain) break;                          // draining: issue nothing more
             tc_fence_after();
-            uint32_t a_lo0 = desc_lo(smem_u32(phi_base + (size_t)pg * phi_bytes), 128u);
-            const uint32_t b_lo0 = desc_lo(smem_u32(g_base + (size_t)pg * g_bytes), 128u);
-            uint32_t d_addr = tmem_base + (uint32_t)(ch * P.mtiles * r);
+            uint32_t a_lo0 = a_tile0 + (uint32_t)pg * (phi_bytes >> 4);
+            const uint32_t b_lo0 = b_ring + (uint32_t)slot * (g_bytes >> 4);
+            uint32_t d_addr = tmem_base + (uint32_t)((ch * P.mtiles + m0) * r);
             const uint32_t first = tp + pg == 0 ? 0u : 1u;
-            for (int mt = 0; mt < P.mtiles; ++mt) {
+            for (int mt = m0; mt < P.mtiles; mt += kDcIssuers) {
 #pragma unroll
               for (int ks = 0; ks < kDcTokens / 16; ++ks)
                 umma_f16_split(d_addr, a_lo0 + (uint32_t)ks * 16u, ab_hi, b_lo0 + (uint32_t)ks * 16u, ab_hi, idesc,
                                ks > 0 ? 1u : first);
-              a_lo0 += (16u * kDcUnit) >> 4;
-              d_addr += (uint32_t)r;
+              a_lo0 += (kDcIssuers * 16u * kDcUnit) >> 4;
+              d_addr += (uint32_t)(kDcIssuers * r);
             }
             umma_commit(pempty + pg);
-            if (ch + 1 == nchunks) umma_commit(gempty + pg);
+            if (ch + 1 == nchunks) umma_commit(gempty + slot);
+            if (++slot == GR) { slot = 0; gpar ^= 1u; }
           }
+          if (ch + 1 == nchunks) { slot0 = slot; gpar0 = gpar; }
         }
       }
       umma_commit(done);
@@ -233,16 +247,19 @@ __global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
     // ------------------------------------------------------------------ gradient-tile loader
     if (elect_one()) {
       const uint8_t* img = reinterpret_cast<const uint8_t*>(P.gimg);
+      int slot = 0;
+      uint32_t par = 1u;                               // a fresh barrier passes a wait for the phase before its first
       for (int ti = 0; ti < ntiles; ++ti) {
-        const int pg = ti % NG, u = ti / NG;
-        if (u > 0) mbar_wait(gempty + pg, (uint32_t)(u - 1) & 1u, wc);
+        mbar_wait(gempty + slot, par, wc);
         if (*abort_flag) break;
-        mbar_arrive_expect_tx(gfull + pg, g_bytes);
+        mbar_arrive_expect_tx(gfull + slot, g_bytes);
         // the image has 128-token tiles [r/8][16 token groups][128 B]; this tile is one half of each channel group
         const int64_t t64 = tile_begin + ti;
         const uint8_t* src = img + (size_t)(t64 >> 1) * 128 * r * 2 + (size_t)(t64 & 1) * kDcUnit;
         for (int cg = 0; cg < r / 8; ++cg)
-          bulk_g2s(g_base + (size_t)pg * g_bytes + (size_t)cg * kDcUnit, src + (size_t)cg * 2 * kDcUnit, kDcUnit, gfull + pg);
+          bulk_g2s(g_base + (size_t)slot * g_bytes + (size_t)cg * kDcUnit, src + (size_t)cg * 2 * kDcUnit, kDcUnit,
+                   gfull + slot);
+        if (++slot == GR) { slot = 0; par ^= 1u; }
       }
       if (*abort_flag) {
         const long long t0 = clock64();
@@ -258,7 +275,7 @@ __global__ void __launch_bounds__(576, 1) tc_dc_kernel(const DcParams P) {
   }
 }
 
-struct DcPlan { int kj, gw, ngroups, mtiles, slab_chunks, slabs, splits; int64_t tiles_total, tiles_per_split; size_t smem; };
+struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, slabs, splits; int64_t tiles_total, tiles_per_split; size_t smem; };
 
 }  // namespace tc
 }  // namespace skv
