@@ -73,7 +73,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         objects.append(obj)
         if force or not _newer(obj, [src, *_headers()]):
             jobs.append([nvcc, *NVCC_FLAGS, *(["-Xptxas", "-v"] if verbose else []), "-c", src, "-o", obj])
-    with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(6, (os.cpu_count() or 2) - 2))) as pool:
         list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
     _run([nvcc, *NVCC_FLAGS, "-shared", "-Xlinker", "-soname=" + os.path.basename(LIB_PATH), *objects, "-o", LIB_PATH])
     _run(_host_command(), verbose)

@@ -202,16 +202,18 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) {
 }
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3FFFu) | (1u << 14); }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand is read from tensor memory (lane = row of A,
-// each 32-bit column holds two consecutive K elements), B from shared memory.
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
-                                            uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem] with a 2:4 sparse A: lane = row of A, each 32-bit column two kept K elements.  K = 32, of
+// which A holds 16 elements (8 columns) per row and the columns at `meta` which ones they are; bit 0 of the
+// instruction descriptor selects the odd one of a pair of metadata columns.
+constexpr uint32_t kSparse = 1u << 2;
+__device__ __forceinline__ void umma_f16_sparse_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
+                                                   uint32_t meta, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.sp.cta_group::1.kind::f16 [%0], [%1], db, [%4], %5, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(meta), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 

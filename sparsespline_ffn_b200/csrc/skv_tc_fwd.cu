@@ -13,23 +13,21 @@ cudaError_t fwd_launch_lin_other(int, int, const FwdParams&, dim3, size_t, cudaS
 namespace {
 
 struct FwdPlan {
-  int groups, words, splits, chunks_per_split, cstages;
+  int groups, fold, splits, chunks_per_split, cstages;
   size_t smem;
 };
 
 size_t fwd_cimg_bytes(const skv_problem& p) {
-  const int lp = (fwd_words(p.L) + 1) / 2 * 4;
-  return align256((size_t)padded_h(p) * lp * padded_r(p) * sizeof(__half));
+  return align256((size_t)padded_h(p) * 4 * fwd_fold(p.L) * padded_r(p) * sizeof(__half));
 }
 
 FwdPlan make_plan(const skv_problem& p) {
   FwdPlan f{};
   const int rp = padded_r(p);
-  f.words = fwd_words(p.L);
-  const int hlp = (f.words + 1) & ~1;
+  const int F = f.fold = fwd_fold(p.L);
   const int chunks = padded_h(p) / kChunkKeys;
   const int64_t N = p.N > 0 ? p.N : 1;
-  const size_t c_bytes = (size_t)kChunkKeys * 2 * hlp * rp * 2;
+  const size_t c_bytes = (size_t)kChunkKeys * 4 * F * rp * 2;
   // Splits are bounded by what their partials may take: below 16 MiB of scratch together with the image, or
   // sixteen of them.  A split of fewer than four chunks is mostly prologue.
   const size_t part = (size_t)N * rp * sizeof(float);
@@ -38,15 +36,15 @@ FwdPlan make_plan(const skv_problem& p) {
   if (most < 16) most = 16;
   if (most > (chunks + 3) / 4) most = (chunks + 3) / 4;
   double best = 0.0;
-  for (int g = fwd_max_groups(f.words, rp); g >= 1; --g) {
-    const size_t stage_bytes = (size_t)128 * g * hlp * 4;
+  for (int g = fwd_max_groups(F, rp); g >= 1; --g) {
+    const size_t stage_bytes = (size_t)128 * g * (F + 1) * 4;
     int cstages = (int)((kSmemLimit - 512 - stage_bytes) / c_bytes);
-    if (cstages > kMaxTaCStages) cstages = kMaxTaCStages;
+    if (cstages > kMaxCStages) cstages = kMaxCStages;
     if (cstages < 2) continue;
     const int64_t tiles = (N + 128 * g - 1) / (128 * g);
     // microseconds: a chunk of g groups (instruction issue, or the MMAs of wide r), a CTA's prologue and
-    // epilogue, and the partials' way through L2 (measured: 1.5 us per chunk of four groups at L = 22)
-    const double issue = (0.25 + 0.31 * g) * (hlp + 8) / 20.0, mma = g * hlp * rp * 0.5 / 1800.0;
+    // epilogue, and the partials' way through L2 (measured: 1.3 us per chunk of four groups at L = 22)
+    const double issue = (0.22 + 0.27 * g) * (F + 14) / 20.0, mma = g * F * rp * 0.5 / 1800.0;
     const double chunk = issue > mma ? issue : mma;
     int last = 0;
     for (int64_t s = 1; s <= most; ++s) {
@@ -83,9 +81,9 @@ size_t fwd_copy_bytes(const skv_problem& p) { return align256((size_t)(p.N > 0 ?
 
 bool fwd_eligible(const skv_problem& p) {
   if (p.dtype != SKV_BF16 || p.r > 128 || p.L < 4 || p.L > 64) return false;
-  const int words = fwd_words(p.L), rp = padded_r(p), hlp = (words + 1) & ~1;
-  return fwd_max_groups(words, rp) >= 1 &&
-         2 * (size_t)kChunkKeys * 2 * hlp * rp * 2 + (size_t)128 * hlp * 4 + 512 <= kSmemLimit;
+  const int F = fwd_fold(p.L), rp = padded_r(p);
+  return fwd_max_groups(F, rp) >= 1 &&
+         2 * (size_t)kChunkKeys * 4 * F * rp * 2 + (size_t)128 * (F + 1) * 4 + 512 <= kSmemLimit;
 }
 
 // `rows_ok`: the token-major arrays can be read and written in place.
@@ -99,7 +97,7 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
             void* delta_out, int64_t ds, void* scratch, bool rows_ok) {
   const skv_problem& p = c.p;
   const FwdPlan& f = plan_forward(p);
-  const int hp = padded_h(p), rp = padded_r(p), lp = (f.words + 1) / 2 * 4;
+  const int hp = padded_h(p), rp = padded_r(p), lp = 4 * f.fold;
   uint8_t* base = static_cast<uint8_t*>(scratch);
   uint32_t* hdr = reinterpret_cast<uint32_t*>(base);
   __half* img = reinterpret_cast<__half*>(base + kHeaderBytes);
@@ -147,7 +145,7 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
   const bool lin = c.g.order == 1, relu = p.activation == SKV_ACT_RELU_SQ;
   auto* launch = lin ? (relu ? fwd_launch_lin_relu : fwd_launch_lin_other)
                      : (relu ? fwd_launch_quad_relu : fwd_launch_quad_other);
-  if (launch(f.groups, f.words, P, grid, f.smem, c.stream) != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
+  if (launch(f.groups, f.fold, P, grid, f.smem, c.stream) != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
   note_launches(1);
   return launch_finalize(partial, f.splits, p.N, p.r, rp, p.lambda_scale, hdr, delta_out, ds, p.delta_f32 != 0, c.stream);
 }

@@ -10,18 +10,19 @@
 #pragma once
 
 #include "skv_tc_prep.cuh"
+#include "skv_tma.cuh"
 
 namespace skv {
 namespace tc {
 
-constexpr int kMaxTaCStages = 8;
+constexpr int kMaxCStages = 8;
 
 struct FwdParams {
   const __nv_bfloat16* z;
   int64_t zs;
   __nv_bfloat16* act_out;
   int64_t as;
-  const __half* cimg;       // [h/8][8*LP/8][r/8][8][8] f16 image of C, LP rows per key
+  const __half* cimg;       // [h/8][8*LP/8][r/8][8][8] f16 image of C, LP = 4 F rows per key
   float* partial;           // [splits][N][r]
   int64_t N;
   int r;                    // code channels, padded to a multiple of 16
@@ -35,68 +36,68 @@ struct FwdParams {
   int skip_copy;            // test hook: the loader leaves out the copy of its first chunk
 };
 
-// Knot rows per key in units of two (f16x2 words) the kernel is instantiated for: the common knot counts
-// (L = 15..16, 21..22, 23..24, 31..32, 41..42) as they are, every other one rounded up (zero rows).
-inline int fwd_words(int L) {
+// Groups of four knot rows per key (see the kernel) the kernel is instantiated for: enough for 2 F - 1 words.
+inline int fwd_fold(int L) {
   const int hl = (L + 1) / 2;
-  for (int v : {4, 6, 8, 11, 12, 16, 21, 22, 32})
-    if (hl <= v) return v;
+  for (int v : {4, 6, 8, 10, 12, 18})
+    if (hl <= 2 * v - 1) return v;
   return 0;
 }
-
-// Token groups (of 128) a CTA can hold: 8 * words columns of Phi and r of accumulator each.
-inline int fwd_max_groups(int words, int r) {
-  const int hlp = (words + 1) & ~1;
-  const int g = 512 / (kChunkKeys * hlp + r);
+// Tensor-memory columns of a token group: Phi of 8 keys, its metadata in two halves, the accumulator.
+__host__ __device__ constexpr int fwd_meta_cols(int F) { return (F / 2 + 1) & ~1; }
+inline int fwd_max_groups(int F, int r) {
+  const int g = 512 / (kChunkKeys * F + 2 * fwd_meta_cols(F) + r);
   return g > 4 ? 4 : g;
 }
 
 // ---------------------------------------------------------------------------------------------
 // Launch shape: grid = (token tiles of 128*GROUPS tokens, key splits).  Each producer thread owns a token: it
-// builds the complete Phi row segment of a key (HL = L/2 f16x2 words, two of them non-zero) in
-// registers and writes it with tcgen05.st into its own tensor-memory lane; the MMA takes A from
-// tensor memory and only the code-table chunk (B) from shared memory.  Nothing has to be
-// cleared: a row segment is overwritten completely every chunk.
+// builds the Phi row segment of a key in registers and writes it with tcgen05.st into its own tensor-memory
+// lane; the MMA takes A from tensor memory and only the code-table chunk (B) from shared memory.  Nothing has
+// to be cleared: a row segment is overwritten completely every chunk.
 //
-// Tensor-memory columns per token group: 8*HL for A (single-buffered) followed by r for the
-// accumulator; with four groups (512 tokens per CTA, 16 producer warps) the other groups keep the
-// SM busy while one group waits for its MMAs.
+// Sparse A.  Of a key's L knot rows a token has weights on three consecutive ones, which always lie in two
+// neighbouring f16x2 words w, w + 1 (rows 2w, 2w + 1).  The table image orders a key's rows in F groups of four, group f
+// = words f and f + F - 1, so that the two words fall into neighbouring groups whichever they are: groups w, w + 1 as
+// their first halves, or (from w = F - 1 on) groups w - F + 1, w - F + 2 as their second.  That is the 2:4 pattern of
+// the sparse MMA: a key is F words of A instead of 2 F (tensor-memory writes, words to place and MMAs all halve), and its
+// metadata is one bit per key, "first or second halves": nibbles 0x4 (elements 0, 1) or 0xE (elements 2, 3).
+// Metadata layout for 16-bit types: the 32-bit word of lane l, K step of 32: lanes with bit 3 clear hold elements 0..15 of
+// rows l and l + 8 (low, high half), lanes with bit 3 set elements 16..31 of rows l - 8 and l; hence one shuffle.
+//
+// Bound: instruction issue of the producers and the load/store data path, which also carries the tensor-memory stores.
+// Tensor-memory columns per token group: 8*F for A, written and consumed in two halves of 4 keys so that the MMAs of
+// one run while the other is built, the metadata of the halves, r for the accumulator.
 // ---------------------------------------------------------------------------------------------
-// Keys of each half chunk (of four) that are placed through the staging row (load/store pipe); the
-// others are placed by multiplying with 0/1 masks in packed f16 arithmetic (FMA pipe).  With the mask
-// arithmetic the d20 shape takes 0.917 / 0.890 / 0.903 ms for 0 / 1 / 2 of four.  (The linear spline
-// stages none: the word behind its last interval's weight would lie past the row.)
-constexpr int kStagedPerHalf = 1;
+// Keys of each half chunk (of four) whose words are placed through a staging row in shared memory: two stores at the
+// dynamic position, F loads, two clearing stores.  The rows of a warp are interleaved by lane, so the bank of
+// every access is the lane and nothing conflicts, whatever the knot intervals are.  The other keys are placed by 0/1 masks in
+// packed f16 arithmetic.
+#ifndef SKV_NSTH
+#define SKV_NSTH 1
+#endif
+constexpr int kStagedPerHalf = SKV_NSTH;
 
-template <int GROUPS, int HL, int ACT, bool LIN>
-__global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(const FwdParams P) {
+template <int GROUPS, int F, int ACT, bool LIN>
+__global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const FwdParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
-  // Keys are padded to HLP words (an even count), so that half a chunk (4 keys) is a whole number
-  // of K = 16 steps; the code-table image has 2*HLP rows per key, the padding rows are zero.
-  constexpr int HLP = (HL + 1) & ~1;
-  constexpr int NSTH = LIN ? 0 : kStagedPerHalf;
   constexpr int kHalfKeys = kChunkKeys / 2;
-  constexpr int kHalfSteps = kHalfKeys * HLP / 8;                  // K = 16 steps per half chunk
+  constexpr int kHalfWords = kHalfKeys * F;                        // words of A per half chunk
+  constexpr int kHalfSteps = kHalfWords / 8;                       // MMAs (K = 32 rows of the table) per half chunk
+  constexpr int kMeta = fwd_meta_cols(F);
+  constexpr int NSTH = kStagedPerHalf;
+  constexpr int SW = F + 1;                                        // staging words per thread (one spare, see LIN)
   const int r = P.r;
-  const uint32_t c_bytes = (uint32_t)(kChunkKeys * 2 * HLP * r * 2);
+  const uint32_t c_bytes = (uint32_t)(kChunkKeys * 4 * F * r * 2);
   const int CS = P.cstages;
   uint8_t* c_base = smem;                                          // [cstage][c_bytes]
-  // One private staging row of HLP words per producer thread.  Placing the two non-zero words of
-  // a row segment costs about thirty compare/select instructions on the half-rate ALU pipe; for
-  // NSTH of the four keys of every half chunk the thread instead stores the two words into its
-  // (zeroed) staging row at the dynamic position, reads the row back and zeroes the two words
-  // again, which moves that work to the load/store pipe.  The rows of a warp are interleaved by
-  // lane (word w of lane l at (w * 32 + l) * 4 bytes of the warp's region), so the bank of every
-  // access is the lane and neither the scattered stores nor the loads conflict, whatever the knot
-  // intervals of the 32 tokens are.
-  constexpr int SW = HLP;
-  uint8_t* stage_base = c_base + (size_t)CS * c_bytes;             // [128*GROUPS][SW words]
+  uint8_t* stage_base = c_base + (size_t)CS * c_bytes;             // [warp][SW][32 lanes]
   uint64_t* bars = reinterpret_cast<uint64_t*>(stage_base + (size_t)128 * GROUPS * SW * 4);
   uint64_t* full = bars;                          // [group][half]  producers -> MMA
   uint64_t* empty = full + 2 * GROUPS;            // [group][half]  MMA -> producers
   uint64_t* cfull = empty + 2 * GROUPS;           // [cstage]       TMA -> MMA
-  uint64_t* cempty = cfull + kMaxTaCStages;       // [cstage]       MMA -> TMA
-  uint64_t* done = cempty + kMaxTaCStages;        // [group]
+  uint64_t* cempty = cfull + kMaxCStages;       // [cstage]       MMA -> TMA
+  uint64_t* done = cempty + kMaxCStages;        // [group]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + GROUPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wc{abort_flag, P.status, kStatusTimeoutFwd, P.wait_cycles};
@@ -105,20 +106,19 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
   const int chunk_begin = blockIdx.y * P.chunks_per_split;
   const int nch = min(P.chunks_per_split, P.chunks_total - chunk_begin);
   const int64_t tile_base = (int64_t)blockIdx.x * (128 * GROUPS);
-  const uint32_t grp_cols = (uint32_t)(kChunkKeys * HLP + r);
+  const uint32_t grp_cols = (uint32_t)(kChunkKeys * F + 2 * kMeta + r);
   uint32_t tmem_cols = 32;
   while (tmem_cols < GROUPS * grp_cols) tmem_cols <<= 1;
 
   if (tid == 0) {
     for (int i = 0; i < 2 * GROUPS; ++i) { mbar_init(full + i, 4); mbar_init(empty + i, 1); }
     for (int i = 0; i < GROUPS; ++i) mbar_init(done + i, 1);
-    for (int i = 0; i < kMaxTaCStages; ++i) { mbar_init(cfull + i, 1); mbar_init(cempty + i, GROUPS); }
+    for (int i = 0; i < kMaxCStages; ++i) { mbar_init(cfull + i, 1); mbar_init(cempty + i, GROUPS); }
     *abort_flag = 0;
     mbar_init_fence();
   }
-  if (NSTH > 0)
-    for (uint32_t i = tid; i < (uint32_t)(128 * GROUPS * SW / 4); i += blockDim.x)
-      reinterpret_cast<uint4*>(stage_base)[i] = make_uint4(0, 0, 0, 0);
+  for (uint32_t i = tid; i < (uint32_t)(128 * GROUPS * SW / 4); i += blockDim.x)
+    reinterpret_cast<uint4*>(stage_base)[i] = make_uint4(0, 0, 0, 0);
   if (warp == 5 * GROUPS) tmem_alloc(tmem_slot, tmem_cols);
   fence_async_smem();
   tc_fence_before();
@@ -138,10 +138,12 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
     __nv_bfloat16* arow = P.act_out ? P.act_out + (valid ? n : 0) * P.as + (int64_t)chunk_begin * kChunkKeys : nullptr;
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)grp * grp_cols;
     uint4 znext = valid && nch > 0 ? ld16(zrow) : make_uint4(0, 0, 0, 0);
-    // word w of this thread's staging row lives at (warp * HLP + w) * 128 + lane * 4: its bank is the
-    // lane, whatever w is, so neither the scattered stores nor the loads conflict
-    const uint32_t srow = smem_u32(stage_base) + (uint32_t)(warp * HLP * 128 + lane * 4);
-    const uint32_t srow_biased = srow - (kWordBias << 7);          // wp carries the bias kWordBias
+    // word w of this thread's staging row; the word index carries the bias kWordBias
+    const uint32_t srow = smem_u32(stage_base) + (uint32_t)(warp * SW * 128 + lane * 4);
+    const uint32_t srow_biased = srow - (kWordBias << 7);
+    const bool up = (lane & 8) != 0;
+    const uint32_t sel_send = up ? 0x5410u : 0x7632u;               // halves of two metadata words the other row needs
+    const uint32_t sel_0 = up ? 0x3254u : 0x5410u, sel_1 = up ? 0x3276u : 0x7610u;
     for (int ci = 0; ci < nch; ++ci) {
       const uint4 zc = znext;
       if (ci + 1 < nch && valid) znext = ld16(zrow + (ci + 1) * kChunkKeys);
@@ -154,81 +156,89 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
         if constexpr (ACT == SKV_ACT_RELU_SQ) aw[i] = relu_sq_bf2(zw[i]);
         else aw[i] = P.act == SKV_ACT_GELU ? pack_bf2(gelu_fwd(bf_lo(zw[i])), gelu_fwd(bf_hi(zw[i]))) : zw[i];
       }
-      // The group's A columns are written and consumed in two halves of 4 keys: the MMAs of one
-      // half run while the other half is being built, so the producers do not wait for them.
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
+        uint32_t W[kHalfWords];
+        uint32_t meta[kHalfSteps];
+#pragma unroll
+        for (int j = 0; j < kHalfSteps; ++j) meta[j] = 0x44444444u;
+        uint32_t x0[kHalfKeys], x1[kHalfKeys], wp[kHalfKeys];
+#pragma unroll
+        for (int pq = 0; pq < kHalfKeys / 2; ++pq) {
+          // knot interval and weights, two keys (one packed z word) at a time; rows past N read z = 0 and their
+          // accumulator rows are never stored
+          uint32_t a0[2], a1[2], aw2[2];
+          phi_pair_words2<LIN>(zw[half * (kHalfKeys / 2) + pq], P.g, a0, a1, aw2);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) { x0[2 * pq + e] = a0[e]; x1[2 * pq + e] = a1[e]; wp[2 * pq + e] = aw2[e]; }
+        }
+#pragma unroll
+        for (int q = 0; q < kHalfKeys; ++q) {
+          // fold: first or second halves, and the word index within the F groups
+          const bool hi = wp[q] >= kWordBias + (uint32_t)(F - 1);
+          if (hi) wp[q] -= (uint32_t)(F - 1);
+#pragma unroll
+          for (int j = 0; j < kHalfSteps; ++j) {                   // nibbles q * F .. q * F + F - 1 of the half's 4 F
+            uint32_t m = 0u;
+#pragma unroll
+            for (int i = 0; i < F; ++i)
+              if ((q * F + i) / 8 == j) m |= 0xAu << (4 * ((q * F + i) % 8));
+            if (m != 0u && hi) meta[j] |= m;
+          }
+          if (q < NSTH) {
+            // (the linear spline's last interval may store a zero word in the spare one)
+            const uint32_t pos = srow_biased + (wp[q] << 7);
+            sts32(pos, x0[q]);
+            sts32(pos + 128u, x1[q]);
+#pragma unroll
+            for (int i = 0; i < F; ++i) W[q * F + i] = lds32(srow + (uint32_t)i * 128u);
+            sts32(pos, 0u);
+            sts32(pos + 128u, 0u);
+          }
+        }
+#pragma unroll
+        for (int q = NSTH; q < kHalfKeys; ++q) {
+          // Placement at word-pair granularity: the word index is 2 * qd + s.  The two words land in pair qd as
+          // (x0, x1) when s = 0, or as (0, x0) there and (x1, 0) in pair qd + 1 when s = 1.  Each word is its value times
+          // a 0/1 mask in packed f16 arithmetic (x * 1 and x * 0 are exact for the non-negative finite weights, and at
+          // most one term of a sum is non-zero), which runs on the FMA pipe; compare/select chains would run on the ALU
+          // pipe.  The biased index >> 1 times 0x10001 is an f16 pair with bit patterns qd (low: a subnormal, or zero) and
+          // (kKnotBias >> 18) + qd (high), distinct per qd; f16 comparisons do not flush subnormals.
+          const bool odd = (wp[q] & 1u) != 0u;
+          const uint32_t y0 = odd ? 0u : x0[q], y1 = odd ? x0[q] : x1[q], y2 = odd ? x1[q] : 0u;
+          const uint32_t q2 = (wp[q] >> 1) * 0x00010001u;
+          const __half2 qh = *reinterpret_cast<const __half2*>(&q2);
+          const __half2 h0 = *reinterpret_cast<const __half2*>(&y0), h1 = *reinterpret_cast<const __half2*>(&y1),
+                        h2 = *reinterpret_cast<const __half2*>(&y2);
+          __half2 m[F / 2];
+#pragma unroll
+          for (int i = 0; i < F / 2; ++i) {
+            const uint32_t c2 = (((kKnotBias >> 18) + (uint32_t)i) << 16) | (uint32_t)i;
+            m[i] = __heq2(qh, *reinterpret_cast<const __half2*>(&c2));
+          }
+#pragma unroll
+          for (int i = 0; i < F / 2; ++i) {
+            __half2 e = __hmul2(m[i], h0);
+            if (i > 0) e = __hfma2(m[i - 1], h2, e);
+            const __half2 o = __hmul2(m[i], h1);
+            W[q * F + 2 * i] = *reinterpret_cast<const uint32_t*>(&e);
+            W[q * F + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&o);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kHalfSteps; j += 2) {
+          const int j1 = j + 1 < kHalfSteps ? j + 1 : j;
+          const uint32_t got = __shfl_xor_sync(0xffffffffu, __byte_perm(meta[j], meta[j1], sel_send), 8);
+          const uint32_t m1 = __byte_perm(meta[j1], got, sel_1);
+          meta[j] = __byte_perm(meta[j], got, sel_0);
+          if (j1 != j) meta[j1] = m1;
+        }
         if (ci > 0) {
           mbar_wait(empty + grp * 2 + half, (uint32_t)(ci - 1) & 1u, wc);
           tc_fence_after();
         }
-        // The first NSTH keys of the half go through the staging row: their stores and loads are
-        // issued first, the select chains of the other keys run while those loads are in flight,
-        // and the staged rows are written to tensor memory last.
-        // The words of two neighbouring keys are stored to tensor memory together (2 * HLP columns:
-        // one 16- and one 8-column store at HLP = 12 instead of two of each).
-        uint32_t WP[kHalfKeys / 2][2 * HLP];
-        // knot interval and weights of the half's four keys, two keys (one packed z word) at a time
-        uint32_t kx0[kHalfKeys], kx1[kHalfKeys], kwp[kHalfKeys];
-#pragma unroll
-        for (int pq = 0; pq < kHalfKeys / 2; ++pq) {
-          uint32_t a0[2], a1[2], aw2[2];
-          phi_pair_words2<LIN>(zw[half * (kHalfKeys / 2) + pq], P.g, a0, a1, aw2);   // rows past N read z = 0; their accumulator rows are never stored
-          kx0[2 * pq] = a0[0]; kx1[2 * pq] = a1[0]; kwp[2 * pq] = aw2[0];
-          kx0[2 * pq + 1] = a0[1]; kx1[2 * pq + 1] = a1[1]; kwp[2 * pq + 1] = aw2[1];
-        }
-#pragma unroll
-        for (int qq = 0; qq < NSTH; ++qq) {
-          const uint32_t x0 = kx0[qq], x1 = kx1[qq], wp = kwp[qq];
-          const uint32_t pos = srow_biased + (wp << 7);
-          sts32(pos, x0);
-          sts32(pos + 128u, x1);
-#pragma unroll
-          for (int i = 0; i < HLP; ++i)
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(WP[qq >> 1][(qq & 1) * HLP + i]) : "r"(srow + (uint32_t)i * 128u) : "memory");
-          sts32(pos, 0u);
-          sts32(pos + 128u, 0u);
-        }
-#pragma unroll
-        for (int qq = NSTH; qq < kHalfKeys; ++qq) {
-          const uint32_t x0 = kx0[qq], x1 = kx1[qq], wp = kwp[qq];
-          // Placement at word-pair granularity: wp = 2 * qd + s.  The two words land in pair qd as
-          // (x0, x1) when s = 0, or as (0, x0) there and (x1, 0) in pair qd + 1 when s = 1.
-          uint32_t* W = &WP[qq >> 1][(qq & 1) * HLP];
-          const bool odd = (wp & 1u) != 0u;
-          const uint32_t y0 = odd ? 0u : x0, y1 = odd ? x0 : x1, y2 = odd ? x1 : 0u;
-          constexpr int kLastPair = (HL - (LIN ? 1 : 2)) >> 1;   // largest qd: bin <= L - 3 (linear: L - 2)
-          // Each word is its value times a 0/1 mask in packed f16 arithmetic (x * 1 and x * 0 are exact
-          // for the non-negative finite weights, and at most one term of a sum is non-zero), so the
-          // placement runs on the FMA pipe instead of compare/select chains on the busier ALU pipe.
-          // wp >> 1 is (kKnotBias >> 2) + qd with qd < 64; times 0x10001 that is the f16 pair with bit
-          // patterns qd (low: a subnormal, or zero) and (kKnotBias >> 18) + qd (high): distinct per qd.
-          // f16 comparisons do not flush subnormals (this file is not built with a flush-to-zero flag).
-          const uint32_t q2 = (wp >> 1) * 0x00010001u;
-          const __half2 qh = *reinterpret_cast<const __half2*>(&q2);
-          const __half2 h0 = *reinterpret_cast<const __half2*>(&y0), h1 = *reinterpret_cast<const __half2*>(&y1),
-                        h2 = *reinterpret_cast<const __half2*>(&y2);
-          __half2 m[HLP / 2];
-#pragma unroll
-          for (int i = 0; i < HLP / 2; ++i) {
-            const uint32_t ci2 = (((kKnotBias >> 18) + (uint32_t)i) << 16) | (uint32_t)i;
-            m[i] = i <= kLastPair ? __heq2(qh, *reinterpret_cast<const __half2*>(&ci2)) : __float2half2_rn(0.0f);
-          }
-#pragma unroll
-          for (int i = 0; i < HLP / 2; ++i) {
-            __half2 e = __hmul2(m[i], h0);
-            if (i > 0) e = __hfma2(m[i - 1], h2, e);
-            const __half2 o = __hmul2(m[i], h1);
-            W[2 * i] = *reinterpret_cast<const uint32_t*>(&e);
-            W[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&o);
-          }
-          if ((qq & 1) && (qq & ~1) >= NSTH)            // a pair of mask-placed keys is complete
-            tmem_st_words<2 * HLP>(lane_addr + (uint32_t)((half * kHalfKeys + (qq & ~1)) * HLP), WP[qq >> 1]);
-        }
-        // (All four keys in one 32- and one 16-column store was slower: 0.909 against 0.890 ms.)
-#pragma unroll
-        for (int pp = 0; 2 * pp < NSTH; ++pp)            // pairs with a staged key: their loads have landed by now
-          tmem_st_words<2 * HLP>(lane_addr + (uint32_t)((half * kHalfKeys + 2 * pp) * HLP), WP[pp]);
+        tmem_st_words<kHalfWords>(lane_addr + (uint32_t)(half * kHalfWords), W);
+        tmem_st_words<kHalfSteps>(lane_addr + (uint32_t)(kChunkKeys * F + half * kMeta), meta);
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive_warp(full + grp * 2 + half);
@@ -239,7 +249,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
     mbar_wait(done + grp, 0, wc);
     tc_fence_after();
     float* prow = P.partial + ((size_t)blockIdx.y * P.N + (valid ? n : 0)) * r;
-    const uint32_t daddr = lane_addr + (uint32_t)(kChunkKeys * HLP);
+    const uint32_t daddr = lane_addr + (uint32_t)(kChunkKeys * F + 2 * kMeta);
     for (int c0 = 0; c0 < r; c0 += 16) {
       float v[16];
       tmem_ld16(daddr + c0, v);
@@ -255,11 +265,12 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
     // (one thread cannot issue N = r MMAs faster than about one per 45 cycles)
     if (elect_one()) {
       const int grp = warp - 4 * GROUPS;
-      const uint32_t idesc = instr_desc(0, 0, 0, 1, 128, r);
+      const uint32_t idesc = instr_desc(0, 0, 0, 1, 128, r) | kSparse;
       const uint32_t b_hi = desc_hi(P.b_sbo);
-      const uint32_t b_step = (2u * (uint32_t)(r / 8) * 128u) >> 4;          // per K=16 step
+      const uint32_t b_step = (4u * (uint32_t)(r / 8) * 128u) >> 4;          // per K=32 step
       const uint32_t a_addr0 = tmem_base + (uint32_t)grp * grp_cols;
-      const uint32_t d_addr = a_addr0 + (uint32_t)(kChunkKeys * HLP);
+      const uint32_t m_addr0 = a_addr0 + (uint32_t)(kChunkKeys * F);
+      const uint32_t d_addr = m_addr0 + (uint32_t)(2 * kMeta);
       for (int ci = 0; ci < nch; ++ci) {
         const int cs = ci % CS;
         bool drain = mbar_wait(cfull + cs, (uint32_t)(ci / CS) & 1u, wc);
@@ -271,8 +282,9 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
           if (drain) break;                          // draining: issue nothing more
           tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < kHalfSteps; ++ks) {     // 8 columns of A (16 K elements) per step
-            umma_f16_ta(d_addr, a_addr, b_lo, b_hi, idesc, (ci > 0 || half > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < kHalfSteps; ++ks) {     // 8 columns of A (16 kept of 32 K elements) per step
+            umma_f16_sparse_ta(d_addr, a_addr, b_lo, b_hi, m_addr0 + (uint32_t)(half * kMeta + (ks & ~1)),
+                               idesc | (uint32_t)(ks & 1), (ci > 0 || half > 0 || ks > 0) ? 1u : 0u);
             a_addr += 8u;
             b_lo += b_step;
           }
@@ -310,27 +322,25 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_ta_kernel(con
   }
 }
 
-template <int G, int HL, int ACT, bool LIN>
+template <int G, int F, int ACT, bool LIN>
 cudaError_t fwd_launch_one(const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-  constexpr int hlp = (HL + 1) & ~1;
-  if constexpr (G * (kChunkKeys * hlp + 16) <= 512)
-    return launch_chained<tc_forward_ta_kernel<G, HL, ACT, LIN>>(grid, 160 * G + 32, smem, stream, P);
+  if constexpr (G * (kChunkKeys * F + 2 * fwd_meta_cols(F) + 16) <= 512)
+    return launch_chained<tc_forward_kernel<G, F, ACT, LIN>>(grid, 160 * G + 32, smem, stream, P);
   else
     return cudaErrorInvalidValue;
 }
 
 template <int ACT, bool LIN>
-cudaError_t fwd_launch(int groups, int words, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-#define SKV_FWD_WORDS(HL_)                                                              \
-  if (words == HL_) {                                                                   \
-    if (groups == 4) return fwd_launch_one<4, HL_, ACT, LIN>(P, grid, smem, stream);    \
-    if (groups == 3) return fwd_launch_one<3, HL_, ACT, LIN>(P, grid, smem, stream);    \
-    if (groups == 2) return fwd_launch_one<2, HL_, ACT, LIN>(P, grid, smem, stream);    \
-    return fwd_launch_one<1, HL_, ACT, LIN>(P, grid, smem, stream);                     \
+cudaError_t fwd_launch(int groups, int fold, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
+#define SKV_FWD_FOLD(F_)                                                               \
+  if (fold == F_) {                                                                    \
+    if (groups == 4) return fwd_launch_one<4, F_, ACT, LIN>(P, grid, smem, stream);    \
+    if (groups == 3) return fwd_launch_one<3, F_, ACT, LIN>(P, grid, smem, stream);    \
+    if (groups == 2) return fwd_launch_one<2, F_, ACT, LIN>(P, grid, smem, stream);    \
+    return fwd_launch_one<1, F_, ACT, LIN>(P, grid, smem, stream);                     \
   }
-  SKV_FWD_WORDS(4) SKV_FWD_WORDS(6) SKV_FWD_WORDS(8) SKV_FWD_WORDS(11) SKV_FWD_WORDS(12)
-  SKV_FWD_WORDS(16) SKV_FWD_WORDS(21) SKV_FWD_WORDS(22) SKV_FWD_WORDS(32)
-#undef SKV_FWD_WORDS
+  SKV_FWD_FOLD(4) SKV_FWD_FOLD(6) SKV_FWD_FOLD(8) SKV_FWD_FOLD(10) SKV_FWD_FOLD(12) SKV_FWD_FOLD(18)
+#undef SKV_FWD_FOLD
   return cudaErrorInvalidValue;
 }
 

@@ -3,8 +3,8 @@
 
 namespace skv {
 namespace tc {
-cudaError_t fwd_launch_lin_other(int groups, int words, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-  return fwd_launch<-1, true>(groups, words, P, grid, smem, stream);
+cudaError_t fwd_launch_lin_other(int groups, int fold, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
+  return fwd_launch<-1, true>(groups, fold, P, grid, smem, stream);
 }
 }  // namespace tc
 }  // namespace skv

@@ -126,7 +126,9 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
       if ((int)j < P.h && left > 0) {
         const __nv_bfloat16* base = P.C + (size_t)j * P.L * P.r + c;
         if (!is_t) {
-          if (b < P.L) o = scaled_h8(ld8(base + (size_t)b * P.r, left, cvec), scale);
+          // group f = b / 4 holds knot rows 2f, 2f + 1 and 2(f + F - 1), 2(f + F - 1) + 1, F = LP / 4 groups
+          const int kr = 2 * (b >> 2) + (b & 1) + ((b & 2) ? LP / 2 - 2 : 0);
+          if (kr < P.L) o = scaled_h8(ld8(base + (size_t)kr * P.r, left, cvec), scale);
         } else if (b < P.L - 1) {
           // b = 0: C[1] - C[0]; b > 0: C[b-1] - 2 C[b] + C[b+1]
           const uint4 v0 = ld8(base + (size_t)(b > 0 ? b - 1 : 0) * P.r, left, cvec);

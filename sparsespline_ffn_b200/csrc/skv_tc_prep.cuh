@@ -41,7 +41,7 @@ struct CopyJob {
 struct PrepParams {
   const __nv_bfloat16* C;
   int h, hp, L, r, rp;
-  int lpc;                   // rows per key of the code-table image, 0: none wanted
+  int lpc;                   // rows per key of the code-table image (4 per group of the forward's order), 0: none wanted
   __half* cimg;
   int lpt;                   // rows per key of the transformed-table image, 0: none wanted
   __half* timg;
