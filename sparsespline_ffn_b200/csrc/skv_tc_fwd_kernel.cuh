@@ -72,11 +72,9 @@ inline int fwd_max_groups(int F, int r) {
 // Keys of each half chunk (of four) whose words are placed through a staging row in shared memory: two stores at the
 // dynamic position, F loads, two clearing stores.  The rows of a warp are interleaved by lane, so the bank of
 // every access is the lane and nothing conflicts, whatever the knot intervals are.  The other keys are placed by 0/1 masks in
-// packed f16 arithmetic.
-#ifndef SKV_NSTH
-#define SKV_NSTH 1
-#endif
-constexpr int kStagedPerHalf = SKV_NSTH;
+// packed f16 arithmetic.  0 / 1 / 2 / 4 staged keys: 0.823 / 0.801 / 0.824 / 0.925 ms at the d20 shape (0.876 with a dense
+// A); with all four the load/store data path is 87 % busy.
+constexpr int kStagedPerHalf = 1;
 
 template <int GROUPS, int F, int ACT, bool LIN>
 __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const FwdParams P) {
