@@ -54,7 +54,7 @@ int resolve(const skv_problem& p) {
   if (p.impl == SKV_IMPL_SIMT) return SKV_IMPL_SIMT;
   const bool ok = tc_eligible(p);
   if (p.impl == SKV_IMPL_TCGEN05) return ok ? (int)SKV_IMPL_TCGEN05 : (int)SKV_ERR_UNSUPPORTED;
-  return ok ? (int)SKV_IMPL_TCGEN05 : (int)SKV_IMPL_SIMT;
+  return ok && tc_worthwhile(p) ? (int)SKV_IMPL_TCGEN05 : (int)SKV_IMPL_SIMT;
 }
 
 // Compute capability and SM count of the current device, cached per device ordinal.

@@ -1,4 +1,5 @@
 // Entry points of the tcgen05 kernel family as seen by the C ABI.
+#include "skv_tc_prep.cuh"
 #include "skv_tma.cuh"
 
 namespace skv {
@@ -37,6 +38,10 @@ bool make_map_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols,
 }  // namespace tc
 
 bool tc_eligible(const skv_problem& p) { return tc::bwd_eligible(p); }
+
+// Split operands double the work, and half a tile of tokens or less leaves most of it to padding; the CUDA-core kernels
+// are as fast there.
+bool tc_worthwhile(const skv_problem& p) { return p.N > 64 || !tc::split_operands(p); }
 
 size_t tc_scratch_bytes(const skv_problem& p, int op, bool rows_ok) {
   return op == SKV_OP_FORWARD ? tc::fwd_scratch_bytes(p, rows_ok) : tc::bwd_scratch_bytes(p, rows_ok);

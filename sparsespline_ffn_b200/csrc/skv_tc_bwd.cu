@@ -14,7 +14,7 @@ namespace tc {
 bool fwd_eligible(const skv_problem& p);
 cudaError_t dz_launch_quad(const DzPlan&, int L, bool relu, const DzParams&, dim3, cudaStream_t);
 cudaError_t dz_launch_lin(const DzPlan&, int L, bool relu, const DzParams&, dim3, cudaStream_t);
-cudaError_t dc_launch(const DcPlan&, bool lin, const DcParams&, dim3, cudaStream_t);
+cudaError_t dc_launch(const DcPlan&, bool lin, bool split, const DcParams&, dim3, cudaStream_t);
 
 namespace {
 
@@ -36,6 +36,7 @@ Split best_split(int64_t tiles, int64_t units, int64_t most, double unit, double
 
 bool make_dz_plan(const skv_problem& p, DzPlan* o) {
   const int lb = (p.L - 1 + 7) / 8, rp = padded_r(p);    // 8-column blocks per key; columns L-1.. are padding
+  const int parts = split_operands(p) ? 2 : 1;
   if (lb < 1 || lb > 8) return false;
   o->lb = lb;
   // two token groups where their rows, g and the table ring fit shared memory
@@ -47,7 +48,7 @@ bool make_dz_plan(const skv_problem& p, DzPlan* o) {
         o->rstages = rs;
         o->tstages = ts;
         o->smem = 1024 + (size_t)groups * rs * 2 * kBoxBytes + (size_t)groups * 128 * rp * 2 +
-                  (size_t)ts * kChunkKeys * 8 * lb * rp * 2 + 512;
+                  (size_t)ts * kChunkKeys * 8 * lb * rp * parts * 2 + 512;
         fits = o->smem <= kSmemLimit;
       }
   if (!fits) return false;
@@ -89,7 +90,7 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     o->tiles_total = ((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens;
     // 0.38 us per tile and chunk of 16 keys at L = 22, r = 32, and the wait for a tile's g; a
     // CTA's prologue and epilogue; a split's partials written and read again through L2 or HBM
-    const double unit = 0.38 * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
+    const double unit = 0.38 * (split_operands(p) ? 1.6 : 1.0) * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
     const double per_split = (double)hp * p.L * rp * 8.0 / 5.0e6;
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
@@ -112,17 +113,17 @@ struct BwdPlan { bool ok; DzPlan dz; DcPlan dc; };
 
 // The plans of the last problem this thread asked about: a call asks several times (eligibility, scratch, launch).
 const BwdPlan& plan_backward(const skv_problem& p) {
-  static thread_local struct { int64_t N; int h, L, r; BwdPlan b; } last{-1, 0, 0, 0, {}};
-  if (last.N != p.N || last.h != p.h || last.L != p.L || last.r != p.r) {
+  static thread_local struct { int64_t N; int h, L, r, order; BwdPlan b; } last{-1, 0, 0, 0, 0, {}};
+  if (last.N != p.N || last.h != p.h || last.L != p.L || last.r != p.r || last.order != p.spline_order) {
     BwdPlan b{};
     b.ok = make_dz_plan(p, &b.dz) && make_dc_plan(p, &b.dc);
-    last = {p.N, p.h, p.L, p.r, b};
+    last = {p.N, p.h, p.L, p.r, p.spline_order, b};
   }
   return last.b;
 }
 
 size_t timg_bytes(const skv_problem& p) {
-  return align256((size_t)padded_h(p) * 8 * ((p.L - 1 + 7) / 8) * padded_r(p) * sizeof(__half));
+  return align256((size_t)padded_h(p) * 8 * ((p.L - 1 + 7) / 8) * padded_r(p) * sizeof(__half)) * (split_operands(p) ? 2 : 1);
 }
 
 int64_t gimg_tiles(const skv_problem& p) { return ((p.N > 0 ? p.N : 1) + 255) / 256 * 2; }
@@ -152,7 +153,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
              bool rows_ok) {
   const skv_problem& p = c.p;
   const BwdPlan& b = plan_backward(p);
-  const bool want_dC = dC || dC_cast, lin = c.g.order == 1;
+  const bool want_dC = dC || dC_cast, lin = c.g.order == 1, split = split_operands(p);
   const int hp = padded_h(p), rp = padded_r(p);
   uint8_t* base = static_cast<uint8_t*>(scratch);
   uint32_t* hdr = reinterpret_cast<uint32_t*>(base);
@@ -169,6 +170,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Q.h = p.h; Q.hp = hp; Q.L = p.L; Q.r = p.r; Q.rp = rp;
   if (dz) {
     Q.lpt = 8 * b.dz.lb;
+    Q.tparts = split ? 2 : 1;
     Q.timg = timg;
   }
   Q.g = static_cast<const __nv_bfloat16*>(g_delta);
@@ -196,7 +198,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
     }
   }
   FusedPlan fp;
-  const bool fused = fused_backward_roles() && rows_ok && dz && want_dC && plan_fused(p, &fp);
+  const bool fused = fused_backward_roles() && rows_ok && !split && dz && want_dC && plan_fused(p, &fp);
   if (fused) {                                           // C and g one after the other, as it has always run
     PrepParams G = Q;
     G.lpt = 0;
@@ -226,6 +228,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Z.chunks_per_split = b.dz.chunks_per_split;
   Z.tstages = b.dz.tstages;
   Z.rstages = b.dz.rstages;
+  Z.tparts = split ? 2 : 1;
   Z.dz_f32 = p.dz_f32;
   Z.wait_cycles = wait_cycle_limit();
   Z.status = c.status;
@@ -265,7 +268,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.tiles_total = b.dc.tiles_total;
       P.status = c.status;
       P.wait_cycles = wait_cycle_limit();
-      if (dc_launch(b.dc, lin, P, dim3((unsigned)b.dc.slabs, (unsigned)b.dc.splits), c.stream) != cudaSuccess) {
+      if (dc_launch(b.dc, lin, split, P, dim3((unsigned)b.dc.slabs, (unsigned)b.dc.splits), c.stream) != cudaSuccess) {
         cudaGetLastError();
         return SKV_ERR_LAUNCH;
       }

@@ -278,6 +278,11 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
+// What rounding (a, b) to the f16 pair `w` left over, as an f16 pair.
+__device__ __forceinline__ uint32_t rest_h2(uint32_t w, float a, float b) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pack_h2(a - f.x, b - f.y);
+}
 __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -329,9 +334,10 @@ __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-template <bool LIN>
+// SPLIT: r0, r1 receive the same words of the weights' remainders after rounding to f16.
+template <bool LIN, bool SPLIT = false>
 __device__ __forceinline__ void phi_pair_words2(uint32_t zw, const GridParams& g, uint32_t (&x0)[2], uint32_t (&x1)[2],
-                                                uint32_t (&wp)[2]) {
+                                                uint32_t (&wp)[2], uint32_t* r0 = nullptr, uint32_t* r1 = nullptr) {
   unsigned long long v, u2, t2, tau2, omt2, b0, b2, b1;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(f2_pack(bf_lo(zw), bf_hi(zw))), "l"(f2_pack(g.lo, g.lo)));
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(u2) : "l"(v), "l"(f2_pack(g.scale, g.scale)), "l"(0ull));
@@ -374,6 +380,14 @@ __device__ __forceinline__ void phi_pair_words2(uint32_t zw, const GridParams& g
   x0[1] = p01b << shb;
   x1[1] = __funnelshift_l(p01b, p2b, shb);
   wp[1] = tbb >> 1;
+  if constexpr (SPLIT) {
+    const uint32_t q01a = rest_h2(p01a, B0a, B1a), q2a = rest_h2(p2a, B2a, 0.0f);
+    const uint32_t q01b = rest_h2(p01b, B0b, B1b), q2b = rest_h2(p2b, B2b, 0.0f);
+    r0[0] = q01a << sha;
+    r1[0] = __funnelshift_l(q01a, q2a, sha);
+    r0[1] = q01b << shb;
+    r1[1] = __funnelshift_l(q01b, q2b, shb);
+  }
 }
 
 // Store N consecutive 32-bit columns of this thread's tensor-memory lane (lane = 32 * (warp % 4) + lane id).
@@ -412,10 +426,11 @@ template <> __device__ __forceinline__ void tmem_st<32>(uint32_t taddr, const ui
       "r"(w[28]), "r"(w[29]), "r"(w[30]), "r"(w[31])
       : "memory");
 }
-// HL (< 64) consecutive columns as the binary decomposition of HL into x16/x8/x4/x2/x1 stores.
+// HL (< 96) consecutive columns as the binary decomposition of HL into x16/x8/x4/x2/x1 stores.
 template <int HL> __device__ __forceinline__ void tmem_st_words(uint32_t taddr, const uint32_t* w) {
   int o = 0;
-  if constexpr ((HL & 32) != 0) { tmem_st<32>(taddr, w); o += 32; }
+  if constexpr (HL >= 64) { tmem_st<32>(taddr, w); tmem_st<32>(taddr + 32, w + 32); o += 64; }
+  if constexpr ((HL & 32) != 0) { tmem_st<32>(taddr + o, w + o); o += 32; }
   if constexpr ((HL & 16) != 0) { tmem_st<16>(taddr + o, w + o); o += 16; }
   if constexpr ((HL & 8) != 0) { tmem_st<8>(taddr + o, w + o); o += 8; }
   if constexpr ((HL & 4) != 0) { tmem_st<4>(taddr + o, w + o); o += 4; }

@@ -47,8 +47,9 @@ constexpr int kDcIssuers = 3;                        // warps that issue MMAs, e
 // One unit behind a stage: the linear spline's last interval stores a zero word there.
 __host__ __device__ constexpr uint32_t dc_stage_bytes(int mtiles) { return (uint32_t)mtiles * 16u * kDcUnit + kDcUnit; }
 
-// KJ = keys per lane and token (a chunk is 4 * KJ keys), GW = warps per producer group.
-template <int KJ, int GW, bool LIN>
+// KJ = keys per lane and token (a chunk is 4 * KJ keys), GW = warps per producer group.  SPLIT: a stage is filled twice, with
+// the weights and with their remainders at the same places.
+template <int KJ, int GW, bool LIN, bool SPLIT>
 __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int KCH = 4 * KJ;
@@ -138,13 +139,13 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
     load_z(pg, 0, znext);
     int ti = pg, ch = 0;
     for (int use = 0; ti < ntiles; ++use) {
-      uint32_t x0[TI][KJ], x1[TI][KJ], ad[TI][KJ];
+      uint32_t x0[TI][KJ], x1[TI][KJ], ad[TI][KJ], r0[SPLIT ? TI : 1][KJ], r1[SPLIT ? TI : 1][KJ];
 #pragma unroll
       for (int i = 0; i < TI; ++i)
 #pragma unroll
         for (int q = 0; q < KJ / 2; ++q) {
           uint32_t a0[2], a1[2], wp[2];
-          phi_pair_words2<LIN>(znext[i][q], P.g, a0, a1, wp);
+          phi_pair_words2<LIN, SPLIT>(znext[i][q], P.g, a0, a1, wp, &r0[SPLIT ? i : 0][2 * q], &r1[SPLIT ? i : 0][2 * q]);
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             x0[i][2 * q + e] = a0[e];
@@ -175,6 +176,19 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
         }
       fence_async_smem();
       mbar_arrive_warp(pfull + pg);
+      if constexpr (SPLIT) {
+        ++use;
+        mbar_wait(pempty + pg, (uint32_t)(use - 1) & 1u, wc);
+#pragma unroll
+        for (int i = 0; i < TI; ++i)
+#pragma unroll
+          for (int j = 0; j < KJ; ++j) {
+            sts32(ad[i][j], r0[i][j]);
+            sts32(ad[i][j] + kDcUnit, r1[i][j]);
+          }
+        fence_async_smem();
+        mbar_arrive_warp(pfull + pg);
+      }
     }
     // ---- epilogue: accumulators -> float32 partial of this token split
     mbar_wait(done, 0, wc);
@@ -214,18 +228,21 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
       bool drain = false;
       for (int tp = 0; tp < ntiles && !drain; tp += NG) {
         const int npg = min(NG, ntiles - tp);
-        for (int ch = 0; ch < nchunks && !drain; ++ch, ++fills) {
+        constexpr int kParts = SPLIT ? 2 : 1;
+        for (int cp = 0; cp < nchunks * kParts && !drain; ++cp, ++fills) {
+          const int ch = cp / kParts, part = cp % kParts;
+          const bool last = cp + 1 == nchunks * kParts;
           int slot = slot0;
           uint32_t gpar = gpar0;
           for (int pg = 0; pg < npg; ++pg) {
-            if (ch == 0) drain = drain || mbar_wait(gfull + slot, gpar, wc);
+            if (cp == 0) drain = drain || mbar_wait(gfull + slot, gpar, wc);
             drain = drain || mbar_wait(pfull + pg, fills & 1u, wc);
             if (drain) break;                          // draining: issue nothing more
             tc_fence_after();
             uint32_t a_lo0 = a_tile0 + (uint32_t)pg * (phi_bytes >> 4);
             const uint32_t b_lo0 = b_ring + (uint32_t)slot * (g_bytes >> 4);
             uint32_t d_addr = tmem_base + (uint32_t)((ch * P.mtiles + m0) * r);
-            const uint32_t first = tp + pg == 0 ? 0u : 1u;
+            const uint32_t first = tp + pg + part == 0 ? 0u : 1u;
             for (int mt = m0; mt < P.mtiles; mt += kDcIssuers) {
 #pragma unroll
               for (int ks = 0; ks < kDcTokens / 16; ++ks)
@@ -235,10 +252,10 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
               d_addr += (uint32_t)(kDcIssuers * r);
             }
             umma_commit(pempty + pg);
-            if (ch + 1 == nchunks) umma_commit(gempty + slot);
+            if (last) umma_commit(gempty + slot);
             if (++slot == GR) { slot = 0; gpar ^= 1u; }
           }
-          if (ch + 1 == nchunks) { slot0 = slot; gpar0 = gpar; }
+          if (last) { slot0 = slot; gpar0 = gpar; }
         }
       }
       umma_commit(done);

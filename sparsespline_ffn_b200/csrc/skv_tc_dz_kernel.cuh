@@ -34,6 +34,7 @@ struct DzParams {
   float coef;                // lambda * scale
   int chunks_total, chunks_per_split;
   int tstages;               // depth of the transformed-table ring (2..kTStages)
+  int tparts;                // f16 parts of the table's values (1 or 2): K runs over tparts * r channels, g repeats
   int rstages;               // boxes of z and g_act per token group (2 or 3)
   int dz_f32;                // dz is float32 [N][dzs] instead of bf16
   int32_t* status;
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
   constexpr int NBLK = kChunkKeys / KB;                              // blocks per chunk
   constexpr bool DB = LB <= 4;                                       // two keys' columns in registers
   const uint32_t g_bytes = (uint32_t)(128 * r * 2);
-  const uint32_t t_bytes = (uint32_t)(kChunkKeys * LP * r * 2);
+  const uint32_t t_bytes = (uint32_t)(kChunkKeys * LP * r * 2 * P.tparts);
   constexpr uint32_t bcols = (uint32_t)(KB * LP);                    // columns of one S block
   uint8_t* g_base = smem;                                             // [group][g_bytes]
   uint8_t* t_base = smem + (size_t)GROUPS * g_bytes;                  // [kTStages][t_bytes]
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
     if (elect_one()) {
       const int grp = warp - 8 * GROUPS;
       mbar_wait(gfull, 0, wc);
-      const uint32_t rb = (uint32_t)(r / 8) * 128u;          // bytes between 8-row groups of the T image
+      const uint32_t rb = (uint32_t)(r * P.tparts / 8) * 128u;   // bytes between 8-row groups of the T image
       const uint32_t a_hi = desc_hi(128u), b_hi = desc_hi(rb);
       constexpr uint32_t idesc = instr_desc(0, 0, 0, 0, 128, (int)bcols);
       const uint32_t a_lo0 = desc_lo(smem_u32(g_base + (size_t)grp * g_bytes), 2048u);
@@ -318,12 +319,15 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
           if (use > 0) drain = drain || mbar_wait(se + (b & 1), (use - 1u) & 1u, wc);
           if (drain) break;                            // draining: issue nothing more
           tc_fence_after();
-          uint32_t a_lo = a_lo0, b_lo = b_blk;
+          uint32_t b_lo = b_blk;
           const uint32_t d_addr = d0 + (uint32_t)(b & 1) * bcols;
-          for (int ks = 0; ks < ksteps; ++ks) {
-            umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, ks > 0 ? 1u : 0u);
-            a_lo += 4096u >> 4;
-            b_lo += 256u >> 4;
+          for (int part = 0; part < P.tparts; ++part) {
+            uint32_t a_lo = a_lo0;
+            for (int ks = 0; ks < ksteps; ++ks) {
+              umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, ks + part > 0 ? 1u : 0u);
+              a_lo += 4096u >> 4;
+              b_lo += 256u >> 4;
+            }
           }
           umma_commit(sf + (b & 1));
           b_blk += ((bcols / 8u) * rb) >> 4;

@@ -7,6 +7,8 @@ namespace tc {
 
 cudaError_t fwd_launch_quad_relu(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
 cudaError_t fwd_launch_quad_other(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
+cudaError_t fwd_launch_split_relu(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
+cudaError_t fwd_launch_split_other(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
 cudaError_t fwd_launch_lin_relu(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
 cudaError_t fwd_launch_lin_other(int, int, const FwdParams&, dim3, size_t, cudaStream_t);
 
@@ -36,7 +38,7 @@ FwdPlan make_plan(const skv_problem& p) {
   if (most < 16) most = 16;
   if (most > (chunks + 3) / 4) most = (chunks + 3) / 4;
   double best = 0.0;
-  for (int g = fwd_max_groups(F, rp); g >= 1; --g) {
+  for (int g = fwd_max_groups(F, rp, split_operands(p)); g >= 1; --g) {
     const size_t stage_bytes = (size_t)128 * g * (F + 1) * 4;
     int cstages = (int)((kSmemLimit - 512 - stage_bytes) / c_bytes);
     if (cstages > kMaxCStages) cstages = kMaxCStages;
@@ -44,7 +46,7 @@ FwdPlan make_plan(const skv_problem& p) {
     const int64_t tiles = (N + 128 * g - 1) / (128 * g);
     // microseconds: a chunk of g groups (instruction issue, or the MMAs of wide r), a CTA's prologue and
     // epilogue, and the partials' way through L2 (measured: 1.3 us per chunk of four groups at L = 22)
-    const double issue = (0.22 + 0.27 * g) * (F + 14) / 20.0, mma = g * F * rp * 0.5 / 1800.0;
+    const double issue = (0.22 + 0.27 * g) * (F + 14) / 20.0 * (split_operands(p) ? 1.4 : 1.0), mma = g * F * rp * 0.5 / 1800.0;
     const double chunk = issue > mma ? issue : mma;
     int last = 0;
     for (int64_t s = 1; s <= most; ++s) {
@@ -69,8 +71,9 @@ FwdPlan make_plan(const skv_problem& p) {
 
 // The plan of the last problem this thread asked about: a call asks several times (scratch size, launch).
 const FwdPlan& plan_forward(const skv_problem& p) {
-  static thread_local struct { int64_t N; int h, L, r; FwdPlan f; } last{-1, 0, 0, 0, {}};
-  if (last.N != p.N || last.h != p.h || last.L != p.L || last.r != p.r) last = {p.N, p.h, p.L, p.r, make_plan(p)};
+  static thread_local struct { int64_t N; int h, L, r, order; FwdPlan f; } last{-1, 0, 0, 0, 0, {}};
+  if (last.N != p.N || last.h != p.h || last.L != p.L || last.r != p.r || last.order != p.spline_order)
+    last = {p.N, p.h, p.L, p.r, p.spline_order, make_plan(p)};
   return last.f;
 }
 
@@ -82,7 +85,7 @@ size_t fwd_copy_bytes(const skv_problem& p) { return align256((size_t)(p.N > 0 ?
 bool fwd_eligible(const skv_problem& p) {
   if (p.dtype != SKV_BF16 || p.r > 128 || p.L < 4 || p.L > 64) return false;
   const int F = fwd_fold(p.L), rp = padded_r(p);
-  return fwd_max_groups(F, rp) >= 1 &&
+  return fwd_max_groups(F, rp, split_operands(p)) >= 1 &&
          2 * (size_t)kChunkKeys * 4 * F * rp * 2 + (size_t)128 * (F + 1) * 4 + 512 <= kSmemLimit;
 }
 
@@ -143,8 +146,9 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
   P.b_sbo = 128;
   const dim3 grid((unsigned)((p.N + 128 * f.groups - 1) / (128 * f.groups)), (unsigned)f.splits);
   const bool lin = c.g.order == 1, relu = p.activation == SKV_ACT_RELU_SQ;
-  auto* launch = lin ? (relu ? fwd_launch_lin_relu : fwd_launch_lin_other)
-                     : (relu ? fwd_launch_quad_relu : fwd_launch_quad_other);
+  auto* launch = lin                 ? (relu ? fwd_launch_lin_relu : fwd_launch_lin_other)
+                 : split_operands(p) ? (relu ? fwd_launch_split_relu : fwd_launch_split_other)
+                                     : (relu ? fwd_launch_quad_relu : fwd_launch_quad_other);
   if (launch(f.groups, f.fold, P, grid, f.smem, c.stream) != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
   note_launches(1);
   return launch_finalize(partial, f.splits, p.N, p.r, rp, p.lambda_scale, hdr, delta_out, ds, p.delta_f32 != 0, c.stream);

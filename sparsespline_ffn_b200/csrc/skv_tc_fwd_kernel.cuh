@@ -45,8 +45,8 @@ inline int fwd_fold(int L) {
 }
 // Tensor-memory columns of a token group: Phi of 8 keys, its metadata in two halves, the accumulator.
 __host__ __device__ constexpr int fwd_meta_cols(int F) { return (F / 2 + 1) & ~1; }
-inline int fwd_max_groups(int F, int r) {
-  const int g = 512 / (kChunkKeys * F + 2 * fwd_meta_cols(F) + r);
+inline int fwd_max_groups(int F, int r, bool split) {
+  const int g = 512 / (kChunkKeys * F * (split ? 2 : 1) + 2 * fwd_meta_cols(F) + r);
   return g > 4 ? 4 : g;
 }
 
@@ -76,14 +76,16 @@ inline int fwd_max_groups(int F, int r) {
 // A); with all four the load/store data path is 87 % busy.
 constexpr int kStagedPerHalf = 1;
 
-template <int GROUPS, int F, int ACT, bool LIN>
+// SPLIT: the weights' remainders follow the weights, in columns of their own and with the same metadata.
+template <int GROUPS, int F, int ACT, bool LIN, bool SPLIT>
 __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const FwdParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kHalfKeys = kChunkKeys / 2;
   constexpr int kHalfWords = kHalfKeys * F;                        // words of A per half chunk
   constexpr int kHalfSteps = kHalfWords / 8;                       // MMAs (K = 32 rows of the table) per half chunk
   constexpr int kMeta = fwd_meta_cols(F);
-  constexpr int NSTH = kStagedPerHalf;
+  constexpr int kParts = SPLIT ? 2 : 1;
+  constexpr int NSTH = SPLIT ? 0 : kStagedPerHalf;
   constexpr int SW = F + 1;                                        // staging words per thread (one spare, see LIN)
   const int r = P.r;
   const uint32_t c_bytes = (uint32_t)(kChunkKeys * 4 * F * r * 2);
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
   const int chunk_begin = blockIdx.y * P.chunks_per_split;
   const int nch = min(P.chunks_per_split, P.chunks_total - chunk_begin);
   const int64_t tile_base = (int64_t)blockIdx.x * (128 * GROUPS);
-  const uint32_t grp_cols = (uint32_t)(kChunkKeys * F + 2 * kMeta + r);
+  const uint32_t grp_cols = (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta + r);
   uint32_t tmem_cols = 32;
   while (tmem_cols < GROUPS * grp_cols) tmem_cols <<= 1;
 
@@ -160,13 +162,13 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
         uint32_t meta[kHalfSteps];
 #pragma unroll
         for (int j = 0; j < kHalfSteps; ++j) meta[j] = 0x44444444u;
-        uint32_t x0[kHalfKeys], x1[kHalfKeys], wp[kHalfKeys];
+        uint32_t x0[kHalfKeys], x1[kHalfKeys], wp[kHalfKeys], r0[kHalfKeys], r1[kHalfKeys];
 #pragma unroll
         for (int pq = 0; pq < kHalfKeys / 2; ++pq) {
           // knot interval and weights, two keys (one packed z word) at a time; rows past N read z = 0 and their
           // accumulator rows are never stored
           uint32_t a0[2], a1[2], aw2[2];
-          phi_pair_words2<LIN>(zw[half * (kHalfKeys / 2) + pq], P.g, a0, a1, aw2);
+          phi_pair_words2<LIN, SPLIT>(zw[half * (kHalfKeys / 2) + pq], P.g, a0, a1, aw2, r0 + 2 * pq, r1 + 2 * pq);
 #pragma unroll
           for (int e = 0; e < 2; ++e) { x0[2 * pq + e] = a0[e]; x1[2 * pq + e] = a1[e]; wp[2 * pq + e] = aw2[e]; }
         }
@@ -194,16 +196,15 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
             sts32(pos + 128u, 0u);
           }
         }
-#pragma unroll
-        for (int q = NSTH; q < kHalfKeys; ++q) {
+        auto place = [&](int q, uint32_t v0, uint32_t v1) {
           // Placement at word-pair granularity: the word index is 2 * qd + s.  The two words land in pair qd as
-          // (x0, x1) when s = 0, or as (0, x0) there and (x1, 0) in pair qd + 1 when s = 1.  Each word is its value times
-          // a 0/1 mask in packed f16 arithmetic (x * 1 and x * 0 are exact for the non-negative finite weights, and at
+          // (v0, v1) when s = 0, or as (0, v0) there and (v1, 0) in pair qd + 1 when s = 1.  Each word is its value times
+          // a 0/1 mask in packed f16 arithmetic (x * 1 and x * 0 are exact for finite weights, and at
           // most one term of a sum is non-zero), which runs on the FMA pipe; compare/select chains would run on the ALU
           // pipe.  The biased index >> 1 times 0x10001 is an f16 pair with bit patterns qd (low: a subnormal, or zero) and
           // (kKnotBias >> 18) + qd (high), distinct per qd; f16 comparisons do not flush subnormals.
           const bool odd = (wp[q] & 1u) != 0u;
-          const uint32_t y0 = odd ? 0u : x0[q], y1 = odd ? x0[q] : x1[q], y2 = odd ? x1[q] : 0u;
+          const uint32_t y0 = odd ? 0u : v0, y1 = odd ? v0 : v1, y2 = odd ? v1 : 0u;
           const uint32_t q2 = (wp[q] >> 1) * 0x00010001u;
           const __half2 qh = *reinterpret_cast<const __half2*>(&q2);
           const __half2 h0 = *reinterpret_cast<const __half2*>(&y0), h1 = *reinterpret_cast<const __half2*>(&y1),
@@ -222,7 +223,9 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
             W[q * F + 2 * i] = *reinterpret_cast<const uint32_t*>(&e);
             W[q * F + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&o);
           }
-        }
+        };
+#pragma unroll
+        for (int q = NSTH; q < kHalfKeys; ++q) place(q, x0[q], x1[q]);
 #pragma unroll
         for (int j = 0; j < kHalfSteps; j += 2) {
           const int j1 = j + 1 < kHalfSteps ? j + 1 : j;
@@ -236,7 +239,12 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
           tc_fence_after();
         }
         tmem_st_words<kHalfWords>(lane_addr + (uint32_t)(half * kHalfWords), W);
-        tmem_st_words<kHalfSteps>(lane_addr + (uint32_t)(kChunkKeys * F + half * kMeta), meta);
+        tmem_st_words<kHalfSteps>(lane_addr + (uint32_t)(kParts * kChunkKeys * F + half * kMeta), meta);
+        if constexpr (SPLIT) {
+#pragma unroll
+          for (int q = 0; q < kHalfKeys; ++q) place(q, r0[q], r1[q]);
+          tmem_st_words<kHalfWords>(lane_addr + (uint32_t)(kChunkKeys * F + half * kHalfWords), W);
+        }
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive_warp(full + grp * 2 + half);
@@ -247,7 +255,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
     mbar_wait(done + grp, 0, wc);
     tc_fence_after();
     float* prow = P.partial + ((size_t)blockIdx.y * P.N + (valid ? n : 0)) * r;
-    const uint32_t daddr = lane_addr + (uint32_t)(kChunkKeys * F + 2 * kMeta);
+    const uint32_t daddr = lane_addr + (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta);
     for (int c0 = 0; c0 < r; c0 += 16) {
       float v[16];
       tmem_ld16(daddr + c0, v);
@@ -267,7 +275,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
       const uint32_t b_hi = desc_hi(P.b_sbo);
       const uint32_t b_step = (4u * (uint32_t)(r / 8) * 128u) >> 4;          // per K=32 step
       const uint32_t a_addr0 = tmem_base + (uint32_t)grp * grp_cols;
-      const uint32_t m_addr0 = a_addr0 + (uint32_t)(kChunkKeys * F);
+      const uint32_t m_addr0 = a_addr0 + (uint32_t)(kParts * kChunkKeys * F);
       const uint32_t d_addr = m_addr0 + (uint32_t)(2 * kMeta);
       for (int ci = 0; ci < nch; ++ci) {
         const int cs = ci % CS;
@@ -281,8 +289,11 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < kHalfSteps; ++ks) {     // 8 columns of A (16 kept of 32 K elements) per step
-            umma_f16_sparse_ta(d_addr, a_addr, b_lo, b_hi, m_addr0 + (uint32_t)(half * kMeta + (ks & ~1)),
-                               idesc | (uint32_t)(ks & 1), (ci > 0 || half > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+            for (int part = 0; part < kParts; ++part)
+              umma_f16_sparse_ta(d_addr, a_addr + (uint32_t)(part * kChunkKeys * F), b_lo, b_hi,
+                                 m_addr0 + (uint32_t)(half * kMeta + (ks & ~1)), idesc | (uint32_t)(ks & 1),
+                                 (ci > 0 || half > 0 || ks > 0 || part > 0) ? 1u : 0u);
             a_addr += 8u;
             b_lo += b_step;
           }
@@ -320,22 +331,22 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
   }
 }
 
-template <int G, int F, int ACT, bool LIN>
+template <int G, int F, int ACT, bool LIN, bool SPLIT>
 cudaError_t fwd_launch_one(const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-  if constexpr (G * (kChunkKeys * F + 2 * fwd_meta_cols(F) + 16) <= 512)
-    return launch_chained<tc_forward_kernel<G, F, ACT, LIN>>(grid, 160 * G + 32, smem, stream, P);
+  if constexpr (G * ((SPLIT ? 2 : 1) * kChunkKeys * F + 2 * fwd_meta_cols(F) + 16) <= 512)
+    return launch_chained<tc_forward_kernel<G, F, ACT, LIN, SPLIT>>(grid, 160 * G + 32, smem, stream, P);
   else
     return cudaErrorInvalidValue;
 }
 
-template <int ACT, bool LIN>
+template <int ACT, bool LIN, bool SPLIT>
 cudaError_t fwd_launch(int groups, int fold, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
 #define SKV_FWD_FOLD(F_)                                                               \
   if (fold == F_) {                                                                    \
-    if (groups == 4) return fwd_launch_one<4, F_, ACT, LIN>(P, grid, smem, stream);    \
-    if (groups == 3) return fwd_launch_one<3, F_, ACT, LIN>(P, grid, smem, stream);    \
-    if (groups == 2) return fwd_launch_one<2, F_, ACT, LIN>(P, grid, smem, stream);    \
-    return fwd_launch_one<1, F_, ACT, LIN>(P, grid, smem, stream);                     \
+    if (groups == 4) return fwd_launch_one<4, F_, ACT, LIN, SPLIT>(P, grid, smem, stream);    \
+    if (groups == 3) return fwd_launch_one<3, F_, ACT, LIN, SPLIT>(P, grid, smem, stream);    \
+    if (groups == 2) return fwd_launch_one<2, F_, ACT, LIN, SPLIT>(P, grid, smem, stream);    \
+    return fwd_launch_one<1, F_, ACT, LIN, SPLIT>(P, grid, smem, stream);                     \
   }
   SKV_FWD_FOLD(4) SKV_FWD_FOLD(6) SKV_FWD_FOLD(8) SKV_FWD_FOLD(10) SKV_FWD_FOLD(12) SKV_FWD_FOLD(18)
 #undef SKV_FWD_FOLD

@@ -4,7 +4,7 @@
 namespace skv {
 namespace tc {
 cudaError_t fwd_launch_lin_other(int groups, int fold, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-  return fwd_launch<-1, true>(groups, fold, P, grid, smem, stream);
+  return fwd_launch<-1, true, true>(groups, fold, P, grid, smem, stream);
 }
 }  // namespace tc
 }  // namespace skv

@@ -4,7 +4,7 @@
 namespace skv {
 namespace tc {
 cudaError_t fwd_launch_lin_relu(int groups, int fold, const FwdParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
-  return fwd_launch<SKV_ACT_RELU_SQ, true>(groups, fold, P, grid, smem, stream);
+  return fwd_launch<SKV_ACT_RELU_SQ, true, true>(groups, fold, P, grid, smem, stream);
 }
 }  // namespace tc
 }  // namespace skv

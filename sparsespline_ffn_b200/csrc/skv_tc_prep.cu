@@ -113,12 +113,16 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
     float scale, inv;
     pow2_scales(combine(P.hdr + kBlockMax, P.scan_c, words), scale, inv);
     const int LP = is_t ? P.lpt : P.lpc;
-    const int64_t pieces = (int64_t)P.hp * LP * cgs;
+    const int cgi = is_t ? cgs * P.tparts : cgs;        // channel groups of the image
+    const int64_t pieces = (int64_t)P.hp * LP * cgi;
     uint4* img = reinterpret_cast<uint4*>(is_t ? P.timg : P.cimg);
 #pragma unroll 2
     for (int64_t e = (int64_t)blk * blockDim.x + threadIdx.x; e < pieces; e += (int64_t)nblk * blockDim.x) {
       const uint32_t core = (uint32_t)(e >> 3);
-      const uint32_t rg = core / (uint32_t)cgs, cg = core - rg * cgs;
+      const uint32_t rg = core / (uint32_t)cgi;
+      uint32_t cg = core - rg * cgi;
+      const bool rest = cg >= (uint32_t)cgs;            // remainders
+      if (rest) cg -= cgs;
       const uint32_t row = rg * 8u + ((uint32_t)e & 7u);
       const uint32_t j = row / (uint32_t)LP;
       const int b = (int)(row - j * LP), c = (int)cg * 8, left = P.r - c;
@@ -137,10 +141,15 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
           const uint32_t a0[4] = {v0.x, v0.y, v0.z, v0.w}, a1[4] = {v1.x, v1.y, v1.z, v1.w}, a2[4] = {v2.x, v2.y, v2.z, v2.w};
           uint32_t w[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            w[i] = b > 0 ? pack_h2(diff2(bf_lo(a0[i]), bf_lo(a1[i]), bf_lo(a2[i]), scale),
-                                   diff2(bf_hi(a0[i]), bf_hi(a1[i]), bf_hi(a2[i]), scale))
-                         : pack_h2((bf_lo(a1[i]) - bf_lo(a0[i])) * scale, (bf_hi(a1[i]) - bf_hi(a0[i])) * scale);
+          for (int i = 0; i < 4; ++i) {
+            float lo = b > 0 ? diff2(bf_lo(a0[i]), bf_lo(a1[i]), bf_lo(a2[i]), scale) : (bf_lo(a1[i]) - bf_lo(a0[i])) * scale;
+            float hi = b > 0 ? diff2(bf_hi(a0[i]), bf_hi(a1[i]), bf_hi(a2[i]), scale) : (bf_hi(a1[i]) - bf_hi(a0[i])) * scale;
+            if (rest) {
+              lo -= __half2float(__float2half_rn(lo));
+              hi -= __half2float(__float2half_rn(hi));
+            }
+            w[i] = pack_h2(lo, hi);
+          }
           o = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
@@ -285,7 +294,7 @@ int launch_prep(PrepParams& P, cudaStream_t stream) {
   P.scan_c = P.lpc || P.lpt ? blocks_for((int64_t)P.h * P.L * P.r / 8, 8, kPlanSMs * 2) : 0;
   P.scan_g = P.g ? blocks_for(P.N * ((P.r + 7) / 8), 4, kPlanSMs * 2) : 0;
   P.blocks_c = P.lpc ? blocks_for((int64_t)P.hp * P.lpc * cgs, 2, kPlanSMs * 8) : 0;
-  P.blocks_t = P.lpt ? blocks_for((int64_t)P.hp * P.lpt * cgs, 2, kPlanSMs * 8) : 0;
+  P.blocks_t = P.lpt ? blocks_for((int64_t)P.hp * P.lpt * cgs * P.tparts, 2, kPlanSMs * 8) : 0;
   P.blocks_g = P.g ? blocks_for(P.tiles * 128 * cgs, 2, kPlanSMs * 8) : 0;
   P.blocks_copy = 0;
   for (const CopyJob& J : P.copy)

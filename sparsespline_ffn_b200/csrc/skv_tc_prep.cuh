@@ -27,6 +27,14 @@ constexpr int kMaxBlocks = 296;               // scanning blocks per array
 inline int padded_h(const skv_problem& p) { return (p.h + kChunkKeys - 1) / kChunkKeys * kChunkKeys; }
 inline int padded_r(const skv_problem& p) { return (p.r + 15) / 16 * 16; }
 
+// Operands as pairs of f16 (value and remainder), for results as accurate as float32 arithmetic on the same inputs.
+// One f16 per weight is what this family has always given bf16 problems of the plain shapes below; every other problem had
+// the CUDA-core kernels' float32 arithmetic and keeps its accuracy: twice the MMAs, still several times faster
+// (linear spline, 4096 x 1024, r = 32, a training step).
+inline bool split_operands(const skv_problem& p) {
+  return p.spline_order == 1 || p.h % kChunkKeys != 0 || p.r % 16 != 0 || p.L > 49;
+}
+
 inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // One [N][h] bf16 array copied to [N][hp] (pad columns zero); with act_out also phi of it at that pointer.
@@ -44,6 +52,7 @@ struct PrepParams {
   int lpc;                   // rows per key of the code-table image (4 per group of the forward's order), 0: none wanted
   __half* cimg;
   int lpt;                   // rows per key of the transformed-table image, 0: none wanted
+  int tparts;                // f16 parts of its values: 1, or 2 (channels [0, rp) and the remainders in [rp, 2 rp))
   __half* timg;
   const __nv_bfloat16* g;    // null: no gradient image
   int64_t gds, N, tiles;     // tiles of 128 tokens in the image
