@@ -27,8 +27,8 @@ namespace tc {
 bool readout_eligible(const skv_problem& p, int64_t D);
 size_t readout_image_bytes(const skv_problem& p, int64_t D);
 int64_t readout_delta_pitch(const skv_problem& p);
-int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, const void* W, int64_t ws, int64_t D,
-            void* y, int64_t ys, void* wimg);
+int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg);
+int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, int64_t D, void* y, int64_t ys, void* wimg);
 }  // namespace tc
 }  // namespace skv
 
@@ -256,9 +256,10 @@ int skv_feature_readout_forward(const skv_problem* p, const void* z, int64_t z_s
   const int64_t dp = tc::readout_delta_pitch(*p);
   void* wimg = base + fwd_bytes + round256((size_t)p->N * dp * 2);
   if (dp != p->r && cudaMemsetAsync(delta, 0, (size_t)p->N * dp * 2, c.stream) != cudaSuccess) return SKV_ERR_LAUNCH;
+  if (int e = tc::readout_pack(c, w_out, w_stride, d_out, wimg)) return e;
   if (int e = skv_feature_forward(&q, z, z_stride, C, nullptr, 0, delta, dp, scratch, fwd_bytes, status, stream))
     return e;
-  return tc::readout(c, z, z_stride, delta, w_out, w_stride, d_out, y, y_stride, wimg);
+  return tc::readout(c, z, z_stride, delta, d_out, y, y_stride, wimg);
 }
 
 int skv_knot_index(const skv_problem* p, const void* z, int64_t z_stride, int32_t* bins, void* stream) {

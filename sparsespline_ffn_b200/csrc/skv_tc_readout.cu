@@ -9,16 +9,16 @@
 // act(z) nor the concatenated feature is ever written to HBM; delta (bf16, lambda applied) comes from the
 // feature kernel run in its delta-only mode just before.
 //
-// One persistent CTA per SM walks output tiles of 256 tokens x 256 outputs (two 128-row MMAs share each
-// B tile, which halves the L2 traffic per flop of a 128 x 256 tile; all 512 tensor-memory columns hold
-// the two accumulators):
+// One persistent CTA per SM walks output tiles of 256 or 128 tokens x 256 outputs (with 256 two 128-row MMAs share
+// each B tile, which halves the L2 traffic per flop of a 128 x 256 tile; with 128 the two accumulators in tensor
+// memory are of successive tiles), or K slices of them:
 //   warp  9    loader (lane 0): per stage one tiled TMA load of the 256 x 64 z (or delta) tile, 128-byte
 //              swizzle, zero fill past N and h, and one 32 KB bulk copy from the pre-tiled image of W
 //   warps 0-7  ReLU^2 in place on the landed z tile (elementwise, so the swizzled layout does not matter);
 //              nothing to do for the identity activation.  After a tile's last stage the same warps are
 //              its epilogue (accumulator -> bf16 -> y)
 //   warp  8    MMA issue (lane 0): 128 x 256 x 16 per instruction
-// Three stages of (A 32 KB + B 32 KB).  Tiles that share their 256 tokens are adjacent in the walk, so the
+// Three stages of (A 32 KB + B 32 KB), or four of (16 + 32).  Tiles that share their 256 tokens are adjacent in the walk, so the
 // z tile is read from HBM once and from L2 by the other D/256 - 1 CTAs.
 // (Loading the z tile with ordinary 16-byte loads into registers instead cost 37 L1 wavefronts per
 // load instruction and left the kernel bound by the load/store unit at 1.23 ms for the d20 shape,
@@ -29,6 +29,7 @@
 // stores back to shared memory and no A reads from it): 0.72 ms, because a 128 x 256 tile needs 48 KB
 // from L2 per 4.2 MFLOP against 64 KB per 8.4 MFLOP here, and both kernels take in about 90 GB/s per
 // SM, which looks like the limit of the L2-to-SM path.)
+#include "skv_tc_prep.cuh"
 #include "skv_tma.cuh"
 
 namespace skv {
@@ -39,8 +40,9 @@ constexpr int32_t kStatusTimeoutReadout = 0x10;
 namespace {
 
 constexpr int kRoK = 64;                         // K columns per stage: 64 (128-byte swizzle) or 32 (64-byte swizzle)
-constexpr int kRoStages = 192 / kRoK;            // 192 KB of stages
-constexpr uint32_t kRoABytes = 256 * kRoK * 2;   // one A stage: 256 tokens x kRoK
+// Tiles of MT * 128 tokens x 256 outputs, MT = 2 or 1 (see readout_plan).
+__host__ __device__ constexpr uint32_t ro_a_bytes(int mt) { return (uint32_t)mt * 128 * kRoK * 2; }
+__host__ __device__ constexpr int ro_stages(int mt) { return mt == 2 ? 3 : 4; }      // 192 KB of stages
 constexpr uint32_t kRoBBytes = 256 * kRoK * 2;   // one B stage: 256 outputs x kRoK
 constexpr int kRoThreads = 320;
 
@@ -54,6 +56,8 @@ struct RoParams {
   int ks;                        // all stages: ks_z + ceil(r / 32)
   int n_tiles;                   // ceil(D / 256)
   int64_t tiles;                 // m_tiles * n_tiles
+  int slices, ks_per;            // K slices per tile and stages per slice
+  float* partial;                // [slices][N][D] when there is more than one slice
   int32_t* status;
   long long wait_cycles;
   int skip_copy;                 // test hook: the loader leaves out its first stage
@@ -86,10 +90,13 @@ __global__ void tc_pack_w_kernel(const __nv_bfloat16* __restrict__ W, int64_t ws
   }
 }
 
-template <bool RELU>
+template <bool RELU, int MT>
 __global__ void __launch_bounds__(kRoThreads, 1)
     tc_readout_kernel(const RoParams P, const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_d) {
   extern __shared__ uint8_t smem_raw[];
+  constexpr int kRoStages = ro_stages(MT);
+  constexpr uint32_t kRoABytes = ro_a_bytes(MT);
+  constexpr uint32_t NB = MT == 1 ? 2u : 1u;     // accumulators in flight: all 512 tensor-memory columns either way
   // the swizzled A stages need 512-byte alignment (1024 keeps room for the 128-byte mode)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* a_base = smem;
@@ -98,9 +105,9 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   uint64_t* full = bars;                         // [stages] TMA + bulk copy landed
   uint64_t* ready = full + kRoStages;            // [stages] activation applied (one arrival per warp); RELU only
   uint64_t* empty = ready + kRoStages;           // [stages] MMA -> loader
-  uint64_t* acc_full = empty + kRoStages;        // [1] MMA -> epilogue
-  uint64_t* acc_empty = acc_full + 1;            // [1] epilogue -> MMA (one arrival per warp)
-  uint64_t* done = acc_empty + 1;                // [1]
+  uint64_t* acc_full = empty + kRoStages;        // [NB] MMA -> epilogue
+  uint64_t* acc_empty = acc_full + NB;           // [NB] epilogue -> MMA (one arrival per warp)
+  uint64_t* done = acc_empty + NB;               // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wc{abort_flag, P.status, kStatusTimeoutReadout, P.wait_cycles};
@@ -108,8 +115,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < kRoStages; ++i) { mbar_init(full + i, 1); mbar_init(ready + i, 8); mbar_init(empty + i, 1); }
-    mbar_init(acc_full, 1);
-    mbar_init(acc_empty, 8);
+    for (uint32_t i = 0; i < NB; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 8); }
     mbar_init(done, 1);
     *abort_flag = 0;
     mbar_init_fence();
@@ -120,15 +126,18 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int64_t step = gridDim.x;
+  const int64_t step = gridDim.x, items = P.tiles * P.slices;     // item = (K slice, tile)
+  pdl_wait();
 
   if (warp < 8) {
     // ------------------------------------------------------------------ activation in place, then epilogue
     uint32_t it = 0, ti = 0;
     bool drain = false;
-    for (int64_t t = blockIdx.x; t < P.tiles && !drain; t += step, ++ti) {
+    for (int64_t t = blockIdx.x; t < items && !drain; t += step, ++ti) {
+      const int64_t tile = t % P.tiles;
+      const int slice = (int)(t / P.tiles), s_beg = slice * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
       if (RELU) {
-        for (int s = 0; s < P.ks && !drain; ++s, ++it) {
+        for (int s = s_beg; s < s_end && !drain; ++s, ++it) {
           const uint32_t st = it % kRoStages;
           if (mbar_wait(full + st, (it / kRoStages) & 1u, wc)) { drain = true; break; }
           if (s < P.ks_z) {
@@ -150,31 +159,40 @@ __global__ void __launch_bounds__(kRoThreads, 1)
         }
         if (drain) break;
       }
-      // ---- epilogue of this tile: accumulator rows of this warp -> bf16 -> y
-      if (mbar_wait(acc_full, ti & 1u, wc)) break;
+      // ---- epilogue of this item: accumulator rows of this warp -> bf16 -> y, or float32 -> partial
+      const uint32_t ab = ti % NB;
+      if (mbar_wait(acc_full + ab, (ti / NB) & 1u, wc)) break;
       tc_fence_after();
-      const int64_t n = (t / P.n_tiles) * 256 + warp * 32 + lane;
-      const int n0 = (int)(t % P.n_tiles) * 256;
-      const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * 256u;
-      __nv_bfloat16* yrow = P.y + (n < P.N ? n : 0) * P.ys + n0;
+      // MT = 2: warps 0-3 and 4-7 take a token half each; MT = 1: an output half each
+      const int64_t n = (tile / P.n_tiles) * (128 * MT) + (MT == 2 ? warp * 32 : (warp & 3) * 32) + lane;
+      const int col0 = MT == 2 ? 0 : (warp >> 2) * 128;
+      const int n0 = (int)(tile % P.n_tiles) * 256 + col0;
+      const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (MT == 2 ? (uint32_t)(warp >> 2) * 256u : ab * 256u + (uint32_t)col0);
+      const int64_t nn = n < P.N ? n : 0;
 #pragma unroll 1
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < 4 * MT; ++c) {
         float v[32];
         tmem_ld16(taddr + (uint32_t)(c * 32), v);
         tmem_ld16(taddr + (uint32_t)(c * 32 + 16), v + 16);
         if (n < P.N) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const int col = c * 32 + q * 8;
-            if (n0 + col < P.D)
-              *reinterpret_cast<uint4*>(yrow + col) =
+            const int col = n0 + c * 32 + q * 8;
+            if (col >= P.D) continue;
+            if (P.slices > 1) {
+              float4* o = reinterpret_cast<float4*>(P.partial + ((size_t)slice * P.N + nn) * P.D + col);
+              o[0] = make_float4(v[q * 8], v[q * 8 + 1], v[q * 8 + 2], v[q * 8 + 3]);
+              o[1] = make_float4(v[q * 8 + 4], v[q * 8 + 5], v[q * 8 + 6], v[q * 8 + 7]);
+            } else {
+              *reinterpret_cast<uint4*>(P.y + nn * P.ys + col) =
                   make_uint4(pack_bf2(v[q * 8], v[q * 8 + 1]), pack_bf2(v[q * 8 + 2], v[q * 8 + 3]),
                              pack_bf2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf2(v[q * 8 + 6], v[q * 8 + 7]));
+            }
           }
         }
       }
       tc_fence_before();
-      mbar_arrive_warp(acc_empty);
+      mbar_arrive_warp(acc_empty + ab);
     }
   } else if (warp == 8) {
     // ------------------------------------------------------------------ MMA issue
@@ -187,11 +205,14 @@ __global__ void __launch_bounds__(kRoThreads, 1)
       constexpr uint32_t idesc = instr_desc(1, 1, 0, 0, 128, 256);
       uint32_t it = 0, ti = 0;
       bool drain = false;
-      for (int64_t t = blockIdx.x; t < P.tiles && !drain; t += step, ++ti) {
-        if (ti >= 1) drain = mbar_wait(acc_empty, (ti - 1u) & 1u, wc);
+      for (int64_t t = blockIdx.x; t < items && !drain; t += step, ++ti) {
+        const uint32_t ab = ti % NB;
+        if (ti >= NB) drain = mbar_wait(acc_empty + ab, (ti / NB - 1u) & 1u, wc);
         if (drain) break;
         tc_fence_after();
-        for (int s = 0; s < P.ks; ++s, ++it) {
+        const int s_beg = (int)(t / P.tiles) * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
+        const uint32_t d_addr = tmem_base + (MT == 1 ? ab * 256u : 0u);
+        for (int s = s_beg; s < s_end; ++s, ++it) {
           const uint32_t st = it % kRoStages, ph = (it / kRoStages) & 1u;
           drain = mbar_wait((RELU ? ready : full) + st, ph, wc);
           if (drain) break;
@@ -201,15 +222,16 @@ __global__ void __launch_bounds__(kRoThreads, 1)
           uint32_t a_lo = ((smem_u32(a_base + st * kRoABytes) >> 4) & 0x3FFFu) | (1u << 16);
           uint32_t b_lo = desc_lo(smem_u32(b_base + st * kRoBBytes), 4096u);
           for (int k = 0; k < nk; ++k) {
-            const uint32_t accf = (s | k) ? 1u : 0u;
-            umma_f16_split(tmem_base, a_lo, a_hi, b_lo, b_hi, idesc, accf);                        // tokens 0-127
-            umma_f16_split(tmem_base + 256u, a_lo + ((128u * kRowBytes) >> 4), a_hi, b_lo, b_hi, idesc, accf);  // tokens 128-255
+            const uint32_t accf = (s > s_beg || k > 0) ? 1u : 0u;
+            umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, accf);                             // tokens 0-127
+            if constexpr (MT == 2)
+              umma_f16_split(d_addr + 256u, a_lo + ((128u * kRowBytes) >> 4), a_hi, b_lo, b_hi, idesc, accf);  // tokens 128-255
             a_lo += 32u >> 4;
             b_lo += 8192u >> 4;
           }
           umma_commit(empty + st);
         }
-        if (!drain) umma_commit(acc_full);
+        if (!drain) umma_commit(acc_full + ab);
       }
       umma_commit(done);
     }
@@ -218,10 +240,12 @@ __global__ void __launch_bounds__(kRoThreads, 1)
     if (elect_one()) {
       uint32_t it = 0;
       bool stop = false;
-      for (int64_t t = blockIdx.x; t < P.tiles && !stop; t += step) {
-        const uint8_t* src = P.wimg + (size_t)(t % P.n_tiles) * P.ks * kRoBBytes;
-        const int m0 = (int)((t / P.n_tiles) * 256);
-        for (int s = 0; s < P.ks; ++s, ++it) {
+      for (int64_t t = blockIdx.x; t < items && !stop; t += step) {
+        const int64_t tile = t % P.tiles;
+        const uint8_t* src = P.wimg + (size_t)(tile % P.n_tiles) * P.ks * kRoBBytes;
+        const int m0 = (int)((tile / P.n_tiles) * (128 * MT));
+        const int s_beg = (int)(t / P.tiles) * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
+        for (int s = s_beg; s < s_end; ++s, ++it) {
           const uint32_t st = it % kRoStages;
           if (it == 0 && P.skip_copy) continue;      // test hook: nothing ever completes full[0]
           if (it >= kRoStages && mbar_wait(empty + st, ((it / kRoStages) - 1u) & 1u, wc)) { stop = true; break; }
@@ -246,9 +270,60 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   }
 }
 
-// Boxes of 256 rows x kRoK columns, the swizzle span of one row.
-bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch) {
-  return make_map_2d(m, base, rows, cols, pitch, kRoK, 256, kRoK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+// Boxes of 128 * mt rows x kRoK columns, the swizzle span of one row.
+bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch, int mt) {
+  return make_map_2d(m, base, rows, cols, pitch, kRoK, 128 * mt, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// y = bf16 of the sum of the K slices' partials, in order; four outputs per thread.
+__global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partial, int slices, int64_t N, int D,
+                                                             __nv_bfloat16* y, int64_t ys) {
+  pdl_wait();
+  const int q4 = D / 4;
+  const int64_t total = N * q4;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4* src = reinterpret_cast<const float4*>(partial) + i;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int k = 0; k < slices; ++k) {
+      const float4 v = src[(size_t)k * total];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    const int64_t n = i / q4;
+    *reinterpret_cast<uint2*>(y + n * ys + (i - n * q4) * 4) = make_uint2(pack_bf2(s.x, s.y), pack_bf2(s.z, s.w));
+  }
+}
+
+// Tile height and K slices.  Microseconds: a stage of 256 tokens costs 0.91 with ReLU^2 (0.70 without), one of 128 tokens
+// more than half of that (it reads as much of W); an item's fill and epilogue; partials through L2.  256 tokens give the
+// best rate, 128 fill a last wave better (8192 x 5120 -> 1280: 160 tiles of 256 on 148 SMs took two rounds), and slices
+// spread few tokens over the chip.
+struct RoPlan { int mt, slices, ks_per; };
+RoPlan readout_plan(const skv_problem& p, int64_t D) {
+  const int ks = (p.h + kRoK - 1) / kRoK + (p.r + kRoK - 1) / kRoK;
+  const bool relu = p.activation == SKV_ACT_RELU_SQ;
+  const double N = (double)(p.N > 0 ? p.N : 1);
+  RoPlan best{2, 1, ks};
+  double best_t = 0.0;
+  for (int mt = 2; mt >= 1; --mt) {
+    const int64_t tiles = ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256);
+    const double stage = mt == 2 ? (relu ? 0.91 : 0.70) : (relu ? 0.50 : 0.40);
+    int last = 0;
+    for (int s = 1; s <= 16 && s <= (ks + 3) / 4; ++s) {
+      const int per = (ks + s - 1) / s, slices = (ks + per - 1) / per;
+      if (slices == last) continue;
+      last = slices;
+      const double t = (double)((tiles * slices + kPlanSMs - 1) / kPlanSMs) * (per * stage + 3.0 * mt) +
+                       (slices > 1 ? 4.0 + slices * N * (double)D * 8.0 / 4.0e6 : 0.0);
+      if (best_t == 0.0 || t < best_t) { best_t = t; best = {mt, slices, per}; }
+    }
+  }
+  return best;
+}
+
+size_t wimg_bytes(const skv_problem& p, int64_t D) {
+  const size_t ks = (size_t)(p.h + kRoK - 1) / kRoK + (size_t)(p.r + kRoK - 1) / kRoK;
+  return (size_t)((D + 255) / 256) * ks * kRoBBytes;
 }
 
 }  // namespace
@@ -258,19 +333,32 @@ bool readout_eligible(const skv_problem& p, int64_t D) {
          p.r % 8 == 0 && D >= 8 && D % 8 == 0 && D <= (1 << 24);
 }
 
+// Image of W, then the K slices' partials.
 size_t readout_image_bytes(const skv_problem& p, int64_t D) {
-  const size_t ks = (size_t)(p.h + kRoK - 1) / kRoK + (size_t)(p.r + kRoK - 1) / kRoK;
-  return (size_t)((D + 255) / 256) * ks * kRoBBytes;
+  const RoPlan f = readout_plan(p, D);
+  return wimg_bytes(p, D) + (f.slices > 1 ? (size_t)f.slices * (p.N > 0 ? p.N : 1) * D * sizeof(float) : 0);
 }
 
 // Row pitch (elements) of the delta buffer the GEMM reads: whole stages of kRoK columns, pad columns zero.
 int64_t readout_delta_pitch(const skv_problem& p) { return (int64_t)((p.r + kRoK - 1) / kRoK) * kRoK; }
 
+// Tiled image of W; a plain launch in front of the feature kernels, so that the GEMM can be chained to them.
+int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg) {
+  const skv_problem& p = c.p;
+  const int ks_z = (p.h + kRoK - 1) / kRoK, ks = ks_z + (p.r + kRoK - 1) / kRoK;
+  const int64_t chunks = (D + 255) / 256 * ks * (kRoBBytes / 16);
+  const int pgrid = (int)((chunks + 255) / 256 < 4096 ? (chunks + 255) / 256 : 4096);
+  tc_pack_w_kernel<<<pgrid, 256, 0, c.stream>>>(static_cast<const __nv_bfloat16*>(W), ws, (int)D, p.h, p.r, ks_z, ks, chunks,
+                                                 static_cast<uint4*>(wimg));
+  note_launches(1);
+  return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+}
+
 // y = [act(z) | delta] * W^T; `delta` is [N][readout_delta_pitch()] bf16 with zero pad columns, `wimg`
 // has readout_image_bytes().
-int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, const void* W, int64_t ws, int64_t D,
-            void* y, int64_t ys, void* wimg) {
+int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, int64_t D, void* y, int64_t ys, void* wimg) {
   const skv_problem& p = c.p;
+  const RoPlan f = readout_plan(p, D);
   RoParams P;
   P.wimg = static_cast<const uint8_t*>(wimg);
   P.y = static_cast<__nv_bfloat16*>(y);
@@ -282,33 +370,38 @@ int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, co
   P.ks_z = (int)((p.h + kRoK - 1) / kRoK);
   P.ks = P.ks_z + (int)((p.r + kRoK - 1) / kRoK);
   P.n_tiles = (int)((D + 255) / 256);
-  P.tiles = ((p.N + 255) / 256) * P.n_tiles;
+  P.tiles = ((p.N + 128 * f.mt - 1) / (128 * f.mt)) * P.n_tiles;
+  P.slices = f.slices;
+  P.ks_per = f.ks_per;
+  P.partial = reinterpret_cast<float*>(static_cast<uint8_t*>(wimg) + wimg_bytes(p, D));
   P.status = c.status;
   P.wait_cycles = wait_cycle_limit();
   P.skip_copy = debug_skip_copy() == 2;
   CUtensorMap map_z, map_d;
-  if (!make_map(&map_z, z, (uint64_t)p.N, (uint64_t)p.h, (uint64_t)zs) ||
-      !make_map(&map_d, delta, (uint64_t)p.N, (uint64_t)readout_delta_pitch(p), (uint64_t)readout_delta_pitch(p)))
+  if (!make_map(&map_z, z, (uint64_t)p.N, (uint64_t)p.h, (uint64_t)zs, f.mt) ||
+      !make_map(&map_d, delta, (uint64_t)p.N, (uint64_t)readout_delta_pitch(p), (uint64_t)readout_delta_pitch(p), f.mt))
     return SKV_ERR_LAUNCH;
-
-  const int64_t chunks = (int64_t)P.n_tiles * P.ks * (kRoBBytes / 16);
-  const int pgrid = (int)((chunks + 255) / 256 < 4096 ? (chunks + 255) / 256 : 4096);
-  tc_pack_w_kernel<<<pgrid, 256, 0, c.stream>>>(static_cast<const __nv_bfloat16*>(W), ws, P.D, P.h, P.r, P.ks_z, P.ks,
-                                                 chunks, static_cast<uint4*>(wimg));
-  if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
-
-  const size_t smem = (size_t)kRoStages * (kRoABytes + kRoBBytes) + 1024 + 256;
-  const int grid = (int)(P.tiles < c.num_sms ? P.tiles : c.num_sms);
-  cudaError_t err;
-  if (p.activation == SKV_ACT_RELU_SQ) {
-    err = cudaFuncSetAttribute(tc_readout_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess) tc_readout_kernel<true><<<grid, kRoThreads, smem, c.stream>>>(P, map_z, map_d);
-  } else {
-    err = cudaFuncSetAttribute(tc_readout_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess) tc_readout_kernel<false><<<grid, kRoThreads, smem, c.stream>>>(P, map_z, map_d);
+  const size_t smem = (size_t)ro_stages(f.mt) * (ro_a_bytes(f.mt) + kRoBBytes) + 1024 + 256;
+  const int64_t items = P.tiles * P.slices;
+  const dim3 grid((unsigned)(items < c.num_sms ? items : c.num_sms));
+  const bool relu = p.activation == SKV_ACT_RELU_SQ;
+  const cudaError_t err =
+      f.mt == 2 ? (relu ? launch_chained<tc_readout_kernel<true, 2>>(grid, kRoThreads, smem, c.stream, P, map_z, map_d)
+                        : launch_chained<tc_readout_kernel<false, 2>>(grid, kRoThreads, smem, c.stream, P, map_z, map_d))
+                : (relu ? launch_chained<tc_readout_kernel<true, 1>>(grid, kRoThreads, smem, c.stream, P, map_z, map_d)
+                        : launch_chained<tc_readout_kernel<false, 1>>(grid, kRoThreads, smem, c.stream, P, map_z, map_d));
+  note_launches(1);
+  if (err != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
+  if (P.slices > 1) {
+    const int64_t blocks = (p.N * (D / 4) + 255) / 256;
+    const dim3 sgrid((unsigned)(blocks < kPlanSMs * 16 ? blocks : kPlanSMs * 16));
+    if (launch_chained<tc_readout_sum_kernel>(sgrid, 256, 0, c.stream, (const float*)P.partial, P.slices, P.N, P.D, P.y,
+                                              P.ys) != cudaSuccess) {
+      cudaGetLastError();
+      return SKV_ERR_LAUNCH;
+    }
+    note_launches(1);
   }
-  if (err != cudaSuccess || cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
-  note_launches(2);
   return SKV_OK;
 }
 
