@@ -45,6 +45,7 @@ template <typename T>
 __device__ __forceinline__ void stage_rows(T* dst, const T* __restrict__ src, int rows, int r, int pitch) {
   if (r == pitch && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
     const int n16 = (int)((size_t)rows * r * sizeof(T) / 16);
+#pragma unroll 8
     for (int i = threadIdx.x; i < n16; i += blockDim.x)
       reinterpret_cast<uint4*>(dst)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
   } else {
@@ -52,6 +53,7 @@ __device__ __forceinline__ void stage_rows(T* dst, const T* __restrict__ src, in
     int per = 32;
     while (per > r) per >>= 1;
     const int c0 = threadIdx.x & (per - 1);
+#pragma unroll 4
     for (int row = threadIdx.x / per; row < rows; row += blockDim.x / per)
       for (int c = c0; c < r; c += per) dst[(size_t)row * pitch + c] = src[(size_t)row * r + c];
   }
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const F
   constexpr int V = Vec<T>::n;
   constexpr int TPW = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
+  constexpr int kPre = TPW < 8 ? TPW : 8;                                 // tokens of the next group loaded ahead
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float4* wbuf = reinterpret_cast<float4*>(smem_raw);                     // [warp][TPW][32]
   T* Cs = reinterpret_cast<T*>(wbuf + kWarps * TPW * kWarp);               // [kch][L][pitch]
@@ -128,17 +131,30 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const F
     __syncthreads();
     stage_rows(Cs, static_cast<const T*>(P.C) + (size_t)j0 * P.L * P.r, kc * P.L, P.r, pitch);
     __syncthreads();
+    float zn[kPre];
+    auto load_z = [&](int m) {
+#pragma unroll
+      for (int t = 0; t < kPre; ++t) {
+        const int64_t n = tile0 + (int64_t)(m * kWarps + warp) * TPW + t;
+        zn[t] = m < P.groups && lane < kc && n < P.N ? ld_f32<T>(z + n * P.zs + j0 + lane) : 0.0f;
+      }
+    };
+    load_z(0);
 #pragma unroll
     for (int m = 0; m < kGroups; ++m) {
       if (m >= P.groups) break;
       const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
       if (n0 >= P.N) break;
+      float zc[kPre];
+#pragma unroll
+      for (int t = 0; t < kPre; ++t) zc[t] = zn[t];
+      load_z(m + 1);                                  // the next group's pre-activations are requested now
       __syncwarp();
-#pragma unroll 4
+#pragma unroll
       for (int t = 0; t < TPW; ++t) {
         float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (lane < kc && n0 + t < P.N) {
-          const float zz = ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
+          const float zz = t < kPre ? zc[t < kPre ? t : 0] : ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
           w = pair_weights(zz, P.g, lane * P.L, pitch);
           if (act_out) st_f32<T>(act_out + (n0 + t) * P.as + j0 + lane, act_fwd(zz, P.act));
         }
@@ -352,6 +368,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
   constexpr int V = 4;
   constexpr int TPW = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
+  constexpr int kPre = TPW < 8 ? TPW : 8;                                  // tokens of the next group loaded ahead
   constexpr int kRes = kWarp + 4;                                          // pitch of the result rows
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float2* wbuf = reinterpret_cast<float2*>(smem_raw);                     // [warp][TPW][32]  (tau, row offset)
@@ -375,6 +392,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
     int per = 32;
     while (per > P.r) per >>= 1;
     const int c0 = threadIdx.x & (per - 1);
+#pragma unroll 4
     for (int row = threadIdx.x / per; row < kc * R; row += blockDim.x / per) {
       const T* src = C + ((size_t)(j0 + row / R) * P.L + row % R) * P.r;
       for (int c = c0; c < pitch; c += per)
@@ -383,31 +401,52 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
   }
   __syncthreads();
 
+  // rows of z, g_delta and g_act of the next group are requested while this one is worked on
+  float zn[kPre], an[kPre], gn[CV][V];
+  auto load_group = [&](int m) {
+    const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+    const bool on = m < P.groups && lane < kc;
+#pragma unroll
+    for (int t = 0; t < kPre; ++t) {
+      zn[t] = on && n0 + t < P.N ? ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane) : 0.0f;
+      an[t] = on && g_act && n0 + t < P.N ? ld_f32<T>(g_act + (n0 + t) * P.gas + j0 + lane) : 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int col = c * (LPT * V) + sl * V + i;
+        gn[c][i] = m < P.groups && n0 + sub < P.N && col < P.r ? ld_f32<T>(g_delta + (n0 + sub) * P.gds + col) : 0.0f;
+      }
+  };
+  load_group(0);
   for (int m = 0; m < P.groups; ++m) {
     const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
     if (n0 >= P.N) break;
-    float zz[TPW];
+    float zz[TPW], ga[kPre];
+    float gd[CV][V];
+#pragma unroll
+    for (int t = 0; t < TPW; ++t)
+      zz[t] = t < kPre ? zn[t < kPre ? t : 0]
+                       : (lane < kc && n0 + t < P.N ? ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane) : 0.0f);
+#pragma unroll
+    for (int t = 0; t < kPre; ++t) ga[t] = an[t];
+#pragma unroll
+    for (int c = 0; c < CV; ++c)
+#pragma unroll
+      for (int i = 0; i < V; ++i) gd[c][i] = gn[c][i];
+    load_group(m + 1);
     uint32_t live = 0u;                                                    // bit t: 0 <= u <= G-1 for (t, lane)
 #pragma unroll
     for (int t = 0; t < TPW; ++t) {
       float2 w = make_float2(0.0f, 0.0f);
-      zz[t] = 0.0f;
       if (lane < kc && n0 + t < P.N) {
-        zz[t] = ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
         const Knot k = knot_of(zz[t], P.g);
         w = make_float2(k.tau, __int_as_float(STAGED ? (lane * R + k.bin) * pitch : (lane * P.L + k.bin) * P.r));
         if (k.clamp_active) live |= 1u << t;
       }
       my[t * kWarp + lane] = w;
     }
-    float gd[CV][V];
-#pragma unroll
-    for (int c = 0; c < CV; ++c)
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const int col = c * (LPT * V) + sl * V + i;
-        gd[c][i] = (n0 + sub < P.N && col < P.r) ? ld_f32<T>(g_delta + (n0 + sub) * P.gds + col) : 0.0f;
-      }
     __syncwarp();
 #pragma unroll 1
     for (int q0 = 0; q0 < kc; q0 += LPT) {
@@ -464,7 +503,8 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
     for (int t = 0; t < TPW; ++t) {
       if (lane < kc && n0 + t < P.N) {
         float o = (live >> t) & 1u ? P.coef * res[t * kRes + lane] : 0.0f;
-        if (g_act) o = fmaf(ld_f32<T>(g_act + (n0 + t) * P.gas + j0 + lane), act_grad(zz[t], P.act), o);
+        if (g_act)
+          o = fmaf(t < kPre ? ga[t < kPre ? t : 0] : ld_f32<T>(g_act + (n0 + t) * P.gas + j0 + lane), act_grad(zz[t], P.act), o);
         st_f32<T>(dz + (n0 + t) * P.dzs + j0 + lane, o);
       }
     }
@@ -542,8 +582,10 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
   for (int64_t t0 = nbeg; t0 < nend; t0 += TT) {
     const int tt = (int)min((int64_t)TT, nend - t0);
     __syncthreads();
+#pragma unroll 8
     for (int t = threadIdx.x / per; t < tt; t += blockDim.x / per)
       for (int c = c0; c < r; c += per) gs[(size_t)t * pitch + c] = ld_f32<T>(g_delta + (t0 + t) * P.gds + c);
+#pragma unroll 8
     for (int i = threadIdx.x; i < tt * W; i += blockDim.x) {
       const int t = i / W, k = i % W;
       zt[t * zp + k] = k < kd ? ld_f32<T>(z + (t0 + t) * P.zs + j0 + k) : 0.0f;
