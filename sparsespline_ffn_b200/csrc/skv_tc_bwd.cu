@@ -13,6 +13,7 @@ namespace tc {
 
 bool fwd_eligible(const skv_problem& p);
 cudaError_t dz_launch_quad(const DzPlan&, int L, bool relu, const DzParams&, dim3, cudaStream_t);
+cudaError_t dz_launch_split(const DzPlan&, int L, bool relu, const DzParams&, dim3, cudaStream_t);
 cudaError_t dz_launch_lin(const DzPlan&, int L, bool relu, const DzParams&, dim3, cudaStream_t);
 cudaError_t dc_launch(const DcPlan&, bool lin, bool split, const DcParams&, dim3, cudaStream_t);
 
@@ -228,7 +229,6 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Z.chunks_per_split = b.dz.chunks_per_split;
   Z.tstages = b.dz.tstages;
   Z.rstages = b.dz.rstages;
-  Z.tparts = split ? 2 : 1;
   Z.dz_f32 = p.dz_f32;
   Z.wait_cycles = wait_cycle_limit();
   Z.status = c.status;
@@ -241,7 +241,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   } else {
     if (dz) {
       const dim3 grid((unsigned)((p.N + 128 * b.dz.groups - 1) / (128 * b.dz.groups)), (unsigned)b.dz.splits);
-      if ((lin ? dz_launch_lin : dz_launch_quad)(b.dz, p.L, p.activation == SKV_ACT_RELU_SQ, Z, grid, c.stream) !=
+      if ((lin ? dz_launch_lin : split ? dz_launch_split : dz_launch_quad)(b.dz, p.L, p.activation == SKV_ACT_RELU_SQ, Z, grid, c.stream) !=
           cudaSuccess) {
         cudaGetLastError();
         return SKV_ERR_LAUNCH;

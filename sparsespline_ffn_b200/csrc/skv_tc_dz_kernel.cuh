@@ -34,7 +34,6 @@ struct DzParams {
   float coef;                // lambda * scale
   int chunks_total, chunks_per_split;
   int tstages;               // depth of the transformed-table ring (2..kTStages)
-  int tparts;                // f16 parts of the table's values (1 or 2): K runs over tparts * r channels, g repeats
   int rstages;               // boxes of z and g_act per token group (2 or 3)
   int dz_f32;                // dz is float32 [N][dzs] instead of bf16
   int32_t* status;
@@ -152,7 +151,9 @@ __host__ __device__ constexpr int dz_block_keys(int lb) { return lb <= 4 ? 4 : 2
 // out of the hot loop); otherwise P.act (identity or gelu) is evaluated at run time.
 // LIN: the derivative of the linear spline is C[bin+1] - C[bin]; with the same table its column weights
 // are the steps 1[bin >= m + 1] = sat(bin - m), so the only change is bin in the place of u_c.
-template <int GROUPS, int LB, int NC, bool RELU, bool LIN>
+// SPLIT: the table's values are two f16 (K runs over 2 r channels of it, over g twice).  A template case: a run-time count in the
+// issuing thread's loop cost 4 % (0.964 -> 1.003 ms at the d20 shape).
+template <int GROUPS, int LB, int NC, bool RELU, bool LIN, bool SPLIT>
 __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
     tc_dz_kernel(const DzParams P, const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_ga,
                  const __grid_constant__ CUtensorMap map_dz) {
@@ -163,10 +164,11 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
   const int r = P.r;
   constexpr int LP = 8 * LB;                                         // padded knot columns per key
   constexpr int KB = dz_block_keys(LB);
+  constexpr int kParts = SPLIT ? 2 : 1;
   constexpr int NBLK = kChunkKeys / KB;                              // blocks per chunk
   constexpr bool DB = LB <= 4;                                       // two keys' columns in registers
   const uint32_t g_bytes = (uint32_t)(128 * r * 2);
-  const uint32_t t_bytes = (uint32_t)(kChunkKeys * LP * r * 2 * P.tparts);
+  const uint32_t t_bytes = (uint32_t)(kChunkKeys * LP * r * 2 * kParts);
   constexpr uint32_t bcols = (uint32_t)(KB * LP);                    // columns of one S block
   uint8_t* g_base = smem;                                             // [group][g_bytes]
   uint8_t* t_base = smem + (size_t)GROUPS * g_bytes;                  // [kTStages][t_bytes]
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
     if (elect_one()) {
       const int grp = warp - 8 * GROUPS;
       mbar_wait(gfull, 0, wc);
-      const uint32_t rb = (uint32_t)(r * P.tparts / 8) * 128u;   // bytes between 8-row groups of the T image
+      const uint32_t rb = (uint32_t)(r * kParts / 8) * 128u;   // bytes between 8-row groups of the T image
       const uint32_t a_hi = desc_hi(128u), b_hi = desc_hi(rb);
       constexpr uint32_t idesc = instr_desc(0, 0, 0, 0, 128, (int)bcols);
       const uint32_t a_lo0 = desc_lo(smem_u32(g_base + (size_t)grp * g_bytes), 2048u);
@@ -321,7 +323,8 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
           tc_fence_after();
           uint32_t b_lo = b_blk;
           const uint32_t d_addr = d0 + (uint32_t)(b & 1) * bcols;
-          for (int part = 0; part < P.tparts; ++part) {
+#pragma unroll
+          for (int part = 0; part < kParts; ++part) {
             uint32_t a_lo = a_lo0;
             for (int ks = 0; ks < ksteps; ++ks) {
               umma_f16_split(d_addr, a_lo, a_hi, b_lo, b_hi, idesc, ks + part > 0 ? 1u : 0u);
@@ -403,7 +406,7 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
 struct DzPlan { int groups, lb, splits, chunks_per_split, tstages, rstages; size_t smem; };
 
 // NC_ = L - 1 useful columns per key for the knot counts in common use, all 8 * LB_ otherwise.
-template <bool LIN>
+template <bool LIN, bool SPLIT>
 cudaError_t dz_launch(const DzPlan& zp, int L, bool relu, const DzParams& P, dim3 grid, cudaStream_t stream) {
   CUtensorMap mz, mg, md;
   if (!make_box_map(&mz, P.z, P.N, P.h, P.zs) || (P.g_act && !make_box_map(&mg, P.g_act, P.N, P.h, P.gas)) ||
@@ -414,8 +417,8 @@ cudaError_t dz_launch(const DzPlan& zp, int L, bool relu, const DzParams& P, dim
   const unsigned threads = 320 * zp.groups + 32;
 #define SKV_DZ_CASE(G_, LB_, NC_, COND_)                                                                           \
   if (zp.groups == G_ && zp.lb == LB_ && (COND_))                                                                  \
-    return relu ? launch_chained<tc_dz_kernel<G_, LB_, NC_, true, LIN>>(grid, threads, zp.smem, stream, P, mz, mg, md)         \
-                : launch_chained<tc_dz_kernel<G_, LB_, NC_, false, LIN>>(grid, threads, zp.smem, stream, P, mz, mg, md);
+    return relu ? launch_chained<tc_dz_kernel<G_, LB_, NC_, true, LIN, SPLIT>>(grid, threads, zp.smem, stream, P, mz, mg, md)         \
+                : launch_chained<tc_dz_kernel<G_, LB_, NC_, false, LIN, SPLIT>>(grid, threads, zp.smem, stream, P, mz, mg, md);
   if constexpr (LIN) {
     SKV_DZ_CASE(2, 3, 20, L == 21)
   } else {

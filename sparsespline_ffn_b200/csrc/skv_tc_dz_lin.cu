@@ -4,7 +4,7 @@
 namespace skv {
 namespace tc {
 cudaError_t dz_launch_lin(const DzPlan& zp, int L, bool relu, const DzParams& P, dim3 grid, cudaStream_t stream) {
-  return dz_launch<true>(zp, L, relu, P, grid, stream);
+  return dz_launch<true, true>(zp, L, relu, P, grid, stream);
 }
 }  // namespace tc
 }  // namespace skv
