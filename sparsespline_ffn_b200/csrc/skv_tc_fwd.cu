@@ -42,6 +42,8 @@ FwdPlan make_plan(const skv_problem& p) {
     const size_t stage_bytes = (size_t)128 * g * (F + 1) * 4;
     int cstages = (int)((kSmemLimit - 512 - stage_bytes) / c_bytes);
     if (cstages > kMaxCStages) cstages = kMaxCStages;
+    // what the ring does not need is L1 for the strided rows of z and phi(z)
+    while (cstages > 3 && cstages * c_bytes + stage_bytes + 512 > kSmemOnePerSM) --cstages;
     if (cstages < 2) continue;
     const int64_t tiles = (N + 128 * g - 1) / (128 * g);
     // microseconds: a chunk of g groups (instruction issue, or the MMAs of wide r), a CTA's prologue and

@@ -86,7 +86,7 @@ def _warn_if_slow_family(lib, p: _lib.Problem, z: torch.Tensor, aligned_fn) -> N
     import warnings
     why = ("a tensor whose base address or row stride is not 16-byte aligned" if not aligned else
            f"a shape outside the tcgen05 kernels' range (h={p.h}, L={p.L}, r={p.r}: need r <= 128, L <= 64)")
-    warnings.warn(f"splinekv_b200: {p.N} x {p.h} bf16 problem runs on the CUDA-core fallback kernels because of "
+    warnings.warn(f"splinekv_b200: {p.N} x {p.h} bf16 problem runs on the CUDA-core kernels because of "
                   f"{why}; expect it to be several times slower", RuntimeWarning, stacklevel=3)
 
 
@@ -134,7 +134,7 @@ def feature_forward(z, C, grid_lo, grid_hi, G, activation="relu_sq", lambda_scal
     With ``delta_f32`` the residual comes back in float32 whatever the dtype of ``z`` (the
     key-sharded mode sums partial residuals across GPUs before the one rounding to bf16); the two
     halves then cannot share a tensor, so the result is ``(phi(z) or None, delta_f32)``.
-    ``spline_order=1`` selects the linear B-spline (``C`` is ``[h, G + 1, r]``; CUDA-core kernels)."""
+    ``spline_order=1`` selects the linear B-spline (``C`` is ``[h, G + 1, r]``)."""
     lib = _lib.load()
     C = C.to(z.dtype) if C.dtype != z.dtype else C
     p = _problem(z, C, grid_lo, grid_hi, G, activation, lambda_scale, impl, spline_order)

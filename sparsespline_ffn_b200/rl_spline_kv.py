@@ -13,7 +13,7 @@ reference module loads, and the same three forward graphs:
 What differs, on purpose: the operator always runs on the sm_100a kernels (there is no eager path, so
 ``use_kernel`` is accepted and must not be asked to be False on this package's behalf: a CPU input
 raises), ``spline_order = 1`` (the linear spline, additive mode only, as in the reference, ``:303, 323``)
-runs on the library's CUDA-core kernels instead of PyTorch code, and the per-forward diagnostics of the reference (``:376-481``) are not computed, which
+runs on the library's kernels instead of PyTorch code, and the per-forward diagnostics of the reference (``:376-481``) are not computed, which
 also removes the host synchronisations they cause.  The two GEMMs around the operator are
 ``torch.nn.Linear``.
 """
