@@ -259,7 +259,6 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.L = p.L;
       P.r = rp;
       P.g = c.g;
-      P.after_dz = dz ? 1 : 0;
       P.words = (p.L + 1) / 2;
       P.ngroups = b.dc.ngroups;
       P.gring = b.dc.gring;

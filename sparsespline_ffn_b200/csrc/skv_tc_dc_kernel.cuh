@@ -28,10 +28,6 @@ struct DcParams {
   int64_t N;
   int h, L, r;
   GridParams g;
-  // Launched behind this call's dz kernel, of which nothing is needed: dz lets its dependents start only after its own wait
-  // for the packing kernel, so once a CTA of this kernel runs the g image is complete, and it fills the SMs that dz's
-  // last wave leaves idle.  The wait for dz moves to the end, so that this kernel's completion still implies dz's.
-  int after_dz;
   int words;                 // f16x2 words per key in the Phi^T tile: L / 2 rounded up (an odd L's last row is zero)
   int ngroups;               // producer groups, one stage each
   int gring;                 // slots of the ring of g tiles, more than groups
@@ -108,7 +104,7 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch();
-  if (!P.after_dz) pdl_wait();
+  pdl_wait();
 
   if (warp < mma_warp) {
     // ------------------------------------------------------------------ producers
@@ -288,7 +284,6 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
       }
     }
   }
-  if (P.after_dz) pdl_wait();
   __syncthreads();
   if (warp == mma_warp) {
     mbar_wait_drain(done, 0, P.wait_cycles);

@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch();
   pdl_wait();
-  pdl_launch();                                        // after the wait: see DcParams::after_dz
 
   if (warp < 8 * GROUPS) {
     // ------------------------------------------------------------------ two threads per token, one per S buffer
