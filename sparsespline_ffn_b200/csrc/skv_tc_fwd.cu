@@ -47,8 +47,9 @@ FwdPlan make_plan(const skv_problem& p) {
     if (cstages < 2) continue;
     const int64_t tiles = (N + 128 * g - 1) / (128 * g);
     // microseconds: a chunk of g groups (instruction issue, or the MMAs of wide r), a CTA's prologue and
-    // epilogue, and the partials' way through L2 (measured: 1.3 us per chunk of four groups at L = 22)
-    const double issue = (0.22 + 0.27 * g) * (F + 14) / 20.0 * (split_operands(p) ? 1.4 : 1.0), mma = g * F * rp * 0.5 / 1800.0;
+    // epilogue, and the partials' way through L2 and their sum, eight loads at a time (measured: 1.3 us per chunk of four groups at L = 22, 0.9
+    // of one: four warps cannot hide their own latencies)
+    const double issue = (0.75 + 0.14 * g) * (F + 14) / 20.0 * (split_operands(p) ? 1.4 : 1.0), mma = g * F * rp * 0.5 / 1800.0;
     const double chunk = issue > mma ? issue : mma;
     int last = 0;
     for (int64_t s = 1; s <= most; ++s) {
@@ -56,7 +57,7 @@ FwdPlan make_plan(const skv_problem& p) {
       if (splits == last) continue;
       last = splits;
       const double t = (double)((tiles * splits + kPlanSMs - 1) / kPlanSMs) * (per * chunk + 4.5) +
-                       (double)splits * part * 2.0 / 4.0e6;
+                       splits * (part * 2.0 / 4.0e6 + 0.08);
       if (best == 0.0 || t < best) {
         best = t;
         f.groups = g;

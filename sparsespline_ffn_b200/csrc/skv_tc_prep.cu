@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(partial) + i;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
+#pragma unroll 8
     for (int k = 0; k < splits; ++k) {
       const float4 v = src[(size_t)k * total];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, in
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(part) + i;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
+#pragma unroll 8
     for (int k = 0; k < splits; ++k) {
       const float4 v = __ldcs(src + (size_t)k * pitch);
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
@@ -291,8 +291,8 @@ int blocks_for(int64_t items, int64_t per_thread, int most) {
 
 int launch_prep(PrepParams& P, cudaStream_t stream) {
   const int cgs = P.rp / 8;
-  P.scan_c = P.lpc || P.lpt ? blocks_for((int64_t)P.h * P.L * P.r / 8, 8, kPlanSMs * 2) : 0;
-  P.scan_g = P.g ? blocks_for(P.N * ((P.r + 7) / 8), 4, kPlanSMs * 2) : 0;
+  P.scan_c = P.lpc || P.lpt ? blocks_for((int64_t)P.h * P.L * P.r / 8, 2, kPlanSMs * 2) : 0;
+  P.scan_g = P.g ? blocks_for(P.N * ((P.r + 7) / 8), 2, kPlanSMs * 2) : 0;
   P.blocks_c = P.lpc ? blocks_for((int64_t)P.hp * P.lpc * cgs, 2, kPlanSMs * 8) : 0;
   P.blocks_t = P.lpt ? blocks_for((int64_t)P.hp * P.lpt * cgs * P.tparts, 2, kPlanSMs * 8) : 0;
   P.blocks_g = P.g ? blocks_for(P.tiles * 128 * cgs, 2, kPlanSMs * 8) : 0;
