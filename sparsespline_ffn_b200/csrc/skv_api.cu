@@ -99,6 +99,9 @@ int make_ctx(const skv_problem* p, void* stream, int32_t* status, LaunchCtx* c) 
   return SKV_OK;
 }
 
+// A forward of so few tokens that gathering table rows beats packing the table.
+bool small_forward(const skv_problem& p) { return p.impl == SKV_IMPL_AUTO && p.N <= small_forward_tokens(p); }
+
 bool aligned(const void* p, size_t a) { return ((uintptr_t)p % a) == 0; }
 
 // Whether the token-major rows of this shape ([N][h] and [N][h + r] tensors) start on 16-byte boundaries and hold
@@ -164,7 +167,12 @@ size_t skv_scratch_bytes(const skv_problem* p, int op) {
   const int impl = resolve(*p);
   if (impl == SKV_IMPL_SIMT) return simt_scratch_bytes(*p, op);
   if (impl != SKV_IMPL_TCGEN05) return 0;
-  return tc_scratch_bytes(*p, op, rows_fit(*p));
+  size_t need = tc_scratch_bytes(*p, op, rows_fit(*p));
+  if (op == SKV_OP_FORWARD && small_forward(*p)) {
+    const size_t small = simt_scratch_bytes(*p, op);
+    if (small > need) need = small;
+  }
+  return need;
 }
 
 int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, void* act_out,
@@ -177,7 +185,7 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
   if (z_stride < p->h || delta_stride < p->r || (act_out && act_stride < p->h)) return SKV_ERR_SHAPE;
   const int impl = resolve(*p);
   if (impl < 0) return impl;
-  const bool small = p->impl == SKV_IMPL_AUTO && p->N <= small_forward_tokens(*p);
+  const bool small = small_forward(*p);
   if (impl == SKV_IMPL_TCGEN05 && !small) {
     const bool ok = p->h % 8 == 0 && row_ok(z, z_stride, 8) && row_ok(act_out, act_stride, 8);
     const bool copies = !ok && scratch_bytes >= tc_scratch_bytes(*p, SKV_OP_FORWARD, false);
