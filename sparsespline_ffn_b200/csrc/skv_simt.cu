@@ -516,9 +516,9 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
 // dC: grid = (key groups, token splits), one warp per key.  A tile of up to 256 tokens is staged (g rows in
 // float32 and the CTA's columns of z); the warp sorts the tile's tokens by knot interval (a counting sort
 // over warp votes, so the order, and with it the result, is always the same) and walks the intervals: the
-// order + 1 rows of an interval are summed in registers over all of its tokens and added to the key's
-// accumulator once per interval, where adding every token to its rows would read and write three rows
-// of shared memory for each.  Tokens outside the grid have no weight and leave the lists.
+// rows of an interval are summed in registers over all of its tokens, in a window that slides from interval to
+// interval and adds one finished row to the key's accumulator each time, where adding every token to its rows would
+// read and write three rows of shared memory for each.  Tokens outside the grid have no weight and leave the lists.
 //
 // Bound: instruction issue (about seven warp instructions per pair at r = 32) and one row of g per pair.
 // ---------------------------------------------------------------------------------------------
@@ -643,60 +643,65 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
       }
     }
     __syncwarp();
-    // ---- one interval at a time
-    int end = off[0];
+    // ---- one interval at a time; the window of rows b, b + 1, b + 2 slides along, so each interval finishes one row
+    float a[3][CV][V];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int c = 0; c < CV; ++c)
+#pragma unroll
+        for (int i = 0; i < V; ++i) a[k][c][i] = 0.0f;
+    auto finish_row = [&](int row) {                  // a[0] added to the key's accumulator, the window moved on
+#pragma unroll
+      for (int c = 0; c < CV; ++c) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+#pragma unroll
+          for (int s = LPT; s < kWarp; s <<= 1) a[0][c][i] += __shfl_xor_sync(kFull, a[0][c][i], s);
+        }
+        if (sub == 0) {
+          float* dst = acc + (size_t)row * ap + sl * V + c * (LPT * V);
+          if constexpr (GACC) {
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+              if (sl * V + c * (LPT * V) + i < r) dst[i] += a[0][c][i];
+          } else {
+            float4 d = *reinterpret_cast<float4*>(dst);
+            d.x += a[0][c][0]; d.y += a[0][c][1]; d.z += a[0][c][2]; d.w += a[0][c][3];
+            *reinterpret_cast<float4*>(dst) = d;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) { a[0][c][i] = a[1][c][i]; a[1][c][i] = a[2][c][i]; a[2][c][i] = 0.0f; }
+      }
+    };
+    int end = off[0], dirty = 0;                      // rows of the window that hold something
     for (int b = 0; b < nb; ++b) {
       const int beg = end;
       end = off[b + 1];
-      if (beg == end) continue;
-      float a[3][CV][V];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int c = 0; c < CV; ++c)
-#pragma unroll
-          for (int i = 0; i < V; ++i) a[k][c][i] = 0.0f;
+      if (beg != end) {
+        dirty = 3;
 #pragma unroll 2
-      for (int p = beg + sub; p < end; p += S) {
-        const float4 e = ent[p];
-        const float* gr = gs + (size_t)__float_as_int(e.w) * pitch + sl * V;
+        for (int p = beg + sub; p < end; p += S) {
+          const float4 e = ent[p];
+          const float* gr = gs + (size_t)__float_as_int(e.w) * pitch + sl * V;
 #pragma unroll
-        for (int c = 0; c < CV; ++c) {
-          const float4 g4 = *reinterpret_cast<const float4*>(gr + c * (LPT * V));
-          const float gv[V] = {g4.x, g4.y, g4.z, g4.w};
+          for (int c = 0; c < CV; ++c) {
+            const float4 g4 = *reinterpret_cast<const float4*>(gr + c * (LPT * V));
+            const float gv[V] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
-          for (int i = 0; i < V; ++i) {
-            a[0][c][i] = fmaf(e.x, gv[i], a[0][c][i]);
-            a[1][c][i] = fmaf(e.y, gv[i], a[1][c][i]);
-            a[2][c][i] = fmaf(e.z, gv[i], a[2][c][i]);
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (k == 2 && !three) break;
-#pragma unroll
-        for (int c = 0; c < CV; ++c) {
-#pragma unroll
-          for (int i = 0; i < V; ++i) {
-#pragma unroll
-            for (int s = LPT; s < kWarp; s <<= 1) a[k][c][i] += __shfl_xor_sync(kFull, a[k][c][i], s);
-          }
-          if (sub == 0) {
-            float* dst = acc + (size_t)(b + k) * ap + sl * V + c * (LPT * V);
-            if constexpr (GACC) {
-#pragma unroll
-              for (int i = 0; i < V; ++i)
-                if (sl * V + c * (LPT * V) + i < r) dst[i] += a[k][c][i];
-            } else {
-              float4 d = *reinterpret_cast<float4*>(dst);
-              d.x += a[k][c][0]; d.y += a[k][c][1]; d.z += a[k][c][2]; d.w += a[k][c][3];
-              *reinterpret_cast<float4*>(dst) = d;
+            for (int i = 0; i < V; ++i) {
+              a[0][c][i] = fmaf(e.x, gv[i], a[0][c][i]);
+              a[1][c][i] = fmaf(e.y, gv[i], a[1][c][i]);
+              a[2][c][i] = fmaf(e.z, gv[i], a[2][c][i]);
             }
           }
         }
       }
+      if (dirty > 0) { finish_row(b); --dirty; }
     }
+    if (dirty > 0) finish_row(nb);
+    if (three && dirty > 1) finish_row(nb + 1);
     __syncwarp();
   }
   __syncthreads();
