@@ -88,22 +88,36 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     int most = 512 / (mtiles * rp);
     if (most > 8) most = 8;
     const int chunks = (hp + kch - 1) / kch;
-    o->tiles_total = ((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens;
-    // 0.38 us per tile and chunk of 16 keys at L = 22, r = 32, and the wait for a tile's g; a
-    // CTA's prologue and epilogue; a split's partials written and read again through L2 or HBM
+    o->tiles = (uint32_t)(((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens);
+    // 0.38 us per tile and chunk of 16 keys at L = 22, r = 32, and the wait for a tile's g; a CTA's prologue, an epilogue per
+    // segment; a segment's partials written and read again through L2 or HBM
     const double unit = 0.38 * (split_operands(p) ? 1.6 : 1.0) * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
-    const double per_split = (double)hp * p.L * rp * 8.0 / 5.0e6;
+    const double per_part = (double)hp * p.L * rp * 8.0 / 5.0e6 + 0.1;
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
-      const int64_t slabs = (chunks + slab - 1) / slab;
-      const Split s = best_split(slabs, o->tiles_total, 32, unit * slab + tile, 4.0 + 0.8 * slab, per_split);
-      if (best == 0.0 || s.time < best) {
-        best = s.time;
+      const uint64_t slabs = (chunks + slab - 1) / slab, T = o->tiles;
+      auto take = [&](double t, uint64_t run, uint64_t pitch, uint64_t parts) {
+        if (best != 0.0 && t >= best) return;
+        best = t;
         o->slab_chunks = slab;
-        o->slabs = (int)slabs;
-        o->splits = s.splits;
-        o->tiles_per_split = s.per;
+        o->pitch = (uint32_t)pitch;
+        o->run = (uint32_t)run;
+        o->total = (uint32_t)(slabs * pitch);
+        o->parts = (int)parts;
+      };
+      // runs within a slab
+      uint64_t last = 0;
+      for (uint64_t n = 1; n <= 32; ++n) {
+        const uint64_t run = (T + n - 1) / n, s = (T + run - 1) / run;
+        if (s == last) continue;
+        last = s;
+        const double waves = (double)((slabs * s + kPlanSMs - 1) / kPlanSMs);
+        take(waves * (run * (unit * slab + tile) + 4.0 + 0.8 * slab) + s * per_part, run, run * s, s);
       }
+      // one run per SM over all slabs
+      const uint64_t run = (slabs * T + kPlanSMs - 1) / kPlanSMs;
+      const double segs = (double)((run + T - 1) / T) + 1.0;
+      take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + ((double)T / run + 1.0) * per_part, run, T, (T - 1) / run + 2);
     }
     return true;
   }
@@ -131,7 +145,7 @@ int64_t gimg_tiles(const skv_problem& p) { return ((p.N > 0 ? p.N : 1) + 255) / 
 size_t gimg_bytes(const skv_problem& p) { return align256((size_t)gimg_tiles(p) * 128 * padded_r(p) * 2); }
 
 size_t part_bytes(const skv_problem& p) {
-  int splits = plan_backward(p).dc.splits;
+  int splits = plan_backward(p).dc.parts;
   FusedPlan f;
   if (fused_backward_roles() && plan_fused(p, &f) && f.splits > splits) splits = f.splits;
   return align256((size_t)splits * padded_h(p) * p.L * padded_r(p) * sizeof(float));
@@ -233,11 +247,11 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Z.wait_cycles = wait_cycle_limit();
   Z.status = c.status;
 
-  int dc_splits = 0;
+  DcParts parts{1, 0, 0, 0};
   if (fused) {
     if (fused_launch(fp, p.L, Z, part, c.stream) != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
     note_launches(1);
-    dc_splits = fp.splits;
+    parts.count = fp.splits;
   } else {
     if (dz) {
       const dim3 grid((unsigned)((p.N + 128 * b.dz.groups - 1) / (128 * b.dz.groups)), (unsigned)b.dz.splits);
@@ -264,22 +278,25 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.gring = b.dc.gring;
       P.mtiles = b.dc.mtiles;
       P.slab_chunks = b.dc.slab_chunks;
-      P.tiles_per_split = b.dc.tiles_per_split;
-      P.tiles_total = b.dc.tiles_total;
+      P.tiles = b.dc.tiles;
+      P.pitch = b.dc.pitch;
+      P.run = b.dc.run;
+      P.total = b.dc.total;
       P.status = c.status;
       P.wait_cycles = wait_cycle_limit();
-      if (dc_launch(b.dc, lin, split, P, dim3((unsigned)b.dc.slabs, (unsigned)b.dc.splits), c.stream) != cudaSuccess) {
+      if (dc_launch(b.dc, lin, split, P, dim3((b.dc.total + b.dc.run - 1) / b.dc.run), c.stream) != cudaSuccess) {
         cudaGetLastError();
         return SKV_ERR_LAUNCH;
       }
       note_launches(1);
-      dc_splits = b.dc.splits;
+      parts = {b.dc.pitch % b.dc.run ? 0 : b.dc.parts, b.dc.pitch, b.dc.run,
+               (uint32_t)(b.dc.slab_chunks * 4 * b.dc.kj * p.L)};
     }
   }
   if (dz != user_dz)
     if (int e = launch_unpad(dz, dzs, user_dz, user_dzs, p.N, p.h, p.dz_f32 != 0, c.stream)) return e;
   if (want_dC)
-    return launch_dc_reduce(part, dc_splits, (int64_t)p.h * p.L, (int64_t)hp * p.L, p.r, rp, p.lambda_scale, hdr, dC,
+    return launch_dc_reduce(part, parts, (int64_t)p.h * p.L, (int64_t)hp * p.L, p.r, rp, p.lambda_scale, hdr, dC,
                             dC_cast, c.stream);
   return SKV_OK;
 }

@@ -3,7 +3,9 @@
 //   A CTA owns a slab of keys, keeps the slab's accumulators in tensor memory and streams
 //   64-token tiles: producer groups take turns, each building the f16 Phi tile of its token
 //   tile for one key chunk in its own shared-memory stage while the MMAs of the others run.
-//   The token range is split over CTAs; a reduce kernel sums the splits in a fixed order.
+//   The work, slab after slab and tile after tile within a slab, is cut into equal runs, one per CTA: a run may end one
+//   slab and begin the next (two segments), which fills the chip evenly, or stay within a slab, which saves the
+//   second segment's epilogue and refill where there is little to do (make_dc_plan weighs the two).  A reduce kernel sums the segments of a slab in a fixed order.
 //
 // Where a weight goes.  A pair's three weights are two neighbouring f16x2 words (knot rows 2w, 2w+1 and the next
 // two).  The operand layout (MN-major, un-swizzled) wants 16-byte pieces of eight M rows of one token, four banks
@@ -24,7 +26,7 @@ struct DcParams {
   const __nv_bfloat16* z;
   int64_t zs;
   const __half* gimg;
-  float* part;               // [splits][h*L][r]
+  float* part;               // [segments of a slab][h*L][r]
   int64_t N;
   int h, L, r;
   GridParams g;
@@ -33,8 +35,9 @@ struct DcParams {
   int gring;                 // slots of the ring of g tiles, more than groups
   int mtiles;                // 128-row MMA tiles per chunk
   int slab_chunks;           // chunks per CTA slab
-  int64_t tiles_per_split;   // 64-token tiles per token split
-  int64_t tiles_total;
+  uint32_t tiles;            // 64-token tiles
+  uint32_t pitch;            // places per slab in the runs' count: the tiles, or whole runs (then no run crosses slabs)
+  uint32_t run, total;       // places of a CTA's run, and of all slabs together
   int32_t* status;
   long long wait_cycles;     // limit of every bounded wait, in clock cycles
 };
@@ -48,8 +51,9 @@ constexpr int kDcIssuers = 3;                        // warps that issue MMAs, e
 __host__ __device__ constexpr uint32_t dc_stage_bytes(int mtiles) { return (uint32_t)mtiles * 16u * kDcUnit + kDcUnit; }
 
 // KJ = keys per lane and token (a chunk is 4 * KJ keys), GW = warps per producer group.  SPLIT: a stage is filled twice, with
-// the weights and with their remainders at the same places.
-template <int KJ, int GW, bool LIN, bool SPLIT>
+// the weights and with their remainders at the same places.  RUNS: a run may cross slabs; without it the segment loop is
+// gone at compile time (5 % on the cases that stay within a slab).
+template <int KJ, int GW, bool LIN, bool SPLIT, bool RUNS>
 __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int KCH = 4 * KJ;
@@ -72,10 +76,6 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int mma_warp = NG * GW;
-  const int key0 = blockIdx.x * P.slab_chunks * KCH;
-  const int nchunks = min(P.slab_chunks, (P.h - key0 + KCH - 1) / KCH);
-  const int64_t tile_begin = (int64_t)blockIdx.y * P.tiles_per_split;
-  const int ntiles = (int)min(P.tiles_per_split, P.tiles_total - tile_begin);
   uint32_t tmem_cols = 32;
   while (tmem_cols < (uint32_t)(P.slab_chunks * P.mtiles * r)) tmem_cols <<= 1;
 
@@ -106,193 +106,210 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   pdl_launch();
   pdl_wait();
 
-  if (warp < mma_warp) {
-    // ------------------------------------------------------------------ producers
-    const int pg = warp / GW, wi = warp % GW;
-    const int tq = lane >> 2, kq = lane & 3;
-    // address of this lane's word 0 of key j and token i, less the bias that the word index carries
-    const uint32_t row = smem_u32(phi_base + (size_t)pg * phi_bytes) + (uint32_t)(wi * TI * 128 + tq * 16 + kq * 4) -
-                         kWordBias * kDcUnit;
-    const uint32_t jstep = (uint32_t)P.words * kDcUnit;
-    const int tk0 = wi * TI * 8 + tq;                                // the lane's first token of the tile
-    auto load_z = [&](int ti, int ch, uint32_t (&zv)[TI][KJ / 2]) {
-      const int key = key0 + ch * KCH + KJ * kq;
+  const uint32_t lin_end = min(P.total, (blockIdx.x + 1) * P.run);
+  int seg = 0;
+  // what each role carries from segment to segment
+  int use = 0;                                         // producers: fills of the group's stage
+  uint32_t old[TI][KJ];
+  uint32_t ppar = 0u, gpar0 = 0u, lpar = 1u;           // MMA issuers: phase per group, ring phase; loader: ring phase
+  int slot0 = 0, lslot = 0;
 #pragma unroll
-      for (int i = 0; i < TI; ++i) {
-        const int64_t n = (tile_begin + ti) * kDcTokens + tk0 + 8 * i;
-        const bool ok = ti < ntiles && n < P.N && key < P.h;         // g is zero past N; keys past h are never stored
-        const __nv_bfloat16* src = P.z + n * P.zs + key;
-        if constexpr (KJ == 4) {
-          const uint2 v = ok ? ld8(src) : make_uint2(0, 0);
-          zv[i][0] = v.x;
-          zv[i][1] = v.y;
-        } else {
-          zv[i][0] = ok ? ld4(src) : 0u;
-        }
-      }
-    };
-    uint32_t znext[TI][KJ / 2], old[TI][KJ];
+  for (int i = 0; i < TI; ++i)
 #pragma unroll
-    for (int i = 0; i < TI; ++i)
+    for (int j = 0; j < KJ; ++j) old[i][j] = 0u;
+  for (uint32_t lin = blockIdx.x * P.run; RUNS ? lin < lin_end : seg == 0; ++seg) {
+    const uint32_t slab = lin / P.pitch, tile_begin = lin - slab * P.pitch;
+    const uint32_t places = min(P.pitch - tile_begin, lin_end - lin);
+    const int ntiles = (int)min(P.tiles - tile_begin, places);
+    const int key0 = (int)slab * P.slab_chunks * KCH;
+    const int nchunks = min(P.slab_chunks, (P.h - key0 + KCH - 1) / KCH);
+    lin += places;
+    if (warp < mma_warp) {
+      // ------------------------------------------------------------------ producers
+      const int pg = warp / GW, wi = warp % GW;
+      const int tq = lane >> 2, kq = lane & 3;
+      // address of this lane's word 0 of key j and token i, less the bias that the word index carries
+      const uint32_t row = smem_u32(phi_base + (size_t)pg * phi_bytes) + (uint32_t)(wi * TI * 128 + tq * 16 + kq * 4) -
+                           kWordBias * kDcUnit;
+      const uint32_t jstep = (uint32_t)P.words * kDcUnit;
+      const int tk0 = wi * TI * 8 + tq;                                // the lane's first token of the tile
+      auto load_z = [&](int ti, int ch, uint32_t (&zv)[TI][KJ / 2]) {
+        const int key = key0 + ch * KCH + KJ * kq;
 #pragma unroll
-      for (int j = 0; j < KJ; ++j) old[i][j] = 0u;
-    load_z(pg, 0, znext);
-    int ti = pg, ch = 0;
-    for (int use = 0; ti < ntiles; ++use) {
-      uint32_t x0[TI][KJ], x1[TI][KJ], ad[TI][KJ], r0[SPLIT ? TI : 1][KJ], r1[SPLIT ? TI : 1][KJ];
-#pragma unroll
-      for (int i = 0; i < TI; ++i)
-#pragma unroll
-        for (int q = 0; q < KJ / 2; ++q) {
-          uint32_t a0[2], a1[2], wp[2];
-          phi_pair_words2<LIN, SPLIT>(znext[i][q], P.g, a0, a1, wp, &r0[SPLIT ? i : 0][2 * q], &r1[SPLIT ? i : 0][2 * q]);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            x0[i][2 * q + e] = a0[e];
-            x1[i][2 * q + e] = a1[e];
-            ad[i][2 * q + e] = row + (uint32_t)(i * 128) + (uint32_t)(2 * q + e) * jstep + wp[e] * kDcUnit;
+        for (int i = 0; i < TI; ++i) {
+          const int64_t n = (int64_t)(tile_begin + (uint32_t)ti) * kDcTokens + tk0 + 8 * i;
+          const bool ok = ti < ntiles && n < P.N && key < P.h;         // g is zero past N; keys past h are never stored
+          const __nv_bfloat16* src = P.z + n * P.zs + key;
+          if constexpr (KJ == 4) {
+            const uint2 v = ok ? ld8(src) : make_uint2(0, 0);
+            zv[i][0] = v.x;
+            zv[i][1] = v.y;
+          } else {
+            zv[i][0] = ok ? ld4(src) : 0u;
           }
         }
-      if (++ch == nchunks) { ch = 0; ti += NG; }
-      load_z(ti, ch, znext);                          // the next fill's rows are requested now
-      if (use > 0) {
-        mbar_wait(pempty + pg, (uint32_t)(use - 1) & 1u, wc);
+      };
+      uint32_t znext[TI][KJ / 2];
+      load_z(pg, 0, znext);
+      int ti = pg, ch = 0;
+      for (; ti < ntiles; ++use) {
+        uint32_t x0[TI][KJ], x1[TI][KJ], ad[TI][KJ], r0[SPLIT ? TI : 1][KJ], r1[SPLIT ? TI : 1][KJ];
+#pragma unroll
+        for (int i = 0; i < TI; ++i)
+#pragma unroll
+          for (int q = 0; q < KJ / 2; ++q) {
+            uint32_t a0[2], a1[2], wp[2];
+            phi_pair_words2<LIN, SPLIT>(znext[i][q], P.g, a0, a1, wp, &r0[SPLIT ? i : 0][2 * q], &r1[SPLIT ? i : 0][2 * q]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              x0[i][2 * q + e] = a0[e];
+              x1[i][2 * q + e] = a1[e];
+              ad[i][2 * q + e] = row + (uint32_t)(i * 128) + (uint32_t)(2 * q + e) * jstep + wp[e] * kDcUnit;
+            }
+          }
+        if (++ch == nchunks) { ch = 0; ti += NG; }
+        load_z(ti, ch, znext);                          // the next fill's rows are requested now
+        if (use > 0) {
+          mbar_wait(pempty + pg, (uint32_t)(use - 1) & 1u, wc);
+#pragma unroll
+          for (int i = 0; i < TI; ++i)
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+              sts32(old[i][j], 0u);
+              sts32(old[i][j] + kDcUnit, 0u);
+            }
+        }
+        // keys in ascending order: the linear spline's zero word of a last interval falls on the next key's first
 #pragma unroll
         for (int i = 0; i < TI; ++i)
 #pragma unroll
           for (int j = 0; j < KJ; ++j) {
-            sts32(old[i][j], 0u);
-            sts32(old[i][j] + kDcUnit, 0u);
-          }
-      }
-      // keys in ascending order: the linear spline's zero word of a last interval falls on the next key's first
-#pragma unroll
-      for (int i = 0; i < TI; ++i)
-#pragma unroll
-        for (int j = 0; j < KJ; ++j) {
-          sts32(ad[i][j], x0[i][j]);
-          sts32(ad[i][j] + kDcUnit, x1[i][j]);
-          old[i][j] = ad[i][j];
-        }
-      fence_async_smem();
-      mbar_arrive_warp(pfull + pg);
-      if constexpr (SPLIT) {
-        ++use;
-        mbar_wait(pempty + pg, (uint32_t)(use - 1) & 1u, wc);
-#pragma unroll
-        for (int i = 0; i < TI; ++i)
-#pragma unroll
-          for (int j = 0; j < KJ; ++j) {
-            sts32(ad[i][j], r0[i][j]);
-            sts32(ad[i][j] + kDcUnit, r1[i][j]);
+            sts32(ad[i][j], x0[i][j]);
+            sts32(ad[i][j] + kDcUnit, x1[i][j]);
+            old[i][j] = ad[i][j];
           }
         fence_async_smem();
         mbar_arrive_warp(pfull + pg);
-      }
-    }
-    // ---- epilogue: accumulators -> float32 partial of this token split
-    mbar_wait(done, 0, wc);
-    tc_fence_after();
-    const int lane_row = (warp & 3) * 32 + lane;
-    float* part = P.part + (size_t)blockIdx.y * P.h * L * r;
-    for (int e = warp >> 2; e < nchunks * P.mtiles; e += mma_warp >> 2) {
-      const int c = e / P.mtiles, mt = e - c * P.mtiles;
-      const int unit = mt * 16 + (lane_row >> 3), j = unit / P.words;
-      const int bb = 2 * (unit - j * P.words) + (lane_row & 1);
-      const int key = key0 + c * KCH + KJ * ((lane_row & 7) >> 1) + j;
-      const bool ok = j < KJ && key < P.h && bb < L;                   // the pad row of an odd L is dropped
-      float* dst = part + ((size_t)key * L + bb) * r;
-      const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(e * r);
-      for (int c0 = 0; c0 < r; c0 += 16) {
-        float v[16];
-        tmem_ld16(taddr + c0, v);
-        if (ok) {
+        if constexpr (SPLIT) {
+          ++use;
+          mbar_wait(pempty + pg, (uint32_t)(use - 1) & 1u, wc);
 #pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          for (int i = 0; i < TI; ++i)
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+              sts32(ad[i][j], r0[i][j]);
+              sts32(ad[i][j] + kDcUnit, r1[i][j]);
+            }
+          fence_async_smem();
+          mbar_arrive_warp(pfull + pg);
+        }
+      }
+      // ---- epilogue: accumulators -> float32 partial of this token split
+      mbar_wait(done, (uint32_t)seg & 1u, wc);
+      tc_fence_after();
+      const int lane_row = (warp & 3) * 32 + lane;
+      float* part = P.part + (size_t)(blockIdx.x - slab * P.pitch / P.run) * P.h * L * r;
+      for (int e = warp >> 2; e < nchunks * P.mtiles; e += mma_warp >> 2) {
+        const int c = e / P.mtiles, mt = e - c * P.mtiles;
+        const int unit = mt * 16 + (lane_row >> 3), j = unit / P.words;
+        const int bb = 2 * (unit - j * P.words) + (lane_row & 1);
+        const int key = key0 + c * KCH + KJ * ((lane_row & 7) >> 1) + j;
+        const bool ok = j < KJ && key < P.h && bb < L;                   // the pad row of an odd L is dropped
+        float* dst = part + ((size_t)key * L + bb) * r;
+        const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(e * r);
+        for (int c0 = 0; c0 < r; c0 += 16) {
+          float v[16];
+          tmem_ld16(taddr + c0, v);
+          if (ok) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+              *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          }
+        }
+      }
+      tc_fence_before();
+    } else if (warp < mma_warp + kDcIssuers) {
+      // ------------------------------------------------------------------ MMA issue
+      if (elect_one()) {
+        const int m0 = warp - mma_warp;
+        const uint32_t idesc = instr_desc(0, 0, 1, 1, 128, r);
+        const uint32_t ab_hi = desc_hi(kDcUnit);
+        const uint32_t a_tile0 = desc_lo(smem_u32(phi_base) + (uint32_t)m0 * 16u * kDcUnit, 128u);
+        const uint32_t b_ring = desc_lo(smem_u32(g_base), 128u);
+        bool drain = false;
+        for (int tp = 0; tp < ntiles && !drain; tp += NG) {
+          const int npg = min(NG, ntiles - tp);
+          constexpr int kParts = SPLIT ? 2 : 1;
+          for (int cp = 0; cp < nchunks * kParts && !drain; ++cp) {
+            const int ch = cp / kParts, part = cp % kParts;
+            const bool last = cp + 1 == nchunks * kParts;
+            int slot = slot0;
+            uint32_t gpar = gpar0;
+            for (int pg = 0; pg < npg; ++pg) {
+              if (cp == 0) drain = drain || mbar_wait(gfull + slot, gpar, wc);
+              drain = drain || mbar_wait(pfull + pg, (ppar >> pg) & 1u, wc);
+              ppar ^= 1u << pg;
+              if (drain) break;                          // draining: issue nothing more
+              tc_fence_after();
+              uint32_t a_lo0 = a_tile0 + (uint32_t)pg * (phi_bytes >> 4);
+              const uint32_t b_lo0 = b_ring + (uint32_t)slot * (g_bytes >> 4);
+              uint32_t d_addr = tmem_base + (uint32_t)((ch * P.mtiles + m0) * r);
+              const uint32_t first = tp + pg + part == 0 ? 0u : 1u;
+              for (int mt = m0; mt < P.mtiles; mt += kDcIssuers) {
+#pragma unroll
+                for (int ks = 0; ks < kDcTokens / 16; ++ks)
+                  umma_f16_split(d_addr, a_lo0 + (uint32_t)ks * 16u, ab_hi, b_lo0 + (uint32_t)ks * 16u, ab_hi, idesc,
+                                 ks > 0 ? 1u : first);
+                a_lo0 += (kDcIssuers * 16u * kDcUnit) >> 4;
+                d_addr += (uint32_t)(kDcIssuers * r);
+              }
+              umma_commit(pempty + pg);
+              if (last) umma_commit(gempty + slot);
+              if (++slot == GR) { slot = 0; gpar ^= 1u; }
+            }
+            if (last) { slot0 = slot; gpar0 = gpar; }
+          }
+        }
+        umma_commit(done);
+      }
+    } else {
+      // ------------------------------------------------------------------ gradient-tile loader
+      if (elect_one()) {
+        const uint8_t* img = reinterpret_cast<const uint8_t*>(P.gimg);
+        int slot = lslot;
+        uint32_t par = lpar;                             // a fresh barrier passes a wait for the phase before its first
+        for (int ti = 0; ti < ntiles; ++ti) {
+          mbar_wait(gempty + slot, par, wc);
+          if (*abort_flag) break;
+          mbar_arrive_expect_tx(gfull + slot, g_bytes);
+          // the image has 128-token tiles [r/8][16 token groups][128 B]; this tile is one half of each channel group
+          const int64_t t64 = (int64_t)tile_begin + ti;
+          const uint8_t* src = img + (size_t)(t64 >> 1) * 128 * r * 2 + (size_t)(t64 & 1) * kDcUnit;
+          for (int cg = 0; cg < r / 8; ++cg)
+            bulk_g2s(g_base + (size_t)slot * g_bytes + (size_t)cg * kDcUnit, src + (size_t)cg * 2 * kDcUnit, kDcUnit,
+                     gfull + slot);
+          if (++slot == GR) { slot = 0; par ^= 1u; }
+        }
+        lslot = slot;
+        lpar = par;
+        if (*abort_flag) {
+          const long long t0 = clock64();
+          while (clock64() - t0 < 2000000) {}
         }
       }
     }
     tc_fence_before();
-  } else if (warp < mma_warp + kDcIssuers) {
-    // ------------------------------------------------------------------ MMA issue
-    if (elect_one()) {
-      const int m0 = warp - mma_warp;
-      const uint32_t idesc = instr_desc(0, 0, 1, 1, 128, r);
-      const uint32_t ab_hi = desc_hi(kDcUnit);
-      const uint32_t a_tile0 = desc_lo(smem_u32(phi_base) + (uint32_t)m0 * 16u * kDcUnit, 128u);
-      const uint32_t b_ring = desc_lo(smem_u32(g_base), 128u);
-      uint32_t fills = 0;                              // of every group so far
-      int slot0 = 0;                                   // ring slot and phase of the round's first tile
-      uint32_t gpar0 = 0u;
-      bool drain = false;
-      for (int tp = 0; tp < ntiles && !drain; tp += NG) {
-        const int npg = min(NG, ntiles - tp);
-        constexpr int kParts = SPLIT ? 2 : 1;
-        for (int cp = 0; cp < nchunks * kParts && !drain; ++cp, ++fills) {
-          const int ch = cp / kParts, part = cp % kParts;
-          const bool last = cp + 1 == nchunks * kParts;
-          int slot = slot0;
-          uint32_t gpar = gpar0;
-          for (int pg = 0; pg < npg; ++pg) {
-            if (cp == 0) drain = drain || mbar_wait(gfull + slot, gpar, wc);
-            drain = drain || mbar_wait(pfull + pg, fills & 1u, wc);
-            if (drain) break;                          // draining: issue nothing more
-            tc_fence_after();
-            uint32_t a_lo0 = a_tile0 + (uint32_t)pg * (phi_bytes >> 4);
-            const uint32_t b_lo0 = b_ring + (uint32_t)slot * (g_bytes >> 4);
-            uint32_t d_addr = tmem_base + (uint32_t)((ch * P.mtiles + m0) * r);
-            const uint32_t first = tp + pg + part == 0 ? 0u : 1u;
-            for (int mt = m0; mt < P.mtiles; mt += kDcIssuers) {
-#pragma unroll
-              for (int ks = 0; ks < kDcTokens / 16; ++ks)
-                umma_f16_split(d_addr, a_lo0 + (uint32_t)ks * 16u, ab_hi, b_lo0 + (uint32_t)ks * 16u, ab_hi, idesc,
-                               ks > 0 ? 1u : first);
-              a_lo0 += (kDcIssuers * 16u * kDcUnit) >> 4;
-              d_addr += (uint32_t)(kDcIssuers * r);
-            }
-            umma_commit(pempty + pg);
-            if (last) umma_commit(gempty + slot);
-            if (++slot == GR) { slot = 0; gpar ^= 1u; }
-          }
-          if (last) { slot0 = slot; gpar0 = gpar; }
-        }
-      }
-      umma_commit(done);
-    }
-  } else {
-    // ------------------------------------------------------------------ gradient-tile loader
-    if (elect_one()) {
-      const uint8_t* img = reinterpret_cast<const uint8_t*>(P.gimg);
-      int slot = 0;
-      uint32_t par = 1u;                               // a fresh barrier passes a wait for the phase before its first
-      for (int ti = 0; ti < ntiles; ++ti) {
-        mbar_wait(gempty + slot, par, wc);
-        if (*abort_flag) break;
-        mbar_arrive_expect_tx(gfull + slot, g_bytes);
-        // the image has 128-token tiles [r/8][16 token groups][128 B]; this tile is one half of each channel group
-        const int64_t t64 = tile_begin + ti;
-        const uint8_t* src = img + (size_t)(t64 >> 1) * 128 * r * 2 + (size_t)(t64 & 1) * kDcUnit;
-        for (int cg = 0; cg < r / 8; ++cg)
-          bulk_g2s(g_base + (size_t)slot * g_bytes + (size_t)cg * kDcUnit, src + (size_t)cg * 2 * kDcUnit, kDcUnit,
-                   gfull + slot);
-        if (++slot == GR) { slot = 0; par ^= 1u; }
-      }
-      if (*abort_flag) {
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000) {}
-      }
-    }
+    __syncthreads();                                     // the accumulators have been read
+    tc_fence_after();
   }
-  __syncthreads();
   if (warp == mma_warp) {
-    mbar_wait_drain(done, 0, P.wait_cycles);
+    mbar_wait_drain(done, (uint32_t)(seg - 1) & 1u, P.wait_cycles);
     tc_fence_after();
     tmem_free(tmem_base, tmem_cols);
   }
 }
 
-struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, slabs, splits; int64_t tiles_total, tiles_per_split; size_t smem; };
+struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, parts; uint32_t tiles, pitch, run, total; size_t smem; };
 
 }  // namespace tc
 }  // namespace skv

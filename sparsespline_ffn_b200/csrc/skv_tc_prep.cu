@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
   }
 }
 
-__global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, int splits, int64_t rows,
+__global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, const DcParts parts, int64_t rows,
                                                            int64_t rows_padded, int r, int rp, float lambda,
                                                            const uint32_t* hdr, float* dC,
                                                            __nv_bfloat16* dC_cast) {
@@ -245,6 +245,11 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, in
   const bool vec = r == rp && ((reinterpret_cast<uintptr_t>(dC) | reinterpret_cast<uintptr_t>(dC_cast)) & 15) == 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(part) + i;
+    int splits = parts.count;
+    if (splits == 0) {
+      const uint32_t slab = (uint32_t)(i / q4) / parts.slab_rows;
+      splits = (int)(((slab + 1) * parts.pitch - 1) / parts.run - slab * parts.pitch / parts.run) + 1;
+    }
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 8
     for (int k = 0; k < splits; ++k) {
@@ -319,11 +324,11 @@ int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, 
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }
 
-int launch_dc_reduce(const float* part, int splits, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
+int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
                      const uint32_t* hdr, float* dC, void* dC_cast, cudaStream_t stream) {
   const dim3 grid((unsigned)blocks_for(rows * (rp / 4), 1, kPlanSMs * 16));
   const cudaError_t e =
-      launch_chained<tc_dc_reduce_kernel>(grid, 256, 0, stream, part, splits, rows, rows_padded, r, rp, lambda, hdr, dC,
+      launch_chained<tc_dc_reduce_kernel>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda, hdr, dC,
                                           static_cast<__nv_bfloat16*>(dC_cast));
   note_launches(1);
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;

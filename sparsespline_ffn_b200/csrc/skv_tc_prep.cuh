@@ -71,8 +71,12 @@ int launch_prep(PrepParams& P, cudaStream_t stream);
 int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,
                     void* out, int64_t ds, bool out_f32, cudaStream_t stream);
 
-// dC = lambda * 2^-k * sum over splits of part[split][row][c] for `rows` knot rows.
-int launch_dc_reduce(const float* part, int splits, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
+// How many partials a knot row of dC has: `count`, or (count = 0) the number of runs of `run` places that touch the row's slab of
+// `slab_rows` rows and `pitch` places.
+struct DcParts { int count; uint32_t pitch, run, slab_rows; };
+
+// dC = lambda * 2^-k * sum over the partials part[i][row][c] for `rows` knot rows.
+int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
                      const uint32_t* hdr, float* dC, void* dC_cast, cudaStream_t stream);
 
 // dst[n][j] = src[n][j], j < h, from padded rows.
