@@ -190,6 +190,15 @@ int skv_feature_forward_noalloc(const skv_problem *p, const void *z, int64_t z_s
 enum skv_debug { SKV_DEBUG_WAIT_CYCLES = 0, SKV_DEBUG_SKIP_FIRST_COPY = 1, SKV_DEBUG_FUSED_BACKWARD = 2 };
 int skv_debug_set(int what, int64_t value);
 
+/* How the tcgen05 dC kernel would cut this problem's work, for tests of the planner; needs no GPU.  The work is
+ * slab after slab (a slab = some keys) of `pitch` places each, cut into runs of `run` places, one per CTA;
+ * place t < `tiles` of a slab is 64 tokens.  A run leaves one partial of dC for every slab that it touches, in slot
+ * (its index - index of the first run that touches the slab).
+ *   out[8] = { 1 if a run may cross slabs, tiles, pitch, run, places of all slabs, slots the scratch has room for,
+ *              keys per slab, partials that are added for the rows of `slab` }
+ * SKV_ERR_UNSUPPORTED when the problem does not run on the tcgen05 kernels. */
+int skv_debug_dc_plan(const skv_problem *p, int64_t slab, int64_t *out);
+
 /* Number of kernels this library has launched in this process so far (host-side counter).  No
  * counterpart in the reference; benchmarks use the difference around a timed region to report
  * how many of the library's own kernels ran inside it. */

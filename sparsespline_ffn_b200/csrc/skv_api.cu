@@ -24,6 +24,7 @@ int fused_backward_roles() { return g_fused_bwd.load(std::memory_order_relaxed);
 
 namespace skv {
 namespace tc {
+void describe_dc_plan(const skv_problem& p, int64_t slab, int64_t* out);
 bool readout_eligible(const skv_problem& p, int64_t D);
 size_t readout_image_bytes(const skv_problem& p, int64_t D);
 int64_t readout_delta_pitch(const skv_problem& p);
@@ -155,6 +156,14 @@ int skv_debug_set(int what, int64_t value) {
     default:
       return SKV_ERR_UNSUPPORTED;
   }
+}
+
+int skv_debug_dc_plan(const skv_problem* p, int64_t slab, int64_t* out) {
+  if (int e = validate(p)) return e;
+  if (!out) return SKV_ERR_NULL;
+  if (resolve(*p) != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;
+  tc::describe_dc_plan(*p, slab, out);
+  return SKV_OK;
 }
 
 int skv_resolve_impl(const skv_problem* p) {

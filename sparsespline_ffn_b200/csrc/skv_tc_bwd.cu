@@ -96,10 +96,11 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
       const uint64_t slabs = (chunks + slab - 1) / slab, T = o->tiles;
-      auto take = [&](double t, uint64_t run, uint64_t pitch, uint64_t parts) {
+      auto take = [&](double t, bool runs, uint64_t run, uint64_t pitch, uint64_t parts) {
         if (best != 0.0 && t >= best) return;
         best = t;
         o->slab_chunks = slab;
+        o->runs = runs;
         o->pitch = (uint32_t)pitch;
         o->run = (uint32_t)run;
         o->total = (uint32_t)(slabs * pitch);
@@ -112,12 +113,15 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
         if (s == last) continue;
         last = s;
         const double waves = (double)((slabs * s + kPlanSMs - 1) / kPlanSMs);
-        take(waves * (run * (unit * slab + tile) + 4.0 + 0.8 * slab) + s * per_part, run, run * s, s);
+        take(waves * (run * (unit * slab + tile) + 4.0 + 0.8 * slab) + s * per_part, false, run, run * s, s);
       }
-      // one run per SM over all slabs
+      // One run per SM over all slabs.  Where a slab is a whole number of runs none crosses: as many partials as runs then,
+      // else up to one more than fit, the first and the last of them shorter.
       const uint64_t run = (slabs * T + kPlanSMs - 1) / kPlanSMs;
       const double segs = (double)((run + T - 1) / T) + 1.0;
-      take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + ((double)T / run + 1.0) * per_part, run, T, (T - 1) / run + 2);
+      const bool cross = T % run != 0;
+      take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + ((double)T / run + 1.0) * per_part, cross, run, T,
+           cross ? (T - 1) / run + 2 : T / run);
     }
     return true;
   }
@@ -135,6 +139,11 @@ const BwdPlan& plan_backward(const skv_problem& p) {
     last = {p.N, p.h, p.L, p.r, p.spline_order, b};
   }
   return last.b;
+}
+
+// What the reduce adds for the knot rows of a slab under this plan.
+DcParts dc_parts(const DcPlan& d, int L) {
+  return {d.runs ? 0 : d.parts, d.pitch, d.run, (uint32_t)(d.slab_chunks * 4 * d.kj * L)};
 }
 
 size_t timg_bytes(const skv_problem& p) {
@@ -157,6 +166,13 @@ size_t row_bytes(const skv_problem& p, int esz) { return align256((size_t)(p.N >
 }  // namespace
 
 bool bwd_eligible(const skv_problem& p) { return fwd_eligible(p) && plan_backward(p).ok; }
+
+void describe_dc_plan(const skv_problem& p, int64_t slab, int64_t* out) {
+  const DcPlan& d = plan_backward(p).dc;
+  const int64_t v[8] = {d.runs, d.tiles, d.pitch, d.run, d.total, d.parts, d.slab_chunks * 4 * d.kj,
+                        dc_parts(d, p.L).of((uint32_t)slab)};
+  for (int i = 0; i < 8; ++i) out[i] = v[i];
+}
 
 size_t bwd_scratch_bytes(const skv_problem& p, bool rows_ok) {
   return kHeaderBytes + gimg_bytes(p) + timg_bytes(p) + part_bytes(p) +
@@ -289,8 +305,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
         return SKV_ERR_LAUNCH;
       }
       note_launches(1);
-      parts = {b.dc.pitch % b.dc.run ? 0 : b.dc.parts, b.dc.pitch, b.dc.run,
-               (uint32_t)(b.dc.slab_chunks * 4 * b.dc.kj * p.L)};
+      parts = dc_parts(b.dc, p.L);
     }
   }
   if (dz != user_dz)

@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   }
 }
 
-struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, parts; uint32_t tiles, pitch, run, total; size_t smem; };
+// `runs`: a run may cross slabs; the template case, the number of partials of a slab and the room for them all follow it.
+struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, parts; bool runs; uint32_t tiles, pitch, run, total; size_t smem; };
 
 }  // namespace tc
 }  // namespace skv

@@ -245,11 +245,7 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
   const bool vec = r == rp && ((reinterpret_cast<uintptr_t>(dC) | reinterpret_cast<uintptr_t>(dC_cast)) & 15) == 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(part) + i;
-    int splits = parts.count;
-    if (splits == 0) {
-      const uint32_t slab = (uint32_t)(i / q4) / parts.slab_rows;
-      splits = (int)(((slab + 1) * parts.pitch - 1) / parts.run - slab * parts.pitch / parts.run) + 1;
-    }
+    const int splits = parts.count ? parts.count : parts.of((uint32_t)(i / q4) / parts.slab_rows);
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 8
     for (int k = 0; k < splits; ++k) {

@@ -73,7 +73,13 @@ int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, 
 
 // How many partials a knot row of dC has: `count`, or (count = 0) the number of runs of `run` places that touch the row's slab of
 // `slab_rows` rows and `pitch` places.
-struct DcParts { int count; uint32_t pitch, run, slab_rows; };
+struct DcParts {
+  int count;
+  uint32_t pitch, run, slab_rows;
+  __host__ __device__ int of(uint32_t slab) const {
+    return count ? count : (int)(((slab + 1) * pitch - 1) / run - slab * pitch / run) + 1;
+  }
+};
 
 // dC = lambda * 2^-k * sum over the partials part[i][row][c] for `rows` knot rows.
 int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
