@@ -43,7 +43,7 @@ enum skv_dtype { SKV_BF16 = 0, SKV_F32 = 1 };
 enum skv_activation { SKV_ACT_RELU_SQ = 0, SKV_ACT_IDENTITY = 1, SKV_ACT_GELU = 2 };
 /* SKV_IMPL_AUTO picks the tcgen05 kernels when the shape is eligible (bf16, r up to 128, L up to 64, either
  * spline order; other h and r than multiples of 8 and 16 are padded inside the scratch) and the CUDA-core
- * kernels otherwise, and for forwards of a few tokens.  The CUDA-core kernels are the float32 tier and the path of
+ * kernels otherwise, for forwards of a few tokens and for backwards of 2^31 - 256 tokens or more.  The CUDA-core kernels are the float32 tier and the path of
  * the remaining shapes, several times slower at production sizes: skv_resolve_impl tells which family a
  * problem gets. */
 enum skv_impl { SKV_IMPL_AUTO = 0, SKV_IMPL_SIMT = 1, SKV_IMPL_TCGEN05 = 2 };

@@ -51,9 +51,9 @@ int validate(const skv_problem* p) {
   return SKV_OK;
 }
 
-int resolve(const skv_problem& p) {
+int resolve(const skv_problem& p, int op) {
   if (p.impl == SKV_IMPL_SIMT) return SKV_IMPL_SIMT;
-  const bool ok = tc_eligible(p);
+  const bool ok = tc_eligible(p, op);
   if (p.impl == SKV_IMPL_TCGEN05) return ok ? (int)SKV_IMPL_TCGEN05 : (int)SKV_ERR_UNSUPPORTED;
   return ok && tc_worthwhile(p) ? (int)SKV_IMPL_TCGEN05 : (int)SKV_IMPL_SIMT;
 }
@@ -161,19 +161,19 @@ int skv_debug_set(int what, int64_t value) {
 int skv_debug_dc_plan(const skv_problem* p, int64_t slab, int64_t* out) {
   if (int e = validate(p)) return e;
   if (!out) return SKV_ERR_NULL;
-  if (resolve(*p) != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;
+  if (resolve(*p, SKV_OP_BACKWARD) != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;
   tc::describe_dc_plan(*p, slab, out);
   return SKV_OK;
 }
 
 int skv_resolve_impl(const skv_problem* p) {
   if (int e = validate(p)) return e;
-  return resolve(*p);
+  return resolve(*p, SKV_OP_BACKWARD);
 }
 
 size_t skv_scratch_bytes(const skv_problem* p, int op) {
   if (validate(p) != SKV_OK) return 0;
-  const int impl = resolve(*p);
+  const int impl = resolve(*p, op);
   if (impl == SKV_IMPL_SIMT) return simt_scratch_bytes(*p, op);
   if (impl != SKV_IMPL_TCGEN05) return 0;
   size_t need = tc_scratch_bytes(*p, op, rows_fit(*p));
@@ -192,7 +192,7 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
   if (p->N == 0) return SKV_OK;
   if (!z || !C || !delta_out) return SKV_ERR_NULL;
   if (z_stride < p->h || delta_stride < p->r || (act_out && act_stride < p->h)) return SKV_ERR_SHAPE;
-  const int impl = resolve(*p);
+  const int impl = resolve(*p, SKV_OP_FORWARD);
   if (impl < 0) return impl;
   const bool small = small_forward(*p);
   if (impl == SKV_IMPL_TCGEN05 && !small) {
@@ -225,7 +225,7 @@ int skv_feature_backward(const skv_problem* p, const void* z, int64_t z_stride, 
   if (!dz && !dC_f32 && !dC_cast) return SKV_OK;
   if (z_stride < p->h || gdelta_stride < p->r || (g_act && gact_stride < p->h) || (dz && dz_stride < p->h))
     return SKV_ERR_SHAPE;
-  const int impl = resolve(*p);
+  const int impl = resolve(*p, SKV_OP_BACKWARD);
   if (impl < 0) return impl;
   const bool dz32 = p->dz_f32 && p->dtype == SKV_BF16;          // float32 dz of a bf16 problem: tcgen05 kernels only
   if (dz32 && impl != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;

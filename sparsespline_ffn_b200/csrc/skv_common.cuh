@@ -133,7 +133,7 @@ int simt_knot_index(const LaunchCtx& c, const void* z, int64_t zs, int32_t* bins
 
 // tcgen05 kernel family (bf16, eligible shapes only).  `rows_ok`: the rows of z, act_out, g_act and dz start
 // on 16-byte boundaries and hold whole chunks of eight keys; otherwise they are copied to rows that do.
-bool tc_eligible(const skv_problem& p);
+bool tc_eligible(const skv_problem& p, int op);
 bool tc_worthwhile(const skv_problem& p);    // of an eligible problem
 size_t tc_scratch_bytes(const skv_problem& p, int op, bool rows_ok);
 int tc_forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* act_out, int64_t as,

@@ -37,7 +37,11 @@ bool make_map_2d(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols,
 }
 }  // namespace tc
 
-bool tc_eligible(const skv_problem& p) { return tc::bwd_eligible(p); }
+// A forward on these kernels is for a backward on them, but only the backward's count of tokens is limited: dz addresses the
+// rows of a token tile by a 32-bit TMA coordinate (tiles are of 256 tokens at most).
+bool tc_eligible(const skv_problem& p, int op) {
+  return tc::bwd_eligible(p) && (op == SKV_OP_FORWARD || p.N < (1ll << 31) - 256);
+}
 
 // Split operands double the work, and half a tile of tokens or less leaves most of it to padding; the CUDA-core kernels
 // are as fast there.

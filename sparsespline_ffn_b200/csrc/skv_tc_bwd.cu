@@ -88,7 +88,9 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     int most = 512 / (mtiles * rp);
     if (most > 8) most = 8;
     const int chunks = (hp + kch - 1) / kch;
-    o->tiles = (uint32_t)(((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens);
+    const int64_t tiles = ((p.N > 0 ? p.N : 1) + kDcTokens - 1) / kDcTokens;
+    if (tiles >= 1ll << 31) return false;                    // places are counted in 32 bits
+    o->tiles = (uint32_t)tiles;
     // 0.38 us per tile and chunk of 16 keys at L = 22, r = 32, and the wait for a tile's g; a CTA's prologue, an epilogue per
     // segment; a segment's partials written and read again through L2 or HBM
     const double unit = 0.38 * (split_operands(p) ? 1.6 : 1.0) * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
@@ -97,7 +99,7 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
       const uint64_t slabs = (chunks + slab - 1) / slab, T = o->tiles;
       auto take = [&](double t, bool runs, uint64_t run, uint64_t pitch, uint64_t parts) {
-        if (best != 0.0 && t >= best) return;
+        if ((best != 0.0 && t >= best) || slabs * pitch >= 1ull << 31) return;
         best = t;
         o->slab_chunks = slab;
         o->runs = runs;
@@ -123,7 +125,7 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
       take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + ((double)T / run + 1.0) * per_part, cross, run, T,
            cross ? (T - 1) / run + 2 : T / run);
     }
-    return true;
+    return best != 0.0;
   }
   return false;
 }

@@ -70,3 +70,24 @@ def test_partials_over_the_range_of_shapes(lib):
         checked += _check(lib, N, int(2 ** rng.uniform(0, 12.5)), rng.randint(4, 64),
                           rng.choice([1, 16, 20, 32, 64, 96, 128]), order)
     assert checked > 200
+
+
+def test_token_and_place_counts_stay_within_32_bits(lib):
+    def problem(N, h, r=16, impl=0):
+        return _lib.Problem(N=N, h=h, L=22, r=r, grid_lo=-3.0, scale=1.0, lambda_scale=1.0, activation=0, dtype=0, impl=impl)
+
+    def resolve(*a, **k):
+        return lib.skv_resolve_impl(ctypes.byref(problem(*a, **k)))
+
+    # dz addresses a tile's rows by a 32-bit coordinate: beyond it, the CUDA-core kernels
+    last = 2**31 - 257
+    assert resolve(last, 8) == _lib.SKV_IMPL["tcgen05"]
+    for N in (last + 1, 2**31, 2**32, 2**40):
+        assert resolve(N, 8) == _lib.SKV_IMPL["simt"] and resolve(N, 8, impl=2) == -3
+        for op in (_lib.SKV_OP_FORWARD, _lib.SKV_OP_BACKWARD):
+            assert lib.skv_scratch_bytes(ctypes.byref(problem(N, 8)), op) < 2**63
+    # dC counts 64-token tiles of all slabs in 32 bits
+    for N, h in ((last, 5120), (2**30, 1 << 20), (2**28, 1 << 24)):
+        if resolve(N, h, r=128) == _lib.SKV_IMPL["tcgen05"]:
+            d = _plan(lib, problem(N, h, r=128))
+            assert d["total"] == -(-h // d["keys"]) * d["pitch"] < 2**31 and d["tiles"] <= d["pitch"]
