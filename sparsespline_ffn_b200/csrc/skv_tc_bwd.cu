@@ -95,6 +95,13 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     // segment; a segment's partials written and read again through L2 or HBM
     const double unit = 0.38 * (split_operands(p) ? 1.6 : 1.0) * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
     const double per_part = (double)hp * p.L * rp * 8.0 / 5.0e6 + 0.1;
+    o->chain = split_operands(p) ? kDcSplitChain : kDcChain;
+    // what a CTA pays for the segments of a slab after its first: its accumulators' way to the partial (10 us for 480
+    // columns of tensor memory, 3.4 us for 96)
+    auto flush = [&](uint64_t run, uint64_t T, int slab) {
+      const uint64_t len = run < T ? run : T;
+      return (double)((len - 1) / o->chain * (run / len)) * (1.5 + 0.018 * slab * mtiles * rp);
+    };
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {
       const uint64_t slabs = (chunks + slab - 1) / slab, T = o->tiles;
@@ -115,15 +122,16 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
         if (s == last) continue;
         last = s;
         const double waves = (double)((slabs * s + kPlanSMs - 1) / kPlanSMs);
-        take(waves * (run * (unit * slab + tile) + 4.0 + 0.8 * slab) + s * per_part, false, run, run * s, s);
+        take(waves * (run * (unit * slab + tile) + 4.0 + 0.8 * slab + flush(run, T, slab)) + s * per_part, false, run,
+             run * s, s);
       }
       // One run per SM over all slabs.  Where a slab is a whole number of runs none crosses: as many partials as runs then,
       // else up to one more than fit, the first and the last of them shorter.
       const uint64_t run = (slabs * T + kPlanSMs - 1) / kPlanSMs;
       const double segs = (double)((run + T - 1) / T) + 1.0;
       const bool cross = T % run != 0;
-      take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + ((double)T / run + 1.0) * per_part, cross, run, T,
-           cross ? (T - 1) / run + 2 : T / run);
+      take(run * (unit * slab + tile) + 4.0 + segs * (0.8 * slab + 6.0) + flush(run, T, slab) +
+               ((double)T / run + 1.0) * per_part, cross, run, T, cross ? (T - 1) / run + 2 : T / run);
     }
     return best != 0.0;
   }
@@ -300,6 +308,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       P.pitch = b.dc.pitch;
       P.run = b.dc.run;
       P.total = b.dc.total;
+      P.chain = b.dc.chain;
       P.status = c.status;
       P.wait_cycles = wait_cycle_limit();
       if (dc_launch(b.dc, lin, split, P, dim3((b.dc.total + b.dc.run - 1) / b.dc.run), c.stream) != cudaSuccess) {

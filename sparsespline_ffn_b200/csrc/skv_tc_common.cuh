@@ -238,6 +238,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Four float32 added (one rounding each) to four in global memory, without waiting for them.
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 // Shared-memory matrix descriptor of an un-swizzled canonical tile: 8 x 16-byte core matrices,
 // `lbo` = byte stride between core matrices along K, `sbo` = byte stride along M/N.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {

@@ -15,10 +15,11 @@ cudaError_t dc_launch_case(const DcPlan& dp, bool lin, bool split, const DcParam
 }  // namespace
 
 cudaError_t dc_launch(const DcPlan& dp, bool lin, bool split, const DcParams& P, dim3 grid, cudaStream_t stream) {
+  const bool segments = dp.runs || dp.run > dp.chain;
 #define SKV_DC_CASE(KJ_, GW_)                                                                   \
   if (dp.kj == KJ_ && dp.gw == GW_)                                                             \
-    return dp.runs ? dc_launch_case<KJ_, GW_, true>(dp, lin, split, P, grid, stream)            \
-                   : dc_launch_case<KJ_, GW_, false>(dp, lin, split, P, grid, stream);
+    return segments ? dc_launch_case<KJ_, GW_, true>(dp, lin, split, P, grid, stream)           \
+                    : dc_launch_case<KJ_, GW_, false>(dp, lin, split, P, grid, stream);
   SKV_DC_CASE(4, 4) SKV_DC_CASE(4, 8) SKV_DC_CASE(2, 4) SKV_DC_CASE(2, 8)
 #undef SKV_DC_CASE
   return cudaErrorInvalidValue;

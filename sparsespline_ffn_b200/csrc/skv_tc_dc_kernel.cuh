@@ -4,8 +4,10 @@
 //   64-token tiles: producer groups take turns, each building the f16 Phi tile of its token
 //   tile for one key chunk in its own shared-memory stage while the MMAs of the others run.
 //   The work, slab after slab and tile after tile within a slab, is cut into equal runs, one per CTA: a run may end one
-//   slab and begin the next (two segments), which fills the chip evenly, or stay within a slab, which saves the
-//   second segment's epilogue and refill where there is little to do (make_dc_plan weighs the two).  A reduce kernel sums the segments of a slab in a fixed order.
+//   slab and begin the next, which fills the chip evenly, or stay within a slab, which saves an epilogue and a refill where
+//   there is little to do (make_dc_plan weighs the two).  A run is worked off in segments that end with the slab or after a chain
+//   of tiles (kDcChain); a CTA's segments of one slab go to one partial, and a reduce kernel sums a slab's
+//   partials in a fixed order.
 //
 // Where a weight goes.  A pair's three weights are two neighbouring f16x2 words (knot rows 2w, 2w+1 and the next
 // two).  The operand layout (MN-major, un-swizzled) wants 16-byte pieces of eight M rows of one token, four banks
@@ -26,7 +28,7 @@ struct DcParams {
   const __nv_bfloat16* z;
   int64_t zs;
   const __half* gimg;
-  float* part;               // [segments of a slab][h*L][r]
+  float* part;               // [runs that touch a slab][h*L][r]
   int64_t N;
   int h, L, r;
   GridParams g;
@@ -38,6 +40,7 @@ struct DcParams {
   uint32_t tiles;            // 64-token tiles
   uint32_t pitch;            // places per slab in the runs' count: the tiles, or whole runs (then no run crosses slabs)
   uint32_t run, total;       // places of a CTA's run, and of all slabs together
+  uint32_t chain;            // tiles of a segment at most
   int32_t* status;
   long long wait_cycles;     // limit of every bounded wait, in clock cycles
 };
@@ -46,13 +49,21 @@ constexpr int kDcTokens = 64;                        // tokens per tile
 constexpr uint32_t kDcUnit = kDcTokens * 16;         // bytes of one 8-row group of a tile
 constexpr int kDcMaxGroups = 4;
 constexpr int kDcMaxRing = 8;                        // slots of the ring of g tiles
+// Tiles whose MMAs follow one another in an accumulator; what they gave is then added to the partial in float32.  The tensor
+// core cuts a sum off at the accumulator's last bit, always towards zero: the error grows with the number of MMAs
+// and does not average out.  Error of dC against 64 bits at 65536 x 5120, r = 32 / r = 128, all gradients positive (so that
+// every bit lost counts): one accumulator for 443 / 1024 tiles 6.8e-5 / 1.9e-4, 256 tiles 5.0e-5 / 5.4e-5, 192 tiles
+// 4.7e-5 / 4.7e-5 (what rounding the operands to f16 gives), dC alone 0.82 / 1.54, 0.83 / 1.61, 0.84 / 1.65 ms.
+// With pairs of f16 there is no such floor: 65536 x 5113, r = 32: 443 tiles 9.9e-5, 32 tiles 7.0e-6, 16 tiles 3.4e-6,
+// 8 tiles 1.8e-6; 1.82, 1.97, 2.12, 2.44 ms.
+constexpr uint32_t kDcChain = 192, kDcSplitChain = 8;
 constexpr int kDcIssuers = 3;                        // warps that issue MMAs, each for every third M tile
 // One unit behind a stage: the linear spline's last interval stores a zero word there.
 __host__ __device__ constexpr uint32_t dc_stage_bytes(int mtiles) { return (uint32_t)mtiles * 16u * kDcUnit + kDcUnit; }
 
 // KJ = keys per lane and token (a chunk is 4 * KJ keys), GW = warps per producer group.  SPLIT: a stage is filled twice, with
-// the weights and with their remainders at the same places.  RUNS: a run may cross slabs; without it the segment loop is
-// gone at compile time (5 % on the cases that stay within a slab).
+// the weights and with their remainders at the same places.  RUNS: a run may have several segments; without it their loop is
+// gone at compile time (5 % on the cases of one segment).
 template <int KJ, int GW, bool LIN, bool SPLIT, bool RUNS>
 __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -119,7 +130,9 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
     for (int j = 0; j < KJ; ++j) old[i][j] = 0u;
   for (uint32_t lin = blockIdx.x * P.run; RUNS ? lin < lin_end : seg == 0; ++seg) {
     const uint32_t slab = lin / P.pitch, tile_begin = lin - slab * P.pitch;
-    const uint32_t places = min(P.pitch - tile_begin, lin_end - lin);
+    if (RUNS && tile_begin >= P.tiles) break;            // places past the tiles end the last run of a slab
+    const uint32_t places = min(min(P.pitch - tile_begin, lin_end - lin), RUNS ? P.chain : ~0u);
+    const bool more = RUNS && seg > 0 && tile_begin > 0; // this CTA's partial of the slab has been begun
     const int ntiles = (int)min(P.tiles - tile_begin, places);
     const int key0 = (int)slab * P.slab_chunks * KCH;
     const int nchunks = min(P.slab_chunks, (P.h - key0 + KCH - 1) / KCH);
@@ -222,8 +235,10 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
           tmem_ld16(taddr + c0, v);
           if (ok) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 4)
-              *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            for (int i = 0; i < 16; i += 4) {
+              if (more) red_add4(dst + c0 + i, v[i], v[i + 1], v[i + 2], v[i + 3]);   // to what this thread has put there
+              else *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
           }
         }
       }
@@ -309,8 +324,13 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
   }
 }
 
-// `runs`: a run may cross slabs; the template case, the number of partials of a slab and the room for them all follow it.
-struct DcPlan { int kj, gw, ngroups, gring, mtiles, slab_chunks, parts; bool runs; uint32_t tiles, pitch, run, total; size_t smem; };
+// `runs`: a run may cross slabs; the number of partials of a slab and the room for them follow it.
+struct DcPlan {
+  int kj, gw, ngroups, gring, mtiles, slab_chunks, parts;
+  bool runs;
+  uint32_t tiles, pitch, run, total, chain;
+  size_t smem;
+};
 
 }  // namespace tc
 }  // namespace skv

@@ -76,6 +76,13 @@ inline int fwd_max_groups(int F, int r, bool split) {
 // A); with all four the load/store data path is 87 % busy.
 constexpr int kStagedPerHalf = 1;
 
+// Chunks whose MMAs follow one another in an accumulator of the SPLIT cases; what they gave is then added to the partial in
+// float32.  The tensor core cuts a sum off at the accumulator's last bit, always towards zero, so the error grows with the
+// number of MMAs and does not average out: 65536 x 5113, r = 32, error of delta against 64 bits with every chunk
+// in one accumulator 1.8e-5 (2.6e-5 where all summands are positive), with 16 chunks 2.3e-6, with 8 1.2e-6 (1.4e-6); the call 1.42,
+// 1.48 and 1.56 ms.  (Single f16 operands are off by 2e-4 already.)
+constexpr int kSplitChain = 8;
+
 // SPLIT: the weights' remainders follow the weights, in columns of their own and with the same metadata.
 template <int GROUPS, int F, int ACT, bool LIN, bool SPLIT>
 __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const FwdParams P) {
@@ -98,7 +105,8 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
   uint64_t* cfull = empty + 2 * GROUPS;           // [cstage]       TMA -> MMA
   uint64_t* cempty = cfull + kMaxCStages;       // [cstage]       MMA -> TMA
   uint64_t* done = cempty + kMaxCStages;        // [group]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + GROUPS);
+  uint64_t* part = done + GROUPS;               // [group]        MMA -> producers: kSplitChain chunks are complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part + GROUPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wc{abort_flag, P.status, kStatusTimeoutFwd, P.wait_cycles};
 
@@ -112,7 +120,7 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
 
   if (tid == 0) {
     for (int i = 0; i < 2 * GROUPS; ++i) { mbar_init(full + i, 4); mbar_init(empty + i, 1); }
-    for (int i = 0; i < GROUPS; ++i) mbar_init(done + i, 1);
+    for (int i = 0; i < 2 * GROUPS; ++i) mbar_init(done + i, 1);
     for (int i = 0; i < kMaxCStages; ++i) { mbar_init(cfull + i, 1); mbar_init(cempty + i, GROUPS); }
     *abort_flag = 0;
     mbar_init_fence();
@@ -144,7 +152,31 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
     const bool up = (lane & 8) != 0;
     const uint32_t sel_send = up ? 0x5410u : 0x7632u;               // halves of two metadata words the other row needs
     const uint32_t sel_0 = up ? 0x3254u : 0x5410u, sel_1 = up ? 0x3276u : 0x7610u;
+    float* prow = P.partial + ((size_t)blockIdx.y * P.N + (valid ? n : 0)) * r;
+    const uint32_t daddr = lane_addr + (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta);
+    // accumulator -> float32 partial of this key split; `more`: added to what this thread has put there
+    auto drain_acc = [&](bool more) {
+      for (int c0 = 0; c0 < r; c0 += 16) {
+        float v[16];
+        tmem_ld16(daddr + c0, v);
+        if (valid) {
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            if (SPLIT && more) red_add4(prow + c0 + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+            else *reinterpret_cast<float4*>(prow + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          }
+        }
+      }
+    };
     for (int ci = 0; ci < nch; ++ci) {
+      if constexpr (SPLIT) {
+        if (ci > 0 && ci % kSplitChain == 0) {           // the MMAs of this chunk wait for its words, hence for this
+          mbar_wait(part + grp, (uint32_t)(ci / kSplitChain - 1) & 1u, wc);
+          tc_fence_after();
+          drain_acc(ci > kSplitChain);
+          tc_fence_before();
+        }
+      }
       const uint4 zc = znext;
       if (ci + 1 < nch && valid) znext = ld16(zrow + (ci + 1) * kChunkKeys);
       const uint32_t zw[4] = {zc.x, zc.y, zc.z, zc.w};
@@ -251,20 +283,9 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
       }
       if (arow && valid) *reinterpret_cast<uint4*>(arow + ci * kChunkKeys) = make_uint4(aw[0], aw[1], aw[2], aw[3]);
     }
-    // epilogue: accumulator -> float32 partial of this key split
     mbar_wait(done + grp, 0, wc);
     tc_fence_after();
-    float* prow = P.partial + ((size_t)blockIdx.y * P.N + (valid ? n : 0)) * r;
-    const uint32_t daddr = lane_addr + (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta);
-    for (int c0 = 0; c0 < r; c0 += 16) {
-      float v[16];
-      tmem_ld16(daddr + c0, v);
-      if (valid) {
-#pragma unroll
-        for (int i = 0; i < 16; i += 4)
-          *reinterpret_cast<float4*>(prow + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-      }
-    }
+    drain_acc(nch > kSplitChain);
     tc_fence_before();
   } else if (warp < 5 * GROUPS) {
     // ------------------------------------------------------------------ MMA issue, one warp per token group
@@ -279,6 +300,8 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
       const uint32_t d_addr = m_addr0 + (uint32_t)(2 * kMeta);
       for (int ci = 0; ci < nch; ++ci) {
         const int cs = ci % CS;
+        const bool fresh = SPLIT ? ci % kSplitChain == 0 : ci == 0;      // the accumulator starts anew
+        if (SPLIT && fresh && ci > 0) umma_commit(part + grp);
         bool drain = mbar_wait(cfull + cs, (uint32_t)(ci / CS) & 1u, wc);
         uint32_t b_lo = desc_lo(smem_u32(c_base + (size_t)cs * c_bytes), P.b_lbo);
         uint32_t a_addr = a_addr0;
@@ -290,10 +313,10 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
 #pragma unroll
           for (int ks = 0; ks < kHalfSteps; ++ks) {     // 8 columns of A (16 kept of 32 K elements) per step
 #pragma unroll
-            for (int part = 0; part < kParts; ++part)
-              umma_f16_sparse_ta(d_addr, a_addr + (uint32_t)(part * kChunkKeys * F), b_lo, b_hi,
+            for (int p = 0; p < kParts; ++p)
+              umma_f16_sparse_ta(d_addr, a_addr + (uint32_t)(p * kChunkKeys * F), b_lo, b_hi,
                                  m_addr0 + (uint32_t)(half * kMeta + (ks & ~1)), idesc | (uint32_t)(ks & 1),
-                                 (ci > 0 || half > 0 || ks > 0 || part > 0) ? 1u : 0u);
+                                 (!fresh || half > 0 || ks > 0 || p > 0) ? 1u : 0u);
             a_addr += 8u;
             b_lo += b_step;
           }
