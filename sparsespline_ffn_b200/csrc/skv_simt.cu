@@ -697,6 +697,12 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
             }
           }
         }
+        if (!three) {                                 // zero weights, but zero times an infinity is not zero
+#pragma unroll
+          for (int c = 0; c < CV; ++c)
+#pragma unroll
+            for (int i = 0; i < V; ++i) a[2][c][i] = 0.0f;
+        }
       }
       if (dirty > 0) { finish_row(b); --dirty; }
     }

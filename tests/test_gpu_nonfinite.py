@@ -1,0 +1,70 @@
+"""Infinities and NaN in C and g_delta reach what touches them and nothing else, on the CUDA-core kernels.  Against the CPU oracle, which adds up the touched rows alone."""
+import numpy as np
+import pytest
+import torch
+
+from tests import util
+
+pytestmark = pytest.mark.gpu
+
+ops = pytest.importorskip("sparsespline_ffn_b200.ops")
+
+INF, NAN = float("inf"), float("nan")
+# (N, h, r, G, spline_order)
+CASES = [(300, 40, 32, 20, 1), (257, 9, 17, 20, 2), (1000, 101, 20, 12, 2), (200, 16, 32, 48, 2), (129, 33, 1, 6, 2),
+         (4100, 24, 16, 20, 1)]
+IDS = ["N%d_h%d_r%d_G%d_order%d" % c for c in CASES]
+
+
+def _inputs(N, h, r, G, order, bad, z_std=None):
+    gen = torch.Generator().manual_seed(N)
+    # inside the grid and below its last interval, where the oracle and the kernels mask alike
+    z = (torch.rand(N, h, generator=gen) * 4.8 - 2.8) if z_std is None else torch.randn(N, h, generator=gen) * z_std
+    C = torch.randn(h, G + order, r, generator=gen) * 0.1
+    go = torch.randn(N, h + r, generator=gen)
+    if bad in ("C", "both"):
+        C[h // 2, (G + order) // 2, 0] = INF
+        C[0, 3, r - 1] = -INF
+        C[h - 1, G // 2, r // 2] = NAN
+    if bad in ("g", "both"):
+        go[N // 3, h] = INF
+        go[N - 1, h + r - 1] = NAN
+        go[0, h + r // 2] = -INF
+    return z.bfloat16().cuda(), C.bfloat16().cuda(), go.bfloat16().cuda()
+
+
+def _check(name, got, ref, dtype, gate):
+    got, ref = util.f32(got), np.asarray(ref, dtype=np.float64)
+    fin = np.isfinite(ref)
+    assert fin.any()
+    extra, missing = np.argwhere(~np.isfinite(got) & fin), np.argwhere(np.isfinite(got) & ~fin)
+    assert not len(extra) and not len(missing), f"{name}: {len(extra)} too many, {len(missing)} too few, {extra[:3]} {missing[:3]}"
+    util.assert_parity(name, np.where(fin, got, 0.0), np.where(fin, ref, 0.0), dtype, rel_gate=gate)
+
+
+@pytest.mark.parametrize("impl", ["simt"])
+@pytest.mark.parametrize("bad", ["C", "g", "both"])
+@pytest.mark.parametrize("case", CASES, ids=IDS)
+def test_nonfinite_inputs_stay_where_they_are_touched(case, bad, impl):
+    N, h, r, G, order = case
+    lo, hi, lam = -3.0, 3.0, 0.75
+    z, C, go = _inputs(N, h, r, G, order, bad)
+    kw = dict(impl=impl, spline_order=order)
+    tc = impl == "tcgen05"
+    f = ops.feature_forward(z, C, lo, hi, G, "relu_sq", lam, **kw)
+    dz, dC, dC_cast = ops.feature_backward(z, C, go, lo, hi, G, "relu_sq", lam, dz_f32=tc, **kw)
+    gf = util.f32(go)
+    a_ref, d_ref = util.oc.feature_forward(util.f32(z), util.f32(C), lo, hi, G, "relu_sq", lam, spline_order=order)
+    dz_ref, dC_ref = util.oc.feature_backward(util.f32(z), util.f32(C), gf[:, h:], gf[:, :h], lo, hi, G, "relu_sq", lam,
+                                              spline_order=order)
+    # pairs of f16: 22 bits; bf16 results: half a unit in the eighth bit
+    _check("delta", f[:, h:], d_ref, torch.bfloat16, 4e-3)
+    _check("dz", dz, dz_ref, torch.float32 if tc else torch.bfloat16, 2e-5 if tc else 4e-3)
+    _check("dC", dC, dC_ref, torch.float32, 2e-5)
+    _check("dC (bf16)", dC_cast, dC_ref, torch.bfloat16, 4e-3)
+    # one result alone, and dz in bf16
+    dz1 = ops.feature_backward(z, C, go, lo, hi, G, "relu_sq", lam, need_dC=False, **kw)[0]
+    dC1 = ops.feature_backward(z, C, go, lo, hi, G, "relu_sq", lam, need_dz=False, **kw)[1]
+    _check("dz alone", dz1, dz_ref, torch.bfloat16, 4e-3)
+    _check("dC alone", dC1, dC_ref, torch.float32, 2e-5)
+    ops.check_status(z.device)
