@@ -220,6 +220,7 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   Q.tiles = gimg_tiles(p);
   Q.gimg = gimg;
   Q.hdr = hdr;
+  Q.contain = split;
   void* user_dz = dz;
   const int64_t user_dzs = dzs;
   if (!rows_ok) {
@@ -321,10 +322,16 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
   }
   if (dz != user_dz)
     if (int e = launch_unpad(dz, dzs, user_dz, user_dzs, p.N, p.h, p.dz_f32 != 0, c.stream)) return e;
+  Contain K{};
+  if (split) {
+    K.z = Z.z; K.zs = zs; K.C = Q.C; K.g = Q.g; K.gds = gds; K.N = p.N;
+    K.h = p.h; K.L = p.L; K.r = p.r; K.grid = c.g;
+    K.dz = user_dz; K.dzs = user_dzs; K.coef = Z.coef; K.dz_f32 = p.dz_f32 != 0;
+  }
   if (want_dC)
     return launch_dc_reduce(part, parts, (int64_t)p.h * p.L, (int64_t)hp * p.L, p.r, rp, p.lambda_scale, hdr, dC,
-                            dC_cast, c.stream);
-  return SKV_OK;
+                            dC_cast, K, c.stream);
+  return split ? launch_dz_contain(K, hdr, c.stream) : (int)SKV_OK;
 }
 
 }  // namespace tc

@@ -275,8 +275,9 @@ __device__ __forceinline__ void pow2_scales(uint32_t amax_bits, float& scale, fl
   scale = __uint_as_float((uint32_t)se << 23);
   inv = __uint_as_float((uint32_t)(254 - se) << 23);
 }
-// Words of the 256-byte header at the start of a call's scratch: bit patterns of max|g_delta| and max|C|.
-constexpr int kAmaxG = 0, kAmaxC = 8;
+// Words of the 256-byte header at the start of a call's scratch: bit patterns of the largest finite |g_delta| and |C|, and
+// whether either holds an infinity or a NaN.
+constexpr int kAmaxG = 0, kAmaxC = 8, kBadG = 1, kBadC = 9;
 
 // Two float32 -> packed f16x2 (low half = a) as a 32-bit word.
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {

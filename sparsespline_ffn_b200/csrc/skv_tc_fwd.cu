@@ -117,6 +117,7 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
   Q.N = p.N;
   Q.act = p.activation;
   Q.hdr = hdr;
+  Q.contain = split_operands(p);
   if (!rows_ok) {
     __nv_bfloat16* zp = reinterpret_cast<__nv_bfloat16*>(
         base + kHeaderBytes + fwd_cimg_bytes(p) + align256((size_t)f.splits * p.N * rp * sizeof(float)));
@@ -154,7 +155,12 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
                                      : (relu ? fwd_launch_quad_relu : fwd_launch_quad_other);
   if (launch(f.groups, f.fold, P, grid, f.smem, c.stream) != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
   note_launches(1);
-  return launch_finalize(partial, f.splits, p.N, p.r, rp, p.lambda_scale, hdr, delta_out, ds, p.delta_f32 != 0, c.stream);
+  Contain K{};
+  if (Q.contain) {
+    K.z = P.z; K.zs = zs; K.C = Q.C; K.N = p.N;
+    K.h = p.h; K.L = p.L; K.r = p.r; K.grid = c.g;
+  }
+  return launch_finalize(partial, f.splits, p.N, p.r, rp, p.lambda_scale, hdr, delta_out, ds, p.delta_f32 != 0, K, c.stream);
 }
 
 }  // namespace tc

@@ -11,13 +11,19 @@ namespace skv {
 namespace tc {
 namespace {
 
-__device__ __forceinline__ uint32_t absmax_bf2(uint32_t m, uint32_t w) {
-  // |x| of a bf16 as a float32 bit pattern; NaN patterns lie above infinity and are skipped
-  const uint32_t lo = (w << 16) & 0x7fff0000u, hi = w & 0x7fff0000u;
-  if (lo <= 0x7f800000u) m = max(m, lo);
-  if (hi <= 0x7f800000u) m = max(m, hi);
-  return m;
-}
+// Largest |x| seen, as float32 bit patterns: of the finite values, and of all (infinity and the NaN patterns above it
+// included).
+struct AbsMax {
+  uint32_t finite = 0, all = 0;
+  __device__ __forceinline__ void add(uint32_t w) {       // two packed bf16
+    const uint32_t lo = (w << 16) & 0x7fff0000u, hi = w & 0x7fff0000u;
+    all = max(all, max(lo, hi));
+    if (lo < 0x7f800000u) finite = max(finite, lo);
+    if (hi < 0x7f800000u) finite = max(finite, hi);
+  }
+  __device__ __forceinline__ void add(const uint4& v) { add(v.x); add(v.y); add(v.z); add(v.w); }
+};
+constexpr uint32_t kBadBit = 0x80000000u;                 // of a block's word: it has seen an infinity or a NaN
 
 // Maximum over the block; valid in every thread.  `words` is shared scratch of 32 words.
 __device__ __forceinline__ uint32_t block_max(uint32_t m, uint32_t* words) {
@@ -42,7 +48,7 @@ __device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p, int n, bool vec) { 
 __global__ void __launch_bounds__(256) tc_scan_kernel(const PrepParams P) {
   __shared__ uint32_t words[32];
   pdl_launch();
-  uint32_t m = 0;
+  AbsMax m;
   const bool is_c = (int)blockIdx.x < P.scan_c;
   const int blk = is_c ? blockIdx.x : blockIdx.x - P.scan_c, nblk = is_c ? P.scan_c : P.scan_g;
   const int64_t first = (int64_t)blk * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
@@ -51,11 +57,10 @@ __global__ void __launch_bounds__(256) tc_scan_kernel(const PrepParams P) {
     const int64_t n8 = (reinterpret_cast<uintptr_t>(P.C) & 15) == 0 ? total / 8 : 0;
 #pragma unroll 4
     for (int64_t i = first; i < n8; i += step) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(P.C) + i);
-      m = absmax_bf2(absmax_bf2(absmax_bf2(absmax_bf2(m, v.x), v.y), v.z), v.w);
+      m.add(__ldg(reinterpret_cast<const uint4*>(P.C) + i));
     }
     for (int64_t i = n8 * 8 + first; i < total; i += step)
-      m = absmax_bf2(m, __ldg(reinterpret_cast<const unsigned short*>(P.C) + i));
+      m.add(__ldg(reinterpret_cast<const unsigned short*>(P.C) + i));
   } else {
     const bool vec = P.r % 8 == 0 && P.gds % 8 == 0 && (reinterpret_cast<uintptr_t>(P.g) & 15) == 0;
     const int cgs = (P.r + 7) / 8;
@@ -64,18 +69,30 @@ __global__ void __launch_bounds__(256) tc_scan_kernel(const PrepParams P) {
     for (int64_t i = first; i < pieces; i += step) {
       const int64_t n = i / cgs;
       const int c = (int)(i - n * cgs) * 8;
-      const uint4 v = ld8(P.g + n * P.gds + c, P.r - c, vec);
-      m = absmax_bf2(absmax_bf2(absmax_bf2(absmax_bf2(m, v.x), v.y), v.z), v.w);
+      m.add(ld8(P.g + n * P.gds + c, P.r - c, vec));
     }
   }
-  m = block_max(m, words);
-  if (threadIdx.x == 0) P.hdr[kBlockMax + (is_c ? 0 : kMaxBlocks) + blk] = m;
+  const uint32_t top = block_max(m.finite, words);
+  const int bad = __syncthreads_or(m.all >= 0x7f800000u);
+  if (threadIdx.x == 0) P.hdr[kBlockMax + (is_c ? 0 : kMaxBlocks) + blk] = top | (bad ? kBadBit : 0u);
 }
 
-__device__ __forceinline__ uint32_t combine(const uint32_t* part, int n, uint32_t* words) {
-  uint32_t m = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) m = max(m, part[i]);
+__device__ __forceinline__ uint32_t combine(const uint32_t* part, int n, uint32_t* words, bool& bad) {
+  uint32_t m = 0, all = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    m = max(m, part[i] & ~kBadBit);
+    all |= part[i];
+  }
+  bad = __syncthreads_or((int)(all & kBadBit)) != 0;
   return block_max(m, words);
+}
+
+// Eight bf16 with zeros in the place of infinities and NaN.
+__device__ __forceinline__ uint32_t finite2(uint32_t w) {
+  return ((w & 0x7f80u) == 0x7f80u ? 0u : w & 0xffffu) | ((w & 0x7f800000u) == 0x7f800000u ? 0u : w & 0xffff0000u);
+}
+__device__ __forceinline__ uint4 finite8(const uint4& v, bool bad) {
+  return bad ? make_uint4(finite2(v.x), finite2(v.y), finite2(v.z), finite2(v.w)) : v;
 }
 
 __device__ __forceinline__ uint4 scaled_h8(const uint4& v, float s) {
@@ -97,13 +114,14 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
   const int cgs = P.rp / 8;
   const bool cvec = P.r % 8 == 0 && (reinterpret_cast<uintptr_t>(P.C) & 15) == 0;
   if (blk == 0) {                                       // final maxima for the kernels that follow
+    bool bad;
     if (P.scan_c) {
-      const uint32_t m = combine(P.hdr + kBlockMax, P.scan_c, words);
-      if (threadIdx.x == 0) P.hdr[kAmaxC] = m;
+      const uint32_t m = combine(P.hdr + kBlockMax, P.scan_c, words, bad);
+      if (threadIdx.x == 0) { P.hdr[kAmaxC] = m; P.hdr[kBadC] = bad; }
     }
     if (P.scan_g) {
-      const uint32_t m = combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words);
-      if (threadIdx.x == 0) P.hdr[kAmaxG] = m;
+      const uint32_t m = combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words, bad);
+      if (threadIdx.x == 0) { P.hdr[kAmaxG] = m; P.hdr[kBadG] = bad; }
     }
   }
   if (blk < P.blocks_c + P.blocks_t) {
@@ -111,7 +129,9 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
     const int nblk = is_t ? P.blocks_t : P.blocks_c;
     if (is_t) blk -= P.blocks_c;
     float scale, inv;
-    pow2_scales(combine(P.hdr + kBlockMax, P.scan_c, words), scale, inv);
+    bool bad;
+    pow2_scales(combine(P.hdr + kBlockMax, P.scan_c, words, bad), scale, inv);
+    bad = bad && P.contain;
     const int LP = is_t ? P.lpt : P.lpc;
     const int cgi = is_t ? cgs * P.tparts : cgs;        // channel groups of the image
     const int64_t pieces = (int64_t)P.hp * LP * cgi;
@@ -132,12 +152,12 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
         if (!is_t) {
           // group f = b / 4 holds knot rows 2f, 2f + 1 and 2(f + F - 1), 2(f + F - 1) + 1, F = LP / 4 groups
           const int kr = 2 * (b >> 2) + (b & 1) + ((b & 2) ? LP / 2 - 2 : 0);
-          if (kr < P.L) o = scaled_h8(ld8(base + (size_t)kr * P.r, left, cvec), scale);
+          if (kr < P.L) o = scaled_h8(finite8(ld8(base + (size_t)kr * P.r, left, cvec), bad), scale);
         } else if (b < P.L - 1) {
           // b = 0: C[1] - C[0]; b > 0: C[b-1] - 2 C[b] + C[b+1]
-          const uint4 v0 = ld8(base + (size_t)(b > 0 ? b - 1 : 0) * P.r, left, cvec);
-          const uint4 v1 = ld8(base + (size_t)(b > 0 ? b : 1) * P.r, left, cvec);
-          const uint4 v2 = b > 0 ? ld8(base + (size_t)(b + 1) * P.r, left, cvec) : make_uint4(0, 0, 0, 0);
+          const uint4 v0 = finite8(ld8(base + (size_t)(b > 0 ? b - 1 : 0) * P.r, left, cvec), bad);
+          const uint4 v1 = finite8(ld8(base + (size_t)(b > 0 ? b : 1) * P.r, left, cvec), bad);
+          const uint4 v2 = b > 0 ? finite8(ld8(base + (size_t)(b + 1) * P.r, left, cvec), bad) : make_uint4(0, 0, 0, 0);
           const uint32_t a0[4] = {v0.x, v0.y, v0.z, v0.w}, a1[4] = {v1.x, v1.y, v1.z, v1.w}, a2[4] = {v2.x, v2.y, v2.z, v2.w};
           uint32_t w[4];
 #pragma unroll
@@ -160,7 +180,9 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
   blk -= P.blocks_c + P.blocks_t;
   if (blk < P.blocks_g) {
     float scale, inv;
-    pow2_scales(combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words), scale, inv);
+    bool bad;
+    pow2_scales(combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words, bad), scale, inv);
+    bad = bad && P.contain;
     const bool vec = P.r % 8 == 0 && P.gds % 8 == 0 && (reinterpret_cast<uintptr_t>(P.g) & 15) == 0;
     const int64_t pieces = P.tiles * 128 * cgs;
     uint4* img = reinterpret_cast<uint4*>(P.gimg);
@@ -170,7 +192,8 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
       const int64_t tile = tc_ / cgs;
       const int c = (int)(tc_ - tile * cgs) * 8;
       const int64_t n = tile * 128 + (e & 127);
-      img[e] = n < P.N && c < P.r ? scaled_h8(ld8(P.g + n * P.gds + c, P.r - c, vec), scale) : make_uint4(0, 0, 0, 0);
+      img[e] = n < P.N && c < P.r ? scaled_h8(finite8(ld8(P.g + n * P.gds + c, P.r - c, vec), bad), scale)
+                                  : make_uint4(0, 0, 0, 0);
     }
     return;
   }
@@ -196,16 +219,143 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
   }
 }
 
+__device__ __forceinline__ bool is_bad(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+
+__device__ __forceinline__ float pair_weight(const Knot& k, int row, int order) {
+  float B0, B1, B2;
+  basis_weights(k, B0, B1, B2, order);
+  return row == 0 ? B0 : row == 1 ? B1 : B2;
+}
+
+// delta[n][c .. c + 3]: the contributions of infinities and NaN in C (a zero weight times one is NaN here too, as it is
+// when the touched rows alone are added up); true when there is one.
+__device__ __noinline__ bool contain_delta(const Contain& K, int64_t n, int c, float (&s)[4]) {
+  bool any = false;
+  for (int j = 0; j < K.h; ++j) {
+    const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j]), K.grid);
+    for (int row = 0; row <= K.grid.order; ++row) {
+      const __nv_bfloat16* src = K.C + ((size_t)j * K.L + k.bin + row) * K.r + c;
+      for (int i = 0; i < 4 && c + i < K.r; ++i) {
+        const float v = __bfloat162float(src[i]);
+        if (is_bad(v)) {
+          s[i] = fmaf(pair_weight(k, row, K.grid.order), v, s[i]);
+          any = true;
+        }
+      }
+    }
+  }
+  return any;
+}
+
+// dC: the same for infinities and NaN in g_delta.  A block lists the tokens that have any, 256 tokens at a time, and its
+// threads, one per four columns of a knot row, walk the list.
+__device__ __noinline__ void contain_dC(const Contain& K, int rp, float lambda, float* dC, __nv_bfloat16* dC_cast) {
+  __shared__ int list[256];
+  __shared__ int count;
+  const int q4 = rp / 4;
+  const int64_t total = (int64_t)K.h * K.L * q4;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = base + threadIdx.x;
+    const int64_t row = i / q4;
+    const int c = (int)(i - row * q4) * 4, j = (int)(row / K.L), l = (int)(row - (int64_t)j * K.L);
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    bool any[4] = {false, false, false, false};
+    for (int64_t n0 = 0; n0 < K.N; n0 += 256) {
+      __syncthreads();
+      if (threadIdx.x == 0) count = 0;
+      __syncthreads();
+      if (n0 + threadIdx.x < K.N) {
+        const __nv_bfloat16* g = K.g + (n0 + threadIdx.x) * K.gds;
+        bool bad = false;
+        for (int e = 0; e < K.r; ++e) bad = bad || is_bad(__bfloat162float(g[e]));
+        if (bad) list[atomicAdd(&count, 1)] = threadIdx.x;
+      }
+      __syncthreads();
+      if (i < total) {
+        for (int e = 0; e < count; ++e) {
+          const int64_t n = n0 + list[e];
+          const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j]), K.grid);
+          if (!k.in_range || l < k.bin || l > k.bin + K.grid.order) continue;
+          const float w = pair_weight(k, l - k.bin, K.grid.order);
+          for (int x = 0; x < 4 && c + x < K.r; ++x) {
+            const float v = __bfloat162float(K.g[n * K.gds + c + x]);
+            if (is_bad(v)) {
+              s[x] = fmaf(w, v, s[x]);
+              any[x] = true;
+            }
+          }
+        }
+      }
+    }
+    for (int x = 0; x < 4; ++x) {
+      if (!any[x]) continue;
+      if (dC) dC[row * K.r + c + x] = lambda * s[x];
+      if (dC_cast) dC_cast[row * K.r + c + x] = __float2bfloat16_rn(lambda * s[x]);
+    }
+  }
+}
+
+// dz: the channels of a pair in which g_delta or a touched row of C is infinite or NaN.  A block takes 256 tokens (one per
+// thread) x 32 keys and first marks the knot rows of its keys and the tokens that have any.
+__device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c) {
+  __shared__ unsigned long long rows[32];
+  const int key_groups = (K.h + 31) / 32;
+  const int64_t tiles = (K.N + 255) / 256 * key_groups;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int64_t n = t / key_groups * 256 + threadIdx.x;
+    const int j0 = (int)(t % key_groups) * 32, keys = min(32, K.h - j0);
+    __syncthreads();
+    if (threadIdx.x < 32) rows[threadIdx.x] = 0ull;
+    __syncthreads();
+    if (bad_c)
+      for (int e = threadIdx.x; e < keys * K.L; e += blockDim.x) {
+        const __nv_bfloat16* src = K.C + ((size_t)j0 * K.L + e) * K.r;
+        bool bad = false;
+        for (int c = 0; c < K.r; ++c) bad = bad || is_bad(__bfloat162float(src[c]));
+        if (bad) atomicOr(&rows[e / K.L], 1ull << (e % K.L));
+      }
+    const __nv_bfloat16* g = K.g + (n < K.N ? n : 0) * K.gds;
+    bool token = false;
+    if (bad_g && n < K.N)
+      for (int c = 0; c < K.r; ++c) token = token || is_bad(__bfloat162float(g[c]));
+    __syncthreads();
+    for (int q = 0; q < keys && n < K.N; ++q) {
+      const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j0 + q]), K.grid);
+      const bool two = K.grid.order != 1;
+      if (!k.clamp_active || !(token || ((rows[q] >> k.bin) & (two ? 7ull : 3ull)))) continue;
+      const __nv_bfloat16* src = K.C + ((size_t)(j0 + q) * K.L + k.bin) * K.r;
+      float s = 0.0f;
+      bool any = false;
+      for (int c = 0; c < K.r; ++c) {
+        const float gv = __bfloat162float(g[c]), c0 = __bfloat162float(src[c]), c1 = __bfloat162float(src[K.r + c]);
+        const float c2 = two ? __bfloat162float(src[2 * K.r + c]) : 0.0f;
+        if (!is_bad(gv) && !is_bad(c0) && !is_bad(c1) && !is_bad(c2)) continue;
+        float d = c1 - c0;
+        if (two) d = fmaf(k.tau, (c2 - c1) - d, d);
+        s = fmaf(gv, d, s);
+        any = true;
+      }
+      if (!any) continue;
+      if (K.dz_f32) static_cast<float*>(K.dz)[n * K.dzs + j0 + q] += K.coef * s;
+      else {
+        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(K.dz) + n * K.dzs + j0 + q;
+        *o = __float2bfloat16_rn(__bfloat162float(*o) + K.coef * s);
+      }
+    }
+  }
+}
+
 // Four consecutive columns per thread; the splits of an element are added in order, four loads in flight.
-template <typename TD>
+template <typename TD, bool CONTAIN>
 __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, int splits, int64_t N, int r,
                                                           int rp, float lambda, const uint32_t* hdr,
-                                                          TD* out, int64_t ds) {
+                                                          TD* out, int64_t ds, const Contain K) {
   pdl_launch();
   pdl_wait();
   float cscale, cinv;
   pow2_scales(hdr[kAmaxC], cscale, cinv);
-  lambda *= cinv;                                       // undo the code-table image's range scaling
+  const bool bad = CONTAIN && hdr[kBadC] != 0u;
+  const float f = lambda * cinv;                        // undo the code-table image's range scaling
   const int q4 = rp / 4;
   const int64_t total = N * q4;
   const bool vec = ds % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && r == rp;
@@ -220,7 +370,14 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
     const int64_t n = i / q4;
     const int c = (int)(i - n * q4) * 4;
     TD* o = out + n * ds + c;
-    const float v[4] = {lambda * s.x, lambda * s.y, lambda * s.z, lambda * s.w};
+    float v[4] = {f * s.x, f * s.y, f * s.z, f * s.w};
+    if constexpr (CONTAIN) {
+      if (bad) {
+        float extra[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (contain_delta(K, n, c, extra))
+          for (int k = 0; k < 4; ++k) v[k] += lambda * extra[k];
+      }
+    }
     if (vec) {
       if constexpr (sizeof(TD) == 4) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
       else *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf2(v[0], v[1]), pack_bf2(v[2], v[3]));
@@ -232,10 +389,11 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
   }
 }
 
+template <bool CONTAIN>
 __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, const DcParts parts, int64_t rows,
                                                            int64_t rows_padded, int r, int rp, float lambda,
                                                            const uint32_t* hdr, float* dC,
-                                                           __nv_bfloat16* dC_cast) {
+                                                           __nv_bfloat16* dC_cast, const Contain K) {
   pdl_wait();
   float gscale, ginv;
   pow2_scales(hdr[kAmaxG], gscale, ginv);
@@ -268,6 +426,20 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
       }
     }
   }
+  if constexpr (CONTAIN) {
+    const bool bad_g = hdr[kBadG] != 0u;
+    if (bad_g) contain_dC(K, rp, lambda, dC, dC_cast);      // the elements of a thread are those it has written above
+    if (K.dz) {
+      const bool bad_c = hdr[kBadC] != 0u;
+      if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) tc_dz_contain_kernel(const uint32_t* hdr, const Contain K) {
+  pdl_wait();
+  const bool bad_g = hdr[kBadG] != 0u, bad_c = hdr[kBadC] != 0u;
+  if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
 }
 
 template <typename T>
@@ -308,24 +480,40 @@ int launch_prep(PrepParams& P, cudaStream_t stream) {
   return SKV_OK;
 }
 
+namespace {
+template <typename TD, bool CONTAIN>
+cudaError_t finalize(dim3 grid, cudaStream_t stream, const float* partial, int splits, int64_t N, int r, int rp, float lambda,
+                     const uint32_t* hdr, void* out, int64_t ds, const Contain& K) {
+  return launch_chained<tc_finalize_kernel<TD, CONTAIN>>(grid, 256, 0, stream, partial, splits, N, r, rp, lambda, hdr,
+                                                         static_cast<TD*>(out), ds, K);
+}
+}  // namespace
+
 int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,
-                    void* out, int64_t ds, bool out_f32, cudaStream_t stream) {
+                    void* out, int64_t ds, bool out_f32, const Contain& K, cudaStream_t stream) {
   const dim3 grid((unsigned)blocks_for(N * (rp / 4), 1, kPlanSMs * 16));
-  const cudaError_t e =
-      out_f32 ? launch_chained<tc_finalize_kernel<float>>(grid, 256, 0, stream, partial, splits, N, r, rp, lambda, hdr,
-                                                          static_cast<float*>(out), ds)
-              : launch_chained<tc_finalize_kernel<__nv_bfloat16>>(grid, 256, 0, stream, partial, splits, N, r, rp, lambda,
-                                                                  hdr, static_cast<__nv_bfloat16*>(out), ds);
+  auto* run = out_f32 ? (K.z ? finalize<float, true> : finalize<float, false>)
+                      : (K.z ? finalize<__nv_bfloat16, true> : finalize<__nv_bfloat16, false>);
+  const cudaError_t e = run(grid, stream, partial, splits, N, r, rp, lambda, hdr, out, ds, K);
   note_launches(1);
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }
 
 int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
-                     const uint32_t* hdr, float* dC, void* dC_cast, cudaStream_t stream) {
+                     const uint32_t* hdr, float* dC, void* dC_cast, const Contain& K, cudaStream_t stream) {
   const dim3 grid((unsigned)blocks_for(rows * (rp / 4), 1, kPlanSMs * 16));
   const cudaError_t e =
-      launch_chained<tc_dc_reduce_kernel>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda, hdr, dC,
-                                          static_cast<__nv_bfloat16*>(dC_cast));
+      K.z ? launch_chained<tc_dc_reduce_kernel<true>>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda, hdr,
+                                                      dC, static_cast<__nv_bfloat16*>(dC_cast), K)
+          : launch_chained<tc_dc_reduce_kernel<false>>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda,
+                                                       hdr, dC, static_cast<__nv_bfloat16*>(dC_cast), K);
+  note_launches(1);
+  return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+}
+
+int launch_dz_contain(const Contain& K, const uint32_t* hdr, cudaStream_t stream) {
+  const dim3 grid((unsigned)blocks_for(K.N * ((K.h + 31) / 32), 1, kPlanSMs * 4));
+  const cudaError_t e = launch_chained<tc_dz_contain_kernel>(grid, 256, 0, stream, hdr, K);
   note_launches(1);
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }

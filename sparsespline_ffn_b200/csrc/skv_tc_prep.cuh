@@ -46,6 +46,24 @@ struct CopyJob {
   int64_t as;
 };
 
+// Infinities and NaN in C and g_delta.  A (token, key) pair touches order + 1 knot rows, but the contractions multiply all rows by
+// weights most of which are zero, and zero times an infinity is NaN: one such element of C would reach every token, one
+// of g_delta every row of dC.  The problems with split operands are contained: their images hold zeros in such
+// places, and where a scan has found any, the last kernels of a call add what the pairs that touch them contribute.
+struct Contain {
+  const __nv_bfloat16* z;    // null: not contained
+  int64_t zs;
+  const __nv_bfloat16* C;
+  const __nv_bfloat16* g;
+  int64_t gds, N;
+  int h, L, r;
+  GridParams grid;
+  void* dz;                  // null: no dz wanted
+  int64_t dzs;
+  float coef;                // lambda * scale, of dz
+  bool dz_f32;
+};
+
 struct PrepParams {
   const __nv_bfloat16* C;
   int h, hp, L, r, rp;
@@ -58,6 +76,7 @@ struct PrepParams {
   int64_t gds, N, tiles;     // tiles of 128 tokens in the image
   __half* gimg;
   CopyJob copy[2];
+  bool contain;              // infinities and NaN become zeros in the images
   int act;
   uint32_t* hdr;
   int scan_c, scan_g;        // blocks that scan each array
@@ -69,7 +88,7 @@ int launch_prep(PrepParams& P, cudaStream_t stream);
 
 // out[n][c] = lambda * 2^-k * sum over splits of partial[split][n][c], c < r of the rp partial columns.
 int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,
-                    void* out, int64_t ds, bool out_f32, cudaStream_t stream);
+                    void* out, int64_t ds, bool out_f32, const Contain& K, cudaStream_t stream);
 
 // How many partials a knot row of dC has: `count`, or (count = 0) the number of runs of `run` places that touch the row's slab of
 // `slab_rows` rows and `pitch` places.
@@ -83,7 +102,10 @@ struct DcParts {
 
 // dC = lambda * 2^-k * sum over the partials part[i][row][c] for `rows` knot rows.
 int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
-                     const uint32_t* hdr, float* dC, void* dC_cast, cudaStream_t stream);
+                     const uint32_t* hdr, float* dC, void* dC_cast, const Contain& K, cudaStream_t stream);
+
+// What infinities and NaN add to dz, for a call without dC (launch_dc_reduce does the same for the others).
+int launch_dz_contain(const Contain& K, const uint32_t* hdr, cudaStream_t stream);
 
 // dst[n][j] = src[n][j], j < h, from padded rows.
 int launch_unpad(const void* src, int64_t ss, void* dst, int64_t ds, int64_t N, int h, bool f32, cudaStream_t stream);

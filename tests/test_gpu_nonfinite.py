@@ -1,4 +1,6 @@
-"""Infinities and NaN in C and g_delta reach what touches them and nothing else, on the CUDA-core kernels.  Against the CPU oracle, which adds up the touched rows alone."""
+"""Infinities and NaN in C and g_delta reach what touches them and nothing else, on the kernels that promise it: the CUDA-core
+family, and the tcgen05 family where it holds operands as pairs of f16 (linear spline, h no multiple of 8, r no multiple
+of 16, more than 49 knot rows).  Against the CPU oracle, which adds up the touched rows alone."""
 import numpy as np
 import pytest
 import torch
@@ -42,7 +44,7 @@ def _check(name, got, ref, dtype, gate):
     util.assert_parity(name, np.where(fin, got, 0.0), np.where(fin, ref, 0.0), dtype, rel_gate=gate)
 
 
-@pytest.mark.parametrize("impl", ["simt"])
+@pytest.mark.parametrize("impl", ["simt", "tcgen05"])
 @pytest.mark.parametrize("bad", ["C", "g", "both"])
 @pytest.mark.parametrize("case", CASES, ids=IDS)
 def test_nonfinite_inputs_stay_where_they_are_touched(case, bad, impl):
@@ -68,3 +70,16 @@ def test_nonfinite_inputs_stay_where_they_are_touched(case, bad, impl):
     _check("dz alone", dz1, dz_ref, torch.bfloat16, 4e-3)
     _check("dC alone", dC1, dC_ref, torch.float32, 2e-5)
     ops.check_status(z.device)
+
+
+@pytest.mark.parametrize("case", CASES, ids=IDS)
+def test_nonfinite_inputs_and_tokens_outside_the_grid(case):
+    N, h, r, G, order = case
+    z, C, go = _inputs(N, h, r, G, order, "both", z_std=2.5)
+    got = {}
+    for impl in ("simt", "tcgen05"):
+        f = ops.feature_forward(z, C, -3.0, 3.0, G, "gelu", 0.5, impl=impl, spline_order=order)
+        dz, dC, _ = ops.feature_backward(z, C, go, -3.0, 3.0, G, "gelu", 0.5, impl=impl, spline_order=order)
+        got[impl] = f, dz, dC
+    for name, a, b in zip(("f", "dz", "dC"), got["tcgen05"], got["simt"]):
+        _check(name, a, util.f32(b), torch.bfloat16, 1e-2)
