@@ -43,9 +43,9 @@ enum skv_dtype { SKV_BF16 = 0, SKV_F32 = 1 };
 enum skv_activation { SKV_ACT_RELU_SQ = 0, SKV_ACT_IDENTITY = 1, SKV_ACT_GELU = 2 };
 /* SKV_IMPL_AUTO picks the tcgen05 kernels when the shape is eligible (bf16, r up to 128, L up to 64, either
  * spline order; other h and r than multiples of 8 and 16 are padded inside the scratch) and the CUDA-core
- * kernels otherwise, for forwards of a few tokens and for backwards of 2^31 - 256 tokens or more.  The CUDA-core kernels are the float32 tier and the path of
- * the remaining shapes, several times slower at production sizes: skv_resolve_impl tells which family a
- * problem gets. */
+ * kernels otherwise, for forwards of a few tokens (512 at most) and for backwards of 2^31 - 256 tokens or more.  The
+ * CUDA-core kernels are the float32 tier and the path of the remaining shapes, several times slower at production
+ * sizes: skv_resolve_impl tells which family a problem gets, skv_resolve_impl_op which one a call gets. */
 enum skv_impl { SKV_IMPL_AUTO = 0, SKV_IMPL_SIMT = 1, SKV_IMPL_TCGEN05 = 2 };
 enum skv_op { SKV_OP_FORWARD = 0, SKV_OP_BACKWARD = 1 };
 
@@ -84,10 +84,15 @@ const char *skv_error_string(int code);
  * Replaces the capability gates of the reference loaders (src/sparsespline_ffn/cuda_ext/__init__.py:31-60). */
 int skv_device_ok(void);
 
-/* Which kernels SKV_IMPL_AUTO resolves to for this problem: SKV_IMPL_SIMT or SKV_IMPL_TCGEN05
+/* Which kernels SKV_IMPL_AUTO resolves to for this problem: SKV_IMPL_SIMT or SKV_IMPL_TCGEN05.  The family is that of
+ * the backward; a forward of so few tokens that reading the table in place is faster than packing it runs on the
+ * CUDA-core kernels all the same (skv_resolve_impl_op)
  * (negative SKV_ERR_* when the problem is invalid).  Replaces the eligibility tests of
  * FlashSplineFeature.forward (src/sparsespline_ffn/kernels/flash_spline_feature_autograd.py:64-82). */
 int skv_resolve_impl(const skv_problem *p);
+
+/* Which kernels a call of op (enum skv_op) with this problem runs on, for rows on 16-byte boundaries. */
+int skv_resolve_impl_op(const skv_problem *p, int op);
 
 /* Bytes of caller-owned scratch that op (enum skv_op) needs for this problem.  The reference
  * kernels allocate theirs internally (src/sparsespline_ffn/cuda_ext/spline_kv_fwd_v11.cu:372-375,

@@ -171,6 +171,13 @@ int skv_resolve_impl(const skv_problem* p) {
   return resolve(*p, SKV_OP_BACKWARD);
 }
 
+int skv_resolve_impl_op(const skv_problem* p, int op) {
+  if (int e = validate(p)) return e;
+  if (op != SKV_OP_FORWARD && op != SKV_OP_BACKWARD) return SKV_ERR_UNSUPPORTED;
+  const int impl = resolve(*p, op);
+  return op == SKV_OP_FORWARD && impl == SKV_IMPL_TCGEN05 && small_forward(*p) ? (int)SKV_IMPL_SIMT : impl;
+}
+
 size_t skv_scratch_bytes(const skv_problem* p, int op) {
   if (validate(p) != SKV_OK) return 0;
   const int impl = resolve(*p, op);

@@ -117,11 +117,16 @@ def _scratch(lib, p: _lib.Problem, op: int, device) -> tuple[torch.Tensor | None
     return torch.empty(need, dtype=torch.uint8, device=device), need
 
 
-def resolve_impl(z, C, grid_lo, grid_hi, G, impl="auto") -> str:
-    """Name of the kernel family the library would use for this problem: 'simt' or 'tcgen05'."""
+def resolve_impl(z, C, grid_lo, grid_hi, G, impl="auto", op: str | None = None, spline_order: int = 2) -> str:
+    """Name of the kernel family the library would use for this problem, 'simt' or 'tcgen05'; with ``op`` 'forward' or
+    'backward' the one that this call runs on (a forward of few tokens reads the table in place on the
+    CUDA cores)."""
     lib = _lib.load()
-    p = _problem(z, C, grid_lo, grid_hi, G, "relu_sq", 1.0, impl)
-    code = lib.skv_resolve_impl(ctypes.byref(p))
+    p = _problem(z, C, grid_lo, grid_hi, G, "relu_sq", 1.0, impl, spline_order)
+    if op is None:
+        code = lib.skv_resolve_impl(ctypes.byref(p))
+    else:
+        code = lib.skv_resolve_impl_op(ctypes.byref(p), {"forward": _lib.SKV_OP_FORWARD, "backward": _lib.SKV_OP_BACKWARD}[op])
     if code < 0:
         _lib.check(code)
     return {1: "simt", 2: "tcgen05"}[code]

@@ -68,6 +68,20 @@ def test_validation_without_a_gpu(lib):
     assert lib.skv_resolve_impl(ctypes.byref(p32)) == -3
 
 
+def test_resolve_per_call_knows_the_small_forward(lib):
+    def family(N, op, **kw):
+        p = _lib.Problem(**{**dict(N=N, h=256, L=22, r=32, grid_lo=-3.0, scale=1.0, lambda_scale=1.0), **kw})
+        return lib.skv_resolve_impl_op(ctypes.byref(p), op)
+
+    fwd, bwd = _lib.SKV_OP_FORWARD, _lib.SKV_OP_BACKWARD
+    simt, tc = _lib.SKV_IMPL["simt"], _lib.SKV_IMPL["tcgen05"]
+    assert family(512, fwd) == simt and family(512, bwd) == tc           # few tokens: the table is read in place
+    assert family(513, fwd) == tc and family(512, fwd, impl=tc) == tc
+    assert family(88, fwd, h=1 << 20) == simt and family(89, fwd, h=1 << 20) == tc
+    assert family(1000, fwd, dtype=1) == simt and family(1000, bwd, dtype=1, impl=tc) == -3
+    assert family(1000, 2) == -3 and family(-1, fwd) == -2
+
+
 @pytest.mark.skipif(torch.cuda.is_available(), reason="checks the no-GPU behaviour")
 def test_no_device_is_an_error_not_a_fallback(lib):
     assert lib.skv_device_ok() == -6
