@@ -2,7 +2,8 @@
 the C ABI, against the reference's own outputs (tests/golden/b1_golden.npz, written by
 tests/golden/make_golden.py from flash_spline_feature_reference(spline_order=1) and autograd,
 src/sparsespline_ffn/rl_spline_kv_reference.py:125-142, 178-187) and against the CPU oracle on larger
-seeded inputs.  It runs on the CUDA-core kernels (float32 arithmetic, bf16 or float32 I/O)."""
+seeded inputs.  float32 runs on the CUDA-core kernels, bf16 from 65 tokens on (forwards: from a few hundred) on the
+tcgen05 kernels with operands as pairs of f16."""
 import os
 
 import numpy as np

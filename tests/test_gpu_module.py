@@ -36,6 +36,17 @@ def fixture():
     return out
 
 
+def _order(case):
+    return CASES[case].get("spline_order", 2)
+
+
+def _twice(rec):
+    """The fixture with its tokens twice: the linear spline's tcgen05 kernels start at 65 tokens, and it has 48."""
+    out = {k: np.concatenate([v, v]) if k in ("x", "gy", "y", "dx") else 2.0 * v if k.startswith("grad.") else v
+           for k, v in rec.items()}
+    return out
+
+
 def _bf(a):
     return torch.from_numpy(np.asarray(a, dtype=np.float32)).to(torch.bfloat16).float().numpy()
 
@@ -47,8 +58,8 @@ def _expected_with_bf16_operator(rec, case):
     z = x @ rec["param.K.weight"].T
     zb, Cb, W = _bf(z), _bf(rec["param.C"]), rec["param.W_out.weight"]
     act = "gelu" if case == "additive_gelu" else "relu_sq"
-    if case in ("additive", "additive_gelu"):
-        a, d = util.oc.feature_forward(zb, Cb, -3.0, 3.0, 20, act, 0.5)
+    if case.startswith("additive"):
+        a, d = util.oc.feature_forward(zb, Cb, -3.0, 3.0, 20, act, 0.5, spline_order=_order(case))
         y = _bf(np.concatenate([a, d], axis=1)) @ W.T
     else:
         _, d = util.oc.feature_forward(zb, Cb, -3.0, 3.0, 20, "identity", 0.5)
@@ -68,10 +79,10 @@ def _expected_dC_with_bf16_operator(rec, case):
     z = x @ rec["param.K.weight"].T
     zb, Cb, W = _bf(z), _bf(rec["param.C"]), rec["param.W_out.weight"]
     g = rec["gy"].reshape(-1, 32) @ W                                  # gradient at the read-out's input
-    if case in ("additive", "additive_gelu"):
+    if case.startswith("additive"):
         act = "gelu" if case == "additive_gelu" else "relu_sq"
         g = _bf(g)
-        return util.oc.feature_backward(zb, Cb, g[:, 64:], g[:, :64], -3.0, 3.0, 20, act, 0.5)[1]
+        return util.oc.feature_backward(zb, Cb, g[:, 64:], g[:, :64], -3.0, 3.0, 20, act, 0.5, spline_order=_order(case))[1]
     if case == "multiplicative":
         g = (g * np.where(z > 0, z * z, 0.0)) @ rec["param.W_d_proj.weight"]
     return util.oc.feature_backward(zb, Cb, _bf(g), None, -3.0, 3.0, 20, "identity", 0.5)[1]
@@ -81,6 +92,8 @@ def _expected_dC_with_bf16_operator(rec, case):
 @pytest.mark.parametrize("case", sorted(CASES))
 def test_module_matches_the_reference_module(fixture, case, dtype):
     rec = fixture[case]
+    if dtype == torch.bfloat16 and _order(case) == 1:
+        rec = _twice(rec)
     cfg = skv_module.RLSplineKVConfig(d=32, h_ratio=2.0, r=16, G=20, grid_lo=-3.0, grid_hi=3.0, lambda_scale=0.5,
                                       c_init_std=0.05, **CASES[case])
     m = skv_module.RLSplineKV(cfg)
@@ -89,7 +102,7 @@ def test_module_matches_the_reference_module(fixture, case, dtype):
     assert not missing.unexpected_keys
     assert set(missing.missing_keys) <= {"grid_lo_buf", "grid_hi_buf"}          # buffers, not parameters
     # float32 throughout runs the CUDA-core kernels: tight gate.  The bf16 variant keeps float32
-    # weights and GEMMs and runs the operator alone in bf16 (the tensor-core kernels): z is rounded to
+    # weights and GEMMs and runs the operator alone in bf16 (its backward on the tensor-core kernels): z is rounded to
     # bf16 on entry, which moves the result by a few 1e-3 of its largest value
     m = m.to(device="cuda")
     m.operator_dtype = None if dtype == torch.float32 else dtype
@@ -97,12 +110,10 @@ def test_module_matches_the_reference_module(fixture, case, dtype):
     y = m(x)
     y.backward(torch.from_numpy(rec["gy"]).to(device="cuda"))
     gate = 2e-4 if dtype == torch.float32 else 2e-2
-    if dtype == torch.bfloat16 and case == "additive_linear":
-        pytest.skip("the linear spline runs on the CUDA-core kernels: the float32 variant covers it")
     if dtype == torch.bfloat16:
         from sparsespline_ffn_b200 import ops as _ops
         z = m.K(x.detach().reshape(-1, 32)).to(dtype)
-        assert _ops.resolve_impl(z, m.C.detach().to(dtype), -3.0, 3.0, 20) == "tcgen05"
+        assert _ops.resolve_impl(z, m.C.detach().to(dtype), -3.0, 3.0, 20, spline_order=_order(case)) == "tcgen05"
         # Rounding z to bf16 moves the result of this fixture by up to 8 % of its largest value (the
         # random code table makes the spline rough), so the forward is checked against the same chain
         # evaluated by the CPU oracle on the rounded z and C, and the gradients only loosely against
