@@ -72,16 +72,6 @@ __device__ __forceinline__ void basis_weights(const Knot& k, float& B0, float& B
   B2 = 0.5f * t * t * m;
 }
 
-// Derivative weights dB_k/dtau (flash_spline_feature_backward_ref.py:64-66), clamp mask applied.
-__device__ __forceinline__ void basis_derivs(const Knot& k, float& d0, float& d1, float& d2, int order = 2) {
-  float t = k.tau;
-  float m = k.clamp_active ? 1.0f : 0.0f;
-  if (order == 1) { d0 = -m; d1 = m; d2 = 0.0f; return; }
-  d0 = -(1.0f - t) * m;
-  d1 = (1.0f - 2.0f * t) * m;
-  d2 = t * m;
-}
-
 // phi and phi' of the base path (rl_spline_kv_reference.py:78-85,
 // flash_spline_feature_autograd.py:227-237).
 // gelu is the exact erf form of torch.nn.functional.gelu; its derivative Phi(z) + z * pdf(z) is what

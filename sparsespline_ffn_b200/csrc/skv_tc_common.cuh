@@ -14,13 +14,9 @@ constexpr int32_t kStatusTimeoutDz = 0x2;
 constexpr int32_t kStatusTimeoutDc = 0x4;
 constexpr int32_t kStatusTimeoutBwd = 0x8;
 
-// A wait gives up after this many clock cycles unless the host set another limit (about two
-// seconds at 2 GHz).  The limit travels in the kernel parameters so that a test can make a wait
-// run out within a millisecond.
-constexpr long long kDefaultWaitCycles = 4000000000LL;
-
 // Test hooks, set through skv_debug_set (host side, read at launch time).
-long long wait_cycle_limit();        // current limit of every bounded wait
+long long wait_cycle_limit();        // current limit of every bounded wait, in clock cycles (by default about two seconds at
+                                     // 2 GHz); it travels in the kernel parameters, so a test can make a wait run out
 int debug_skip_copy();               // 1: the forward's loader leaves out its first code-table copy;
                                      // 2: the read-out GEMM's loader leaves out its first stage
 int fused_backward_roles();          // 0: two kernels (default); 3: dz and dC as one kernel where its plan fits
@@ -172,18 +168,9 @@ __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem], both operands 16-bit, float32 accumulate; issued by one thread.
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with the two descriptors given as 32-bit halves, so that an issue loop only has to
-// advance the low words (start address field) by a constant per K step.
+// D[tmem] (+)= A[smem] * B[smem], both operands 16-bit, float32 accumulate; issued by one thread.  The two
+// descriptors are given as 32-bit halves, so that an issue loop only has to advance the low words (start address
+// field) by a constant per K step.
 __device__ __forceinline__ void umma_f16_split(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                                uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -195,8 +182,9 @@ __device__ __forceinline__ void umma_f16_split(uint32_t tmem_d, uint32_t a_lo, u
       "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Halves of an un-swizzled descriptor (see smem_desc): low word = start address and K stride,
-// high word = M/N stride and the sm_100 version bit.
+// Halves of the shared-memory matrix descriptor of an un-swizzled canonical tile (core matrices of 8 x 16 bytes, layout
+// type 0): low word = start address and `lbo`, the byte stride between core matrices along K; high word = `sbo`, the
+// byte stride along M/N, and the sm_100 version bit.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) {
   return ((addr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);
 }
@@ -241,17 +229,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 // Four float32 added (one rounding each) to four in global memory, without waiting for them.
 __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-// Shared-memory matrix descriptor of an un-swizzled canonical tile: 8 x 16-byte core matrices,
-// `lbo` = byte stride between core matrices along K, `sbo` = byte stride along M/N.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;   // descriptor version of sm_100
-  return d;                 // layout type 0 (no swizzle), base offset 0
 }
 
 // Instruction descriptor for kind::f16: float32 accumulate, A/B element formats (0 = f16, 1 = bf16),
