@@ -3,13 +3,15 @@
 // of microseconds at small sizes, about what the same steps cost in Python for each direction.
 //
 // Only plain calls are served (CUDA tensors of one dtype the kernels take, shapes that agree, unit
-// inner strides).  For anything else an entry returns None and the Python operators take the call: they
+// inner strides, no tracing and no forward-mode tangents: a tracer would record the empty output alone, and a
+// tangent would be dropped without a word).  For anything else an entry returns None and the Python operators take the call: they
 // convert what can be converted and raise what has to be raised.  Nothing is decided differently here.
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -68,6 +70,7 @@ bool plain_problem(const Tensor& z, const Tensor& C, double lo, double hi, long 
   if ((dt != at::kBFloat16 && dt != at::kFloat) || C.scalar_type() != dt) return false;
   if (z.dim() != 2 || C.dim() != 3 || !C.is_contiguous() || z.is_conj() || z.is_neg() || C.is_neg()) return false;
   if (z.stride(1) != 1 || z.stride(0) < z.size(1)) return false;
+  if (z._fw_grad(0).defined() || C._fw_grad(0).defined() || torch::jit::tracer::isTracing()) return false;
   if (C.size(0) != z.size(1) || (order != 1 && order != 2) || C.size(1) != G + order || !(hi > lo)) return false;
   if (z.size(1) > (1 << 24) || C.size(1) > 4096 || C.size(2) > 256 || C.size(2) < 1) return false;
   *p = skv_problem{};
