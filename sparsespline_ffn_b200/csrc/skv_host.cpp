@@ -131,7 +131,16 @@ struct SplineFeatureBackward : public torch::autograd::Node {
     torch::autograd::variable_list out(2);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
-    const Tensor z = z_.unpack(shared_from_this()), C = C_.unpack(shared_from_this());
+    Tensor z = z_.unpack(shared_from_this());
+    const Tensor C = C_.unpack(shared_from_this());
+    // a saved-tensor hook may hand back other strides or another dtype than it was given
+    TORCH_CHECK(z.is_cuda() && C.device() == z.device(), "CUDA-only: the saved z and C must be on one CUDA device");
+    TORCH_CHECK(z.dim() == 2 && z.size(0) == p.N && z.size(1) == p.h && C.dim() == 3 && C.size(0) == p.h &&
+                C.size(1) == p.L && C.size(2) == p.r, "the saved z or C has another shape than the forward's");
+    const auto dt = p.dtype == SKV_F32 ? at::kFloat : at::kBFloat16;
+    if (z.scalar_type() != dt) z = z.to(dt);
+    if (z.stride(1) != 1 || z.stride(0) < z.size(1)) z = z.contiguous();
+    const Tensor table = (C.scalar_type() != dt ? C.to(dt) : C).contiguous();
     const bool need_dz = task_should_compute_output(0), need_dC = task_should_compute_output(1);
     const int64_t width = with_base ? (int64_t)p.h + p.r : p.r;
     c10::cuda::CUDAGuard guard(z.device());
@@ -144,12 +153,12 @@ struct SplineFeatureBackward : public torch::autograd::Node {
     char* gbase = static_cast<char*>(go.data_ptr());
     Tensor dz, dC;
     if (need_dz) dz = at::empty({p.N, p.h}, z.options().requires_grad(false));
-    if (need_dC) dC = at::empty({p.h, p.L, p.r}, C.options().requires_grad(false));
+    if (need_dC) dC = at::empty({p.h, p.L, p.r}, z.options().requires_grad(false));
     const size_t need = skv_scratch_bytes(&p, SKV_OP_BACKWARD);
     Tensor scratch = scratch_for(need, z);
     const bool f32 = p.dtype == SKV_F32;
     const int code = skv_feature_backward(
-        &p, z.data_ptr(), z.stride(0), C.data_ptr(), with_base ? gbase : nullptr, go.stride(0),
+        &p, z.data_ptr(), z.stride(0), table.data_ptr(), with_base ? gbase : nullptr, go.stride(0),
         gbase + (with_base ? p.h * esz : 0), go.stride(0), need_dz ? dz.data_ptr() : nullptr, p.h,
         need_dC && f32 ? static_cast<float*>(dC.data_ptr()) : nullptr, need_dC && !f32 ? dC.data_ptr() : nullptr,
         need ? scratch.data_ptr() : nullptr, need,
