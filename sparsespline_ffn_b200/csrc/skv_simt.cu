@@ -672,7 +672,11 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
           }
         }
 #pragma unroll
-        for (int i = 0; i < V; ++i) { a[0][c][i] = a[1][c][i]; a[1][c][i] = a[2][c][i]; a[2][c][i] = 0.0f; }
+        for (int i = 0; i < V; ++i) {
+          a[0][c][i] = a[1][c][i];
+          a[1][c][i] = three ? a[2][c][i] : 0.0f;     // the linear spline's third weight is zero, but zero times an
+          a[2][c][i] = 0.0f;                          // infinity is not
+        }
       }
     };
     int end = off[0], dirty = 0;                      // rows of the window that hold something
@@ -696,12 +700,6 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
               a[2][c][i] = fmaf(e.z, gv[i], a[2][c][i]);
             }
           }
-        }
-        if (!three) {                                 // zero weights, but zero times an infinity is not zero
-#pragma unroll
-          for (int c = 0; c < CV; ++c)
-#pragma unroll
-            for (int i = 0; i < V; ++i) a[2][c][i] = 0.0f;
         }
       }
       if (dirty > 0) { finish_row(b); --dirty; }

@@ -11,19 +11,21 @@ namespace skv {
 namespace tc {
 namespace {
 
-// Largest |x| seen, as float32 bit patterns: of the finite values, and of all (infinity and the NaN patterns above it
-// included).
-struct AbsMax {
-  uint32_t finite = 0, all = 0;
-  __device__ __forceinline__ void add(uint32_t w) {       // two packed bf16
-    const uint32_t lo = (w << 16) & 0x7fff0000u, hi = w & 0x7fff0000u;
-    all = max(all, max(lo, hi));
-    if (lo < 0x7f800000u) finite = max(finite, lo);
-    if (hi < 0x7f800000u) finite = max(finite, hi);
-  }
-  __device__ __forceinline__ void add(const uint4& v) { add(v.x); add(v.y); add(v.z); add(v.w); }
-};
+constexpr uint32_t kInf = 0x7f800000u;                    // NaN patterns lie above it
 constexpr uint32_t kBadBit = 0x80000000u;                 // of a block's word: it has seen an infinity or a NaN
+
+// Largest |x| of packed bf16 as a float32 bit pattern: of all values, or (FINITE) of the finite ones.
+template <bool FINITE>
+__device__ __forceinline__ uint32_t absmax(uint32_t m, uint32_t w) {
+  const uint32_t lo = (w << 16) & 0x7fff0000u, hi = w & 0x7fff0000u;
+  if (!FINITE || lo < kInf) m = max(m, lo);
+  if (!FINITE || hi < kInf) m = max(m, hi);
+  return m;
+}
+template <bool FINITE>
+__device__ __forceinline__ uint32_t absmax(uint32_t m, const uint4& v) {
+  return absmax<FINITE>(absmax<FINITE>(absmax<FINITE>(absmax<FINITE>(m, v.x), v.y), v.z), v.w);
+}
 
 // Maximum over the block; valid in every thread.  `words` is shared scratch of 32 words.
 __device__ __forceinline__ uint32_t block_max(uint32_t m, uint32_t* words) {
@@ -45,22 +47,17 @@ __device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p, int n, bool vec) { 
   return make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
 }
 
-__global__ void __launch_bounds__(256) tc_scan_kernel(const PrepParams P) {
-  __shared__ uint32_t words[32];
-  pdl_launch();
-  AbsMax m;
-  const bool is_c = (int)blockIdx.x < P.scan_c;
-  const int blk = is_c ? blockIdx.x : blockIdx.x - P.scan_c, nblk = is_c ? P.scan_c : P.scan_g;
-  const int64_t first = (int64_t)blk * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
+// This thread's share of the array that its block scans.
+template <bool FINITE>
+__device__ __forceinline__ uint32_t scan_share(const PrepParams& P, bool is_c, int64_t first, int64_t step) {
+  uint32_t m = 0;
   if (is_c) {
     const int64_t total = (int64_t)P.h * P.L * P.r;
     const int64_t n8 = (reinterpret_cast<uintptr_t>(P.C) & 15) == 0 ? total / 8 : 0;
 #pragma unroll 4
-    for (int64_t i = first; i < n8; i += step) {
-      m.add(__ldg(reinterpret_cast<const uint4*>(P.C) + i));
-    }
+    for (int64_t i = first; i < n8; i += step) m = absmax<FINITE>(m, __ldg(reinterpret_cast<const uint4*>(P.C) + i));
     for (int64_t i = n8 * 8 + first; i < total; i += step)
-      m.add(__ldg(reinterpret_cast<const unsigned short*>(P.C) + i));
+      m = absmax<FINITE>(m, (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(P.C) + i));
   } else {
     const bool vec = P.r % 8 == 0 && P.gds % 8 == 0 && (reinterpret_cast<uintptr_t>(P.g) & 15) == 0;
     const int cgs = (P.r + 7) / 8;
@@ -69,12 +66,21 @@ __global__ void __launch_bounds__(256) tc_scan_kernel(const PrepParams P) {
     for (int64_t i = first; i < pieces; i += step) {
       const int64_t n = i / cgs;
       const int c = (int)(i - n * cgs) * 8;
-      m.add(ld8(P.g + n * P.gds + c, P.r - c, vec));
+      m = absmax<FINITE>(m, ld8(P.g + n * P.gds + c, P.r - c, vec));
     }
   }
-  const uint32_t top = block_max(m.finite, words);
-  const int bad = __syncthreads_or(m.all >= 0x7f800000u);
-  if (threadIdx.x == 0) P.hdr[kBlockMax + (is_c ? 0 : kMaxBlocks) + blk] = top | (bad ? kBadBit : 0u);
+  return m;
+}
+
+__global__ void __launch_bounds__(256) tc_scan_kernel(const __grid_constant__ PrepParams P) {
+  __shared__ uint32_t words[32];
+  pdl_launch();
+  const bool is_c = (int)blockIdx.x < P.scan_c;
+  const int blk = is_c ? blockIdx.x : blockIdx.x - P.scan_c, nblk = is_c ? P.scan_c : P.scan_g;
+  const int64_t first = (int64_t)blk * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
+  uint32_t m = block_max(scan_share<false>(P, is_c, first, step), words);
+  if (m >= kInf) m = block_max(scan_share<true>(P, is_c, first, step), words) | kBadBit;   // once more, without them
+  if (threadIdx.x == 0) P.hdr[kBlockMax + (is_c ? 0 : kMaxBlocks) + blk] = m;
 }
 
 __device__ __forceinline__ uint32_t combine(const uint32_t* part, int n, uint32_t* words, bool& bad) {
@@ -227,24 +233,33 @@ __device__ __forceinline__ float pair_weight(const Knot& k, int row, int order) 
   return row == 0 ? B0 : row == 1 ? B1 : B2;
 }
 
-// delta[n][c .. c + 3]: the contributions of infinities and NaN in C (a zero weight times one is NaN here too, as it is
-// when the touched rows alone are added up); true when there is one.
-__device__ __noinline__ bool contain_delta(const Contain& K, int64_t n, int c, float (&s)[4]) {
-  bool any = false;
-  for (int j = 0; j < K.h; ++j) {
-    const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j]), K.grid);
-    for (int row = 0; row <= K.grid.order; ++row) {
-      const __nv_bfloat16* src = K.C + ((size_t)j * K.L + k.bin + row) * K.r + c;
-      for (int i = 0; i < 4 && c + i < K.r; ++i) {
-        const float v = __bfloat162float(src[i]);
-        if (is_bad(v)) {
-          s[i] = fmaf(pair_weight(k, row, K.grid.order), v, s[i]);
-          any = true;
+// delta: the contributions of infinities and NaN in C (a zero weight times one is NaN here too, as it is when the
+// touched rows alone are added up).  A thread takes the elements that it has written.
+template <typename TD>
+__device__ __noinline__ void contain_delta(const Contain& K, int rp, float lambda, TD* out, int64_t ds) {
+  const int q4 = rp / 4;
+  const int64_t total = K.N * q4;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n = i / q4;
+    const int c = (int)(i - n * q4) * 4;
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    bool any[4] = {false, false, false, false};
+    for (int j = 0; j < K.h; ++j) {
+      const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j]), K.grid);
+      for (int row = 0; row <= K.grid.order; ++row) {
+        const __nv_bfloat16* src = K.C + ((size_t)j * K.L + k.bin + row) * K.r + c;
+        for (int x = 0; x < 4 && c + x < K.r; ++x) {
+          const float v = __bfloat162float(src[x]);
+          if (is_bad(v)) {
+            s[x] = fmaf(pair_weight(k, row, K.grid.order), v, s[x]);
+            any[x] = true;
+          }
         }
       }
     }
+    for (int x = 0; x < 4; ++x)
+      if (any[x]) st_f32<TD>(out + n * ds + c + x, lambda * s[x]);
   }
-  return any;
 }
 
 // dC: the same for infinities and NaN in g_delta.  A block lists the tokens that have any, 256 tokens at a time, and its
@@ -349,12 +364,11 @@ __device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c
 template <typename TD, bool CONTAIN>
 __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, int splits, int64_t N, int r,
                                                           int rp, float lambda, const uint32_t* hdr,
-                                                          TD* out, int64_t ds, const Contain K) {
+                                                          TD* out, int64_t ds, const __grid_constant__ Contain K) {
   pdl_launch();
   pdl_wait();
   float cscale, cinv;
   pow2_scales(hdr[kAmaxC], cscale, cinv);
-  const bool bad = CONTAIN && hdr[kBadC] != 0u;
   const float f = lambda * cinv;                        // undo the code-table image's range scaling
   const int q4 = rp / 4;
   const int64_t total = N * q4;
@@ -370,14 +384,7 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
     const int64_t n = i / q4;
     const int c = (int)(i - n * q4) * 4;
     TD* o = out + n * ds + c;
-    float v[4] = {f * s.x, f * s.y, f * s.z, f * s.w};
-    if constexpr (CONTAIN) {
-      if (bad) {
-        float extra[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (contain_delta(K, n, c, extra))
-          for (int k = 0; k < 4; ++k) v[k] += lambda * extra[k];
-      }
-    }
+    const float v[4] = {f * s.x, f * s.y, f * s.z, f * s.w};
     if (vec) {
       if constexpr (sizeof(TD) == 4) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
       else *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf2(v[0], v[1]), pack_bf2(v[2], v[3]));
@@ -387,13 +394,15 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
         if (c + k < r) st_f32<TD>(o + k, v[k]);
     }
   }
+  if constexpr (CONTAIN)
+    if (hdr[kBadC] != 0u) contain_delta(K, rp, lambda, out, ds);
 }
 
 template <bool CONTAIN>
 __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, const DcParts parts, int64_t rows,
                                                            int64_t rows_padded, int r, int rp, float lambda,
                                                            const uint32_t* hdr, float* dC,
-                                                           __nv_bfloat16* dC_cast, const Contain K) {
+                                                           __nv_bfloat16* dC_cast, const __grid_constant__ Contain K) {
   pdl_wait();
   float gscale, ginv;
   pow2_scales(hdr[kAmaxG], gscale, ginv);
@@ -436,7 +445,7 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
   }
 }
 
-__global__ void __launch_bounds__(256) tc_dz_contain_kernel(const uint32_t* hdr, const Contain K) {
+__global__ void __launch_bounds__(256) tc_dz_contain_kernel(const uint32_t* hdr, const __grid_constant__ Contain K) {
   pdl_wait();
   const bool bad_g = hdr[kBadG] != 0u, bad_c = hdr[kBadC] != 0u;
   if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
