@@ -96,11 +96,11 @@ bool make_dc_plan(const skv_problem& p, DcPlan* o) {
     const double unit = 0.38 * (split_operands(p) ? 1.6 : 1.0) * kch / 16.0 * words / 11.0 * (0.8 + rp / 160.0), tile = 0.002 * rp;
     const double per_part = (double)hp * p.L * rp * 8.0 / 5.0e6 + 0.1;
     o->chain = split_operands(p) ? kDcSplitChain : kDcChain;
-    // what a CTA pays for the segments of a slab after its first: its accumulators' way to the partial (10 us for 480
-    // columns of tensor memory, 3.4 us for 96)
+    // what a CTA pays for the segments of a slab after its first: its accumulators' way to the partial (8 to 10 us for 480
+    // columns of tensor memory, 1.5 to 3 for 96)
     auto flush = [&](uint64_t run, uint64_t T, int slab) {
       const uint64_t len = run < T ? run : T;
-      return (double)((len - 1) / o->chain * (run / len)) * (1.5 + 0.018 * slab * mtiles * rp);
+      return (double)((len - 1) / o->chain * (run / len)) * (1.0 + 0.017 * slab * mtiles * rp);
     };
     double best = 0.0;
     for (int slab = most < chunks ? most : chunks; slab >= 1; --slab) {

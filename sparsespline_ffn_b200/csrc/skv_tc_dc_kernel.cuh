@@ -53,10 +53,11 @@ constexpr int kDcMaxRing = 8;                        // slots of the ring of g t
 // core cuts a sum off at the accumulator's last bit, always towards zero: the error grows with the number of MMAs
 // and does not average out.  Error of dC against 64 bits at 65536 x 5120, r = 32 / r = 128, all gradients positive (so that
 // every bit lost counts): one accumulator for 443 / 1024 tiles 6.8e-5 / 1.9e-4, 256 tiles 5.0e-5 / 5.4e-5, 192 tiles
-// 4.7e-5 / 4.7e-5 (what rounding the operands to f16 gives), dC alone 0.82 / 1.54, 0.83 / 1.61, 0.84 / 1.65 ms.
+// 4.7e-5 / 4.7e-5 (what rounding the operands to f16 gives), dC alone 0.81 / 1.53, 0.82 / 1.57, 0.83 / 1.60 ms.
 // With pairs of f16 there is no such floor: 65536 x 5113, r = 32: 443 tiles 9.9e-5, 32 tiles 7.0e-6, 16 tiles 3.4e-6,
-// 8 tiles 1.8e-6; 1.82, 1.97, 2.12, 2.44 ms.
-constexpr uint32_t kDcChain = 192, kDcSplitChain = 8;
+// 8 tiles 1.8e-6; 1.94, 2.03, 2.14, 2.36 ms; 4096 x 1024, linear: 37, 37, 38, 45 us.  (float32 arithmetic on the CUDA
+// cores: 3.2e-6 at the former size, 13.7 ms.)
+constexpr uint32_t kDcChain = 192, kDcSplitChain = 16;
 constexpr int kDcIssuers = 3;                        // warps that issue MMAs, each for every third M tile
 // One unit behind a stage: the linear spline's last interval stores a zero word there.
 __host__ __device__ constexpr uint32_t dc_stage_bytes(int mtiles) { return (uint32_t)mtiles * 16u * kDcUnit + kDcUnit; }
@@ -228,16 +229,20 @@ __global__ void __launch_bounds__(640, 1) tc_dc_kernel(const DcParams P) {
         const int bb = 2 * (unit - j * P.words) + (lane_row & 1);
         const int key = key0 + c * KCH + KJ * ((lane_row & 7) >> 1) + j;
         const bool ok = j < KJ && key < P.h && bb < L;                   // the pad row of an odd L is dropped
-        float* dst = part + ((size_t)key * L + bb) * r;
+        const uint32_t at = ok ? (uint32_t)(key * L + bb) : ~0u;         // row of the partial
         const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(e * r);
         for (int c0 = 0; c0 < r; c0 += 16) {
           float v[16];
           tmem_ld16(taddr + c0, v);
-          if (ok) {
+          quad_transpose(v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              if (more) red_add4(dst + c0 + i, v[i], v[i + 1], v[i + 2], v[i + 3]);   // to what this thread has put there
-              else *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          for (int j4 = 0; j4 < 4; ++j4) {
+            const uint32_t row4 = __shfl_sync(0xffffffffu, at, (lane & ~3) + j4);
+            if (row4 != ~0u) {
+              float* dst = part + (size_t)row4 * r + c0 + 4 * (lane & 3);
+              const float* q = v + 4 * j4;
+              if (more) red_add4(dst, q[0], q[1], q[2], q[3]);             // to what this thread has put there
+              else *reinterpret_cast<float4*>(dst) = make_float4(q[0], q[1], q[2], q[3]);
             }
           }
         }

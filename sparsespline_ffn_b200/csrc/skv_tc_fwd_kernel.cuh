@@ -79,8 +79,8 @@ constexpr int kStagedPerHalf = 1;
 // Chunks whose MMAs follow one another in an accumulator of the SPLIT cases; what they gave is then added to the partial in
 // float32.  The tensor core cuts a sum off at the accumulator's last bit, always towards zero, so the error grows with the
 // number of MMAs and does not average out: 65536 x 5113, r = 32, error of delta against 64 bits with every chunk
-// in one accumulator 1.8e-5 (2.6e-5 where all summands are positive), with 16 chunks 2.3e-6, with 8 1.2e-6 (1.4e-6); the call 1.42,
-// 1.48 and 1.56 ms.  (Single f16 operands are off by 2e-4 already.)
+// in one accumulator 1.8e-5 (2.6e-5 where all summands are positive), with 16 chunks 2.3e-6, with 8 1.2e-6 (1.4e-6); the call 1.41,
+// 1.43 and 1.47 ms.  (Single f16 operands are off by 2e-4 already.)
 constexpr int kSplitChain = 8;
 
 // SPLIT: the weights' remainders follow the weights, in columns of their own and with the same metadata.
@@ -152,18 +152,22 @@ __global__ void __launch_bounds__(160 * GROUPS + 32, 1) tc_forward_kernel(const 
     const bool up = (lane & 8) != 0;
     const uint32_t sel_send = up ? 0x5410u : 0x7632u;               // halves of two metadata words the other row needs
     const uint32_t sel_0 = up ? 0x3254u : 0x5410u, sel_1 = up ? 0x3276u : 0x7610u;
-    float* prow = P.partial + ((size_t)blockIdx.y * P.N + (valid ? n : 0)) * r;
-    const uint32_t daddr = lane_addr + (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta);
     // accumulator -> float32 partial of this key split; `more`: added to what this thread has put there
     auto drain_acc = [&](bool more) {
+      const int64_t n4 = n & ~(int64_t)3;
+      float* prow = P.partial + ((size_t)blockIdx.y * P.N + n4) * r + 4 * (lane & 3);
+      const uint32_t daddr = lane_addr + (uint32_t)(kParts * kChunkKeys * F + 2 * kMeta);
       for (int c0 = 0; c0 < r; c0 += 16) {
         float v[16];
         tmem_ld16(daddr + c0, v);
-        if (valid) {
+        quad_transpose(v);
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            if (SPLIT && more) red_add4(prow + c0 + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
-            else *reinterpret_cast<float4*>(prow + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        for (int j = 0; j < 4; ++j) {
+          if (n4 + j < P.N) {
+            float* dst = prow + (size_t)j * r + c0;
+            const float* q = v + 4 * j;
+            if (SPLIT && more) red_add4(dst, q[0], q[1], q[2], q[3]);
+            else *reinterpret_cast<float4*>(dst) = make_float4(q[0], q[1], q[2], q[3]);
           }
         }
       }

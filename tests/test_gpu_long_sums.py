@@ -43,8 +43,8 @@ def test_dC_of_many_tokens_per_accumulator(N, h, r):
 @pytest.mark.parametrize("N,h,r,G,order", [(20000, 5113, 32, 20, 2), (33000, 4096, 32, 20, 1), (2000, 1001, 20, 12, 2),
                                            (9000, 1536, 33, 20, 2), (600, 8 * 8 * 16 + 1, 20, 48, 2)])
 def test_pairs_of_f16_keep_their_accuracy(N, h, r, G, order):
-    # forward: 8 chunks of 8 keys, dC: 8 tiles of 64 tokens to an accumulator, 64 to 256 MMAs, each at most 2^-23 of
-    # the sum so far; 22 bits of the operands
+    # forward: 8 chunks of 8 keys, dC: 16 tiles of 64 tokens to an accumulator, 64 to 256 MMAs, each at most 2^-23 of
+    # the sum so far, 2^-24 of the final one on the average: 128 x 2^-24 x 1/2 = 4e-6 for dC, and 22 bits of the operands
     z, g = _normal(N, h, seed=1), _normal(N, r, seed=2).abs()
     C = (_normal(h, G + order, r, seed=3) * 0.02).abs()
     kw = dict(impl="tcgen05", spline_order=order, with_base=False)
