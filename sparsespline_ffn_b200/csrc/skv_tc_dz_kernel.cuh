@@ -40,29 +40,15 @@ struct DzParams {
   long long wait_cycles;     // limit of every bounded wait, in clock cycles
 };
 
-// Tensor-memory loads of one key's S columns: the first NC of its LB blocks of 8 float32 columns of
-// this warp's lanes (the padding columns are never read: the kernel's time follows the bytes it moves
-// out of tensor memory, 4 * NC per pair).  The loads are issued without waiting; tmem_wait_key waits
-// for all outstanding loads and ties the destination registers to the wait so that no use can be
-// scheduled ahead of it.
+// Tensor-memory loads of one key's S columns, LB blocks of 8 float32 columns of this warp's lanes.  The loads are issued
+// without waiting; tmem_wait_key waits for all outstanding loads and ties the destination registers to the wait so that
+// no use can be scheduled ahead of it.
 template <int N> __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r);
 template <> __device__ __forceinline__ void tmem_ld_cols<8>(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr)
                : "memory");
-}
-template <> __device__ __forceinline__ void tmem_ld_cols<4>(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr)
-               : "memory");
-}
-template <> __device__ __forceinline__ void tmem_ld_cols<2>(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
-}
-template <> __device__ __forceinline__ void tmem_ld_cols<1>(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[0]) : "r"(taddr) : "memory");
 }
 template <> __device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -73,9 +59,9 @@ template <> __device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uin
       : "r"(taddr)
       : "memory");
 }
-// All 8 * LB columns of the key, in as few instructions as possible (a load instruction costs more
-// than the columns it moves: loading only the NC useful columns as 8 + 8 + 4 + 1 was slower, 1.16 ms
-// against 1.11 ms at the d20 shape).
+// All 8 * LB columns of the key, in as few instructions as possible: a load instruction costs more than the columns it
+// moves.  (Measured on an earlier form of the kernel with one S block of 8 keys: the NC useful columns as 8 + 8 + 4 + 1
+// took 1.16 ms at the d20 shape, all 24 as 16 + 8 1.11 ms.)
 template <int LB, int NC>
 __device__ __forceinline__ void tmem_ld_key(uint32_t taddr, uint32_t (&r)[LB][8]) {
   uint32_t* flat = &r[0][0];
@@ -140,8 +126,8 @@ __host__ __device__ constexpr int dz_block_keys(int lb) { return lb <= 4 ? 4 : 2
 //   one warp (lane 0)    moves the group's boxes: loads of z and g_act, stores of dz
 // and one loader warp for the transformed table.
 //
-// Bound: instruction issue of the consumers (64 instructions per 32 pairs, 42 of them the saturating adds and the
-// packed FMAs).  What it took to get near it, at the d20 shape: MMAs issued by an elected thread (300-400 cycles
+// Bound: instruction issue of the consumers (71 instructions per 32 pairs at L = 22, 32 of them the saturating adds and the
+// packed FMAs; 72 % of the issue slots).  What it took to get near it, at the d20 shape: MMAs issued by an elected thread (300-400 cycles
 // per pair of MMAs before, 150 now), which is what makes smaller S blocks affordable; two blocks per group, so that
 // one is computed while the other is read (with one block of 8 keys a group waited 670 cycles per chunk); a
 // block given back as soon as its last key is in registers; the boxes' copies on a warp of their own (a consumer
@@ -405,7 +391,10 @@ __global__ void __launch_bounds__(320 * GROUPS + 32, 1)
 
 struct DzPlan { int groups, lb, splits, chunks_per_split, tstages, rstages; size_t smem; };
 
-// NC_ = L - 1 useful columns per key for the knot counts in common use, all 8 * LB_ otherwise.
+// Columns whose weights are formed: the L - 1 useful ones, known at compile time, where that spares three to seven of
+// 8 * LB and the spline is one that the package's defaults and sweeps use; all 8 * LB otherwise (the padding's weights are
+// zero).  dz at 65536 x 5120, r = 32, exact against all: L = 22 0.973 / 1.043 ms, L = 42 1.70 / 1.83 ms, linear L = 21
+// 1.10 / 1.17 ms.  One column spared (L = 16, 15 of 16) costs a pair its partner: 0.888 / 0.854 ms.
 template <bool LIN, bool SPLIT>
 cudaError_t dz_launch(const DzPlan& zp, int L, bool relu, const DzParams& P, dim3 grid, cudaStream_t stream) {
   CUtensorMap mz, mg, md;
@@ -422,7 +411,7 @@ cudaError_t dz_launch(const DzPlan& zp, int L, bool relu, const DzParams& P, dim
   if constexpr (LIN) {
     SKV_DZ_CASE(2, 3, 20, L == 21)
   } else {
-    SKV_DZ_CASE(2, 3, 21, L == 22) SKV_DZ_CASE(2, 2, 15, L == 16) SKV_DZ_CASE(2, 6, 41, L == 42)
+    SKV_DZ_CASE(2, 3, 21, L == 22) SKV_DZ_CASE(2, 6, 41, L == 42)
   }
   SKV_DZ_CASE(2, 1, 8, true) SKV_DZ_CASE(2, 2, 16, true) SKV_DZ_CASE(2, 3, 24, true) SKV_DZ_CASE(2, 4, 32, true)
   SKV_DZ_CASE(2, 5, 40, true) SKV_DZ_CASE(2, 6, 48, true) SKV_DZ_CASE(2, 7, 56, true) SKV_DZ_CASE(2, 8, 64, true)
