@@ -99,6 +99,13 @@ int skv_resolve_impl_op(const skv_problem *p, int op);
  * src/sparsespline_ffn/cuda_ext/spline_kv_bwd_wgmma_v5.cu:588-598). */
 size_t skv_scratch_bytes(const skv_problem *p, int op);
 
+/* Infinities and NaN.  In z: a value outside the grid (or NaN) has no spline weight.  In C and g_delta: the CUDA-core
+ * kernels, and the tcgen05 kernels where they hold operands as pairs of f16 (linear spline, h no multiple of 8, r no
+ * multiple of 16, more than 49 knot rows), let such an element reach only the results of the (token, key) pairs that touch
+ * it.  On the other shapes the tcgen05 kernels multiply knot rows that a pair does not touch by zero weights, so a
+ * non-finite element of C can make delta of its code channel and dz of its key non-finite for all tokens, and one of
+ * g_delta dC of its channel in all rows. */
+
 /* Forward.  Replaces spline_kv_fwd_cuda / spline_kv_fwd_v11_cuda
  * (src/sparsespline_ffn/cuda_ext/__init__.py:529-555, src/sparsespline_ffn/cuda_ext/spline_kv_fwd_v11.cu:349-402)
  * and the Triton forward flash_spline_feature_forward
