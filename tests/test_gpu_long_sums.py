@@ -56,3 +56,31 @@ def test_pairs_of_f16_keep_their_accuracy(N, h, r, G, order):
     for keys in (slice(0, 4), slice(h - 4, h)):
         util.assert_parity("dC", dC[keys], _dC_of(z, C, g, G, order, keys), torch.float32, bias=True, rel_gate=5e-6)
     ops.check_status(z.device)
+
+
+# one CTA per slab or more slabs than SMs, so that a run has all the tiles: on both sides of 16 and 32 tiles of 64 tokens
+@pytest.mark.parametrize("N", [1023, 1024, 1025, 2048, 2049, 2113])
+def test_dC_at_the_ends_of_its_segments(N):
+    h, r, G = 12008, 16, 20
+    z, g = _normal(N, h, seed=4), _normal(N, r, seed=5)
+    C = torch.zeros(h, G + 1, r, dtype=torch.bfloat16, device="cuda")
+    _, dC, dC_cast = ops.feature_backward(z, C, g, LO, HI, G, "identity", 1.0, with_base=False, need_dz=False, impl="tcgen05",
+                                          spline_order=1)
+    for keys in (slice(0, 4), slice(6000, 6004), slice(h - 4, h)):
+        util.assert_parity("dC", dC[keys], _dC_of(z, C, g, G, 1, keys), torch.float32, bias=True, rel_gate=5e-6)
+    assert torch.equal(dC_cast, dC.bfloat16())
+    ops.check_status(z.device)
+
+
+# a tile of 384 tokens for each of 148 SMs, so that one split has all the keys: on both sides of 8, 16 and 24 chunks of 8
+@pytest.mark.parametrize("h", [57, 64, 65, 72, 128, 129, 192, 193])
+def test_forward_at_the_ends_of_its_chains(h):
+    N, r, G = 148 * 384 - 3, 20, 12
+    z = _normal(N, h, seed=6)
+    C = _normal(h, G + 2, r, seed=7) * 0.02
+    a, delta = ops.feature_forward(z, C, LO, HI, G, "identity", 1.0, delta_f32=True, impl="tcgen05")
+    assert torch.equal(a, z)
+    for rows in (slice(0, 64), slice(N // 2, N // 2 + 64), slice(N - 64, N)):
+        _, ref = util.oc.feature_forward(util.f32(z[rows]), util.f32(C), LO, HI, G, "identity", 1.0)
+        util.assert_parity("delta", delta[rows], ref, torch.float32, rel_gate=5e-6)
+    ops.check_status(z.device)
