@@ -69,3 +69,26 @@ def test_debug_set_rejects_unknown_settings():
     lib = _lib.load()
     assert lib.skv_debug_set(99, 1) < 0
     assert lib.skv_debug_set(_lib.SKV_DEBUG_WAIT_CYCLES, 5) < 0   # a limit too short to be useful
+
+
+def test_a_forward_with_paired_operands_drains_too():
+    # 25 chunks: the accumulator would be added to the partial three times before the end
+    lib = _lib.load()
+    N, h, r, G = 60000, 200, 32, 20
+    z, C, _ = util.make_inputs(N, h, r, G - 1, torch.bfloat16)            # G + 1 knot rows
+    ops.check_status(z.device)
+    assert lib.skv_debug_set(_lib.SKV_DEBUG_WAIT_CYCLES, 2_000_000) == 0
+    assert lib.skv_debug_set(_lib.SKV_DEBUG_SKIP_FIRST_COPY, 1) == 0
+    try:
+        ops.feature_forward(z, C, -3.0, 3.0, G, impl="tcgen05", spline_order=1)
+        torch.cuda.synchronize()
+    finally:
+        lib.skv_debug_set(_lib.SKV_DEBUG_SKIP_FIRST_COPY, 0)
+        lib.skv_debug_set(_lib.SKV_DEBUG_WAIT_CYCLES, 4_000_000_000)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        ops.check_status(z.device)
+    f = ops.feature_forward(z, C, -3.0, 3.0, G, "relu_sq", 0.75, impl="tcgen05", spline_order=1)
+    rows = slice(N - 100, N)
+    _, d_ref = util.oc.feature_forward(util.f32(z[rows]), util.f32(C), -3.0, 3.0, G, "relu_sq", 0.75, spline_order=1)
+    util.assert_parity("lambda*delta", f[rows, h:], d_ref, torch.bfloat16)
+    ops.check_status(z.device)
