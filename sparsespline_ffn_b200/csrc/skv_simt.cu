@@ -13,9 +13,16 @@ namespace {
 
 constexpr int kWarp = 32;
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kWarps = 8;             // warps per CTA of the token-major kernels
+constexpr int kWarps = 8;             // warps per CTA of the kernels below, but for staged_warps
 constexpr int kGroups = 4;            // token groups a warp of the staged forward keeps accumulators for
 constexpr int kSmallEntries = 256;    // pair weights per warp of the small forward (tokens x keys of a pass)
+
+// Warps per CTA of the kernels over a staged table, two CTAs per SM.  What a lane waits for is a chain of two shared-memory reads per
+// key (weights, then rows), so warps are what hides it: sixteen where a lane's registers allow it (64 of them: float32 rows
+// of up to 128 channels, and four to sixteen lanes per token, so that their staging buffers leave room for the table).
+__host__ __device__ constexpr int staged_warps(int lpt, int cv, int row_bytes_per_lane) {
+  return row_bytes_per_lane == 4 && cv == 1 && lpt >= 4 ? 16 : 8;
+}
 
 __host__ __device__ inline int64_t cdiv64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -99,20 +106,21 @@ __device__ __forceinline__ float4 pair_weights(float zz, const GridParams& g, in
 // bf16 table stays bf16 there.
 // ---------------------------------------------------------------------------------------------
 template <typename T, typename TD, int LPT, int CV>
-__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const FwdArgs P) {
-  constexpr int V = Vec<T>::n;
+__global__ void __launch_bounds__(staged_warps(LPT, CV, sizeof(T)) * kWarp, 2) simt_forward_kernel(const FwdArgs P) {
+  constexpr int V = Vec<T>::n, W = staged_warps(LPT, CV, sizeof(T));
   constexpr int TPW = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
-  constexpr int kPre = TPW < 8 ? TPW : 8;                                 // tokens of the next group loaded ahead
+  constexpr int kPre = TPW < 8 ? TPW : 8;                                 // tokens of a group loaded ahead
+  constexpr int kAhead = TPW * kGroups <= 8 ? kGroups : 1;                // groups loaded ahead: all where that is eight values
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float4* wbuf = reinterpret_cast<float4*>(smem_raw);                     // [warp][TPW][32]
-  T* Cs = reinterpret_cast<T*>(wbuf + kWarps * TPW * kWarp);               // [kch][L][pitch]
+  T* Cs = reinterpret_cast<T*>(wbuf + W * TPW * kWarp);               // [kch][L][pitch]
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const int sub = lane / LPT, sl = lane % LPT;
   float4* my = wbuf + warp * TPW * kWarp;
   const T* z = static_cast<const T*>(P.z);
   T* act_out = static_cast<T*>(P.act_out);
-  const int64_t tile0 = (int64_t)blockIdx.x * (kWarps * TPW * P.groups);
+  const int64_t tile0 = (int64_t)blockIdx.x * (W * TPW * P.groups);
   const int kbeg = blockIdx.y * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
   const int rowstep = pitch;
   const bool three = P.g.order != 1;
@@ -128,38 +136,45 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const F
 
   for (int j0 = kbeg; j0 < kend; j0 += P.kch) {
     const int kc = min(P.kch, kend - j0);
+    // rows of the first token of the group whose pre-activations are loaded next, and of the group that is worked on
+    // (running pointers: as offsets of the group number the compiler would keep every group's in registers)
+    const int64_t first = tile0 + (int64_t)warp * TPW;
+    const T* zp = z + first * P.zs + j0 + lane;
+    T* ap = act_out ? act_out + first * P.as + j0 + lane : nullptr;
+    float zn[kAhead][kPre];
+    auto load_z = [&](int m) {
+      asm volatile("" : "+l"(zp));
+      const int64_t n0 = first + (int64_t)m * (W * TPW);
+#pragma unroll
+      for (int t = 0; t < kPre; ++t)
+        zn[m % kAhead][t] = m < P.groups && lane < kc && n0 + t < P.N ? ld_f32<T>(zp + t * P.zs) : 0.0f;
+      if (kPre == TPW) zp += (int64_t)(W * TPW) * P.zs;
+    };
+#pragma unroll
+    for (int m = 0; m < kAhead; ++m) load_z(m);
     __syncthreads();
     stage_rows(Cs, static_cast<const T*>(P.C) + (size_t)j0 * P.L * P.r, kc * P.L, P.r, pitch);
     __syncthreads();
-    float zn[kPre];
-    auto load_z = [&](int m) {
-#pragma unroll
-      for (int t = 0; t < kPre; ++t) {
-        const int64_t n = tile0 + (int64_t)(m * kWarps + warp) * TPW + t;
-        zn[t] = m < P.groups && lane < kc && n < P.N ? ld_f32<T>(z + n * P.zs + j0 + lane) : 0.0f;
-      }
-    };
-    load_z(0);
 #pragma unroll
     for (int m = 0; m < kGroups; ++m) {
       if (m >= P.groups) break;
-      const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+      const int64_t n0 = first + (int64_t)m * (W * TPW);
       if (n0 >= P.N) break;
-      float zc[kPre];
-#pragma unroll
-      for (int t = 0; t < kPre; ++t) zc[t] = zn[t];
-      load_z(m + 1);                                  // the next group's pre-activations are requested now
+      asm volatile("" : "+l"(ap));
       __syncwarp();
 #pragma unroll
       for (int t = 0; t < TPW; ++t) {
         float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (lane < kc && n0 + t < P.N) {
-          const float zz = t < kPre ? zc[t < kPre ? t : 0] : ld_f32<T>(z + (n0 + t) * P.zs + j0 + lane);
+          const float zz = t < kPre ? zn[m % kAhead][t < kPre ? t : 0] : ld_f32<T>(zp + t * P.zs);
           w = pair_weights(zz, P.g, lane * P.L, pitch);
-          if (act_out) st_f32<T>(act_out + (n0 + t) * P.as + j0 + lane, act_fwd(zz, P.act));
+          if (act_out) st_f32<T>(ap + t * P.as, act_fwd(zz, P.act));
         }
         my[t * kWarp + lane] = w;
       }
+      if (kPre < TPW) zp += (int64_t)(W * TPW) * P.zs;
+      if (act_out) ap += (int64_t)(W * TPW) * P.as;
+      if (kAhead < kGroups) load_z(m + kAhead);       // the next group's pre-activations are requested now
       __syncwarp();
 #pragma unroll 2
       for (int q = 0; q < kc; ++q) {
@@ -185,7 +200,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_forward_kernel(const F
 #pragma unroll
   for (int m = 0; m < kGroups; ++m) {
     if (m >= P.groups) break;
-    const int64_t n = tile0 + (int64_t)(m * kWarps + warp) * TPW + sub;
+    const int64_t n = tile0 + (int64_t)(m * W + warp) * TPW + sub;
     if (n >= P.N) continue;
 #pragma unroll
     for (int c = 0; c < CV; ++c)
@@ -337,7 +352,7 @@ __global__ void __launch_bounds__(256) simt_finalize_kernel(const float* __restr
 // dz: grid = (token tiles, key slabs).  The derivative of the quadratic spline is linear between the knots,
 //     sum_k B_k' C[bin + k] = (1 - tau) D[bin] + tau D[bin + 1],   D[b] = C[b + 1] - C[b]
 // (the linear spline: D[bin] alone), so the slab is staged as its differences D in float32 and a pair
-// reads two rows instead of three.  The lanes of a token hold partial sums of LPT keys and one
+// reads two rows instead of three.  The lanes of a token hold partial sums of eight keys and one
 // transpose-reduce turns them into one key's sum per lane; 32 keys' results go through shared memory so
 // that z, g_act and dz are read and written by whole rows of 32 keys.
 //
@@ -364,16 +379,17 @@ struct DzArgs {
 
 // STAGED = false: a key's differences do not fit shared memory; they are formed from the table itself.
 template <typename T, int LPT, int CV, bool STAGED>
-__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs P) {
-  constexpr int V = 4;
+__global__ void __launch_bounds__(staged_warps(LPT, CV, 4) * kWarp, 2) simt_dz_kernel(const DzArgs P) {
+  constexpr int V = 4, W = staged_warps(LPT, CV, 4);
+  constexpr int Q = LPT < 8 ? LPT : 8;                                     // keys of a transpose
   constexpr int TPW = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
   constexpr int kPre = TPW < 8 ? TPW : 8;                                  // tokens of the next group loaded ahead
   constexpr int kRes = kWarp + 4;                                          // pitch of the result rows
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float2* wbuf = reinterpret_cast<float2*>(smem_raw);                     // [warp][TPW][32]  (tau, row offset)
-  float* rbuf = reinterpret_cast<float*>(wbuf + kWarps * TPW * kWarp);     // [warp][TPW][kRes]
-  float* Ds = rbuf + kWarps * TPW * kRes;                                  // [kch][rows][pitch]
+  float* rbuf = reinterpret_cast<float*>(wbuf + W * TPW * kWarp);     // [warp][TPW][kRes]
+  float* Ds = rbuf + W * TPW * kRes;                                  // [kch][rows][pitch]
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const int sub = lane / LPT, sl = lane % LPT;
   float2* my = wbuf + warp * TPW * kWarp;
@@ -385,7 +401,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
   T* dz = static_cast<T*>(P.dz);
   const bool two = P.g.order != 1;
   const int R = P.L - 1;                                                   // difference rows per key
-  const int64_t tile0 = (int64_t)blockIdx.x * (kWarps * TPW * P.groups);
+  const int64_t tile0 = (int64_t)blockIdx.x * (W * TPW * P.groups);
   const int j0 = blockIdx.y * P.kch, kc = min(P.kch, P.h - j0);
 
   if constexpr (STAGED) {
@@ -404,7 +420,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
   // rows of z, g_delta and g_act of the next group are requested while this one is worked on
   float zn[kPre], an[kPre], gn[CV][V];
   auto load_group = [&](int m) {
-    const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+    const int64_t n0 = tile0 + (int64_t)(m * W + warp) * TPW;
     const bool on = m < P.groups && lane < kc;
 #pragma unroll
     for (int t = 0; t < kPre; ++t) {
@@ -421,7 +437,7 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
   };
   load_group(0);
   for (int m = 0; m < P.groups; ++m) {
-    const int64_t n0 = tile0 + (int64_t)(m * kWarps + warp) * TPW;
+    const int64_t n0 = tile0 + (int64_t)(m * W + warp) * TPW;
     if (n0 >= P.N) break;
     float zz[TPW], ga[kPre];
     float gd[CV][V];
@@ -449,12 +465,12 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
     }
     __syncwarp();
 #pragma unroll 1
-    for (int q0 = 0; q0 < kc; q0 += LPT) {
-      float v[LPT];
+    for (int q0 = 0; q0 < kc; q0 += Q) {
+      float v[Q];
 #pragma unroll
-      for (int q = 0; q < LPT; ++q) {
+      for (int q = 0; q < Q; ++q) {
         const float2 w = my[sub * kWarp + q0 + q];                          // keys past kc: row 0, result unused
-        float s = 0.0f;
+        float s = 0.0f, s1 = 0.0f;                                          // g times either row
 #pragma unroll
         for (int c = 0; c < CV; ++c) {
           float d[V], e[V];
@@ -476,18 +492,18 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
               e[i] = two && col < P.r ? ld_f32<T>(row + 2 * P.r + col) - c1 : 0.0f;
             }
           }
-          if (two) {
-#pragma unroll
-            for (int i = 0; i < V; ++i) d[i] = fmaf(w.x, e[i] - d[i], d[i]);
-          }
 #pragma unroll
           for (int i = 0; i < V; ++i) s = fmaf(gd[c][i], d[i], s);
-        }
-        v[q] = s;
-      }
-      // afterwards v[0] of lane sl is the sum over the token's lanes of v[sl]
+          if (two) {
 #pragma unroll
-      for (int s = LPT / 2; s >= 1; s >>= 1) {
+            for (int i = 0; i < V; ++i) s1 = fmaf(gd[c][i], e[i], s1);
+          }
+        }
+        v[q] = two ? fmaf(w.x, s1 - s, s) : s;
+      }
+      // afterwards v[0] of lane sl is the sum over the token's lanes of v[sl % Q]
+#pragma unroll
+      for (int s = Q / 2; s >= 1; s >>= 1) {
 #pragma unroll
         for (int i = 0; i < s; ++i) {
           const bool up = (sl & s) != 0;
@@ -496,7 +512,9 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dz_kernel(const DzArgs
           v[i] = keep + __shfl_xor_sync(kFull, send, s);
         }
       }
-      res[sub * kRes + q0 + sl] = v[0];
+#pragma unroll
+      for (int s = Q; s < LPT; s <<= 1) v[0] += __shfl_xor_sync(kFull, v[0], s);
+      if (sl < Q) res[sub * kRes + q0 + sl] = v[0];
     }
     __syncwarp();
 #pragma unroll
@@ -539,18 +557,37 @@ struct DcArgs {
 };
 
 constexpr int kMaxTile = 256;
+constexpr int kDcMaxWarps = 24;
+constexpr int kDcAhead = 4;                // pieces of four gradients that a thread requests before a tile is worked on
+
+// Four neighbouring elements, aligned.
+template <typename T> struct Quad;
+template <> struct Quad<float> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+  __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Quad<__nv_bfloat16> {
+  uint2 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = __ldg(reinterpret_cast<const uint2*>(p)); }
+  __device__ __forceinline__ float4 get() const {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+  }
+};
 
 // GACC = true: a key's accumulator does not fit shared memory and lives in the partial buffer.
 template <typename T, int LPT, int CV, bool GACC>
-__global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs P) {
+__global__ void __launch_bounds__(kDcMaxWarps * kWarp, 1) simt_dc_kernel(const DcArgs P) {
   constexpr int V = 4;
   constexpr int S = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
+  constexpr int kPer = kMaxTile / kWarp;                                   // tokens of a tile per lane, at most
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int W = blockDim.x / kWarp, TT = P.TT, nb = P.L - P.g.order, r = P.r;
-  const int zp = W + 1;
+  const int zp = W | 1;                                                    // odd: a column of z has no bank conflicts
   float* gs = reinterpret_cast<float*>(smem_raw);                          // [TT][pitch]
-  float4* ent_all = reinterpret_cast<float4*>(gs + (size_t)TT * pitch);    // [W][TT]  (w0, w1, w2, token)
+  float4* ent_all = reinterpret_cast<float4*>(gs + (size_t)TT * pitch);    // [W][TT]  (w0, w1, w2, offset of the token's row)
   float* acc_all = reinterpret_cast<float*>(ent_all + (size_t)W * TT);     // [W][L][pitch] unless GACC
   float* zt = acc_all + (GACC ? 0 : (size_t)W * P.L * pitch);              // [TT][zp]
   int* off_all = reinterpret_cast<int*>(zt + (size_t)TT * zp);             // [W][nb + 1]
@@ -574,31 +611,64 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
   } else {
     zero16(acc_all, (size_t)W * P.L * pitch * sizeof(float));
   }
-  int per = 32;
-  while (per > r) per >>= 1;
-  const int c0 = threadIdx.x & (per - 1);
   if (r != pitch) zero16(gs, (size_t)TT * pitch * sizeof(float));
+
+  // A tile's gradients and pre-activations are requested before the tile in front of it is worked on: the first
+  // kDcAhead pieces of four gradients of every thread, and one column of z per thread.
+  const bool quads = r % 4 == 0 && P.gds % 4 == 0 && (reinterpret_cast<uintptr_t>(g_delta) & (4 * sizeof(T) - 1)) == 0;
+  const int rq = r / 4, zk = threadIdx.x % W, zt0 = threadIdx.x / W;       // a thread's key and first token of z: every 32nd
+  Quad<T> gn[kDcAhead];
+  float zn[kPer];
+  auto request = [&](int64_t t0) {
+    const int tt = (int)min((int64_t)TT, nend - t0);
+    if (quads) {
+#pragma unroll
+      for (int i = 0; i < kDcAhead; ++i) {
+        const int e = threadIdx.x + i * blockDim.x, t = e / rq;
+        if (t < tt) gn[i].load(g_delta + (t0 + t) * P.gds + (e - t * rq) * 4);
+      }
+    }
+    const T* src = z + (t0 + zt0) * P.zs + j0 + zk;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      zn[i] = zt0 + i * kWarp < tt && zk < kd ? ld_f32<T>(src + (int64_t)(i * kWarp) * P.zs) : 0.0f;
+  };
+  request(nbeg);
 
   for (int64_t t0 = nbeg; t0 < nend; t0 += TT) {
     const int tt = (int)min((int64_t)TT, nend - t0);
     __syncthreads();
-#pragma unroll 8
-    for (int t = threadIdx.x / per; t < tt; t += blockDim.x / per)
-      for (int c = c0; c < r; c += per) gs[(size_t)t * pitch + c] = ld_f32<T>(g_delta + (t0 + t) * P.gds + c);
-#pragma unroll 8
-    for (int i = threadIdx.x; i < tt * W; i += blockDim.x) {
-      const int t = i / W, k = i % W;
-      zt[t * zp + k] = k < kd ? ld_f32<T>(z + (t0 + t) * P.zs + j0 + k) : 0.0f;
+    if (quads) {
+#pragma unroll
+      for (int i = 0; i < kDcAhead; ++i) {
+        const int e = threadIdx.x + i * blockDim.x, t = e / rq;
+        if (t < tt) *reinterpret_cast<float4*>(gs + (size_t)t * pitch + (e - t * rq) * 4) = gn[i].get();
+      }
+      for (int e = threadIdx.x + kDcAhead * blockDim.x; e < tt * rq; e += blockDim.x) {
+        const int t = e / rq;
+        Quad<T> q;
+        q.load(g_delta + (t0 + t) * P.gds + (e - t * rq) * 4);
+        *reinterpret_cast<float4*>(gs + (size_t)t * pitch + (e - t * rq) * 4) = q.get();
+      }
+    } else {
+      for (int e = threadIdx.x; e < tt * r; e += blockDim.x) {
+        const int t = e / r, c = e - t * r;
+        gs[(size_t)t * pitch + c] = ld_f32<T>(g_delta + (t0 + t) * P.gds + c);
+      }
     }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      if (zt0 + i * kWarp < tt) zt[(zt0 + i * kWarp) * zp + zk] = zn[i];
     for (int i = lane; i <= nb; i += kWarp) off[i] = 0;
     __syncthreads();
+    if (t0 + TT < nend) request(t0 + TT);
     if (!mine) continue;
 
     // ---- rank of every token within its interval, counts per interval
-    int bins[kMaxTile / kWarp], pos[kMaxTile / kWarp];
-    float tau[kMaxTile / kWarp];
+    int bins[kPer], pos[kPer];
+    float tau[kPer];
 #pragma unroll
-    for (int i = 0; i < kMaxTile / kWarp; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       bins[i] = -1;
       if (i * kWarp < tt) {
         const int t = i * kWarp + lane;
@@ -632,18 +702,19 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
     }
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < kMaxTile / kWarp; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       if (bins[i] >= 0) {
         Knot k;
         k.tau = tau[i];
         k.in_range = true;
         float B0, B1, B2;
         basis_weights(k, B0, B1, B2, P.g.order);
-        ent[off[bins[i]] + pos[i]] = make_float4(B0, B1, B2, __int_as_float(i * kWarp + lane));
+        ent[off[bins[i]] + pos[i]] = make_float4(B0, B1, B2, __int_as_float((i * kWarp + lane) * pitch));
       }
     }
     __syncwarp();
-    // ---- one interval at a time; the window of rows b, b + 1, b + 2 slides along, so each interval finishes one row
+    // ---- one interval at a time; the window of rows b, b + 1, b + 2 slides along, so each interval finishes one row.  The
+    // three sums take the three places in turn (the loop is unrolled by three) instead of moving.
     float a[3][CV][V];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -651,36 +722,47 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
       for (int c = 0; c < CV; ++c)
 #pragma unroll
         for (int i = 0; i < V; ++i) a[k][c][i] = 0.0f;
-    auto finish_row = [&](int row) {                  // a[0] added to the key's accumulator, the window moved on
+    auto finish_row = [&](float (&w)[CV][V], int row) {  // a finished sum goes to the key's accumulator, its place is free
 #pragma unroll
       for (int c = 0; c < CV; ++c) {
+        // the lane groups' sums are added while the channels are shared out among them: V -> V / 2 -> 1 per lane
+        int col = sl * V + c * (LPT * V), n = V;
+        bool write = true;
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
+        for (int s = S / 2; s >= 1; s >>= 1) {
+          const bool up = (sub & s) != 0;
+          if (n > 1) {
+            n /= 2;
 #pragma unroll
-          for (int s = LPT; s < kWarp; s <<= 1) a[0][c][i] += __shfl_xor_sync(kFull, a[0][c][i], s);
+            for (int i = 0; i < V / 2; ++i) {
+              if (i >= n) continue;
+              const float send = up ? w[c][i] : w[c][i + n], keep = up ? w[c][i + n] : w[c][i];
+              w[c][i] = keep + __shfl_xor_sync(kFull, send, s * LPT);
+            }
+            if (up) col += n;
+          } else {
+            w[c][0] += __shfl_xor_sync(kFull, w[c][0], s * LPT);
+            write = write && !up;
+          }
         }
-        if (sub == 0) {
-          float* dst = acc + (size_t)row * ap + sl * V + c * (LPT * V);
-          if constexpr (GACC) {
+        float* dst = acc + (size_t)row * ap + col;
+        if (write) {
+          if constexpr (S == 1 && !GACC) {
+            float4 d = *reinterpret_cast<float4*>(dst);
+            d.x += w[c][0]; d.y += w[c][1]; d.z += w[c][2]; d.w += w[c][3];
+            *reinterpret_cast<float4*>(dst) = d;
+          } else {
 #pragma unroll
             for (int i = 0; i < V; ++i)
-              if (sl * V + c * (LPT * V) + i < r) dst[i] += a[0][c][i];
-          } else {
-            float4 d = *reinterpret_cast<float4*>(dst);
-            d.x += a[0][c][0]; d.y += a[0][c][1]; d.z += a[0][c][2]; d.w += a[0][c][3];
-            *reinterpret_cast<float4*>(dst) = d;
+              if (i < n && (!GACC || col + i < r)) dst[i] += w[c][i];
           }
         }
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          a[0][c][i] = a[1][c][i];
-          a[1][c][i] = three ? a[2][c][i] : 0.0f;     // the linear spline's third weight is zero, but zero times an
-          a[2][c][i] = 0.0f;                          // infinity is not
-        }
+        for (int i = 0; i < V; ++i) w[c][i] = 0.0f;
       }
     };
     int end = off[0], dirty = 0;                      // rows of the window that hold something
-    for (int b = 0; b < nb; ++b) {
+    auto interval = [&](int b, float (&w0)[CV][V], float (&w1)[CV][V], float (&w2)[CV][V]) {
       const int beg = end;
       end = off[b + 1];
       if (beg != end) {
@@ -688,24 +770,44 @@ __global__ void __launch_bounds__(kWarps * kWarp, 2) simt_dc_kernel(const DcArgs
 #pragma unroll 2
         for (int p = beg + sub; p < end; p += S) {
           const float4 e = ent[p];
-          const float* gr = gs + (size_t)__float_as_int(e.w) * pitch + sl * V;
+          const float* gr = gs + __float_as_int(e.w) + sl * V;
 #pragma unroll
           for (int c = 0; c < CV; ++c) {
             const float4 g4 = *reinterpret_cast<const float4*>(gr + c * (LPT * V));
             const float gv[V] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
             for (int i = 0; i < V; ++i) {
-              a[0][c][i] = fmaf(e.x, gv[i], a[0][c][i]);
-              a[1][c][i] = fmaf(e.y, gv[i], a[1][c][i]);
-              a[2][c][i] = fmaf(e.z, gv[i], a[2][c][i]);
+              w0[c][i] = fmaf(e.x, gv[i], w0[c][i]);
+              w1[c][i] = fmaf(e.y, gv[i], w1[c][i]);
+            }
+            if (three) {                               // (a third weight of zero times an infinity is not zero)
+#pragma unroll
+              for (int i = 0; i < V; ++i) w2[c][i] = fmaf(e.z, gv[i], w2[c][i]);
             }
           }
         }
       }
-      if (dirty > 0) { finish_row(b); --dirty; }
+      if (dirty > 0) { finish_row(w0, b); --dirty; }
+    };
+    int b = 0;
+    for (; b + 3 <= nb; b += 3) {
+      interval(b, a[0], a[1], a[2]);
+      interval(b + 1, a[1], a[2], a[0]);
+      interval(b + 2, a[2], a[0], a[1]);
     }
-    if (dirty > 0) finish_row(nb);
-    if (three && dirty > 1) finish_row(nb + 1);
+    if (nb - b == 1) {
+      interval(b, a[0], a[1], a[2]);
+      if (dirty > 0) finish_row(a[1], nb);
+      if (three && dirty > 1) finish_row(a[2], nb + 1);
+    } else if (nb - b == 2) {
+      interval(b, a[0], a[1], a[2]);
+      interval(b + 1, a[1], a[2], a[0]);
+      if (dirty > 0) finish_row(a[2], nb);
+      if (three && dirty > 1) finish_row(a[0], nb + 1);
+    } else {
+      if (dirty > 0) finish_row(a[0], nb);
+      if (three && dirty > 1) finish_row(a[1], nb + 1);
+    }
     __syncwarp();
   }
   __syncthreads();
@@ -755,6 +857,7 @@ __global__ void simt_knot_index_kernel(const T* __restrict__ z, int64_t zs, int6
 constexpr int kPlanSMs = 148;                            // B200; only used to balance launch shapes
 constexpr size_t kSmemHalf = 110 * 1024;                 // two CTAs per SM
 constexpr size_t kSmemFull = 216 * 1024;
+constexpr size_t kSmemMost = 226 * 1024;
 constexpr size_t kFwdScratchCap = SKV_NOALLOC_SCRATCH_BYTES;   // the key splits' partials stay below this
 
 // Lanes per token (a power of two from 2 to 32) and 16-byte pieces per lane for rows of r elements.
@@ -765,7 +868,7 @@ void lanes_for(int r, int v, int* lpt, int* cv) {
   *cv = l * v < r ? 2 : 1;
 }
 
-struct FwdPlan { bool small; int lpt, cv, kch, groups, splits, keys_per_split; int64_t tiles; size_t smem; };
+struct FwdPlan { bool small; int lpt, cv, warps, kch, groups, splits, keys_per_split; int64_t tiles; size_t smem; };
 
 FwdPlan plan_forward(const skv_problem& p) {
   FwdPlan f;
@@ -773,10 +876,13 @@ FwdPlan plan_forward(const skv_problem& p) {
   lanes_for(p.r, v, &f.lpt, &f.cv);
   const int tpw = kWarp / f.lpt, pitch = f.lpt * v * f.cv;
   const int64_t N = p.N > 0 ? p.N : 1;
-  const size_t wb = (size_t)kWarps * tpw * kWarp * 16, per_key = (size_t)p.L * pitch * size;
-  size_t kch = kSmemHalf > wb ? (kSmemHalf - wb) / per_key : 0;
-  if (kch < 8) kch = (kSmemFull - wb) / per_key;
-  f.kch = (int)(kch > 32 ? 32 : kch);
+  const int warps = staged_warps(f.lpt, f.cv, size);
+  const size_t wb = (size_t)warps * tpw * kWarp * 16, per_key = (size_t)p.L * pitch * size;
+  size_t most_keys = kSmemHalf > wb ? (kSmemHalf - wb) / per_key : 0;
+  if (most_keys < 8) most_keys = (kSmemFull - wb) / per_key;
+  if (most_keys > 32) most_keys = 32;
+  f.kch = (int)most_keys;
+  f.warps = warps;
   f.small = f.kch < 1 || N <= small_forward_tokens(p);
   const size_t part_bytes = (size_t)N * p.r * sizeof(float);
   if (f.small) {
@@ -797,59 +903,66 @@ FwdPlan plan_forward(const skv_problem& p) {
     f.smem = 0;
     return f;
   }
-  f.smem = wb + (size_t)f.kch * per_key;
-  const int slots = kPlanSMs * (f.smem <= kSmemHalf + 1024 ? 2 : 1);
-  const int slabs = (int)cdiv64(p.h, f.kch);
-  // clocks: a slab's copy, the work of one token group on it, and the partials' round trip
-  const double copy = (double)f.kch * per_key / 32.0;
-  const double work = (double)kWarps * tpw * f.kch * (pitch * size / 64.0 + 0.5);
+  const int slots = kPlanSMs * (wb + most_keys * per_key <= kSmemHalf + 1024 ? 2 : 1);
   double best = 0.0;
   for (int groups = kGroups; groups >= 1; groups >>= 1) {
-    const int64_t tiles = cdiv64(N, (int64_t)kWarps * tpw * groups);
+    const int64_t tiles = cdiv64(N, (int64_t)warps * tpw * groups);
     int last = 0;
-    for (int s = 1; s <= slabs && s <= 64; ++s) {
-      const int per = (int)cdiv64(slabs, s), splits = (int)cdiv64(slabs, per);
+    for (int s = 1; s <= 64; ++s) {
+      // the keys of a split in equal slabs, and a whole number of them
+      const int64_t share = cdiv64(p.h, s);
+      const int slabs = (int)cdiv64(share, (int64_t)most_keys), kch = (int)cdiv64(share, slabs);
+      const int per = slabs * kch, splits = (int)cdiv64(p.h, per);
       if (splits > 1 && splits * part_bytes > kFwdScratchCap) break;
       if (splits == last) continue;
       last = splits;
-      const double t = (double)cdiv64(tiles * splits, slots) * per * (copy + groups * work) +
+      // clocks: a slab's copy, the work of one token group on it (rows of every pair, weights of every token), and the
+      // partials' round trip
+      const double copy = 1000.0 + (double)kch * per_key / 32.0;
+      const double work = (double)warps * tpw * (kch * (pitch * size / 64.0 + 0.5) + 12.0);
+      const double t = (double)cdiv64(tiles * splits, slots) * slabs * (copy + groups * work) +
                        (splits > 1 ? 4000.0 + (double)splits * part_bytes / 1500.0 : 0.0);
       if (best == 0.0 || t < best) {
         best = t;
         f.groups = groups;
         f.tiles = tiles;
         f.splits = splits;
-        f.keys_per_split = per * f.kch;
+        f.kch = kch;
+        f.keys_per_split = per;
       }
     }
   }
+  f.smem = wb + (size_t)f.kch * per_key;
   return f;
 }
 
-struct DzPlan { bool staged; int lpt, cv, kch, groups; int64_t tiles; size_t smem; };
+struct DzPlan { bool staged; int lpt, cv, warps, kch, groups; int64_t tiles; size_t smem; };
 DzPlan plan_dz(const skv_problem& p) {
   DzPlan d;
   lanes_for(p.r, 4, &d.lpt, &d.cv);
   const int tpw = kWarp / d.lpt, pitch = d.lpt * 4 * d.cv;
-  const size_t bufs = (size_t)kWarps * tpw * (kWarp * 8 + (kWarp + 4) * 4), per_key = (size_t)(p.L - 1) * pitch * 4;
-  size_t kch = (kSmemHalf - bufs) / per_key;
-  if (kch < 8) kch = (kSmemFull - bufs) / per_key;
-  d.staged = kch >= 1;
-  if (kch > 32 || !d.staged) kch = 32;
-  while (kch > 8 && kch % 8) --kch;
-  d.kch = (int)kch;
-  d.smem = bufs + (d.staged ? kch * per_key : 0);
-  const int slots = kPlanSMs * (d.smem <= kSmemHalf + 1024 ? 2 : 1);
-  const int64_t N = p.N > 0 ? p.N : 1, slabs = cdiv64(p.h, d.kch), unit = (int64_t)kWarps * tpw;
-  const double copy = d.staged ? (double)kch * per_key / 24.0 : 0.0;
-  const double work = (double)unit * kch * (pitch / 16.0 + 0.5);
+  d.warps = staged_warps(d.lpt, d.cv, 4);
+  const size_t bufs = (size_t)d.warps * tpw * (kWarp * 8 + (kWarp + 4) * 4), per_key = (size_t)(p.L - 1) * pitch * 4;
+  size_t most_keys = (kSmemHalf - bufs) / per_key;
+  if (most_keys < 8) most_keys = (kSmemFull - bufs) / per_key;
+  d.staged = most_keys >= 1;
+  if (most_keys > 32 || !d.staged) most_keys = 32;
+  const int slots = kPlanSMs * (bufs + (d.staged ? most_keys * per_key : 0) <= kSmemHalf + 1024 ? 2 : 1);
+  const int64_t N = p.N > 0 ? p.N : 1, unit = (int64_t)d.warps * tpw;
   double best = 0.0;
-  for (int64_t groups = 1; groups <= 64; groups <<= 1) {
-    const int64_t tiles = cdiv64(N, unit * groups);
-    const double t = (double)cdiv64(tiles * slabs, slots) * (copy + groups * work);
-    if (best == 0.0 || t < best) { best = t; d.groups = (int)groups; d.tiles = tiles; }
-    if (tiles == 1) break;
+  for (int64_t kch = (int64_t)most_keys; kch >= 1; --kch) {
+    if (kch > 8 && kch % 8) continue;                    // whole transposes, and aligned pieces of z and dz
+    const int64_t slabs = cdiv64(p.h, kch);
+    const double copy = 1000.0 + (d.staged ? (double)kch * per_key / 24.0 : 0.0);
+    const double work = (double)unit * (cdiv64(kch, 8) * 8 * (pitch / 16.0 + 0.5) + 16.0);
+    for (int64_t groups = 1; groups <= 64; groups <<= 1) {
+      const int64_t tiles = cdiv64(N, unit * groups);
+      const double t = (double)cdiv64(tiles * slabs, slots) * (copy + groups * work);
+      if (best == 0.0 || t < best) { best = t; d.groups = (int)groups; d.tiles = tiles; d.kch = (int)kch; }
+      if (tiles == 1) break;
+    }
   }
+  d.smem = bufs + (d.staged ? d.kch * per_key : 0);
   return d;
 }
 
@@ -857,35 +970,42 @@ struct DcPlan { bool gacc; int lpt, cv, W, TT, splits; int64_t tokens_per_split;
 DcPlan plan_dc(const skv_problem& p) {
   DcPlan d;
   lanes_for(p.r, 4, &d.lpt, &d.cv);
-  const int pitch = d.lpt * 4 * d.cv, nb = p.L - 1;
+  const int pitch = d.lpt * 4 * d.cv, nb = p.L - 1, S = kWarp / d.lpt;
   const size_t per_acc = (size_t)p.L * pitch * 4;
   auto bytes = [&](int W, int TT, bool gacc) {
-    return (size_t)TT * pitch * 4 + (size_t)W * TT * 16 + (gacc ? 0 : W * per_acc) + (size_t)TT * (W + 1) * 4 +
+    return (size_t)TT * pitch * 4 + (size_t)W * TT * 16 + (gacc ? 0 : W * per_acc) + (size_t)TT * (W | 1) * 4 +
            (size_t)W * (nb + 2) * 4;
   };
-  // eight keys and 256 tokens with two CTAs per SM where that fits, then smaller tiles, then fewer keys
-  d.gacc = false;
-  d.W = kWarps;
-  d.TT = kMaxTile;
-  while (d.TT > 64 && bytes(d.W, d.TT, false) > kSmemHalf) d.TT >>= 1;
-  if (bytes(d.W, d.TT, false) > kSmemHalf) d.TT = 128;
-  while (d.W > 1 && bytes(d.W, d.TT, false) > kSmemFull) d.W >>= 1;
-  if (bytes(d.W, d.TT, false) > kSmemFull) { d.gacc = true; d.W = kWarps; d.TT = 64; }
-  d.smem = bytes(d.W, d.TT, d.gacc);
-  const int slots = kPlanSMs * (d.smem <= kSmemHalf + 1024 ? 2 : 1);
-  const int64_t N = p.N > 0 ? p.N : 1, groups = cdiv64(p.h, d.W), tiles = cdiv64(N, d.TT);
+  const int64_t N = p.N > 0 ? p.N : 1;
   const double elems = (double)p.h * p.L * p.r;
   double best = 0.0;
-  int64_t last = 0;
-  for (int64_t s = 1; s <= 16; ++s) {
-    const int64_t per = cdiv64(tiles, s), splits = cdiv64(tiles, per);
-    if (splits == last) continue;
-    last = splits;
-    // clocks: a tile per warp about 7 instructions per pair and 40 per interval; partials' round trip
-    const double t = (double)cdiv64(groups * splits, slots) * per * (d.TT * 14.0 * d.cv + 4000.0) +
-                     (splits > 1 ? 4000.0 + splits * elems * 8 / 1500.0 : 0.0);
-    if (best == 0.0 || t < best) { best = t; d.splits = (int)splits; d.tokens_per_split = per * d.TT; }
-  }
+  auto consider = [&](int W, int TT, bool gacc) {
+    const int64_t groups = cdiv64(p.h, W), tiles = cdiv64(N, TT);
+    // warp instructions of a tile and key: the sort, S pairs at a time, a finished row per interval; issued by a chip that
+    // needs about twenty warps per SM to be busy
+    const double tile = (double)W * (TT * 1.5 + TT * (6.0 + 14.0 * d.cv) / S + p.L * (14.0 + 12.0 * d.cv)) / (W < 20 ? W / 20.0 : 1.0);
+    int64_t last = 0;
+    for (int64_t s = 1; s <= 16; ++s) {
+      const int64_t per = cdiv64(tiles, s), splits = cdiv64(tiles, per);
+      if (splits == last) continue;
+      last = splits;
+      // clocks, with a CTA's prologue and epilogue, and the partials' round trip
+      const double t = (double)cdiv64(groups * splits, kPlanSMs) * (per * (tile / 3.0 + 500.0) + 3000.0) +
+                       (splits > 1 ? 3000.0 + splits * elems * 8 / 1500.0 : 0.0);
+      if (best != 0.0 && t >= best) continue;
+      best = t;
+      d.gacc = gacc;
+      d.W = W;
+      d.TT = TT;
+      d.smem = bytes(W, TT, gacc);
+      d.splits = (int)splits;
+      d.tokens_per_split = per * TT;
+    }
+  };
+  for (int TT = kMaxTile; TT >= 64; TT >>= 1)
+    for (int W = kDcMaxWarps; W >= 1; --W)
+      if (bytes(W, TT, false) <= kSmemMost) consider(W, TT, false);
+  if (best == 0.0) consider(kWarps, 64, true);
   return d;
 }
 
@@ -931,7 +1051,7 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
     if (f.small && vec) simt_forward_small_kernel<T, TD, LPT_, CV_, true><<<grid, kWarps * kWarp, 0, c.stream>>>(a);  \
     else if (f.small) simt_forward_small_kernel<T, TD, LPT_, CV_, false><<<grid, kWarps * kWarp, 0, c.stream>>>(a);   \
     else if ((e = set_smem(simt_forward_kernel<T, TD, LPT_, CV_>, f.smem)) == SKV_OK)                           \
-      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, kWarps * kWarp, f.smem, c.stream>>>(a);                     \
+      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, f.warps * kWarp, f.smem, c.stream>>>(a);                     \
   }
   SKV_LANES(f.lpt, f.cv, SKV_CALL)
 #undef SKV_CALL
@@ -963,9 +1083,9 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
   {                                                                                                      \
     if (!d.staged) {                                                                                     \
       if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, false>, d.smem)) == SKV_OK)                         \
-        simt_dz_kernel<T, LPT_, CV_, false><<<grid, kWarps * kWarp, d.smem, c.stream>>>(a);              \
+        simt_dz_kernel<T, LPT_, CV_, false><<<grid, d.warps * kWarp, d.smem, c.stream>>>(a);              \
     } else if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, true>, d.smem)) == SKV_OK)                     \
-      simt_dz_kernel<T, LPT_, CV_, true><<<grid, kWarps * kWarp, d.smem, c.stream>>>(a);                 \
+      simt_dz_kernel<T, LPT_, CV_, true><<<grid, d.warps * kWarp, d.smem, c.stream>>>(a);                 \
   }
     SKV_LANES(d.lpt, d.cv, SKV_CALL)
 #undef SKV_CALL
