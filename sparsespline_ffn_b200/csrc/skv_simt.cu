@@ -15,7 +15,6 @@ constexpr int kWarp = 32;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 8;             // warps per CTA of the kernels below, but for staged_warps
 constexpr int kGroups = 4;            // token groups a warp of the staged forward keeps accumulators for
-constexpr int kSmallEntries = 256;    // pair weights per warp of the small forward (tokens x keys of a pass)
 
 // Warps per CTA of the kernels over a staged table, two CTAs per SM.  What a lane waits for is a chain of two shared-memory reads per
 // key (weights, then rows), so warps are what hides it: sixteen where a lane's registers allow it (64 of them: float32 rows
@@ -84,9 +83,9 @@ struct FwdArgs {
   GridParams g;
   float lambda;
   int act;
-  int kch;                   // staged: keys per slab; small: keys per warp
+  int kch;                   // staged: keys per slab; small: keys of a warp at a time, at most 32
   int keys_per_split;
-  int groups;                // staged: token groups per warp (1..kGroups); small: tokens per warp
+  int groups;                // staged: token groups per warp (1..kGroups); small: CTAs per token
 };
 
 // Weights of one pair for the gather loop: B_0..B_2 and the element offset of row `bin`.
@@ -216,13 +215,15 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, sizeof(T)) * kWarp, 2) s
 }
 
 // ---------------------------------------------------------------------------------------------
-// Forward that reads the table rows where they are: grid = (token groups, key splits).  For few tokens
-// most of the table is never touched, so nothing is copied or packed first; each warp takes `kch` keys
-// of up to 32 / LPT tokens, spare lane groups share the keys of the tokens there are, and the warps'
-// sums are added in shared memory.  Also the path of a table too large per key for shared memory.
+// Forward that reads the table rows where they are: a cluster of CTAs takes a token, each CTA a share of its keys, a warp up
+// to 32 of them at a time.  For few tokens most of the table is never touched, so nothing is copied or packed first.
+// 32 / LPT keys of a warp are worked on at once; the lane groups', the warps' and the CTAs' sums are added in a fixed order,
+// the last of them through the shared memory of the cluster's first CTA.  Also the path of a table too large per key
+// for shared memory.
 //
-// Bound: the latency of one dependent chain (z -> knot -> row), so keys are spread over as many
-// warps as the chip holds and four rows' loads are in flight per lane.
+// Bound: the latency of one dependent chain (z -> knot -> row -> sums), so the keys of a token are spread over as many
+// warps as the chip holds and four rows' loads are in flight per lane; then, from about 64 tokens at h = 5120 on, by what
+// L2 delivers (three rows per pair).
 // ---------------------------------------------------------------------------------------------
 template <typename T, int CV, bool VECLD>
 __device__ __forceinline__ void load_row(const T* __restrict__ row, int col, int r, float (&f)[Vec<T>::n]) {
@@ -234,92 +235,121 @@ __device__ __forceinline__ void load_row(const T* __restrict__ row, int col, int
   }
 }
 
+constexpr int kSmallWarps = 32;       // most warps of a CTA
+constexpr int kSmallCluster = 8;      // most CTAs of a token
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// One float32 into the shared memory of the cluster's first CTA, at the place `p` has in this one's.
+__device__ __forceinline__ void store_first_cta(float* p, float v) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), b;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(b) : "r"(a));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(b), "f"(v) : "memory");
+}
+
 template <typename T, typename TD, int LPT, int CV, bool VECLD>
-__global__ void __launch_bounds__(kWarps * kWarp) simt_forward_small_kernel(const FwdArgs P) {
+__global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_kernel(const FwdArgs P) {
   constexpr int V = Vec<T>::n;
   constexpr int TPW = kWarp / LPT;
   constexpr int pitch = LPT * V * CV;
-  __shared__ float4 wbuf[kWarps][kSmallEntries];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int W = blockDim.x / kWarp, cs = P.groups;
+  float* parts = reinterpret_cast<float*>(smem_raw);                       // [kSmallCluster][pitch], of the first CTA
+  float* red = parts + kSmallCluster * pitch;                              // [warp][pitch], in the place of
+  float4* wbuf = reinterpret_cast<float4*>(red);                           // [warp][32]
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  const int sub = lane / LPT, sl = lane % LPT;
-  const int TG = P.groups;                            // tokens of a warp: a power of two up to TPW
-  const int tok = sub & (TG - 1), ks = sub / TG, kstep = TPW / TG;
+  const int sub = lane / LPT, sl = lane % LPT, rank = blockIdx.x % cs;
   const T* z = static_cast<const T*>(P.z);
   const T* C = static_cast<const T*>(P.C);
   T* act_out = static_cast<T*>(P.act_out);
-  const int64_t n0 = (int64_t)blockIdx.x * TG;
-  const int kbeg = blockIdx.y * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
+  const int kbeg = rank * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
   const bool three = P.g.order != 1;
-  float4* my = wbuf[warp];
+  float4* my = wbuf + warp * kWarp;
+  if (cs > 1) cluster_arrive();                       // the first CTA has started before anything is sent to it
 
-  float acc[CV][V];
+  for (int64_t n = blockIdx.x / cs; n < P.N; n += gridDim.x / cs) {
+    float acc[CV][V];
 #pragma unroll
-  for (int c = 0; c < CV; ++c)
+    for (int c = 0; c < CV; ++c)
 #pragma unroll
-    for (int i = 0; i < V; ++i) acc[c][i] = 0.0f;
-
-  const int kw = P.kch;                               // keys of a warp per pass: 4, 8, 16 or 32
-  for (int j0 = kbeg + warp * kw; j0 < kend; j0 += kWarps * kw) {
-    const int kc = min(kw, kend - j0);
-    __syncwarp();
-    for (int e = lane; e < TG * kw; e += kWarp) {
-      const int t = e / kw, k = e % kw;
-      float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (k < kc && n0 + t < P.N) {
-        const float zz = ld_f32<T>(z + (n0 + t) * P.zs + j0 + k);
-        w = pair_weights(zz, P.g, k * P.L, P.r);
-        if (act_out) st_f32<T>(act_out + (n0 + t) * P.as + j0 + k, act_fwd(zz, P.act));
+      for (int i = 0; i < V; ++i) acc[c][i] = 0.0f;
+    const T* zr = z + n * P.zs;
+    float znext = 0.0f;
+    const int kw = P.kch;
+    int j0 = kbeg + warp * kw;
+    if (lane < kw && j0 + lane < kend) znext = ld_f32<T>(zr + j0 + lane);
+    for (; j0 < kend; j0 += W * kw) {
+      const int kc = min(kw, kend - j0);
+      const float zz = znext;
+      if (lane < kw && j0 + W * kw + lane < kend) znext = ld_f32<T>(zr + j0 + W * kw + lane);
+      __syncwarp();
+      if (lane < kc) {
+        my[lane] = pair_weights(zz, P.g, lane * P.L, P.r);
+        if (act_out) st_f32<T>(act_out + n * P.as + j0 + lane, act_fwd(zz, P.act));
       }
-      my[e] = w;
-    }
-    __syncwarp();
-    const T* base = C + (size_t)j0 * P.L * P.r;
+      __syncwarp();
+      const T* base = C + (size_t)j0 * P.L * P.r;
 #pragma unroll 4
-    for (int q = ks; q < kc; q += kstep) {
-      const float4 w = my[tok * kw + q];
-      const T* row = base + __float_as_int(w.w);
+      for (int q = sub; q < kc; q += TPW) {
+        const float4 w = my[q];
+        const T* row = base + __float_as_int(w.w);
 #pragma unroll
-      for (int c = 0; c < CV; ++c) {
-        const int col = c * (LPT * V) + sl * V;
-        if (col < P.r) {
-          float f0[V], f1[V], f2[V];
-          load_row<T, CV, VECLD>(row, col, P.r, f0);
-          load_row<T, CV, VECLD>(row + P.r, col, P.r, f1);
-          if (three) load_row<T, CV, VECLD>(row + 2 * P.r, col, P.r, f2);
+        for (int c = 0; c < CV; ++c) {
+          const int col = c * (LPT * V) + sl * V;
+          if (col < P.r) {
+            float f0[V], f1[V], f2[V];
+            load_row<T, CV, VECLD>(row, col, P.r, f0);
+            load_row<T, CV, VECLD>(row + P.r, col, P.r, f1);
+            if (three) load_row<T, CV, VECLD>(row + 2 * P.r, col, P.r, f2);
 #pragma unroll
-          for (int i = 0; i < V; ++i) {
-            acc[c][i] = fmaf(w.y, f1[i], fmaf(w.x, f0[i], acc[c][i]));
-            if (three) acc[c][i] = fmaf(w.z, f2[i], acc[c][i]);
+            for (int i = 0; i < V; ++i) {
+              acc[c][i] = fmaf(w.y, f1[i], fmaf(w.x, f0[i], acc[c][i]));
+              if (three) acc[c][i] = fmaf(w.z, f2[i], acc[c][i]);
+            }
           }
         }
       }
     }
+#pragma unroll
+    for (int s = LPT; s < kWarp; s <<= 1) {
+#pragma unroll
+      for (int c = 0; c < CV; ++c)
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[c][i] += __shfl_xor_sync(kFull, acc[c][i], s);
+    }
+    __syncthreads();
+    if (sub == 0) {
+#pragma unroll
+      for (int c = 0; c < CV; ++c)
+#pragma unroll
+        for (int i = 0; i < V; ++i) red[(size_t)warp * pitch + c * (LPT * V) + sl * V + i] = acc[c][i];
+    }
+    __syncthreads();
+    if (cs > 1) cluster_wait();                       // the first CTA is there and has read what it was sent last
+    for (int col = threadIdx.x; col < P.r; col += blockDim.x) {
+      float s = 0.0f;
+#pragma unroll 8
+      for (int w = 0; w < W; ++w) s += red[(size_t)w * pitch + col];
+      if (cs > 1) store_first_cta(parts + rank * pitch + col, s);
+      else st_f32<TD>(static_cast<TD*>(P.delta_out) + n * P.ds + col, P.lambda * s);
+    }
+    if (cs > 1) {
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      if (rank == 0) {
+        for (int col = threadIdx.x; col < P.r; col += blockDim.x) {
+          float s = 0.0f;
+          for (int k = 0; k < cs; ++k) s += parts[k * pitch + col];
+          st_f32<TD>(static_cast<TD*>(P.delta_out) + n * P.ds + col, P.lambda * s);
+        }
+      }
+      __syncwarp();
+      cluster_arrive();
+    }
+    __syncthreads();                                  // the sums have been read
   }
-  // lanes that shared a token, then the warps, in a fixed order
-  for (int s = LPT * TG; s < kWarp; s <<= 1) {
-#pragma unroll
-    for (int c = 0; c < CV; ++c)
-#pragma unroll
-      for (int i = 0; i < V; ++i) acc[c][i] += __shfl_xor_sync(kFull, acc[c][i], s);
-  }
-  float* red = reinterpret_cast<float*>(&wbuf[0][0]);  // [warp][TG][pitch]
-  __syncthreads();
-  if (ks == 0) {
-#pragma unroll
-    for (int c = 0; c < CV; ++c)
-#pragma unroll
-      for (int i = 0; i < V; ++i) red[((size_t)warp * TG + tok) * pitch + c * (LPT * V) + sl * V + i] = acc[c][i];
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < TG * P.r; e += blockDim.x) {
-    const int t = e / P.r, col = e % P.r;
-    if (n0 + t >= P.N) break;
-    float s = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) s += red[((size_t)w * TG + t) * pitch + col];
-    if (P.partial) P.partial[((size_t)blockIdx.y * P.N + n0 + t) * P.r + col] = s;
-    else st_f32<TD>(static_cast<TD*>(P.delta_out) + (n0 + t) * P.ds + col, P.lambda * s);
-  }
+  if (cs > 1) cluster_wait();
 }
 
 // Sum of the key splits' partial residuals in a fixed order, lambda, cast.  A CTA takes 32 elements;
@@ -885,22 +915,34 @@ FwdPlan plan_forward(const skv_problem& p) {
   f.warps = warps;
   f.small = f.kch < 1 || N <= small_forward_tokens(p);
   const size_t part_bytes = (size_t)N * p.r * sizeof(float);
+  f.splits = 1;
   if (f.small) {
-    int tg = 1;
-    while (tg < tpw && tg < N) tg <<= 1;
-    f.groups = tg;
-    f.tiles = cdiv64(N, tg);
-    // the largest pass that still gives two CTAs per SM, so that few partials are left to add
-    int kw = 4;
-    while (kw < tpw / tg) kw <<= 1;
-    while (kw < 32 && 2 * kw * tg <= kSmallEntries && f.tiles * cdiv64(p.h, kWarps * kw * 2) >= 2 * kPlanSMs) kw <<= 1;
-    f.kch = kw;
-    int64_t splits = cdiv64(p.h, kWarps * kw);
-    const int64_t most = (int64_t)(kFwdScratchCap / part_bytes);
-    if (splits > most) splits = most > 1 ? most : 1;
-    f.keys_per_split = (int)(cdiv64(cdiv64(p.h, splits), kWarps * kw) * kWarps * kw);
-    f.splits = (int)cdiv64(p.h, f.keys_per_split);
-    f.smem = 0;
+    // CTAs of a token, warps of a CTA and keys of a warp's pass.  Microseconds: a pass is a chain of latencies, one more for
+    // every 32 / LPT keys, or what an SM takes from L2 (60 KB; it holds 32 of these warps); launch, sums, and the
+    // cluster's exchange.  A cluster lives within a GPC, so large ones do not fill the chip.
+    double best = 0.0;
+    for (int cs = kSmallCluster; cs >= 1; cs >>= 1) {
+      const int64_t keys = cdiv64(p.h, cs), ctas = N * cs;
+      for (int most : {32, 24, 16, 10, 8}) {
+        const int64_t passes = cdiv64(keys, (int64_t)most * kWarp), w = cdiv64(keys, passes * kWarp) < 4 ? cdiv64(keys, passes * kWarp) : most;
+        const int64_t kw = cdiv64(cdiv64(keys, passes * w), tpw) * tpw < kWarp ? cdiv64(cdiv64(keys, passes * w), tpw) * tpw : kWarp;
+        const int64_t per_sm = kSmallWarps / w, sms = cs == 8 ? (per_sm > 1 ? 128 : 120) : cs == 4 ? (per_sm > 1 ? 138 : 132) : kPlanSMs;
+        const int64_t waves = cdiv64(ctas, sms * per_sm);
+        const int64_t resident = cdiv64(ctas, sms) < per_sm ? cdiv64(ctas, sms) : per_sm;
+        const double lat = 0.7 + 0.45 * cdiv64(kw, tpw), load = (double)(resident * w * kw) * 3 * p.r * size / 60000.0;
+        const double t = waves * (passes * (lat > load ? lat : load) + (cs > 1 ? 2.0 : 1.2));
+        if (best == 0.0 || t < best) {
+          best = t;
+          f.groups = cs;
+          f.warps = (int)w;
+          f.kch = (int)kw;
+          f.keys_per_split = (int)keys;
+        }
+      }
+    }
+    f.tiles = N < 1 << 20 ? N : 1 << 20;                 // clusters; each goes on to further tokens
+    const size_t row = (size_t)pitch * 4;
+    f.smem = kSmallCluster * row + f.warps * (row > kWarp * 16 ? row : kWarp * 16);
     return f;
   }
   const int slots = kPlanSMs * (wb + most_keys * per_key <= kSmemHalf + 1024 ? 2 : 1);
@@ -1020,6 +1062,23 @@ int set_smem(K kernel, size_t bytes) {
   return SKV_OK;
 }
 
+// The CTAs of a token as a cluster.
+template <typename K>
+int launch_small(K kernel, const FwdPlan& f, const FwdArgs& a, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(f.tiles * f.groups));
+  cfg.blockDim = dim3((unsigned)(f.warps * kWarp));
+  cfg.dynamicSmemBytes = f.smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)f.groups;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+}
+
 // One case per (lanes per token, pieces per lane) that rows of up to 256 elements need.
 #define SKV_LANES(LPT_, CV_, CALL)                                    \
   if (CV_ == 2) CALL(32, 2)                                           \
@@ -1048,10 +1107,10 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
   int e = SKV_OK;
 #define SKV_CALL(LPT_, CV_)                                                                                     \
   {                                                                                                             \
-    if (f.small && vec) simt_forward_small_kernel<T, TD, LPT_, CV_, true><<<grid, kWarps * kWarp, 0, c.stream>>>(a);  \
-    else if (f.small) simt_forward_small_kernel<T, TD, LPT_, CV_, false><<<grid, kWarps * kWarp, 0, c.stream>>>(a);   \
+    if (f.small && vec) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, true>, f, a, c.stream);    \
+    else if (f.small) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, false>, f, a, c.stream);     \
     else if ((e = set_smem(simt_forward_kernel<T, TD, LPT_, CV_>, f.smem)) == SKV_OK)                           \
-      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, f.warps * kWarp, f.smem, c.stream>>>(a);                     \
+      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, f.warps * kWarp, f.smem, c.stream>>>(a);                    \
   }
   SKV_LANES(f.lpt, f.cv, SKV_CALL)
 #undef SKV_CALL
