@@ -28,7 +28,7 @@ void describe_dc_plan(const skv_problem& p, int64_t slab, int64_t* out);
 bool readout_eligible(const skv_problem& p, int64_t D);
 size_t readout_image_bytes(const skv_problem& p, int64_t D);
 int64_t readout_delta_pitch(const skv_problem& p);
-int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg);
+int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg, bool first);
 int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, int64_t D, void* y, int64_t ys, void* wimg);
 }  // namespace tc
 }  // namespace skv
@@ -191,11 +191,12 @@ size_t skv_scratch_bytes(const skv_problem* p, int op) {
   return need;
 }
 
-int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, void* act_out,
-                        int64_t act_stride, void* delta_out, int64_t delta_stride, void* scratch,
-                        size_t scratch_bytes, int32_t* status, void* stream) {
-  LaunchCtx c;
-  if (int e = make_ctx(p, stream, status, &c)) return e;
+}  // extern "C"
+
+namespace {
+int feature_forward(const LaunchCtx& c, const void* z, int64_t z_stride, const void* C, void* act_out, int64_t act_stride,
+                    void* delta_out, int64_t delta_stride, void* scratch, size_t scratch_bytes) {
+  const skv_problem* p = &c.p;
   if (p->N == 0) return SKV_OK;
   if (!z || !C || !delta_out) return SKV_ERR_NULL;
   if (z_stride < p->h || delta_stride < p->r || (act_out && act_stride < p->h)) return SKV_ERR_SHAPE;
@@ -212,7 +213,20 @@ int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, c
     // rows of a fitting shape passed at odd addresses or strides: there is no room for copies
     if (p->impl == SKV_IMPL_TCGEN05) return SKV_ERR_ALIGN;
   }
+  if (c.beside)
+    if (int e = c.beside(c.beside_arg, true)) return e;
   return simt_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
+}
+}  // namespace
+
+extern "C" {
+
+int skv_feature_forward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, void* act_out,
+                        int64_t act_stride, void* delta_out, int64_t delta_stride, void* scratch,
+                        size_t scratch_bytes, int32_t* status, void* stream) {
+  LaunchCtx c;
+  if (int e = make_ctx(p, stream, status, &c)) return e;
+  return feature_forward(c, z, z_stride, C, act_out, act_stride, delta_out, delta_stride, scratch, scratch_bytes);
 }
 
 int skv_feature_backward(const skv_problem* p, const void* z, int64_t z_stride, const void* C, const void* g_act,
@@ -279,10 +293,15 @@ int skv_feature_readout_forward(const skv_problem* p, const void* z, int64_t z_s
   void* delta = base + fwd_bytes;
   const int64_t dp = tc::readout_delta_pitch(*p);
   void* wimg = base + fwd_bytes + round256((size_t)p->N * dp * 2);
-  if (dp != p->r && cudaMemsetAsync(delta, 0, (size_t)p->N * dp * 2, c.stream) != cudaSuccess) return SKV_ERR_LAUNCH;
-  if (int e = tc::readout_pack(c, w_out, w_stride, d_out, wimg)) return e;
-  if (int e = skv_feature_forward(&q, z, z_stride, C, nullptr, 0, delta, dp, scratch, fwd_bytes, status, stream))
-    return e;
+  const struct PackW { const LaunchCtx& c; const void* w; int64_t ws, D; void* img; } pack{c, w_out, w_stride, d_out, wimg};
+  LaunchCtx f = c;
+  f.p = q;
+  f.beside_arg = &pack;
+  f.beside = [](const void* arg, bool first) {
+    const PackW& a = *static_cast<const PackW*>(arg);
+    return tc::readout_pack(a.c, a.w, a.ws, a.D, a.img, first);
+  };
+  if (int e = feature_forward(f, z, z_stride, C, nullptr, 0, delta, dp, scratch, fwd_bytes)) return e;
   return tc::readout(c, z, z_stride, delta, d_out, y, y_stride, wimg);
 }
 

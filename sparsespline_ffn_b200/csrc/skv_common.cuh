@@ -109,6 +109,10 @@ struct LaunchCtx {
   cudaStream_t stream;
   int32_t* status;
   int num_sms;
+  // Launched by a tensor-core forward behind its first kernel, to run beside it (the read-out's image of W), by a CUDA-core
+  // forward as its first; may be null.
+  int (*beside)(const void* arg, bool first) = nullptr;
+  const void* beside_arg = nullptr;
 };
 
 // CUDA-core kernel family (any N, h, L, r <= 256; bf16 or float32).

@@ -11,7 +11,10 @@ namespace skv {
 // Programmatic dependent launch: a kernel of a call's chain may be scheduled while its predecessor still
 // runs (its CTAs have all started); pdl_wait() returns once the predecessor is complete and its
 // writes are visible.  Every kernel launched through launch_chained() calls it in every thread that touches what earlier
-// kernels wrote; the first kernel of a call is launched plainly and so follows everything before it.
+// kernels wrote.  The first kernel of a call, whose predecessor is whatever was on the stream, waits in every thread before
+// anything else and only then lets its successor start: from there on the call's inputs may be read without a wait.
+// Chained to what was there its launch costs nothing: a plain launch leaves 1.5 us between two calls.  The last kernel of a call
+// lets its successor start after its own wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // (What an earlier kernel of the chain wrote is read through plain pointers or ld16, never through const __restrict__
 // pointers or __ldg: the compiler may move such loads above the wait.)

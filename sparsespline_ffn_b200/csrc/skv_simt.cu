@@ -7,6 +7,7 @@
 // a warp works on 32 / LPT tokens of one key at a time; knot interval and weights of a pair are
 // computed once by one lane and handed to the LPT lanes through shared memory (a 16-byte broadcast).
 #include "skv_common.cuh"
+#include "skv_launch.cuh"
 
 namespace skv {
 namespace {
@@ -119,6 +120,8 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, sizeof(T)) * kWarp, 2) s
   float4* my = wbuf + warp * TPW * kWarp;
   const T* z = static_cast<const T*>(P.z);
   T* act_out = static_cast<T*>(P.act_out);
+  pdl_wait();
+  pdl_launch();
   const int64_t tile0 = (int64_t)blockIdx.x * (W * TPW * P.groups);
   const int kbeg = blockIdx.y * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
   const int rowstep = pitch;
@@ -225,10 +228,15 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, sizeof(T)) * kWarp, 2) s
 // warps as the chip holds and four rows' loads are in flight per lane; then, from about 64 tokens at h = 5120 on, by what
 // L2 delivers (three rows per pair).
 // ---------------------------------------------------------------------------------------------
-template <typename T, int CV, bool VECLD>
+// 16 bytes of a row at element `col`, as one load or (BYTES 8) two, where rows start on such boundaries; 0: element by element.
+template <typename T, int BYTES>
 __device__ __forceinline__ void load_row(const T* __restrict__ row, int col, int r, float (&f)[Vec<T>::n]) {
-  if constexpr (VECLD) {
+  if constexpr (BYTES == 16) {
     Vec<T>::cvt(__ldg(reinterpret_cast<const uint4*>(row + col)), f);
+  } else if constexpr (BYTES == 8) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(row + col));
+    const uint2 b = col + Vec<T>::n / 2 < r ? __ldg(reinterpret_cast<const uint2*>(row + col) + 1) : make_uint2(0, 0);
+    Vec<T>::cvt(make_uint4(a.x, a.y, b.x, b.y), f);
   } else {
 #pragma unroll
     for (int i = 0; i < Vec<T>::n; ++i) f[i] = col + i < r ? ld_f32<T>(row + col + i) : 0.0f;
@@ -247,7 +255,7 @@ __device__ __forceinline__ void store_first_cta(float* p, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(b), "f"(v) : "memory");
 }
 
-template <typename T, typename TD, int LPT, int CV, bool VECLD>
+template <typename T, typename TD, int LPT, int CV, int BYTES>
 __global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_kernel(const FwdArgs P) {
   constexpr int V = Vec<T>::n;
   constexpr int TPW = kWarp / LPT;
@@ -265,6 +273,8 @@ __global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_ker
   const int kbeg = rank * P.keys_per_split, kend = min(P.h, kbeg + P.keys_per_split);
   const bool three = P.g.order != 1;
   float4* my = wbuf + warp * kWarp;
+  pdl_wait();
+  pdl_launch();
   if (cs > 1) cluster_arrive();                       // the first CTA has started before anything is sent to it
 
   for (int64_t n = blockIdx.x / cs; n < P.N; n += gridDim.x / cs) {
@@ -298,9 +308,9 @@ __global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_ker
           const int col = c * (LPT * V) + sl * V;
           if (col < P.r) {
             float f0[V], f1[V], f2[V];
-            load_row<T, CV, VECLD>(row, col, P.r, f0);
-            load_row<T, CV, VECLD>(row + P.r, col, P.r, f1);
-            if (three) load_row<T, CV, VECLD>(row + 2 * P.r, col, P.r, f2);
+            load_row<T, BYTES>(row, col, P.r, f0);
+            load_row<T, BYTES>(row + P.r, col, P.r, f1);
+            if (three) load_row<T, BYTES>(row + 2 * P.r, col, P.r, f2);
 #pragma unroll
             for (int i = 0; i < V; ++i) {
               acc[c][i] = fmaf(w.y, f1[i], fmaf(w.x, f0[i], acc[c][i]));
@@ -355,9 +365,11 @@ __global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_ker
 // Sum of the key splits' partial residuals in a fixed order, lambda, cast.  A CTA takes 32 elements;
 // its eight warps each add every eighth split, so that a sum over many splits is not one serial chain.
 template <typename TD>
-__global__ void __launch_bounds__(256) simt_finalize_kernel(const float* __restrict__ partial, int splits, int64_t N,
-                                                            int r, float lambda, TD* __restrict__ out, int64_t ds) {
+__global__ void __launch_bounds__(256) simt_finalize_kernel(const float* partial, int splits, int64_t N,
+                                                            int r, float lambda, TD* out, int64_t ds) {
   __shared__ float part[8][kWarp];
+  pdl_wait();
+  pdl_launch();
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const int64_t total = N * r;
   for (int64_t b = (int64_t)blockIdx.x * kWarp; b < total; b += (int64_t)gridDim.x * kWarp) {
@@ -431,6 +443,8 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, 4) * kWarp, 2) simt_dz_k
   T* dz = static_cast<T*>(P.dz);
   const bool two = P.g.order != 1;
   const int R = P.L - 1;                                                   // difference rows per key
+  pdl_wait();
+  pdl_launch();
   const int64_t tile0 = (int64_t)blockIdx.x * (W * TPW * P.groups);
   const int j0 = blockIdx.y * P.kch, kc = min(P.kch, P.h - j0);
 
@@ -584,6 +598,7 @@ struct DcArgs {
   float lambda;
   int TT;                    // tokens per tile, a multiple of 32
   int64_t tokens_per_split;
+  bool first;                // the first kernel of a call; else it runs beside dz, which it has nothing to wait for
 };
 
 constexpr int kMaxTile = 256;
@@ -635,6 +650,8 @@ __global__ void __launch_bounds__(kDcMaxWarps * kWarp, 1) simt_dc_kernel(const D
                     : acc_all + (size_t)warp * P.L * pitch;
   const int ap = GACC ? r : pitch;
 
+  if (P.first) pdl_wait();
+  pdl_launch();
   if constexpr (GACC) {
     if (mine)
       for (int i = lane; i < P.L * r; i += kWarp) acc[i] = 0.0f;
@@ -840,6 +857,7 @@ __global__ void __launch_bounds__(kDcMaxWarps * kWarp, 1) simt_dc_kernel(const D
     }
     __syncwarp();
   }
+  if (!P.first) pdl_wait();                            // whoever waits for this kernel has waited for dz
   __syncthreads();
   if (!mine) return;
   const size_t row0 = (size_t)(j0 + warp) * P.L;
@@ -858,8 +876,9 @@ __global__ void __launch_bounds__(kDcMaxWarps * kWarp, 1) simt_dc_kernel(const D
 }
 
 template <typename T>
-__global__ void simt_dc_reduce_kernel(const float* __restrict__ part, int splits, size_t elems, float lambda,
-                                      float* __restrict__ dC, T* __restrict__ dC_cast) {
+__global__ void simt_dc_reduce_kernel(const float* part, int splits, size_t elems, float lambda, float* dC, T* dC_cast) {
+  pdl_wait();
+  pdl_launch();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < elems; i += (size_t)gridDim.x * blockDim.x) {
     float s = 0.0f;
 #pragma unroll 4
@@ -900,7 +919,7 @@ void lanes_for(int r, int v, int* lpt, int* cv) {
 
 struct FwdPlan { bool small; int lpt, cv, warps, kch, groups, splits, keys_per_split; int64_t tiles; size_t smem; };
 
-FwdPlan plan_forward(const skv_problem& p) {
+FwdPlan make_forward_plan(const skv_problem& p) {
   FwdPlan f;
   const int size = p.dtype == SKV_BF16 ? 2 : 4, v = 16 / size;
   lanes_for(p.r, v, &f.lpt, &f.cv);
@@ -979,7 +998,7 @@ FwdPlan plan_forward(const skv_problem& p) {
 }
 
 struct DzPlan { bool staged; int lpt, cv, warps, kch, groups; int64_t tiles; size_t smem; };
-DzPlan plan_dz(const skv_problem& p) {
+DzPlan make_dz_plan(const skv_problem& p) {
   DzPlan d;
   lanes_for(p.r, 4, &d.lpt, &d.cv);
   const int tpw = kWarp / d.lpt, pitch = d.lpt * 4 * d.cv;
@@ -1009,7 +1028,7 @@ DzPlan plan_dz(const skv_problem& p) {
 }
 
 struct DcPlan { bool gacc; int lpt, cv, W, TT, splits; int64_t tokens_per_split; size_t smem; };
-DcPlan plan_dc(const skv_problem& p) {
+DcPlan make_dc_plan(const skv_problem& p) {
   DcPlan d;
   lanes_for(p.r, 4, &d.lpt, &d.cv);
   const int pitch = d.lpt * 4 * d.cv, nb = p.L - 1, S = kWarp / d.lpt;
@@ -1027,7 +1046,7 @@ DcPlan plan_dc(const skv_problem& p) {
     // needs about twenty warps per SM to be busy
     const double tile = (double)W * (TT * 1.5 + TT * (6.0 + 14.0 * d.cv) / S + p.L * (14.0 + 12.0 * d.cv)) / (W < 20 ? W / 20.0 : 1.0);
     int64_t last = 0;
-    for (int64_t s = 1; s <= 16; ++s) {
+    for (int64_t s = 1; s <= 16 && s <= tiles; ++s) {
       const int64_t per = cdiv64(tiles, s), splits = cdiv64(tiles, per);
       if (splits == last) continue;
       last = splits;
@@ -1045,21 +1064,29 @@ DcPlan plan_dc(const skv_problem& p) {
     }
   };
   for (int TT = kMaxTile; TT >= 64; TT >>= 1)
-    for (int W = kDcMaxWarps; W >= 1; --W)
+    for (int W : {24, 20, 16, 12, 8, 6, 4, 2, 1})
       if (bytes(W, TT, false) <= kSmemMost) consider(W, TT, false);
   if (best == 0.0) consider(kWarps, 64, true);
   return d;
 }
 
-template <typename K>
-int set_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return SKV_ERR_LAUNCH;
-    }
-  }
-  return SKV_OK;
+// The plan of the last problem this thread asked about: a call asks for its scratch and again for its launch.
+template <typename Plan, Plan (*Make)(const skv_problem&)>
+const Plan& last_plan(const skv_problem& p) {
+  static thread_local struct { int64_t N; int h, L, r, dtype, order; Plan plan; } last{-1, 0, 0, 0, 0, 0, {}};
+  if (last.N != p.N || last.h != p.h || last.L != p.L || last.r != p.r || last.dtype != p.dtype || last.order != p.spline_order)
+    last = {p.N, p.h, p.L, p.r, p.dtype, p.spline_order, Make(p)};
+  return last.plan;
+}
+const FwdPlan& plan_forward(const skv_problem& p) { return last_plan<FwdPlan, make_forward_plan>(p); }
+const DzPlan& plan_dz(const skv_problem& p) { return last_plan<DzPlan, make_dz_plan>(p); }
+const DcPlan& plan_dc(const skv_problem& p) { return last_plan<DcPlan, make_dc_plan>(p); }
+
+template <auto Kernel, typename... Args>
+int launch(dim3 grid, int warps, size_t smem, cudaStream_t stream, const Args&... args) {
+  if (launch_chained<Kernel>(grid, (unsigned)(warps * kWarp), smem, stream, args...) == cudaSuccess) return SKV_OK;
+  cudaGetLastError();
+  return SKV_ERR_LAUNCH;
 }
 
 // The CTAs of a token as a cluster.
@@ -1070,13 +1097,17 @@ int launch_small(K kernel, const FwdPlan& f, const FwdArgs& a, cudaStream_t stre
   cfg.blockDim = dim3((unsigned)(f.warps * kWarp));
   cfg.dynamicSmemBytes = f.smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)f.groups;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+  cfg.numAttrs = 2;
+  if (cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess) return SKV_OK;
+  cudaGetLastError();
+  return SKV_ERR_LAUNCH;
 }
 
 // One case per (lanes per token, pieces per lane) that rows of up to 256 elements need.
@@ -1103,14 +1134,16 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
   a.N = p.N; a.h = p.h; a.L = p.L; a.r = p.r; a.g = c.g; a.lambda = p.lambda_scale; a.act = p.activation;
   a.kch = f.kch; a.keys_per_split = f.keys_per_split; a.groups = f.groups;
   const dim3 grid((unsigned)f.tiles, (unsigned)f.splits);
-  const bool vec = p.r % Vec<T>::n == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  constexpr int n = Vec<T>::n;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(C);
+  const int bytes = p.r % n == 0 && at % 16 == 0 ? 16 : p.r % (n / 2) == 0 && at % 8 == 0 ? 8 : 0;
   int e = SKV_OK;
 #define SKV_CALL(LPT_, CV_)                                                                                     \
   {                                                                                                             \
-    if (f.small && vec) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, true>, f, a, c.stream);    \
-    else if (f.small) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, false>, f, a, c.stream);     \
-    else if ((e = set_smem(simt_forward_kernel<T, TD, LPT_, CV_>, f.smem)) == SKV_OK)                           \
-      simt_forward_kernel<T, TD, LPT_, CV_><<<grid, f.warps * kWarp, f.smem, c.stream>>>(a);                    \
+    if (f.small && bytes == 16) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 16>, f, a, c.stream);    \
+    else if (f.small && bytes == 8) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 8>, f, a, c.stream);  \
+    else if (f.small) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 0>, f, a, c.stream);     \
+    else e = launch<simt_forward_kernel<T, TD, LPT_, CV_>>(grid, f.warps, f.smem, c.stream, a);                 \
   }
   SKV_LANES(f.lpt, f.cv, SKV_CALL)
 #undef SKV_CALL
@@ -1118,11 +1151,11 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
   note_launches(1);
   if (f.splits > 1) {
     const int64_t blocks = cdiv64(p.N * p.r, kWarp);
-    simt_finalize_kernel<TD><<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, c.stream>>>(
-        a.partial, f.splits, p.N, p.r, p.lambda_scale, static_cast<TD*>(delta_out), ds);
+    e = launch<simt_finalize_kernel<TD>>(dim3((unsigned)(blocks < 4096 ? blocks : 4096)), 8, 0, c.stream, (const float*)a.partial,
+                                         f.splits, p.N, p.r, p.lambda_scale, static_cast<TD*>(delta_out), ds);
     note_launches(1);
   }
-  return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+  return e;
 }
 
 template <typename T>
@@ -1140,17 +1173,13 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
     int e = SKV_OK;
 #define SKV_CALL(LPT_, CV_)                                                                              \
   {                                                                                                      \
-    if (!d.staged) {                                                                                     \
-      if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, false>, d.smem)) == SKV_OK)                         \
-        simt_dz_kernel<T, LPT_, CV_, false><<<grid, d.warps * kWarp, d.smem, c.stream>>>(a);              \
-    } else if ((e = set_smem(simt_dz_kernel<T, LPT_, CV_, true>, d.smem)) == SKV_OK)                     \
-      simt_dz_kernel<T, LPT_, CV_, true><<<grid, d.warps * kWarp, d.smem, c.stream>>>(a);                 \
+    e = d.staged ? launch<simt_dz_kernel<T, LPT_, CV_, true>>(grid, d.warps, d.smem, c.stream, a)        \
+                 : launch<simt_dz_kernel<T, LPT_, CV_, false>>(grid, d.warps, d.smem, c.stream, a);      \
   }
     SKV_LANES(d.lpt, d.cv, SKV_CALL)
 #undef SKV_CALL
     if (e) return e;
     note_launches(1);
-    if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
   }
   if (dC || dC_cast) {
     DcPlan d = plan_dc(p);
@@ -1169,27 +1198,24 @@ int backward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, con
     a.dC = dC; a.dC_cast = dC_cast;
     a.N = p.N; a.h = p.h; a.L = p.L; a.r = p.r; a.g = c.g; a.lambda = p.lambda_scale;
     a.TT = d.TT; a.tokens_per_split = d.tokens_per_split;
+    a.first = !dz;
     const dim3 grid((unsigned)cdiv64(p.h, d.W), (unsigned)d.splits);
     int e = SKV_OK;
 #define SKV_CALL(LPT_, CV_)                                                                              \
   {                                                                                                      \
-    if (d.gacc) {                                                                                        \
-      if ((e = set_smem(simt_dc_kernel<T, LPT_, CV_, true>, d.smem)) == SKV_OK)                          \
-        simt_dc_kernel<T, LPT_, CV_, true><<<grid, d.W * kWarp, d.smem, c.stream>>>(a);                  \
-    } else if ((e = set_smem(simt_dc_kernel<T, LPT_, CV_, false>, d.smem)) == SKV_OK)                    \
-      simt_dc_kernel<T, LPT_, CV_, false><<<grid, d.W * kWarp, d.smem, c.stream>>>(a);                   \
+    e = d.gacc ? launch<simt_dc_kernel<T, LPT_, CV_, true>>(grid, d.W, d.smem, c.stream, a)              \
+               : launch<simt_dc_kernel<T, LPT_, CV_, false>>(grid, d.W, d.smem, c.stream, a);            \
   }
     SKV_LANES(d.lpt, d.cv, SKV_CALL)
 #undef SKV_CALL
     if (e) return e;
     note_launches(1);
-    if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
     if (parts) {
       const unsigned rgrid = (unsigned)((elems + 255) / 256 < 4096 ? (elems + 255) / 256 : 4096);
-      simt_dc_reduce_kernel<T><<<rgrid, 256, 0, c.stream>>>(a.part, d.splits, elems, p.lambda_scale, dC,
-                                                            static_cast<T*>(dC_cast));
+      if (int e2 = launch<simt_dc_reduce_kernel<T>>(dim3(rgrid), 8, 0, c.stream, (const float*)a.part, d.splits, elems, p.lambda_scale,
+                                                    dC, static_cast<T*>(dC_cast)))
+        return e2;
       note_launches(1);
-      if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
     }
   }
   return SKV_OK;

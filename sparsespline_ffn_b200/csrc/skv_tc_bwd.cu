@@ -245,9 +245,9 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
     PrepParams G = Q;
     G.lpt = 0;
     Q.g = nullptr;
-    if (int e = launch_prep(G, c.stream)) return e;
+    if (int e = launch_prep(G, c)) return e;
   }
-  if (int e = launch_prep(Q, c.stream)) return e;
+  if (int e = launch_prep(Q, c)) return e;
 
   DzParams Z;
   Z.z = static_cast<const __nv_bfloat16*>(z);

@@ -126,7 +126,7 @@ int forward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void* 
     zs = hp;
     act_out = nullptr;                                   // written by the copy
   }
-  if (int e = launch_prep(Q, c.stream)) return e;
+  if (int e = launch_prep(Q, c)) return e;
 
   FwdParams P;
   P.z = static_cast<const __nv_bfloat16*>(z);

@@ -3,7 +3,7 @@
 //
 // Each of these is a few microseconds of memory traffic, so launches, not bytes, are what they cost: the
 // scans of C and g_delta share one launch, all images and copies another, and the maximum is combined by
-// every block of the second launch from the block maxima of the first, which needs neither atomics
+// every warp of the second launch from the block maxima of the first, which needs neither atomics
 // nor a cleared word.
 #include "skv_tc_prep.cuh"
 
@@ -74,7 +74,8 @@ __device__ __forceinline__ uint32_t scan_share(const PrepParams& P, bool is_c, i
 
 __global__ void __launch_bounds__(256) tc_scan_kernel(const __grid_constant__ PrepParams P) {
   __shared__ uint32_t words[32];
-  pdl_launch();
+  pdl_wait();
+  pdl_launch();                                         // only now: later kernels may read the call's inputs at once
   const bool is_c = (int)blockIdx.x < P.scan_c;
   const int blk = is_c ? blockIdx.x : blockIdx.x - P.scan_c, nblk = is_c ? P.scan_c : P.scan_g;
   const int64_t first = (int64_t)blk * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
@@ -83,14 +84,17 @@ __global__ void __launch_bounds__(256) tc_scan_kernel(const __grid_constant__ Pr
   if (threadIdx.x == 0) P.hdr[kBlockMax + (is_c ? 0 : kMaxBlocks) + blk] = m;
 }
 
-__device__ __forceinline__ uint32_t combine(const uint32_t* part, int n, uint32_t* words, bool& bad) {
+// Maximum of the block maxima, by every warp for itself: no barrier between the wait for the scan and the first image.
+__device__ __forceinline__ uint32_t combine(const uint32_t* part, int n, bool& bad) {
   uint32_t m = 0, all = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    m = max(m, part[i] & ~kBadBit);
-    all |= part[i];
+#pragma unroll 4
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
+    const uint32_t v = part[i];
+    m = max(m, v & ~kBadBit);
+    all |= v;
   }
-  bad = __syncthreads_or((int)(all & kBadBit)) != 0;
-  return block_max(m, words);
+  bad = __any_sync(0xffffffffu, (all & kBadBit) != 0u);
+  return __reduce_max_sync(0xffffffffu, m);
 }
 
 // Eight bf16 with zeros in the place of infinities and NaN.
@@ -109,67 +113,82 @@ __device__ __forceinline__ uint4 scaled_h8(const uint4& v, float s) {
 // Second difference of one bf16 column triple, scaled by a power of two (exact), as the dz table wants it.
 __device__ __forceinline__ float diff2(float a, float b, float c, float s) { return (a - 2.0f * b + c) * s; }
 
+// Division constants of the packing kernel: channel groups per row of the C image, the T image and g, rows per key of both.
+struct PackDiv { FastDiv cgi_c, cgi_t, cgs, lpc, lpt; };
+
 // Images.  Piece e (16 bytes) of an image is row e & 7 of the core matrix e >> 3; core matrices run over code
 // channels first, then over groups of eight rows, so consecutive threads write consecutive bytes and
 // the threads of a warp read whole rows.
-__global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
-  __shared__ uint32_t words[32];
-  pdl_launch();
-  pdl_wait();
-  int blk = blockIdx.x;
-  const int cgs = P.rp / 8;
+//
+// The sources of a thread's first pieces are requested before the wait for the scan, and rows are copied there (all are inputs of
+// the call); what is left behind it is the maximum, arithmetic and stores.
+constexpr int kPieces = 2;                              // pieces a thread works on at a time
+
+template <bool IS_T>
+__device__ __forceinline__ void pack_table(const PrepParams& P, const PackDiv& F, int blk) {
+  const int cgs = P.rp / 8, cgi = IS_T ? cgs * P.tparts : cgs;             // channel groups of the image
+  const int nblk = IS_T ? P.blocks_t : P.blocks_c, LP = IS_T ? P.lpt : P.lpc;
+  const FastDiv &fc = IS_T ? F.cgi_t : F.cgi_c, &fl = IS_T ? F.lpt : F.lpc;
   const bool cvec = P.r % 8 == 0 && (reinterpret_cast<uintptr_t>(P.C) & 15) == 0;
-  if (blk == 0) {                                       // final maxima for the kernels that follow
-    bool bad;
-    if (P.scan_c) {
-      const uint32_t m = combine(P.hdr + kBlockMax, P.scan_c, words, bad);
-      if (threadIdx.x == 0) { P.hdr[kAmaxC] = m; P.hdr[kBadC] = bad; }
-    }
-    if (P.scan_g) {
-      const uint32_t m = combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words, bad);
-      if (threadIdx.x == 0) { P.hdr[kAmaxG] = m; P.hdr[kBadG] = bad; }
-    }
-  }
-  if (blk < P.blocks_c + P.blocks_t) {
-    const bool is_t = blk >= P.blocks_c;
-    const int nblk = is_t ? P.blocks_t : P.blocks_c;
-    if (is_t) blk -= P.blocks_c;
-    float scale, inv;
-    bool bad;
-    pow2_scales(combine(P.hdr + kBlockMax, P.scan_c, words, bad), scale, inv);
-    bad = bad && P.contain;
-    const int LP = is_t ? P.lpt : P.lpc;
-    const int cgi = is_t ? cgs * P.tparts : cgs;        // channel groups of the image
-    const int64_t pieces = (int64_t)P.hp * LP * cgi;
-    uint4* img = reinterpret_cast<uint4*>(is_t ? P.timg : P.cimg);
-#pragma unroll 2
-    for (int64_t e = (int64_t)blk * blockDim.x + threadIdx.x; e < pieces; e += (int64_t)nblk * blockDim.x) {
-      const uint32_t core = (uint32_t)(e >> 3);
-      const uint32_t rg = core / (uint32_t)cgi;
-      uint32_t cg = core - rg * cgi;
-      const bool rest = cg >= (uint32_t)cgs;            // remainders
+  const int64_t pieces = (int64_t)P.hp * LP * cgi, step = (int64_t)nblk * blockDim.x;
+  uint4* img = reinterpret_cast<uint4*>(IS_T ? P.timg : P.cimg);
+  uint4 v[kPieces][IS_T ? 3 : 1];
+  int bs[kPieces];                                      // row of the key, with kRest: of the remainders; -1: zeros
+  constexpr int kRest = 1 << 16;
+  auto request = [&](int64_t e0) {
+#pragma unroll
+    for (int x = 0; x < kPieces; ++x) {
+      const int64_t e = e0 + x * step;
+      bs[x] = -1;
+      if (e >= pieces) continue;
+      const uint32_t core = (uint32_t)(e >> 3), rg = fc.div(core);
+      uint32_t cg = core - rg * (uint32_t)cgi;
+      const bool rest = IS_T && cg >= (uint32_t)cgs;
       if (rest) cg -= cgs;
-      const uint32_t row = rg * 8u + ((uint32_t)e & 7u);
-      const uint32_t j = row / (uint32_t)LP;
+      const uint32_t row = rg * 8u + ((uint32_t)e & 7u), j = fl.div(row);
       const int b = (int)(row - j * LP), c = (int)cg * 8, left = P.r - c;
+      if ((int)j >= P.h || left <= 0) continue;
+      const __nv_bfloat16* base = P.C + (size_t)j * P.L * P.r + c;
+      if constexpr (!IS_T) {
+        // group f = b / 4 holds knot rows 2f, 2f + 1 and 2(f + F - 1), 2(f + F - 1) + 1, F = LP / 4 groups
+        const int kr = 2 * (b >> 2) + (b & 1) + ((b & 2) ? LP / 2 - 2 : 0);
+        if (kr >= P.L) continue;
+        v[x][0] = ld8(base + (size_t)kr * P.r, left, cvec);
+      } else {
+        // b = 0: C[1] - C[0]; b > 0: C[b-1] - 2 C[b] + C[b+1]
+        if (b >= P.L - 1) continue;
+        v[x][0] = ld8(base + (size_t)(b > 0 ? b - 1 : 0) * P.r, left, cvec);
+        v[x][1] = ld8(base + (size_t)(b > 0 ? b : 1) * P.r, left, cvec);
+        v[x][2] = b > 0 ? ld8(base + (size_t)(b + 1) * P.r, left, cvec) : make_uint4(0, 0, 0, 0);
+      }
+      bs[x] = b + (rest ? kRest : 0);
+    }
+  };
+  const int64_t first = (int64_t)blk * blockDim.x + threadIdx.x;
+  request(first);
+  pdl_wait();
+  float scale, inv;
+  bool bad;
+  pow2_scales(combine(P.hdr + kBlockMax, P.scan_c, bad), scale, inv);
+  bad = bad && P.contain;
+  for (int64_t e0 = first; e0 < pieces; e0 += kPieces * step) {
+    if (e0 != first) request(e0);
+#pragma unroll
+    for (int x = 0; x < kPieces; ++x) {
+      if (e0 + x * step >= pieces) break;
       uint4 o = make_uint4(0, 0, 0, 0);
-      if ((int)j < P.h && left > 0) {
-        const __nv_bfloat16* base = P.C + (size_t)j * P.L * P.r + c;
-        if (!is_t) {
-          // group f = b / 4 holds knot rows 2f, 2f + 1 and 2(f + F - 1), 2(f + F - 1) + 1, F = LP / 4 groups
-          const int kr = 2 * (b >> 2) + (b & 1) + ((b & 2) ? LP / 2 - 2 : 0);
-          if (kr < P.L) o = scaled_h8(finite8(ld8(base + (size_t)kr * P.r, left, cvec), bad), scale);
-        } else if (b < P.L - 1) {
-          // b = 0: C[1] - C[0]; b > 0: C[b-1] - 2 C[b] + C[b+1]
-          const uint4 v0 = finite8(ld8(base + (size_t)(b > 0 ? b - 1 : 0) * P.r, left, cvec), bad);
-          const uint4 v1 = finite8(ld8(base + (size_t)(b > 0 ? b : 1) * P.r, left, cvec), bad);
-          const uint4 v2 = b > 0 ? finite8(ld8(base + (size_t)(b + 1) * P.r, left, cvec), bad) : make_uint4(0, 0, 0, 0);
+      if (bs[x] >= 0) {
+        if constexpr (!IS_T) {
+          o = scaled_h8(finite8(v[x][0], bad), scale);
+        } else {
+          const bool rest = bs[x] >= kRest, b0 = (bs[x] & (kRest - 1)) == 0;
+          const uint4 v0 = finite8(v[x][0], bad), v1 = finite8(v[x][1], bad), v2 = finite8(v[x][2], bad);
           const uint32_t a0[4] = {v0.x, v0.y, v0.z, v0.w}, a1[4] = {v1.x, v1.y, v1.z, v1.w}, a2[4] = {v2.x, v2.y, v2.z, v2.w};
           uint32_t w[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            float lo = b > 0 ? diff2(bf_lo(a0[i]), bf_lo(a1[i]), bf_lo(a2[i]), scale) : (bf_lo(a1[i]) - bf_lo(a0[i])) * scale;
-            float hi = b > 0 ? diff2(bf_hi(a0[i]), bf_hi(a1[i]), bf_hi(a2[i]), scale) : (bf_hi(a1[i]) - bf_hi(a0[i])) * scale;
+            float lo = b0 ? (bf_lo(a1[i]) - bf_lo(a0[i])) * scale : diff2(bf_lo(a0[i]), bf_lo(a1[i]), bf_lo(a2[i]), scale);
+            float hi = b0 ? (bf_hi(a1[i]) - bf_hi(a0[i])) * scale : diff2(bf_hi(a0[i]), bf_hi(a1[i]), bf_hi(a2[i]), scale);
             if (rest) {
               lo -= __half2float(__float2half_rn(lo));
               hi -= __half2float(__float2half_rn(hi));
@@ -179,48 +198,79 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const PrepParams P) {
           o = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
-      img[e] = o;
+      img[e0 + x * step] = o;
     }
-    return;
   }
-  blk -= P.blocks_c + P.blocks_t;
-  if (blk < P.blocks_g) {
+}
+
+__global__ void __launch_bounds__(256) tc_pack_kernel(const __grid_constant__ PrepParams P, const __grid_constant__ PackDiv F) {
+  pdl_launch();
+  int blk = blockIdx.x;
+  if (blk < P.blocks_c + P.blocks_t) {
+    if (blk < P.blocks_c) pack_table<false>(P, F, blk);
+    else pack_table<true>(P, F, blk - P.blocks_c);
+  } else if (blk < P.blocks_c + P.blocks_t + P.blocks_g) {
+    const int cgs = P.rp / 8;
+    const bool vec = P.r % 8 == 0 && P.gds % 8 == 0 && (reinterpret_cast<uintptr_t>(P.g) & 15) == 0;
+    const int64_t pieces = P.tiles * 128 * cgs, step = (int64_t)P.blocks_g * blockDim.x;
+    const int64_t first = (int64_t)(blk - P.blocks_c - P.blocks_t) * blockDim.x + threadIdx.x;
+    uint4* img = reinterpret_cast<uint4*>(P.gimg);
+    uint4 v[kPieces];
+    auto request = [&](int64_t e0) {
+#pragma unroll
+      for (int x = 0; x < kPieces; ++x) {
+        const int64_t e = e0 + x * step;
+        const int64_t tc_ = e >> 7;                     // (tile, channel group)
+        const int64_t tile = P.tiles < (1 << 27) ? (int64_t)F.cgs.div((uint32_t)tc_) : tc_ / cgs;
+        const int c = (int)(tc_ - tile * cgs) * 8;
+        const int64_t n = tile * 128 + (e & 127);
+        v[x] = e < pieces && n < P.N && c < P.r ? ld8(P.g + n * P.gds + c, P.r - c, vec) : make_uint4(0, 0, 0, 0);
+      }
+    };
+    request(first);
+    pdl_wait();
     float scale, inv;
     bool bad;
-    pow2_scales(combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, words, bad), scale, inv);
+    pow2_scales(combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, bad), scale, inv);
     bad = bad && P.contain;
-    const bool vec = P.r % 8 == 0 && P.gds % 8 == 0 && (reinterpret_cast<uintptr_t>(P.g) & 15) == 0;
-    const int64_t pieces = P.tiles * 128 * cgs;
-    uint4* img = reinterpret_cast<uint4*>(P.gimg);
-#pragma unroll 2
-    for (int64_t e = (int64_t)blk * blockDim.x + threadIdx.x; e < pieces; e += (int64_t)P.blocks_g * blockDim.x) {
-      const int64_t tc_ = e >> 7;                       // (tile, channel group)
-      const int64_t tile = tc_ / cgs;
-      const int c = (int)(tc_ - tile * cgs) * 8;
-      const int64_t n = tile * 128 + (e & 127);
-      img[e] = n < P.N && c < P.r ? scaled_h8(finite8(ld8(P.g + n * P.gds + c, P.r - c, vec), bad), scale)
-                                  : make_uint4(0, 0, 0, 0);
-    }
-    return;
-  }
-  blk -= P.blocks_g;
-  for (int q = 0; q < 2; ++q) {
-    const CopyJob& J = P.copy[q];
-    if (!J.dst && !J.act_out) continue;
-    const int w8 = P.hp / 8;
-    const int64_t pieces = P.N * w8;
-    for (int64_t i = (int64_t)blk * blockDim.x + threadIdx.x; i < pieces; i += (int64_t)P.blocks_copy * blockDim.x) {
-      const int64_t n = i / w8;
-      const int c = (int)(i - n * w8) * 8, left = min(8, P.h - c);
-      const uint4 v = ld8(J.src + n * J.ss + c, left, false);
-      if (J.dst) *reinterpret_cast<uint4*>(J.dst + n * P.hp + c) = v;
-      if (J.act_out) {
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        __nv_bfloat16* o = J.act_out + n * J.as + c;
+    for (int64_t e0 = first; e0 < pieces; e0 += kPieces * step) {
+      if (e0 != first) request(e0);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < left) o[k] = __float2bfloat16_rn(act_fwd((k & 1) ? bf_hi(w[k >> 1]) : bf_lo(w[k >> 1]), P.act));
+      for (int x = 0; x < kPieces; ++x)
+        if (e0 + x * step < pieces) img[e0 + x * step] = scaled_h8(finite8(v[x], bad), scale);
+    }
+  } else {
+    blk -= P.blocks_c + P.blocks_t + P.blocks_g;
+    for (int q = 0; q < 2; ++q) {
+      const CopyJob& J = P.copy[q];
+      if (!J.dst && !J.act_out) continue;
+      const int w8 = P.hp / 8;
+      const int64_t pieces = P.N * w8;
+      for (int64_t i = (int64_t)blk * blockDim.x + threadIdx.x; i < pieces; i += (int64_t)P.blocks_copy * blockDim.x) {
+        const int64_t n = i / w8;
+        const int c = (int)(i - n * w8) * 8, left = min(8, P.h - c);
+        const uint4 v = ld8(J.src + n * J.ss + c, left, false);
+        if (J.dst) *reinterpret_cast<uint4*>(J.dst + n * P.hp + c) = v;
+        if (J.act_out) {
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+          __nv_bfloat16* o = J.act_out + n * J.as + c;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k < left) o[k] = __float2bfloat16_rn(act_fwd((k & 1) ? bf_hi(w[k >> 1]) : bf_lo(w[k >> 1]), P.act));
+        }
       }
+    }
+  }
+  pdl_wait();                                           // whoever waits for this kernel has waited for the scan
+  if (blockIdx.x == 0 && threadIdx.x < 32) {            // final maxima for the kernels that follow
+    bool bad;
+    if (P.scan_c) {
+      const uint32_t m = combine(P.hdr + kBlockMax, P.scan_c, bad);
+      if (threadIdx.x == 0) { P.hdr[kAmaxC] = m; P.hdr[kBadC] = bad; }
+    }
+    if (P.scan_g) {
+      const uint32_t m = combine(P.hdr + kBlockMax + kMaxBlocks, P.scan_g, bad);
+      if (threadIdx.x == 0) { P.hdr[kAmaxG] = m; P.hdr[kBadG] = bad; }
     }
   }
 }
@@ -234,12 +284,13 @@ __device__ __forceinline__ float pair_weight(const Knot& k, int row, int order) 
 }
 
 // delta: the contributions of infinities and NaN in C (a zero weight times one is NaN here too, as it is when the
-// touched rows alone are added up).  A thread takes the elements that it has written.
+// touched rows alone are added up).  A block takes the `outputs` groups of four columns that it has written.
 template <typename TD>
-__device__ __noinline__ void contain_delta(const Contain& K, int rp, float lambda, TD* out, int64_t ds) {
+__device__ __noinline__ void contain_delta(const Contain& K, int rp, float lambda, TD* out, int64_t ds, int outputs) {
   const int q4 = rp / 4;
   const int64_t total = K.N * q4;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+  if ((int)threadIdx.x >= outputs) return;
+  for (int64_t i = (int64_t)blockIdx.x * outputs + threadIdx.x; i < total; i += (int64_t)gridDim.x * outputs) {
     const int64_t n = i / q4;
     const int c = (int)(i - n * q4) * 4;
     float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -360,27 +411,44 @@ __device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c
   }
 }
 
-// Four consecutive columns per thread; the splits of an element are added in order, four loads in flight.
-template <typename TD, bool CONTAIN>
+// Four consecutive columns per thread, SG lanes per output: each adds every SG-th split, eight loads in flight, and the
+// SG sums are exchanged within the warp.  What one thread would add alone is a chain of round trips to L2:
+// 1999 x 2560 (36 partials of 16 K outputs) 6.8 us behind the forward with SG = 1.
+template <typename TD, bool CONTAIN, int SG>
 __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, int splits, int64_t N, int r,
                                                           int rp, float lambda, const uint32_t* hdr,
                                                           TD* out, int64_t ds, const __grid_constant__ Contain K) {
-  pdl_launch();
+  constexpr int kOut = 256 / SG;                        // outputs of a block
   pdl_wait();
+  pdl_launch();
   float cscale, cinv;
   pow2_scales(hdr[kAmaxC], cscale, cinv);
   const float f = lambda * cinv;                        // undo the code-table image's range scaling
   const int q4 = rp / 4;
   const int64_t total = N * q4;
   const bool vec = ds % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && r == rp;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const float4* src = reinterpret_cast<const float4*>(partial) + i;
+  constexpr int kPerWarp = 32 / SG;
+  const int me = (int)(threadIdx.x / 32) * kPerWarp + (int)(threadIdx.x % kPerWarp), sg = (int)(threadIdx.x % 32) / kPerWarp;
+  for (int64_t b = (int64_t)blockIdx.x * kOut; b < total; b += (int64_t)gridDim.x * kOut) {
+    const int64_t i = b + me;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i < total) {
+      const float4* src = reinterpret_cast<const float4*>(partial) + i;
 #pragma unroll 8
-    for (int k = 0; k < splits; ++k) {
-      const float4 v = src[(size_t)k * total];
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      for (int k = sg; k < splits; k += SG) {
+        const float4 v = src[(size_t)k * total];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
     }
+#pragma unroll
+    for (int x = kPerWarp; x < 32; x <<= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, x);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, x);
+      s.z += __shfl_xor_sync(0xffffffffu, s.z, x);
+      s.w += __shfl_xor_sync(0xffffffffu, s.w, x);
+    }
+    if (sg > 0) continue;
+    if (i >= total) continue;
     const int64_t n = i / q4;
     const int c = (int)(i - n * q4) * 4;
     TD* o = out + n * ds + c;
@@ -394,8 +462,12 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
         if (c + k < r) st_f32<TD>(o + k, v[k]);
     }
   }
-  if constexpr (CONTAIN)
-    if (hdr[kBadC] != 0u) contain_delta(K, rp, lambda, out, ds);
+  if constexpr (CONTAIN) {
+    if (hdr[kBadC] != 0u) {
+      __syncthreads();                                  // the block's outputs are written: its threads take them in turn
+      contain_delta(K, rp, lambda, out, ds, kOut);
+    }
+  }
 }
 
 template <bool CONTAIN>
@@ -404,6 +476,7 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
                                                            const uint32_t* hdr, float* dC,
                                                            __nv_bfloat16* dC_cast, const __grid_constant__ Contain K) {
   pdl_wait();
+  pdl_launch();
   float gscale, ginv;
   pow2_scales(hdr[kAmaxG], gscale, ginv);
   const float f = lambda * ginv;
@@ -447,6 +520,7 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
 
 __global__ void __launch_bounds__(256) tc_dz_contain_kernel(const uint32_t* hdr, const __grid_constant__ Contain K) {
   pdl_wait();
+  pdl_launch();
   const bool bad_g = hdr[kBadG] != 0u, bad_c = hdr[kBadC] != 0u;
   if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
 }
@@ -471,39 +545,56 @@ int blocks_for(int64_t items, int64_t per_thread, int most) {
 
 }  // namespace
 
-int launch_prep(PrepParams& P, cudaStream_t stream) {
+int launch_prep(PrepParams& P, const LaunchCtx& ctx) {
+  const cudaStream_t stream = ctx.stream;
   const int cgs = P.rp / 8;
-  P.scan_c = P.lpc || P.lpt ? blocks_for((int64_t)P.h * P.L * P.r / 8, 2, kPlanSMs * 2) : 0;
-  P.scan_g = P.g ? blocks_for(P.N * ((P.r + 7) / 8), 2, kPlanSMs * 2) : 0;
+  P.scan_c = P.lpc || P.lpt ? blocks_for((int64_t)P.h * P.L * P.r / 8, 2, kMaxBlocks) : 0;
+  P.scan_g = P.g ? blocks_for(P.N * ((P.r + 7) / 8), 2, kMaxBlocks) : 0;
   P.blocks_c = P.lpc ? blocks_for((int64_t)P.hp * P.lpc * cgs, 2, kPlanSMs * 8) : 0;
   P.blocks_t = P.lpt ? blocks_for((int64_t)P.hp * P.lpt * cgs * P.tparts, 2, kPlanSMs * 8) : 0;
   P.blocks_g = P.g ? blocks_for(P.tiles * 128 * cgs, 2, kPlanSMs * 8) : 0;
   P.blocks_copy = 0;
   for (const CopyJob& J : P.copy)
     if (J.dst || J.act_out) P.blocks_copy = blocks_for(P.N * (P.hp / 8), 1, kPlanSMs * 16);
+  // Not chained to what was on the stream: an SM that never runs empty keeps the split of shared memory and L1 that the last kernel
+  // asked for, and behind a dC (all of it shared memory) the forward's strided rows of z find no L1 (65536 x 5120: 770 -> 977 us).
   tc_scan_kernel<<<(unsigned)(P.scan_c + P.scan_g), 256, 0, stream>>>(P);
   if (cudaGetLastError() != cudaSuccess) return SKV_ERR_LAUNCH;
+  if (ctx.beside)
+    if (int e = ctx.beside(ctx.beside_arg, false)) return e;
   const unsigned grid = (unsigned)(P.blocks_c + P.blocks_t + P.blocks_g + P.blocks_copy);
-  if (launch_chained<tc_pack_kernel>(dim3(grid), 256, 0, stream, P) != cudaSuccess) return SKV_ERR_LAUNCH;
+  const PackDiv F{FastDiv(cgs), FastDiv(cgs * (P.tparts ? P.tparts : 1)), FastDiv(cgs), FastDiv(P.lpc ? P.lpc : 1), FastDiv(P.lpt ? P.lpt : 1)};
+  if (launch_chained<tc_pack_kernel>(dim3(grid), 256, 0, stream, P, F) != cudaSuccess) return SKV_ERR_LAUNCH;
   note_launches(2);
   return SKV_OK;
 }
 
 namespace {
 template <typename TD, bool CONTAIN>
-cudaError_t finalize(dim3 grid, cudaStream_t stream, const float* partial, int splits, int64_t N, int r, int rp, float lambda,
+cudaError_t finalize(cudaStream_t stream, const float* partial, int splits, int64_t N, int r, int rp, float lambda,
                      const uint32_t* hdr, void* out, int64_t ds, const Contain& K) {
-  return launch_chained<tc_finalize_kernel<TD, CONTAIN>>(grid, 256, 0, stream, partial, splits, N, r, rp, lambda, hdr,
-                                                         static_cast<TD*>(out), ds, K);
+  // lanes per output: so many that a lane has two rounds of eight loads, where the outputs alone do not fill the chip
+  // with four blocks per SM (9 splits, 8192 x 5120: 3.5 us with one lane, 4.7 with two)
+  const int64_t outputs = N * (rp / 4);
+  int sg = 1;
+  while (sg < 8 && splits > 16 * sg && outputs * sg < (int64_t)kPlanSMs * 1024) sg *= 2;
+  const dim3 grid((unsigned)blocks_for(outputs * sg, 1, kPlanSMs * 16));
+  auto go = [&](auto n) {
+    return launch_chained<tc_finalize_kernel<TD, CONTAIN, decltype(n)::value>>(grid, 256, 0, stream, partial, splits, N, r, rp, lambda,
+                                                                               hdr, static_cast<TD*>(out), ds, K);
+  };
+  return sg == 1   ? go(std::integral_constant<int, 1>())
+         : sg == 2 ? go(std::integral_constant<int, 2>())
+         : sg == 4 ? go(std::integral_constant<int, 4>())
+                   : go(std::integral_constant<int, 8>());
 }
 }  // namespace
 
 int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,
                     void* out, int64_t ds, bool out_f32, const Contain& K, cudaStream_t stream) {
-  const dim3 grid((unsigned)blocks_for(N * (rp / 4), 1, kPlanSMs * 16));
   auto* run = out_f32 ? (K.z ? finalize<float, true> : finalize<float, false>)
                       : (K.z ? finalize<__nv_bfloat16, true> : finalize<__nv_bfloat16, false>);
-  const cudaError_t e = run(grid, stream, partial, splits, N, r, rp, lambda, hdr, out, ds, K);
+  const cudaError_t e = run(stream, partial, splits, N, r, rp, lambda, hdr, out, ds, K);
   note_launches(1);
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }

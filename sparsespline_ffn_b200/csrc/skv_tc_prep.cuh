@@ -20,7 +20,7 @@ constexpr size_t kSmemOnePerSM = 116 * 1024;
 // that scanned C and g_delta.
 constexpr size_t kHeaderBytes = 4096;
 constexpr int kBlockMax = 64;                 // first word of the block maxima
-constexpr int kMaxBlocks = 296;               // scanning blocks per array
+constexpr int kMaxBlocks = 444;               // scanning blocks per array
 
 // The kernels work on whole chunks of keys and whole K = 16 steps of code channels; the images (and, when the
 // rows of z cannot be read in 16-byte pieces, padded copies of the token-major arrays) carry the padding.
@@ -83,8 +83,25 @@ struct PrepParams {
   int blocks_c, blocks_t, blocks_g, blocks_copy;
 };
 
-// Maxima, then images and copies: two launches.
-int launch_prep(PrepParams& P, cudaStream_t stream);
+// Maxima, then images and copies: two launches, and between them what the context has to be run beside the first.
+int launch_prep(PrepParams& P, const LaunchCtx& c);
+
+// Unsigned division by a constant: n / d for any 32-bit n (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", figure 4.1), for the places within the images.
+struct FastDiv {
+  uint32_t d, mul, s1, s2;
+  explicit FastDiv(uint32_t divisor = 1) : d(divisor) {
+    uint32_t l = 0;
+    while ((1ull << l) < d) ++l;
+    mul = (uint32_t)((((1ull << l) - d) << 32) / d + 1);
+    s1 = l < 1 ? l : 1;
+    s2 = l < 1 ? 0 : l - 1;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const {
+    const uint32_t t = __umulhi(mul, n);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
 
 // out[n][c] = lambda * 2^-k * sum over splits of partial[split][n][c], c < r of the rp partial columns.
 int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, float lambda, const uint32_t* hdr,

@@ -66,8 +66,12 @@ struct RoParams {
 // W[D][ws] (the layout of torch.nn.Linear.weight, columns [0,h) for act(z) and [h,h+r) for delta) ->
 // per (output tile, stage) a 256 x kRoK K-major tile of 8 x 16-byte core matrices, [k core][n core][8 rows],
 // zero where the tile reaches past D, h or r.
-__global__ void tc_pack_w_kernel(const __nv_bfloat16* __restrict__ W, int64_t ws, int D, int h, int r, int ks_z, int ks,
-                                 int64_t chunks, uint4* __restrict__ img) {
+// `first`: the first kernel of a call; else it runs beside the one that is (and writes what the call in front of this one may
+// still read only because that one has waited).
+__global__ void tc_pack_w_kernel(const __nv_bfloat16* W, int64_t ws, int D, int h, int r, int ks_z, int ks,
+                                 int64_t chunks, uint4* img, int first) {
+  if (first) pdl_wait();
+  pdl_launch();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < chunks; idx += (int64_t)gridDim.x * blockDim.x) {
     constexpr int kPer = (int)(kRoBBytes / 16);
     const int c = (int)(idx % kPer);
@@ -86,8 +90,9 @@ __global__ void tc_pack_w_kernel(const __nv_bfloat16* __restrict__ W, int64_t ws
       ok = ok && kd < r;
       k = (int64_t)h + kd;
     }
-    img[idx] = ok ? __ldg(reinterpret_cast<const uint4*>(W + n * ws + k)) : make_uint4(0, 0, 0, 0);
+    img[idx] = ok ? ld16(W + n * ws + k) : make_uint4(0, 0, 0, 0);
   }
+  if (!first) pdl_wait();                            // whoever waits for this kernel has waited for the one in front of it
 }
 
 template <bool RELU, int MT>
@@ -128,6 +133,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
   const int64_t step = gridDim.x, items = P.tiles * P.slices;     // item = (K slice, tile)
   pdl_wait();
+  pdl_launch();
 
   if (warp < 8) {
     // ------------------------------------------------------------------ activation in place, then epilogue
@@ -279,6 +285,7 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
 __global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partial, int slices, int64_t N, int D,
                                                              __nv_bfloat16* y, int64_t ys) {
   pdl_wait();
+  pdl_launch();
   const int q4 = D / 4;
   const int64_t total = N * q4;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -339,22 +346,24 @@ size_t readout_image_bytes(const skv_problem& p, int64_t D) {
   return wimg_bytes(p, D) + (f.slices > 1 ? (size_t)f.slices * (p.N > 0 ? p.N : 1) * D * sizeof(float) : 0);
 }
 
-// Row pitch (elements) of the delta buffer the GEMM reads: whole stages of kRoK columns, pad columns zero.
+// Row pitch (elements) of the delta buffer the GEMM reads: whole stages of kRoK columns.
 int64_t readout_delta_pitch(const skv_problem& p) { return (int64_t)((p.r + kRoK - 1) / kRoK) * kRoK; }
 
-// Tiled image of W; a plain launch in front of the feature kernels, so that the GEMM can be chained to them.
-int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg) {
+// Tiled image of W, in front of the feature kernels or beside their first, so that the GEMM can be chained to them.
+int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg, bool first) {
   const skv_problem& p = c.p;
   const int ks_z = (p.h + kRoK - 1) / kRoK, ks = ks_z + (p.r + kRoK - 1) / kRoK;
   const int64_t chunks = (D + 255) / 256 * ks * (kRoBBytes / 16);
   const int pgrid = (int)((chunks + 255) / 256 < 4096 ? (chunks + 255) / 256 : 4096);
-  tc_pack_w_kernel<<<pgrid, 256, 0, c.stream>>>(static_cast<const __nv_bfloat16*>(W), ws, (int)D, p.h, p.r, ks_z, ks, chunks,
-                                                 static_cast<uint4*>(wimg));
+  const cudaError_t e = launch_chained<tc_pack_w_kernel>(dim3((unsigned)pgrid), 256, 0, c.stream, static_cast<const __nv_bfloat16*>(W),
+                                                         ws, (int)D, p.h, p.r, ks_z, ks, chunks, static_cast<uint4*>(wimg),
+                                                         first ? 1 : 0);
   note_launches(1);
-  return cudaGetLastError() == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
+  return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }
 
-// y = [act(z) | delta] * W^T; `delta` is [N][readout_delta_pitch()] bf16 with zero pad columns, `wimg`
+// y = [act(z) | delta] * W^T; `delta` is [N][readout_delta_pitch()] bf16 (its map ends at column r: what lies behind reads as
+// zeros), `wimg`
 // has readout_image_bytes().
 int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, int64_t D, void* y, int64_t ys, void* wimg) {
   const skv_problem& p = c.p;
@@ -379,7 +388,7 @@ int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, in
   P.skip_copy = debug_skip_copy() == 2;
   CUtensorMap map_z, map_d;
   if (!make_map(&map_z, z, (uint64_t)p.N, (uint64_t)p.h, (uint64_t)zs, f.mt) ||
-      !make_map(&map_d, delta, (uint64_t)p.N, (uint64_t)readout_delta_pitch(p), (uint64_t)readout_delta_pitch(p), f.mt))
+      !make_map(&map_d, delta, (uint64_t)p.N, (uint64_t)p.r, (uint64_t)readout_delta_pitch(p), f.mt))
     return SKV_ERR_LAUNCH;
   const size_t smem = (size_t)ro_stages(f.mt) * (ro_a_bytes(f.mt) + kRoBBytes) + 1024 + 256;
   const int64_t items = P.tiles * P.slices;
