@@ -56,12 +56,22 @@ struct RoParams {
   int ks;                        // all stages: ks_z + ceil(r / 32)
   int n_tiles;                   // ceil(D / 256)
   int64_t tiles;                 // m_tiles * n_tiles
-  int slices, ks_per;            // K slices per tile and stages per slice
-  float* partial;                // [slices][N][D] when there is more than one slice
+  int64_t whole;                 // the first tiles are worked on in one piece, the others in K slices
+  int slices, ks_per;            // of each of the others, and stages per slice
+  float* partial;                // [slices][tiles - whole][128 * MT][256]
   int32_t* status;
   long long wait_cycles;
   int skip_copy;                 // test hook: the loader leaves out its first stage
 };
+
+// What a CTA works on at a time: a whole tile, or a K slice of one.
+struct RoItem { int64_t tile; int slice, s_beg, s_end; };      // slice < 0: whole
+__device__ __forceinline__ RoItem ro_item(const RoParams& P, int64_t t) {
+  if (t < P.whole) return {t, -1, 0, P.ks};
+  const int64_t rest = P.tiles - P.whole, i = t - P.whole;
+  const int slice = (int)(i / rest);
+  return {P.whole + i % rest, slice, slice * P.ks_per, min(P.ks, (slice + 1) * P.ks_per)};
+}
 
 // W[D][ws] (the layout of torch.nn.Linear.weight, columns [0,h) for act(z) and [h,h+r) for delta) ->
 // per (output tile, stage) a 256 x kRoK K-major tile of 8 x 16-byte core matrices, [k core][n core][8 rows],
@@ -131,7 +141,7 @@ __global__ void __launch_bounds__(kRoThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int64_t step = gridDim.x, items = P.tiles * P.slices;     // item = (K slice, tile)
+  const int64_t step = gridDim.x, items = P.whole + (P.tiles - P.whole) * P.slices;
   pdl_wait();
   pdl_launch();
 
@@ -140,10 +150,10 @@ __global__ void __launch_bounds__(kRoThreads, 1)
     uint32_t it = 0, ti = 0;
     bool drain = false;
     for (int64_t t = blockIdx.x; t < items && !drain; t += step, ++ti) {
-      const int64_t tile = t % P.tiles;
-      const int slice = (int)(t / P.tiles), s_beg = slice * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
+      const RoItem item = ro_item(P, t);
+      const int64_t tile = item.tile;
       if (RELU) {
-        for (int s = s_beg; s < s_end && !drain; ++s, ++it) {
+        for (int s = item.s_beg; s < item.s_end && !drain; ++s, ++it) {
           const uint32_t st = it % kRoStages;
           if (mbar_wait(full + st, (it / kRoStages) & 1u, wc)) { drain = true; break; }
           if (s < P.ks_z) {
@@ -175,6 +185,9 @@ __global__ void __launch_bounds__(kRoThreads, 1)
       const int n0 = (int)(tile % P.n_tiles) * 256 + col0;
       const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (MT == 2 ? (uint32_t)(warp >> 2) * 256u : ab * 256u + (uint32_t)col0);
       const int64_t nn = n < P.N ? n : 0;
+      float* part = P.partial;
+      if (item.slice >= 0)
+        part += (((size_t)item.slice * (P.tiles - P.whole) + (tile - P.whole)) * (128 * MT) + (MT == 2 ? warp * 32 : (warp & 3) * 32) + lane) * 256 + col0;
 #pragma unroll 1
       for (int c = 0; c < 4 * MT; ++c) {
         float v[32];
@@ -185,8 +198,8 @@ __global__ void __launch_bounds__(kRoThreads, 1)
           for (int q = 0; q < 4; ++q) {
             const int col = n0 + c * 32 + q * 8;
             if (col >= P.D) continue;
-            if (P.slices > 1) {
-              float4* o = reinterpret_cast<float4*>(P.partial + ((size_t)slice * P.N + nn) * P.D + col);
+            if (item.slice >= 0) {
+              float4* o = reinterpret_cast<float4*>(part + c * 32 + q * 8);
               o[0] = make_float4(v[q * 8], v[q * 8 + 1], v[q * 8 + 2], v[q * 8 + 3]);
               o[1] = make_float4(v[q * 8 + 4], v[q * 8 + 5], v[q * 8 + 6], v[q * 8 + 7]);
             } else {
@@ -216,7 +229,8 @@ __global__ void __launch_bounds__(kRoThreads, 1)
         if (ti >= NB) drain = mbar_wait(acc_empty + ab, (ti / NB - 1u) & 1u, wc);
         if (drain) break;
         tc_fence_after();
-        const int s_beg = (int)(t / P.tiles) * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
+        const RoItem item = ro_item(P, t);
+        const int s_beg = item.s_beg, s_end = item.s_end;
         const uint32_t d_addr = tmem_base + (MT == 1 ? ab * 256u : 0u);
         for (int s = s_beg; s < s_end; ++s, ++it) {
           const uint32_t st = it % kRoStages, ph = (it / kRoStages) & 1u;
@@ -247,10 +261,10 @@ __global__ void __launch_bounds__(kRoThreads, 1)
       uint32_t it = 0;
       bool stop = false;
       for (int64_t t = blockIdx.x; t < items && !stop; t += step) {
-        const int64_t tile = t % P.tiles;
-        const uint8_t* src = P.wimg + (size_t)(tile % P.n_tiles) * P.ks * kRoBBytes;
-        const int m0 = (int)((tile / P.n_tiles) * (128 * MT));
-        const int s_beg = (int)(t / P.tiles) * P.ks_per, s_end = min(P.ks, s_beg + P.ks_per);
+        const RoItem item = ro_item(P, t);
+        const uint8_t* src = P.wimg + (size_t)(item.tile % P.n_tiles) * P.ks * kRoBBytes;
+        const int m0 = (int)((item.tile / P.n_tiles) * (128 * MT));
+        const int s_beg = item.s_beg, s_end = item.s_end;
         for (int s = s_beg; s < s_end; ++s, ++it) {
           const uint32_t st = it % kRoStages;
           if (it == 0 && P.skip_copy) continue;      // test hook: nothing ever completes full[0]
@@ -281,48 +295,58 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
   return make_map_2d(m, base, rows, cols, pitch, kRoK, 128 * mt, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-// y = bf16 of the sum of the K slices' partials, in order; four outputs per thread.
-__global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partial, int slices, int64_t N, int D,
-                                                             __nv_bfloat16* y, int64_t ys) {
+// y = bf16 of the sum of the K slices' partials, in order, for the tiles that were sliced; four outputs per thread.
+__global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partial, int slices, int64_t whole, int64_t rest, int rows,
+                                                             int n_tiles, int64_t N, int D, __nv_bfloat16* y, int64_t ys) {
   pdl_wait();
   pdl_launch();
-  const int q4 = D / 4;
-  const int64_t total = N * q4;
+  const int64_t total = rest * rows * 64;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = i / (rows * 64), tile = whole + b;
+    const int e = (int)(i - b * (rows * 64));
+    const int64_t n = tile / n_tiles * rows + e / 64;
+    const int col = (int)(tile % n_tiles) * 256 + e % 64 * 4;
+    if (n >= N || col >= D) continue;
     const float4* src = reinterpret_cast<const float4*>(partial) + i;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
+#pragma unroll 8
     for (int k = 0; k < slices; ++k) {
       const float4 v = src[(size_t)k * total];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    const int64_t n = i / q4;
-    *reinterpret_cast<uint2*>(y + n * ys + (i - n * q4) * 4) = make_uint2(pack_bf2(s.x, s.y), pack_bf2(s.z, s.w));
+    *reinterpret_cast<uint2*>(y + n * ys + col) = make_uint2(pack_bf2(s.x, s.y), pack_bf2(s.z, s.w));
   }
 }
 
-// Tile height and K slices.  Microseconds: a stage of 256 tokens costs 0.91 with ReLU^2 (0.70 without), one of 128 tokens
-// more than half of that (it reads as much of W); an item's fill and epilogue; partials through L2.  256 tokens give the
-// best rate, 128 fill a last wave better (8192 x 5120 -> 1280: 160 tiles of 256 on 148 SMs took two rounds), and slices
-// spread few tokens over the chip.
-struct RoPlan { int mt, slices, ks_per; };
+// Tile height, how many tiles are worked on whole, and K slices of the others.  Microseconds: a stage of 256 tokens costs 0.91 with
+// ReLU^2 (0.70 without), one of 128 tokens more than half of that (it reads as much of W); an item's fill and epilogue; partials
+// through L2.  256 tokens give the best rate; whole rounds of tiles need no partials; slices spread a last round that
+// is not full, or few tokens, over the chip.  8192 x 5120 -> 1280 (320 tiles of 128 tokens on 148 SMs): in three rounds 127 us,
+// in two and a sixth 105.
+struct RoPlan { int mt, slices, ks_per; int64_t whole; };
 RoPlan readout_plan(const skv_problem& p, int64_t D) {
   const int ks = (p.h + kRoK - 1) / kRoK + (p.r + kRoK - 1) / kRoK;
   const bool relu = p.activation == SKV_ACT_RELU_SQ;
-  const double N = (double)(p.N > 0 ? p.N : 1);
-  RoPlan best{2, 1, ks};
+  RoPlan best{2, 1, ks, 0};
   double best_t = 0.0;
   for (int mt = 2; mt >= 1; --mt) {
-    const int64_t tiles = ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256);
-    const double stage = mt == 2 ? (relu ? 0.91 : 0.70) : (relu ? 0.50 : 0.40);
-    int last = 0;
-    for (int s = 1; s <= 16 && s <= (ks + 3) / 4; ++s) {
-      const int per = (ks + s - 1) / s, slices = (ks + per - 1) / per;
-      if (slices == last) continue;
-      last = slices;
-      const double t = (double)((tiles * slices + kPlanSMs - 1) / kPlanSMs) * (per * stage + 3.0 * mt) +
-                       (slices > 1 ? 4.0 + slices * N * (double)D * 8.0 / 4.0e6 : 0.0);
-      if (best_t == 0.0 || t < best_t) { best_t = t; best = {mt, slices, per}; }
+    const int64_t tiles = ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256), rounds = tiles / kPlanSMs;
+    const double stage = mt == 2 ? (relu ? 0.91 : 0.70) : (relu ? 0.50 : 0.40), fix = 3.0 * mt;
+    auto take = [&](double t, int slices, int per, int64_t whole) {
+      if (best_t == 0.0 || t < best_t) { best_t = t; best = {mt, slices, per, whole}; }
+    };
+    take((double)((tiles + kPlanSMs - 1) / kPlanSMs) * (ks * stage + fix), 1, ks, tiles);
+    for (int64_t full = rounds; full >= 0 && full >= rounds - 1; --full) {
+      const int64_t whole = full * kPlanSMs, rest = tiles - whole;
+      int last = 1;
+      for (int s = 2; s <= 16 && s <= (ks + 3) / 4 && rest > 0; ++s) {
+        const int per = (ks + s - 1) / s, slices = (ks + per - 1) / per;
+        if (slices == last) continue;
+        last = slices;
+        take(full * (ks * stage + fix) + (double)((rest * slices + kPlanSMs - 1) / kPlanSMs) * (per * stage + fix) + 4.0 +
+                 (double)slices * rest * mt * 128 * 256 * 8.0 / 4.0e6,
+             slices, per, whole);
+      }
     }
   }
   return best;
@@ -340,10 +364,14 @@ bool readout_eligible(const skv_problem& p, int64_t D) {
          p.r % 8 == 0 && D >= 8 && D % 8 == 0 && D <= (1 << 24);
 }
 
+int64_t readout_tiles(const skv_problem& p, int64_t D, int mt) {
+  return ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256);
+}
+
 // Image of W, then the K slices' partials.
 size_t readout_image_bytes(const skv_problem& p, int64_t D) {
   const RoPlan f = readout_plan(p, D);
-  return wimg_bytes(p, D) + (f.slices > 1 ? (size_t)f.slices * (p.N > 0 ? p.N : 1) * D * sizeof(float) : 0);
+  return wimg_bytes(p, D) + (size_t)(f.slices > 1 ? f.slices * (readout_tiles(p, D, f.mt) - f.whole) : 0) * f.mt * 128 * 256 * sizeof(float);
 }
 
 // Row pitch (elements) of the delta buffer the GEMM reads: whole stages of kRoK columns.
@@ -379,7 +407,8 @@ int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, in
   P.ks_z = (int)((p.h + kRoK - 1) / kRoK);
   P.ks = P.ks_z + (int)((p.r + kRoK - 1) / kRoK);
   P.n_tiles = (int)((D + 255) / 256);
-  P.tiles = ((p.N + 128 * f.mt - 1) / (128 * f.mt)) * P.n_tiles;
+  P.tiles = readout_tiles(p, D, f.mt);
+  P.whole = f.whole;
   P.slices = f.slices;
   P.ks_per = f.ks_per;
   P.partial = reinterpret_cast<float*>(static_cast<uint8_t*>(wimg) + wimg_bytes(p, D));
@@ -391,7 +420,7 @@ int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, in
       !make_map(&map_d, delta, (uint64_t)p.N, (uint64_t)p.r, (uint64_t)readout_delta_pitch(p), f.mt))
     return SKV_ERR_LAUNCH;
   const size_t smem = (size_t)ro_stages(f.mt) * (ro_a_bytes(f.mt) + kRoBBytes) + 1024 + 256;
-  const int64_t items = P.tiles * P.slices;
+  const int64_t items = P.whole + (P.tiles - P.whole) * P.slices;
   const dim3 grid((unsigned)(items < c.num_sms ? items : c.num_sms));
   const bool relu = p.activation == SKV_ACT_RELU_SQ;
   const cudaError_t err =
@@ -402,10 +431,11 @@ int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, in
   note_launches(1);
   if (err != cudaSuccess) { cudaGetLastError(); return SKV_ERR_LAUNCH; }
   if (P.slices > 1) {
-    const int64_t blocks = (p.N * (D / 4) + 255) / 256;
+    const int rows = 128 * f.mt;
+    const int64_t rest = P.tiles - P.whole, blocks = (rest * rows * 64 + 255) / 256;
     const dim3 sgrid((unsigned)(blocks < kPlanSMs * 16 ? blocks : kPlanSMs * 16));
-    if (launch_chained<tc_readout_sum_kernel>(sgrid, 256, 0, c.stream, (const float*)P.partial, P.slices, P.N, P.D, P.y,
-                                              P.ys) != cudaSuccess) {
+    if (launch_chained<tc_readout_sum_kernel>(sgrid, 256, 0, c.stream, (const float*)P.partial, P.slices, P.whole, rest, rows, P.n_tiles,
+                                              P.N, P.D, P.y, P.ys) != cudaSuccess) {
       cudaGetLastError();
       return SKV_ERR_LAUNCH;
     }
