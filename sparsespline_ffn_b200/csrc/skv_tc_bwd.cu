@@ -320,13 +320,17 @@ int backward(const LaunchCtx& c, const void* z, int64_t zs, const void* C, const
       parts = dc_parts(b.dc, p.L);
     }
   }
-  if (dz != user_dz)
+  // padded rows of dz: brought to their place by the last kernel where there is one that knows how, else by one of its own
+  const bool with_reduce = dz != user_dz && want_dC && split;
+  if (dz != user_dz && !with_reduce)
     if (int e = launch_unpad(dz, dzs, user_dz, user_dzs, p.N, p.h, p.dz_f32 != 0, c.stream)) return e;
   Contain K{};
   if (split) {
     K.z = Z.z; K.zs = zs; K.C = Q.C; K.g = Q.g; K.gds = gds; K.N = p.N;
     K.h = p.h; K.L = p.L; K.r = p.r; K.grid = c.g;
-    K.dz = user_dz; K.dzs = user_dzs; K.coef = Z.coef; K.dz_f32 = p.dz_f32 != 0;
+    K.dz = user_dz; K.dzs = user_dzs;
+    if (with_reduce) { K.dz_rows = dz; K.dz_rows_stride = dzs; }
+    K.coef = Z.coef; K.dz_f32 = p.dz_f32 != 0;
   }
   if (want_dC)
     return launch_dc_reduce(part, parts, (int64_t)p.h * p.L, (int64_t)hp * p.L, p.r, rp, p.lambda_scale, hdr, dC,

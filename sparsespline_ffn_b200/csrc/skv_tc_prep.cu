@@ -315,12 +315,12 @@ __device__ __noinline__ void contain_delta(const Contain& K, int rp, float lambd
 
 // dC: the same for infinities and NaN in g_delta.  A block lists the tokens that have any, 256 tokens at a time, and its
 // threads, one per four columns of a knot row, walk the list.
-__device__ __noinline__ void contain_dC(const Contain& K, int rp, float lambda, float* dC, __nv_bfloat16* dC_cast) {
+__device__ __noinline__ void contain_dC(const Contain& K, int rp, float lambda, float* dC, __nv_bfloat16* dC_cast, int blocks) {
   __shared__ int list[256];
   __shared__ int count;
   const int q4 = rp / 4;
   const int64_t total = (int64_t)K.h * K.L * q4;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total; base += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total; base += (int64_t)blocks * blockDim.x) {
     const int64_t i = base + threadIdx.x;
     const int64_t row = i / q4;
     const int c = (int)(i - row * q4) * 4, j = (int)(row / K.L), l = (int)(row - (int64_t)j * K.L);
@@ -362,12 +362,13 @@ __device__ __noinline__ void contain_dC(const Contain& K, int rp, float lambda, 
 }
 
 // dz: the channels of a pair in which g_delta or a touched row of C is infinite or NaN.  A block takes 256 tokens (one per
-// thread) x 32 keys and first marks the knot rows of its keys and the tokens that have any.
-__device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c) {
+// thread) x 32 keys and first marks the knot rows of its keys and the tokens that have any.  Where dz is still in padded rows,
+// all of it is brought to its place.
+__device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c, int64_t first, int64_t step) {
   __shared__ unsigned long long rows[32];
   const int key_groups = (K.h + 31) / 32;
   const int64_t tiles = (K.N + 255) / 256 * key_groups;
-  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+  for (int64_t t = first; t < tiles; t += step) {
     const int64_t n = t / key_groups * 256 + threadIdx.x;
     const int j0 = (int)(t % key_groups) * 32, keys = min(32, K.h - j0);
     __syncthreads();
@@ -388,11 +389,11 @@ __device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c
     for (int q = 0; q < keys && n < K.N; ++q) {
       const Knot k = knot_of(__bfloat162float(K.z[n * K.zs + j0 + q]), K.grid);
       const bool two = K.grid.order != 1;
-      if (!k.clamp_active || !(token || ((rows[q] >> k.bin) & (two ? 7ull : 3ull)))) continue;
       const __nv_bfloat16* src = K.C + ((size_t)(j0 + q) * K.L + k.bin) * K.r;
       float s = 0.0f;
       bool any = false;
-      for (int c = 0; c < K.r; ++c) {
+      const bool touched = k.clamp_active && (token || ((rows[q] >> k.bin) & (two ? 7ull : 3ull)));
+      for (int c = 0; touched && c < K.r; ++c) {
         const float gv = __bfloat162float(g[c]), c0 = __bfloat162float(src[c]), c1 = __bfloat162float(src[K.r + c]);
         const float c2 = two ? __bfloat162float(src[2 * K.r + c]) : 0.0f;
         if (!is_bad(gv) && !is_bad(c0) && !is_bad(c1) && !is_bad(c2)) continue;
@@ -401,11 +402,16 @@ __device__ __noinline__ void contain_dz(const Contain& K, bool bad_g, bool bad_c
         s = fmaf(gv, d, s);
         any = true;
       }
-      if (!any) continue;
-      if (K.dz_f32) static_cast<float*>(K.dz)[n * K.dzs + j0 + q] += K.coef * s;
-      else {
-        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(K.dz) + n * K.dzs + j0 + q;
-        *o = __float2bfloat16_rn(__bfloat162float(*o) + K.coef * s);
+      if (!any && !K.dz_rows) continue;
+      const int64_t at = n * K.dzs + j0 + q, from = K.dz_rows ? n * K.dz_rows_stride + j0 + q : at;
+      if (K.dz_f32) {
+        float v = static_cast<const float*>(K.dz_rows ? K.dz_rows : K.dz)[from];
+        if (any) v += K.coef * s;
+        static_cast<float*>(K.dz)[at] = v;
+      } else {
+        __nv_bfloat16 v = static_cast<const __nv_bfloat16*>(K.dz_rows ? K.dz_rows : K.dz)[from];
+        if (any) v = __float2bfloat16_rn(__bfloat162float(v) + K.coef * s);
+        static_cast<__nv_bfloat16*>(K.dz)[at] = v;
       }
     }
   }
@@ -470,20 +476,43 @@ __global__ void __launch_bounds__(256) tc_finalize_kernel(const float* partial, 
   }
 }
 
+// Rows of h elements from padded rows, a row per block at a time.
+template <typename T>
+__device__ __forceinline__ void unpad_rows(const void* src, int64_t ss, void* dst, int64_t ds, int64_t N, int h, int64_t first, int64_t step) {
+  for (int64_t n = first; n < N; n += step) {
+    const T* a = static_cast<const T*>(src) + n * ss;
+    T* b = static_cast<T*>(dst) + n * ds;
+#pragma unroll 4
+    for (int j = threadIdx.x; j < h; j += blockDim.x) b[j] = a[j];
+  }
+}
+
+// The first `blocks` blocks add; those behind them bring dz from padded rows to its place (a launch of its own for that cost
+// 5 us of a step of 2000 x 1001 and the host two).  Where infinities or NaN were found contain_dz does both.
 template <bool CONTAIN>
 __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, const DcParts parts, int64_t rows,
                                                            int64_t rows_padded, int r, int rp, float lambda,
                                                            const uint32_t* hdr, float* dC,
-                                                           __nv_bfloat16* dC_cast, const __grid_constant__ Contain K) {
+                                                           __nv_bfloat16* dC_cast, const __grid_constant__ Contain K, int blocks) {
   pdl_wait();
   pdl_launch();
+  if constexpr (CONTAIN) {
+    if ((int)blockIdx.x >= blocks) {
+      const bool bad_g = hdr[kBadG] != 0u, bad_c = hdr[kBadC] != 0u;
+      const int64_t first = blockIdx.x - blocks, step = gridDim.x - blocks;
+      if (bad_g || bad_c) contain_dz(K, bad_g, bad_c, first, step);
+      else if (K.dz_f32) unpad_rows<float>(K.dz_rows, K.dz_rows_stride, K.dz, K.dzs, K.N, K.h, first, step);
+      else unpad_rows<__nv_bfloat16>(K.dz_rows, K.dz_rows_stride, K.dz, K.dzs, K.N, K.h, first, step);
+      return;
+    }
+  }
   float gscale, ginv;
   pow2_scales(hdr[kAmaxG], gscale, ginv);
   const float f = lambda * ginv;
   const int q4 = rp / 4;
   const int64_t total = rows * q4, pitch = rows_padded * q4;
   const bool vec = r == rp && ((reinterpret_cast<uintptr_t>(dC) | reinterpret_cast<uintptr_t>(dC_cast)) & 15) == 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)blocks * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(part) + i;
     const int splits = parts.count ? parts.count : parts.of((uint32_t)(i / q4) / parts.slab_rows);
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -510,10 +539,10 @@ __global__ void __launch_bounds__(256) tc_dc_reduce_kernel(const float* part, co
   }
   if constexpr (CONTAIN) {
     const bool bad_g = hdr[kBadG] != 0u;
-    if (bad_g) contain_dC(K, rp, lambda, dC, dC_cast);      // the elements of a thread are those it has written above
-    if (K.dz) {
+    if (bad_g) contain_dC(K, rp, lambda, dC, dC_cast, blocks);      // the elements of a thread are those it has written above
+    if (K.dz && !K.dz_rows) {
       const bool bad_c = hdr[kBadC] != 0u;
-      if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
+      if (bad_g || bad_c) contain_dz(K, bad_g, bad_c, blockIdx.x, blocks);
     }
   }
 }
@@ -522,7 +551,7 @@ __global__ void __launch_bounds__(256) tc_dz_contain_kernel(const uint32_t* hdr,
   pdl_wait();
   pdl_launch();
   const bool bad_g = hdr[kBadG] != 0u, bad_c = hdr[kBadC] != 0u;
-  if (bad_g || bad_c) contain_dz(K, bad_g, bad_c);
+  if (bad_g || bad_c) contain_dz(K, bad_g, bad_c, blockIdx.x, gridDim.x);
 }
 
 template <typename T>
@@ -601,12 +630,13 @@ int launch_finalize(const float* partial, int splits, int64_t N, int r, int rp, 
 
 int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
                      const uint32_t* hdr, float* dC, void* dC_cast, const Contain& K, cudaStream_t stream) {
-  const dim3 grid((unsigned)blocks_for(rows * (rp / 4), 1, kPlanSMs * 16));
+  const int blocks = blocks_for(rows * (rp / 4), 1, kPlanSMs * 16);
+  const dim3 grid((unsigned)(blocks + (K.z && K.dz_rows ? (K.N < kPlanSMs * 8 ? (int)K.N : kPlanSMs * 8) : 0)));
   const cudaError_t e =
       K.z ? launch_chained<tc_dc_reduce_kernel<true>>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda, hdr,
-                                                      dC, static_cast<__nv_bfloat16*>(dC_cast), K)
+                                                      dC, static_cast<__nv_bfloat16*>(dC_cast), K, blocks)
           : launch_chained<tc_dc_reduce_kernel<false>>(grid, 256, 0, stream, part, parts, rows, rows_padded, r, rp, lambda,
-                                                       hdr, dC, static_cast<__nv_bfloat16*>(dC_cast), K);
+                                                       hdr, dC, static_cast<__nv_bfloat16*>(dC_cast), K, blocks);
   note_launches(1);
   return e == cudaSuccess ? SKV_OK : SKV_ERR_LAUNCH;
 }

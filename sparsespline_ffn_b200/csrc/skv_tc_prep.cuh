@@ -60,6 +60,8 @@ struct Contain {
   GridParams grid;
   void* dz;                  // null: no dz wanted
   int64_t dzs;
+  const void* dz_rows;       // padded rows that dz is in; null: it is in its place
+  int64_t dz_rows_stride;
   float coef;                // lambda * scale, of dz
   bool dz_f32;
 };
@@ -117,7 +119,8 @@ struct DcParts {
   }
 };
 
-// dC = lambda * 2^-k * sum over the partials part[i][row][c] for `rows` knot rows.
+// dC = lambda * 2^-k * sum over the partials part[i][row][c] for `rows` knot rows.  Where K has dz in padded rows, its blocks
+// bring it to its place too.
 int launch_dc_reduce(const float* part, const DcParts& parts, int64_t rows, int64_t rows_padded, int r, int rp, float lambda,
                      const uint32_t* hdr, float* dC, void* dC_cast, const Contain& K, cudaStream_t stream);
 
