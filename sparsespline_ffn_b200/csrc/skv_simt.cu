@@ -362,30 +362,43 @@ __global__ void __launch_bounds__(kSmallWarps * kWarp, 1) simt_forward_small_ker
   if (cs > 1) cluster_wait();
 }
 
-// Sum of the key splits' partial residuals in a fixed order, lambda, cast.  A CTA takes 32 elements;
-// its eight warps each add every eighth split, so that a sum over many splits is not one serial chain.
-template <typename TD>
-__global__ void __launch_bounds__(256) simt_finalize_kernel(const float* partial, int splits, int64_t N,
-                                                            int r, float lambda, TD* out, int64_t ds) {
-  __shared__ float part[8][kWarp];
+// Sum of the key splits' partial residuals in a fixed order, lambda, cast.  A CTA takes 32 times Q neighbouring elements;
+// its eight warps each add every eighth split, so that a sum over many splits is not one serial chain.  Q = 4 where r allows it
+// (4096 x 32 elements, 18 splits: 8.3 us element by element; a step of 4096 x 1024 takes 2.5 us less with fours).
+template <typename TD, int Q>
+__global__ void __launch_bounds__(256) simt_finalize_kernel(const float* partial, int splits, int64_t N, int r, float lambda, TD* out,
+                                                            int64_t ds) {
+  __shared__ float part[8][kWarp][Q];
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const int64_t total = N * r;
-  for (int64_t b = (int64_t)blockIdx.x * kWarp; b < total; b += (int64_t)gridDim.x * kWarp) {
-    const int64_t i = b + lane;
-    float s = 0.0f;
+  for (int64_t b = (int64_t)blockIdx.x * (kWarp * Q); b < total; b += (int64_t)gridDim.x * (kWarp * Q)) {
+    const int64_t i = b + lane * Q;
+    float s[Q] = {};
     if (i < total) {
 #pragma unroll 4
-      for (int k = warp; k < splits; k += 8) s += partial[(size_t)k * total + i];
+      for (int k = warp; k < splits; k += 8) {
+        const float* src = partial + (size_t)k * total + i;
+        if constexpr (Q == 4) {
+          const float4 v = *reinterpret_cast<const float4*>(src);
+          s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+        } else {
+          s[0] += *src;
+        }
+      }
     }
     __syncthreads();
-    part[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && i < total) {
 #pragma unroll
-      for (int w = 1; w < 8; ++w) s += part[w][lane];
-      st_f32<TD>(out + (i / r) * ds + (i % r), lambda * s);
+    for (int q = 0; q < Q; ++q) part[warp][lane][q] = s[q];
+    __syncthreads();
+    // element `warp` of a lane's (of its only one the first warp takes care)
+    if (warp < Q && i < total) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) sum += part[w][lane][warp];
+      const int64_t e = i + warp;
+      st_f32<TD>(out + (e / r) * ds + (e % r), lambda * sum);
     }
   }
 }
@@ -1150,9 +1163,13 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
   if (e) return e;
   note_launches(1);
   if (f.splits > 1) {
-    const int64_t blocks = cdiv64(p.N * p.r, kWarp);
-    e = launch<simt_finalize_kernel<TD>>(dim3((unsigned)(blocks < 4096 ? blocks : 4096)), 8, 0, c.stream, (const float*)a.partial,
-                                         f.splits, p.N, p.r, p.lambda_scale, static_cast<TD*>(delta_out), ds);
+    const bool fours = p.r % 4 == 0 && reinterpret_cast<uintptr_t>(a.partial) % 16 == 0;
+    const int64_t blocks = cdiv64(p.N * p.r, fours ? 4 * kWarp : kWarp);
+    const dim3 fgrid((unsigned)(blocks < 4096 ? blocks : 4096));
+    e = fours ? launch<simt_finalize_kernel<TD, 4>>(fgrid, 8, 0, c.stream, (const float*)a.partial, f.splits, p.N, p.r, p.lambda_scale,
+                                                    static_cast<TD*>(delta_out), ds)
+              : launch<simt_finalize_kernel<TD, 1>>(fgrid, 8, 0, c.stream, (const float*)a.partial, f.splits, p.N, p.r, p.lambda_scale,
+                                                    static_cast<TD*>(delta_out), ds);
     note_launches(1);
   }
   return e;
