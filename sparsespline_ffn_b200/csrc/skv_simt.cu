@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, 4) * kWarp, 2) simt_dz_k
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const float2 w = my[sub * kWarp + q0 + q];                          // keys past kc: row 0, result unused
-        float s = 0.0f, s1 = 0.0f;                                          // g times either row
+        float s = 0.0f;
 #pragma unroll
         for (int c = 0; c < CV; ++c) {
           float d[V], e[V];
@@ -549,14 +549,15 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, 4) * kWarp, 2) simt_dz_k
               e[i] = two && col < P.r ? ld_f32<T>(row + 2 * P.r + col) - c1 : 0.0f;
             }
           }
-#pragma unroll
-          for (int i = 0; i < V; ++i) s = fmaf(gd[c][i], d[i], s);
+          // (interpolated before the product: adjacent differences cancel, and the two products' roundings would not)
           if (two) {
 #pragma unroll
-            for (int i = 0; i < V; ++i) s1 = fmaf(gd[c][i], e[i], s1);
+            for (int i = 0; i < V; ++i) d[i] = fmaf(w.x, e[i] - d[i], d[i]);
           }
+#pragma unroll
+          for (int i = 0; i < V; ++i) s = fmaf(gd[c][i], d[i], s);
         }
-        v[q] = two ? fmaf(w.x, s1 - s, s) : s;
+        v[q] = s;
       }
       // afterwards v[0] of lane sl is the sum over the token's lanes of v[sl % Q]
 #pragma unroll
