@@ -102,7 +102,8 @@ __device__ __forceinline__ float4 pair_weights(float zz, const GridParams& g, in
 // slabs whose table rows it copies to shared memory; a warp owns `groups` groups of 32 / LPT tokens and
 // keeps their residuals in registers over all slabs.
 //
-// Bound: shared-memory bandwidth (three rows of r channels per pair, 128 bytes a clock), which is why a
+// Bound: shared-memory bandwidth (three rows of r channels per pair, 128 bytes a clock; 81 % of it at 4096 x 1024, r = 32, float32, 80 us;
+// 58 % and 103 us with half the warps), which is why a
 // bf16 table stays bf16 there.
 // ---------------------------------------------------------------------------------------------
 template <typename T, typename TD, int LPT, int CV>
@@ -411,7 +412,8 @@ __global__ void __launch_bounds__(256) simt_finalize_kernel(const float* partial
 // transpose-reduce turns them into one key's sum per lane; 32 keys' results go through shared memory so
 // that z, g_act and dz are read and written by whole rows of 32 keys.
 //
-// Bound: shared-memory bandwidth, two float32 rows of r channels per pair.
+// Bound: shared-memory latency and bandwidth, two float32 rows of r channels per pair (52 % of it with 27 warps per SM; 4096 x 1024, r = 32:
+// 84 us, 103 with half the warps).
 // ---------------------------------------------------------------------------------------------
 struct DzArgs {
   const void* z;
@@ -596,7 +598,9 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, 4) * kWarp, 2) simt_dz_k
 // interval and adds one finished row to the key's accumulator each time, where adding every token to its rows would
 // read and write three rows of shared memory for each.  Tokens outside the grid have no weight and leave the lists.
 //
-// Bound: instruction issue (about seven warp instructions per pair at r = 32) and one row of g per pair.
+// Bound: latencies and instruction issue (66 % of the slots with 21 warps per SM): at 4096 x 1024, r = 32, the products of the rows
+// take 49 us of 104, the walk over the intervals and the finished rows 28, staging and the sort 27.  With eight warps per CTA, two
+// CTAs per SM, no request ahead and a full reduction per finished row it took 173.
 // ---------------------------------------------------------------------------------------------
 struct DcArgs {
   const void* z;
@@ -1250,9 +1254,9 @@ size_t simt_scratch_bytes(const skv_problem& p, int op) {
   return f.splits > 1 ? (size_t)f.splits * (p.N > 0 ? p.N : 1) * p.r * sizeof(float) : 0;
 }
 
-// Tokens up to which the forward reads table rows in place.  That takes about 8 us and one for every 1.05 M of N h r; the
-// tensor-core chain 15 us and one for every 0.26 M table elements it has to scan and pack.  128 tokens at h = 5120, r = 32:
-// 29 against 31 us; 65 tokens 18 against 29; 256 tokens 45 against 31.
+// Tokens up to which the forward reads table rows in place.  On the GPU, in place against the tensor-core chain: h = 5120, r = 32: 132 tokens
+// 17.2 and 18.1 us, 160 tokens 26.3 and 17.9; h = 2560: 177 tokens, 200 tokens 14.9 and 15.6; h = 1024: 250 tokens 8.3 and 12.3, 300
+// tokens 13.8 and 12.4; h = 5120, r = 128: 100 tokens 48.9 and 48.8.
 int64_t small_forward_tokens(const skv_problem& p) {
   if (p.dtype != SKV_BF16) return 64;
   const int64_t n = 4 * (int64_t)p.L + 7300000 / ((int64_t)p.h * p.r);
