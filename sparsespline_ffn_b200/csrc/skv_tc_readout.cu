@@ -319,8 +319,8 @@ __global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partia
 }
 
 // Tile height, how many tiles are worked on whole, and K slices of the others.  Microseconds: a stage of 256 tokens costs 0.91 with
-// ReLU^2 (0.70 without), one of 128 tokens more than half of that (it reads as much of W); an item's fill and epilogue; partials
-// through L2.  256 tokens give the best rate; whole rounds of tiles need no partials; slices spread a last round that
+// ReLU^2 (0.70 without), one of 128 tokens more than half of that (it reads as much of W); an item's fill and epilogue; a launch more and
+// partials through L2.  256 tokens give the best rate; whole rounds of tiles need no partials; slices spread a last round that
 // is not full, or few tokens, over the chip.  8192 x 5120 -> 1280 (320 tiles of 128 tokens on 148 SMs): in three rounds 127 us,
 // in two and a sixth 105.
 struct RoPlan { int mt, slices, ks_per; int64_t whole; };
@@ -331,7 +331,7 @@ RoPlan readout_plan(const skv_problem& p, int64_t D) {
   double best_t = 0.0;
   for (int mt = 2; mt >= 1; --mt) {
     const int64_t tiles = ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256), rounds = tiles / kPlanSMs;
-    const double stage = mt == 2 ? (relu ? 0.91 : 0.70) : (relu ? 0.50 : 0.40), fix = 3.0 * mt;
+    const double stage = mt == 2 ? (relu ? 0.91 : 0.70) : (relu ? 0.50 : 0.37), fix = 3.0 * mt;
     auto take = [&](double t, int slices, int per, int64_t whole) {
       if (best_t == 0.0 || t < best_t) { best_t = t; best = {mt, slices, per, whole}; }
     };
@@ -343,7 +343,7 @@ RoPlan readout_plan(const skv_problem& p, int64_t D) {
         const int per = (ks + s - 1) / s, slices = (ks + per - 1) / per;
         if (slices == last) continue;
         last = slices;
-        take(full * (ks * stage + fix) + (double)((rest * slices + kPlanSMs - 1) / kPlanSMs) * (per * stage + fix) + 4.0 +
+        take(full * (ks * stage + fix) + (double)((rest * slices + kPlanSMs - 1) / kPlanSMs) * (per * stage + fix) + 8.0 +
                  (double)slices * rest * mt * 128 * 256 * 8.0 / 4.0e6,
              slices, per, whole);
       }
