@@ -88,10 +88,8 @@ __device__ __forceinline__ float act_grad(float z, int act) {
 }
 
 template <typename T> __device__ __forceinline__ float ld_f32(const T* p);
-template <> __device__ __forceinline__ float ld_f32<float>(const float* p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ld_f32<__nv_bfloat16>(const __nv_bfloat16* p) {
-  return __bfloat162float(__ldg(p));
-}
+template <> __device__ __forceinline__ float ld_f32<float>(const float* p) { return *p; }
+template <> __device__ __forceinline__ float ld_f32<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 template <typename T> __device__ __forceinline__ void st_f32(T* p, float v);
 template <> __device__ __forceinline__ void st_f32<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void st_f32<__nv_bfloat16>(__nv_bfloat16* p, float v) {

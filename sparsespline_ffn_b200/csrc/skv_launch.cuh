@@ -16,25 +16,26 @@ namespace skv {
 // Chained to what was there its launch costs nothing: a plain launch leaves 1.5 us between two calls.  The last kernel of a call
 // lets its successor start after its own wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// (What an earlier kernel of the chain wrote is read through plain pointers or ld16, never through const __restrict__
-// pointers or __ldg: the compiler may move such loads above the wait.)
+// (What an earlier kernel may have written, of the chain or of the call in front of it, is read through plain pointers or ld16, never
+// through const __restrict__ pointers, __ldg or ld.global.nc: those are for memory that nothing writes while the kernel is resident, a
+// chained kernel is resident before its wait returns, and the compiler may move such loads above the wait.)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// 16 bytes through the read-only path, not moved across pdl_wait().
+// 16, 8 and 4 bytes, not moved across pdl_wait().
 __device__ __forceinline__ uint4 ld16(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 
 __device__ __forceinline__ uint2 ld8(const void* p) {
   uint2 v;
-  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint32_t ld4(const void* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 

@@ -6,6 +6,9 @@
 // rows of r channels, nothing else.  A row is read with 16-byte loads by LPT neighbouring lanes, so
 // a warp works on 32 / LPT tokens of one key at a time; knot interval and weights of a pair are
 // computed once by one lane and handed to the LPT lanes through shared memory (a 16-byte broadcast).
+//
+// Every kernel is chained to what was on the stream in front of it and may be resident while its inputs are written, so it reads
+// them, behind its wait, through plain pointers (skv_launch.cuh).
 #include "skv_common.cuh"
 #include "skv_launch.cuh"
 
@@ -49,12 +52,12 @@ template <> struct Vec<__nv_bfloat16> {
 // Rows [0, rows) of r elements, contiguous in global memory, into shared rows of `pitch` elements.
 // The pad columns are not written (the caller zeroes the buffer once).
 template <typename T>
-__device__ __forceinline__ void stage_rows(T* dst, const T* __restrict__ src, int rows, int r, int pitch) {
+__device__ __forceinline__ void stage_rows(T* dst, const T* src, int rows, int r, int pitch) {
   if (r == pitch && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
     const int n16 = (int)((size_t)rows * r * sizeof(T) / 16);
 #pragma unroll 8
     for (int i = threadIdx.x; i < n16; i += blockDim.x)
-      reinterpret_cast<uint4*>(dst)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+      reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
   } else {
     // `per` threads copy one row (the largest power of two not above r, at most a warp)
     int per = 32;
@@ -231,12 +234,12 @@ __global__ void __launch_bounds__(staged_warps(LPT, CV, sizeof(T)) * kWarp, 2) s
 // ---------------------------------------------------------------------------------------------
 // 16 bytes of a row at element `col`, as one load or (BYTES 8) two, where rows start on such boundaries; 0: element by element.
 template <typename T, int BYTES>
-__device__ __forceinline__ void load_row(const T* __restrict__ row, int col, int r, float (&f)[Vec<T>::n]) {
+__device__ __forceinline__ void load_row(const T* row, int col, int r, float (&f)[Vec<T>::n]) {
   if constexpr (BYTES == 16) {
-    Vec<T>::cvt(__ldg(reinterpret_cast<const uint4*>(row + col)), f);
+    Vec<T>::cvt(*reinterpret_cast<const uint4*>(row + col), f);
   } else if constexpr (BYTES == 8) {
-    const uint2 a = __ldg(reinterpret_cast<const uint2*>(row + col));
-    const uint2 b = col + Vec<T>::n / 2 < r ? __ldg(reinterpret_cast<const uint2*>(row + col) + 1) : make_uint2(0, 0);
+    const uint2 a = *reinterpret_cast<const uint2*>(row + col);
+    const uint2 b = col + Vec<T>::n / 2 < r ? reinterpret_cast<const uint2*>(row + col)[1] : make_uint2(0, 0);
     Vec<T>::cvt(make_uint4(a.x, a.y, b.x, b.y), f);
   } else {
 #pragma unroll
@@ -627,12 +630,12 @@ constexpr int kDcAhead = 4;                // pieces of four gradients that a th
 template <typename T> struct Quad;
 template <> struct Quad<float> {
   float4 v;
-  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+  __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
   __device__ __forceinline__ float4 get() const { return v; }
 };
 template <> struct Quad<__nv_bfloat16> {
   uint2 v;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = __ldg(reinterpret_cast<const uint2*>(p)); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
   __device__ __forceinline__ float4 get() const {
     return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
                        __uint_as_float(v.y & 0xffff0000u));
