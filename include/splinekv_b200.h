@@ -211,6 +211,11 @@ int skv_debug_set(int what, int64_t value);
  * SKV_ERR_UNSUPPORTED when the problem does not run on the tcgen05 kernels. */
 int skv_debug_dc_plan(const skv_problem *p, int64_t slab, int64_t *out);
 
+/* How the read-out GEMM would cut its work, for tests that want a certain plan; needs no GPU.
+ *   out[4] = { tokens of a tile (256 or 128), tiles, tiles worked on whole, K slices of each of the others (1: there are none) }
+ * SKV_ERR_UNSUPPORTED when the read-out does not take the problem. */
+int skv_debug_readout_plan(const skv_problem *p, int64_t d_out, int64_t *out);
+
 /* Number of kernels this library has launched in this process so far (host-side counter).  No
  * counterpart in the reference; benchmarks use the difference around a timed region to report
  * how many of the library's own kernels ran inside it. */

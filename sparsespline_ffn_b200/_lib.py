@@ -16,7 +16,7 @@ EXPORTS = (
     "skv_abi_version", "skv_error_string", "skv_device_ok", "skv_resolve_impl", "skv_scratch_bytes",
     "skv_feature_forward", "skv_feature_backward", "skv_knot_index", "skv_kernel_launches",
     "skv_feature_forward_noalloc", "skv_debug_set", "skv_readout_scratch_bytes", "skv_feature_readout_forward",
-    "skv_debug_dc_plan", "skv_resolve_impl_op",
+    "skv_debug_dc_plan", "skv_debug_readout_plan", "skv_resolve_impl_op",
 )
 SKV_DEBUG_WAIT_CYCLES, SKV_DEBUG_SKIP_FIRST_COPY, SKV_DEBUG_FUSED_BACKWARD = 0, 1, 2
 SKV_NOALLOC_SCRATCH_BYTES = 16 << 20
@@ -78,6 +78,8 @@ def load() -> ctypes.CDLL:
     lib.skv_debug_set.restype = i32
     lib.skv_debug_dc_plan.argtypes = [pp, i64, ctypes.POINTER(i64)]
     lib.skv_debug_dc_plan.restype = i32
+    lib.skv_debug_readout_plan.argtypes = [pp, i64, ctypes.POINTER(i64)]
+    lib.skv_debug_readout_plan.restype = i32
     lib.skv_readout_scratch_bytes.argtypes = [pp, i64]
     lib.skv_readout_scratch_bytes.restype = ctypes.c_size_t
     lib.skv_feature_readout_forward.argtypes = [pp, vp, i64, vp, vp, i64, i64, vp, i64, vp, ctypes.c_size_t, vp, vp]

@@ -28,6 +28,7 @@ void describe_dc_plan(const skv_problem& p, int64_t slab, int64_t* out);
 bool readout_eligible(const skv_problem& p, int64_t D);
 size_t readout_image_bytes(const skv_problem& p, int64_t D);
 int64_t readout_delta_pitch(const skv_problem& p);
+void describe_readout_plan(const skv_problem& p, int64_t D, int64_t* out);
 int readout_pack(const LaunchCtx& c, const void* W, int64_t ws, int64_t D, void* wimg, bool first);
 int readout(const LaunchCtx& c, const void* z, int64_t zs, const void* delta, int64_t D, void* y, int64_t ys, void* wimg);
 }  // namespace tc
@@ -163,6 +164,14 @@ int skv_debug_dc_plan(const skv_problem* p, int64_t slab, int64_t* out) {
   if (!out) return SKV_ERR_NULL;
   if (resolve(*p, SKV_OP_BACKWARD) != SKV_IMPL_TCGEN05) return SKV_ERR_UNSUPPORTED;
   tc::describe_dc_plan(*p, slab, out);
+  return SKV_OK;
+}
+
+int skv_debug_readout_plan(const skv_problem* p, int64_t d_out, int64_t* out) {
+  if (int e = validate(p)) return e;
+  if (!out) return SKV_ERR_NULL;
+  if (!tc::readout_eligible(*p, d_out)) return SKV_ERR_UNSUPPORTED;
+  tc::describe_readout_plan(*p, d_out, out);
   return SKV_OK;
 }
 

@@ -368,6 +368,14 @@ int64_t readout_tiles(const skv_problem& p, int64_t D, int mt) {
   return ((p.N > 0 ? p.N : 1) + 128 * mt - 1) / (128 * mt) * ((D + 255) / 256);
 }
 
+void describe_readout_plan(const skv_problem& p, int64_t D, int64_t* out) {
+  const RoPlan f = readout_plan(p, D);
+  out[0] = 128 * f.mt;
+  out[1] = readout_tiles(p, D, f.mt);
+  out[2] = f.whole;
+  out[3] = f.slices;
+}
+
 // Image of W, then the K slices' partials.
 size_t readout_image_bytes(const skv_problem& p, int64_t D) {
   const RoPlan f = readout_plan(p, D);
