@@ -1159,12 +1159,15 @@ int forward_t(const LaunchCtx& c, const void* z, int64_t zs, const void* C, void
   const uintptr_t at = reinterpret_cast<uintptr_t>(C);
   const int bytes = p.r % n == 0 && at % 16 == 0 ? 16 : p.r % (n / 2) == 0 && at % 8 == 0 ? 8 : 0;
   int e = SKV_OK;
+  // (32 lanes take 256 bf16 in one piece: two pieces per lane are for float32)
 #define SKV_CALL(LPT_, CV_)                                                                                     \
   {                                                                                                             \
-    if (f.small && bytes == 16) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 16>, f, a, c.stream);    \
-    else if (f.small && bytes == 8) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 8>, f, a, c.stream);  \
-    else if (f.small) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 0>, f, a, c.stream);     \
-    else e = launch<simt_forward_kernel<T, TD, LPT_, CV_>>(grid, f.warps, f.smem, c.stream, a);                 \
+    if constexpr (CV_ == 1 || n == 4) {                                                                         \
+      if (f.small && bytes == 16) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 16>, f, a, c.stream);    \
+      else if (f.small && bytes == 8) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 8>, f, a, c.stream);  \
+      else if (f.small) e = launch_small(simt_forward_small_kernel<T, TD, LPT_, CV_, 0>, f, a, c.stream);     \
+      else e = launch<simt_forward_kernel<T, TD, LPT_, CV_>>(grid, f.warps, f.smem, c.stream, a);                 \
+    }                                                                                                           \
   }
   SKV_LANES(f.lpt, f.cv, SKV_CALL)
 #undef SKV_CALL
