@@ -27,6 +27,9 @@ F32, BF16 = torch.float32, torch.bfloat16
     (190, 27, 200, 22, 2, F32),    # two pieces per lane
     (190, 27, 200, 22, 2, BF16),
     (140, 19, 256, 22, 2, BF16),
+    (600, 37, 136, 22, 2, BF16),   # wide bf16 rows staged (more tokens than are read in place), a ragged last slab
+    (1025, 19, 200, 22, 2, BF16),
+    (577, 45, 256, 21, 1, BF16),
     (90, 3, 256, 700, 2, F32),     # a key's rows and accumulator do not fit shared memory
 ])
 def test_cuda_core_kernels(N, h, r, L, order, dtype):

@@ -1,6 +1,8 @@
 """Infinities and NaN in C and g_delta reach what touches them and nothing else, on the kernels that promise it: the CUDA-core
 family, and the tcgen05 family where it holds operands as pairs of f16 (linear spline, h no multiple of 8, r no multiple
 of 16, more than 49 knot rows).  Against the CPU oracle, which adds up the touched rows alone."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -83,3 +85,22 @@ def test_nonfinite_inputs_and_tokens_outside_the_grid(case):
         got[impl] = f, dz, dC
     for name, a, b in zip(("f", "dz", "dC"), got["tcgen05"], got["simt"]):
         _check(name, a, util.f32(b), torch.bfloat16, 1e-2)
+
+
+# (N, h, r, lanes that add up the splits of an output): more than 16, 32 and 64 key splits
+@pytest.mark.parametrize("N,h,r,lanes", [(320, 640, 32, 2), (319, 2560, 32, 4), (320, 5120, 16, 8)])
+@pytest.mark.parametrize("delta_f32", [False, True])
+def test_nonfinite_code_tables_and_many_key_splits(N, h, r, lanes, delta_f32):
+    z, C, _ = _inputs(N, h, r, 20, 1, "C")
+    p = ops._problem(z, C, -3.0, 3.0, 20, "relu_sq", 0.75, "tcgen05", 1)
+    image = 4096 + -(-h * 24 * r * 2 // 256) * 256       # header and operand image of C: what is left of the scratch are the partials
+    partials = ops._lib.load().skv_scratch_bytes(ctypes.byref(p), ops._lib.SKV_OP_FORWARD) - image
+    assert partials // (N * r * 4) > 8 * lanes
+    f = ops.feature_forward(z, C, -3.0, 3.0, 20, "relu_sq", 0.75, impl="tcgen05", spline_order=1, delta_f32=delta_f32)
+    _, d_ref = util.oc.feature_forward(util.f32(z), util.f32(C), -3.0, 3.0, 20, "relu_sq", 0.75, spline_order=1)
+    # float32: pairs of f16 and sums of a few thousand products; bf16: half a unit in the eighth bit
+    if delta_f32:
+        _check("delta", f[1], d_ref, torch.float32, 2e-5)
+    else:
+        _check("delta", f[:, h:], d_ref, torch.bfloat16, 4e-3)
+    ops.check_status(z.device)

@@ -11,7 +11,8 @@ ops = pytest.importorskip("sparsespline_ffn_b200.ops")
 
 # (N, h, r, G, spline_order)
 CASES = [(65, 8, 16, 20, 1), (129, 24, 32, 21, 1), (513, 40, 128, 3, 1), (257, 9, 17, 20, 2), (1000, 101, 20, 12, 2),
-         (130, 33, 1, 6, 2), (200, 16, 32, 48, 2), (640, 24, 24, 62, 2), (96, 7, 96, 23, 2)]
+         (130, 33, 1, 6, 2), (200, 16, 32, 48, 2), (640, 24, 24, 62, 2), (96, 7, 96, 23, 2),
+         (2500, 37, 20, 12, 2)]          # padded rows of dz: more than the blocks that bring them to their place
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "N%d_h%d_r%d_G%d_order%d" % c)
