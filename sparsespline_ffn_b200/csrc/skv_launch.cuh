@@ -11,10 +11,11 @@ namespace skv {
 // Programmatic dependent launch: a kernel of a call's chain may be scheduled while its predecessor still
 // runs (its CTAs have all started); pdl_wait() returns once the predecessor is complete and its
 // writes are visible.  Every kernel launched through launch_chained() calls it in every thread that touches what earlier
-// kernels wrote.  The first kernel of a call, whose predecessor is whatever was on the stream, waits in every thread before
-// anything else and only then lets its successor start: from there on the call's inputs may be read without a wait.
-// Chained to what was there its launch costs nothing: a plain launch leaves 1.5 us between two calls.  The last kernel of a call
-// lets its successor start after its own wait.
+// kernels wrote, at its end at the latest, so that whoever waits for it has waited for all in front of it.
+//
+// The first kernel of a call waits in every thread before anything else and only then lets its successor start: from there on the
+// call's inputs may be read without a wait.  In a CUDA-core call it is chained to whatever was on the stream (a plain launch
+// leaves 1.5 us between two calls); in a tensor-core call, where it is the scan, it is launched plainly (launch_prep says why).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // (What an earlier kernel may have written, of the chain or of the call in front of it, is read through plain pointers or ld16, never
 // through const __restrict__ pointers, __ldg or ld.global.nc: those are for memory that nothing writes while the kernel is resident, a

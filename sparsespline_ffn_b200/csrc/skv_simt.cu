@@ -7,8 +7,8 @@
 // a warp works on 32 / LPT tokens of one key at a time; knot interval and weights of a pair are
 // computed once by one lane and handed to the LPT lanes through shared memory (a 16-byte broadcast).
 //
-// Every kernel is chained to what was on the stream in front of it and may be resident while its inputs are written, so it reads
-// them, behind its wait, through plain pointers (skv_launch.cuh).
+// Every kernel of a forward or backward is chained to what was on the stream in front of it and may be resident while its inputs
+// are written, so it reads them through plain pointers (skv_launch.cuh).
 #include "skv_common.cuh"
 #include "skv_launch.cuh"
 
@@ -23,8 +23,8 @@ constexpr int kGroups = 4;            // token groups a warp of the staged forwa
 // Warps per CTA of the kernels over a staged table, two CTAs per SM.  What a lane waits for is a chain of two shared-memory reads per
 // key (weights, then rows), so warps are what hides it: sixteen where a lane's registers allow it (64 of them: float32 rows
 // of up to 128 channels, and four to sixteen lanes per token, so that their staging buffers leave room for the table).
-__host__ __device__ constexpr int staged_warps(int lpt, int cv, int row_bytes_per_lane) {
-  return row_bytes_per_lane == 4 && cv == 1 && lpt >= 4 ? 16 : 8;
+__host__ __device__ constexpr int staged_warps(int lpt, int cv, int element_bytes) {
+  return element_bytes == 4 && cv == 1 && lpt >= 4 ? 16 : 8;
 }
 
 __host__ __device__ inline int64_t cdiv64(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -1260,9 +1260,11 @@ size_t simt_scratch_bytes(const skv_problem& p, int op) {
   return f.splits > 1 ? (size_t)f.splits * (p.N > 0 ? p.N : 1) * p.r * sizeof(float) : 0;
 }
 
-// Tokens up to which the forward reads table rows in place.  On the GPU, in place against the tensor-core chain: h = 5120, r = 32: 132 tokens
-// 17.2 and 18.1 us, 160 tokens 26.3 and 17.9; h = 2560: 177 tokens, 200 tokens 14.9 and 15.6; h = 1024: 250 tokens 8.3 and 12.3, 300
-// tokens 13.8 and 12.4; h = 5120, r = 128: 100 tokens 48.9 and 48.8.
+// Tokens up to which the forward reads table rows in place.  The line was fitted to earlier forms of both sides (in place: 8 us and one
+// for every 1.05 M of N h r; the tensor-core chain: 15 us and one for every 0.26 M table elements).  In place against the
+// tensor-core chain as they are, on the GPU, L = 22: h = 5120, r = 32 (line at 132): 132 tokens 17.2 and 18.1 us, 160 tokens 26.3 and 17.9;
+// h = 5120, r = 128 (99): 100 tokens 48.9 and 48.8.  Elsewhere it is off: h = 2560, r = 32 (177): 200 tokens 14.9 and 15.6; h = 1024, r = 32
+// (310): 250 tokens 8.3 and 12.3, 300 tokens 13.8 and 12.4.  Float32 has no tensor-core side; its 64 is not measured against the staged kernel.
 int64_t small_forward_tokens(const skv_problem& p) {
   if (p.dtype != SKV_BF16) return 64;
   const int64_t n = 4 * (int64_t)p.L + 7300000 / ((int64_t)p.h * p.r);

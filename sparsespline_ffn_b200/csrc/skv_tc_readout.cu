@@ -52,8 +52,8 @@ struct RoParams {
   int64_t ys;
   int64_t N;
   int h, r, D;
-  int ks_z;                      // stages that read z: ceil(h / 32)
-  int ks;                        // all stages: ks_z + ceil(r / 32)
+  int ks_z;                      // stages that read z: ceil(h / kRoK)
+  int ks;                        // all stages: ks_z + ceil(r / kRoK)
   int n_tiles;                   // ceil(D / 256)
   int64_t tiles;                 // m_tiles * n_tiles
   int64_t whole;                 // the first tiles are worked on in one piece, the others in K slices
