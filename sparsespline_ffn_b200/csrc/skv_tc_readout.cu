@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(256) tc_readout_sum_kernel(const float* partia
 // ReLU^2 (0.70 without), one of 128 tokens more than half of that (it reads as much of W); an item's fill and epilogue; a launch more and
 // partials through L2.  256 tokens give the best rate; whole rounds of tiles need no partials; slices spread a last round that
 // is not full, or few tokens, over the chip.  8192 x 5120 -> 1280 (320 tiles of 128 tokens on 148 SMs): in three rounds 127 us,
-// in two and a sixth 105.
+// in two rounds and six slices 105 with the sum; these constants take five slices (the whole call 252 us in three rounds, 233 so).
 struct RoPlan { int mt, slices, ks_per; int64_t whole; };
 RoPlan readout_plan(const skv_problem& p, int64_t D) {
   const int ks = (p.h + kRoK - 1) / kRoK + (p.r + kRoK - 1) / kRoK;
